@@ -29,6 +29,11 @@
 // its own output dimensions over the 32 keys.  Rows of a key block that lie
 // beyond the sequence are zero-filled, never read: a page that is used again may
 // hold anything.
+//
+// Bound by instructions, not by bytes: a key's row is therefore looked up once a block (a lane a key) and handed to the
+// copying lanes by shuffles; a division and a table read for each 16 bytes took longer than the arithmetic (float32, 4 rows
+// of up to 900 keys in one split: 100 us, in four: 18 us; a prompt of 300 tokens with the next block's copies under the
+// arithmetic as well: 78.6 -> 60.9 us).
 #include <math.h>
 
 #include "common.cuh"
@@ -146,38 +151,41 @@ __device__ __forceinline__ void warp_key_block(const T* ks, const T* vs, const f
   __syncwarp();
 }
 
-// Copies key rows [first_key, first_key + 32) of one KV head into shared memory
-// with `nthreads` threads (thread index `tid`); rows at or beyond kv_end become zeros.  A row's first `hd` elements are
-// copied; rows lie `stride` elements apart (values that are the leading columns of wider key rows: stride > hd).
+// Where key `first_key + lane` lies: its row of the cache (cache[page][kv head][offset in page] are the rows), -1 beyond the
+// sequence.  One lookup and one division a key and block of keys; a thread that copies looks its rows up in the other lanes.
+__device__ __forceinline__ long long lane_row(const int* __restrict__ table, int page_size, int nkv, int kvh, int first_key,
+                                              int kv_end) {
+  const int key = first_key + (threadIdx.x & 31);
+  if (key >= kv_end) return -1;
+  const int page = key / page_size;
+  return (static_cast<long long>(table[page]) * nkv + kvh) * page_size + (key - page * page_size);
+}
+
+// Copies the 32 key rows of a block into shared memory with `nthreads` threads (whole warps; thread index `tid`): `mine` is
+// the calling lane's row (lane_row); rows beyond the sequence become zeros.  A row's first `hd` elements are copied; rows lie
+// `stride` elements apart (values that are the leading columns of wider key rows: stride > hd).
 template <typename T>
-__device__ __forceinline__ void load_key_block(T* dst, const T* __restrict__ cache, const int* __restrict__ table,
-                                               int page_size, int nkv, int kvh, int first_key, int kv_end, int hd,
-                                               int stride, int tid, int nthreads) {
+__device__ __forceinline__ void load_key_block(T* dst, const T* __restrict__ cache, long long mine, int hd, int stride, int tid,
+                                               int nthreads) {
   using G = RowGeom<T>;
   if (hd % G::CHUNK == 0 && stride % G::CHUNK == 0) {
     // rows start on 16-byte boundaries: asynchronous 16-byte copies, zeros beyond the row and beyond the sequence
+    // (KB * CHUNKS is a multiple of 32 and so is every step: a warp stays together)
     const int row_chunks = hd / G::CHUNK;
+#pragma unroll 8
     for (int c = tid; c < KB * G::CHUNKS; c += nthreads) {
       const int r = c / G::CHUNKS, part = c - r * G::CHUNKS;
-      const int key = first_key + r;
-      const bool valid = key < kv_end && part < row_chunks;
-      const T* src = cache;
-      if (valid) {
-        const int page = table[key / page_size];       // cache[page][kv head][offset in page][hd]
-        const size_t row = (static_cast<size_t>(page) * nkv + kvh) * page_size + key % page_size;
-        src = cache + row * stride + part * G::CHUNK;
-      }
-      cp_async16(dst + r * G::STRIDE + part * G::CHUNK, src, valid);
+      const long long row = __shfl_sync(0xffffffffu, mine, r);
+      const bool valid = row >= 0 && part < row_chunks;
+      cp_async16(dst + r * G::STRIDE + part * G::CHUNK, valid ? cache + row * stride + part * G::CHUNK : cache, valid);
     }
   } else {
     // an even head size whose rows are not 16-byte aligned: pairs of elements with plain loads
     for (int c = tid; c < KB * (D / 2); c += nthreads) {
       const int r = c / (D / 2), pair = c - r * (D / 2);
-      const int key = first_key + r;
+      const long long row = __shfl_sync(0xffffffffu, mine, r);
       T a = from_f32<T>(0.0f), b = a;
-      if (key < kv_end && 2 * pair < hd) {
-        const int page = table[key / page_size];
-        const size_t row = (static_cast<size_t>(page) * nkv + kvh) * page_size + key % page_size;
+      if (row >= 0 && 2 * pair < hd) {
         a = cache[row * stride + 2 * pair];
         b = cache[row * stride + 2 * pair + 1];
       }
@@ -200,20 +208,19 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
                          const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                          const int* __restrict__ prefix_len, const int* __restrict__ rows, int nh, int nkv,
                          int page_size, int window, float scale, int tile_tokens, int head_chunks, int hd,
-                         int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride) {
+                         int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride, int stages) {
   using G = RowGeom<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* qs = reinterpret_cast<float*>(smem_raw);                        // [32][D]
   float* ps = qs + 32 * D;                                               // [PF_WARPS][32 * NV]
-  T* ks = reinterpret_cast<T*>(ps + PF_WARPS * KB * NV);                 // [32][STRIDE]
-  T* vs = ks + KB * G::STRIDE;
+  T* tiles = reinterpret_cast<T*>(ps + PF_WARPS * KB * NV);              // [stages][K, V][32][STRIDE]
 
   const int row = rows[blockIdx.z];
   const int kvh = blockIdx.y / head_chunks, hc = blockIdx.y - kvh * head_chunks;
   const int head_base = kvh * (nh / nkv) + hc * 32;                      // first query head of this CTA
   const int group = min(32, nh / nkv - hc * 32);                         // query heads of this CTA
   const int q_begin = cu_q[row], q_len = cu_q[row + 1] - q_begin;
-  const int tok0 = blockIdx.x * tile_tokens;
+  const int tok0 = (gridDim.x - 1 - blockIdx.x) * tile_tokens;           // the tiles that see the most keys start first
   if (tok0 >= q_len) return;
   const int ntok = min(tile_tokens, q_len - tok0);
   const int nvec = ntok * group;
@@ -245,17 +252,29 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
   }
   VecState st;
   st.init();
+  // The next block's copies run under this one's arithmetic where two blocks fit (`stages`).
+  auto fetch = [&](int kb, int stage) {
+    T* ks = tiles + stage * 2 * KB * G::STRIDE;
+    const long long mine = lane_row(table, page_size, nkv, kvh, kb, kv_end);
+    load_key_block<T>(ks, k_cache, mine, hd, hd, threadIdx.x, blockDim.x);
+    load_key_block<T>(ks + KB * G::STRIDE, v_cache, mine, hd_v, v_stride, threadIdx.x, blockDim.x);
+  };
+  if (stages > 1) fetch(k_begin, 0);
+  cp_async_commit();
+  int stage = 0;
   for (int kb = k_begin; kb < kv_end; kb += KB) {
-    __syncthreads();                                   // the previous block is no longer read
-    load_key_block<T>(ks, k_cache, table, page_size, nkv, kvh, kb, kv_end, hd, hd, threadIdx.x, blockDim.x);
-    load_key_block<T>(vs, v_cache, table, page_size, nkv, kvh, kb, kv_end, hd_v, v_stride, threadIdx.x, blockDim.x);
+    __syncthreads();                                   // the block before is no longer read
+    if (stages == 1) fetch(kb, 0);
+    else if (kb + KB < kv_end) fetch(kb + KB, stage ^ 1);
     cp_async_commit();
-    cp_async_wait<0>();
+    if (stages == 1) cp_async_wait<0>(); else cp_async_wait<1>();
     __syncthreads();
+    const T* ks = tiles + stage * 2 * KB * G::STRIDE;
     const bool touches = warp_p_max >= kb && (window <= 0 || kb + KB - 1 > warp_p_min - window) &&
                          (chunk <= 0 || kb + KB - 1 >= warp_p_min - warp_p_min % chunk);
     if (touches)
-      warp_key_block<T>(ks, vs, qs + warp * NV * D, qpos, kb, kv_end, window, chunk, st, ps + warp * KB * NV, softcap);
+      warp_key_block<T>(ks, ks + KB * G::STRIDE, qs + warp * NV * D, qpos, kb, kv_end, window, chunk, st, ps + warp * KB * NV, softcap);
+    if (stages > 1) stage ^= 1;
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -334,8 +353,9 @@ decode_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
   for (int s = 0; s < stages - 1; ++s) {
     if (issue < blk_hi) {
       T* t = my_tiles + s * tile_elems;
-      load_key_block<T>(t, k_cache, table, page_size, nkv, kvh, k_begin + issue * KB, kv_end, hd, hd, lane, 32);
-      load_key_block<T>(t + KB * G::STRIDE, v_cache, table, page_size, nkv, kvh, k_begin + issue * KB, kv_end, hd_v, v_stride, lane, 32);
+      const long long mine = lane_row(table, page_size, nkv, kvh, k_begin + issue * KB, kv_end);
+      load_key_block<T>(t, k_cache, mine, hd, hd, lane, 32);
+      load_key_block<T>(t + KB * G::STRIDE, v_cache, mine, hd_v, v_stride, lane, 32);
     }
     cp_async_commit();
     issue += DEC_WARPS;
@@ -346,16 +366,18 @@ decode_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
       const int s_issue = (stage + stages - 1) % stages;
       if (issue < blk_hi) {
         T* t = my_tiles + s_issue * tile_elems;
-        load_key_block<T>(t, k_cache, table, page_size, nkv, kvh, k_begin + issue * KB, kv_end, hd, hd, lane, 32);
-        load_key_block<T>(t + KB * G::STRIDE, v_cache, table, page_size, nkv, kvh, k_begin + issue * KB, kv_end, hd_v, v_stride, lane, 32);
+        const long long mine = lane_row(table, page_size, nkv, kvh, k_begin + issue * KB, kv_end);
+        load_key_block<T>(t, k_cache, mine, hd, hd, lane, 32);
+        load_key_block<T>(t + KB * G::STRIDE, v_cache, mine, hd_v, v_stride, lane, 32);
       }
       cp_async_commit();
       issue += DEC_WARPS;
       cp_async_wait<1>();          // stages is 1 or 2: all but the newest group have landed
     } else {
       T* t = my_tiles;
-      load_key_block<T>(t, k_cache, table, page_size, nkv, kvh, k_begin + blk * KB, kv_end, hd, hd, lane, 32);
-      load_key_block<T>(t + KB * G::STRIDE, v_cache, table, page_size, nkv, kvh, k_begin + blk * KB, kv_end, hd_v, v_stride, lane, 32);
+      const long long mine = lane_row(table, page_size, nkv, kvh, k_begin + blk * KB, kv_end);
+      load_key_block<T>(t, k_cache, mine, hd, hd, lane, 32);
+      load_key_block<T>(t + KB * G::STRIDE, v_cache, mine, hd_v, v_stride, lane, 32);
       cp_async_commit();
       cp_async_wait<0>();
     }
@@ -444,7 +466,10 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   const int group = nh / nkv;
   const int head_chunks = (group + 31) / 32;                  // more than 32 query heads per KV head: several CTAs
   const int tile_tokens = group >= 32 ? 1 : 32 / group;
-  const size_t smem = (32 * D + PF_WARPS * KB * NV) * sizeof(float) + 2 * KB * G::STRIDE * sizeof(T);
+  // Two blocks of keys where two CTAs of that size still share an SM, else one.
+  constexpr size_t fixed = (32 * D + PF_WARPS * KB * NV) * sizeof(float), block = 2 * KB * G::STRIDE * sizeof(T);
+  constexpr int stages = fixed + 2 * block <= 110 * 1024 ? 2 : 1;
+  constexpr size_t smem = fixed + stages * block;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -457,7 +482,7 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   prefill_attention_kernel<T><<<grid, PF_WARPS * 32, smem, stream>>>(
       static_cast<const T*>(q), static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out),
       block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window, scale, tile_tokens,
-      head_chunks, hd, hd_v, softcap, chunk, sinks, v_stride > 0 ? v_stride : hd_v);
+      head_chunks, hd, hd_v, softcap, chunk, sinks, v_stride > 0 ? v_stride : hd_v, stages);
   return b200_check_launch();
 }
 
