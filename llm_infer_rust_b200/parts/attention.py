@@ -14,35 +14,41 @@ _KEYS_PER_CTA_AT_LEAST = 512      # fewer keys per CTA leave its warps' copy pip
 # is busy with far fewer keys (measured at 8 rows x 16 heads on rows of 320 columns, 2,048 keys: 43.0 us in 4 splits,
 # 27.5 us in 16; 32 heads on rows of 448: 128.0 against 91.1 us; one row of 8,192 keys: 246.8 against 82.9 us).
 _LATENT_KEYS_PER_CTA_AT_LEAST = 128
+# (4 rows x 8 KV heads of up to 900 float32 keys: 100 us whole on 32 SMs, 21 us in four splits with their combination.)
+_ALL_SIZES_KEYS_PER_CTA_AT_LEAST = 128
+# A cluster of n splits gives way to more splits where rows may hold n * n times as many keys (see decode_splits).
+_KEYS_FOR_MORE_SPLITS, _LATENT_KEYS_FOR_MORE_SPLITS = 256, 32
 
 
 def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int,
-                  keys_per_cta: int = _KEYS_PER_CTA_AT_LEAST) -> int:
-    """How many CTAs share one row's keys.
+                  keys_per_cta: int = _KEYS_PER_CTA_AT_LEAST, keys_for_more: int = _KEYS_FOR_MORE_SPLITS) -> int:
+    """How many CTAs share one row's keys, ``ctas_per_split`` CTAs for each split.
 
-    With ``ctas_per_split`` CTAs for each split, the number of splits is chosen so that the
-    grid fills whole waves of SMs as well as it can while every CTA keeps at least ``keys_per_cta`` keys.
+    The grid stays within one wave of SMs and every CTA keeps at least ``keys_per_cta`` keys.  Within a wave 2, 4 or 8
+    splits are the CTAs of one cluster, which combine their parts themselves; other counts need a kernel for it and are
+    taken where the cluster would leave half of the SMs idle and the rows may be long (``keys_for_more``).
+    (Measured at 16 query and 8 KV heads of 128, us at 300 / 1,000 / 4,096 / 8,192 keys a row: 8 rows 15 / 20 / 38 / 66 in
+    two splits, 24 / 27 / 47 / 70 in the nine that fill two and a half waves best; 4 rows 13 / 16 / 26 / 38 in four, 17 / 20
+    / 30 / 43 in nine; 12 rows 13 / 22 / 50 / 85 whole, 20 / 26 / 56 / 89 in three.  More than a cluster: 2 rows 21.5 / 29.7
+    / 83 us in four and 21.1 / 27.7 / 68 in seven or nine at 4,096 / 8,192 / 32,768 keys; 1 row 21.5 / 48 in eight and 21.5 /
+    42 in eighteen at 8,192 / 32,768.  ``kv_len_bound`` is what the rows may grow to when the step is captured, so the
+    choice has to serve short rows too.)
     """
     ctas_per_split = max(1, ctas_per_split)
-    if 8 * ctas_per_split >= 7 * sm_count:
-        # A grid that fills the SMs without splits stays whole: with several waves the splits are combined by a kernel
-        # of its own, which costs more than the last wave's idle SMs (measured at 4,096 keys a row: 32 rows x 8 KV
-        # heads 90.8 us whole against 103.8 us in the four splits that fill the waves best, 64 rows 177.5 against
-        # 182.3 us in two).
-        return 1
-    most = max(1, min(64, kv_len_bound // max(1, keys_per_cta)))
-    best, best_fill = 1, 0.0
-    for splits in range(1, most + 1):
-        if splits == 8 and 2 * ctas_per_split * splits > sm_count:
-            # Eight splits of a grid that fits one wave are the CTAs of one cluster, and more than a handful of clusters
-            # of eight do not find room side by side: measured at 2 rows x 8 KV heads, 18.1 us against 12.4 us with six
-            # splits (one row: 8 clusters of eight, 9.6 us, the best there).
-            continue
-        ctas = ctas_per_split * splits
-        fill = ctas / (sm_count * -(-ctas // sm_count))
-        if fill > best_fill * 1.05:
-            best, best_fill = splits, fill
-    return best
+    most = max(1, min(64, kv_len_bound // max(1, keys_per_cta), sm_count // ctas_per_split))
+    # More than a handful of clusters of eight do not find room side by side: measured at 2 rows x 8 KV heads, 18.1 us
+    # against 12.4 us with six splits (one row: 8 clusters of eight, 9.6 us, the best there).
+    cluster = max(s for s in (1, 2, 4, 8) if s <= most and (s < 8 or 2 * ctas_per_split * s <= sm_count))
+    if 2 * cluster * ctas_per_split <= sm_count and kv_len_bound >= cluster * cluster * keys_for_more:
+        return 7 if most == 8 else most                   # (a cluster of eight was turned down above)
+    return cluster
+
+
+def _keys_per_cta(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim=None) -> int:
+    """The fewest keys worth a CTA: the all-sizes kernel's takes in 128 at a time, a tenth as fast as the tensor-core one."""
+    if ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim):
+        return _KEYS_PER_CTA_AT_LEAST
+    return _ALL_SIZES_KEYS_PER_CTA_AT_LEAST
 
 
 class GQAttention(Part):
@@ -123,7 +129,8 @@ class GQAttention(Part):
         if ctx.num_decode:
             bound = min(ctx.kv_len_bound, self.window) if self.window else ctx.kv_len_bound
             per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page)
-            splits = decode_splits(per_split, bound, ctx.sm_count)
+            splits = decode_splits(per_split, bound, ctx.sm_count,
+                                   _keys_per_cta(q.dtype, self.nh, self.nkv, self.d, page))
             need = ops.decode_scratch_floats(ctx.num_decode, self.nh, self.d, splits)
             scratch = ctx.scratch(need) if need else None
             ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,
@@ -233,7 +240,8 @@ class GatedConvAttention(Part):
         if ctx.num_decode:
             bound = min(ctx.kv_len_bound, self.window) if self.window else ctx.kv_len_bound
             per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page, self.dv)
-            splits = decode_splits(per_split, bound, ctx.sm_count)
+            splits = decode_splits(per_split, bound, ctx.sm_count,
+                                   _keys_per_cta(q.dtype, self.nh, self.nkv, self.d, page, self.dv))
             need = ops.decode_scratch_floats(ctx.num_decode, self.nh, max(self.d, self.dv), splits)
             scratch = ctx.scratch(need) if need else None
             ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,
@@ -264,13 +272,14 @@ def _masked_attention(part, q, out, ctx, cache, num_heads, num_kv_heads, head_di
         for limit in (part.window, part.chunk):
             if limit:
                 bound = min(bound, limit)
-        keys_per_cta = _KEYS_PER_CTA_AT_LEAST
+        keys_per_cta, keys_for_more = _KEYS_PER_CTA_AT_LEAST, _KEYS_FOR_MORE_SPLITS
         if shared_values and ops.latent_uses_tensor_cores(q.dtype, num_heads, head_dim, v_head_dim, page):
             per_split = ctx.num_decode * (num_heads // ops.latent_head_group(num_heads))
-            keys_per_cta = _LATENT_KEYS_PER_CTA_AT_LEAST
+            keys_per_cta, keys_for_more = _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS
         else:
             per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, num_heads, num_kv_heads, head_dim, page, v_head_dim)
-        splits = decode_splits(per_split, bound, ctx.sm_count, keys_per_cta)
+            keys_per_cta = _keys_per_cta(q.dtype, num_heads, num_kv_heads, head_dim, page, v_head_dim)
+        splits = decode_splits(per_split, bound, ctx.sm_count, keys_per_cta, keys_for_more)
         need = ops.decode_scratch_floats(ctx.num_decode, num_heads, max(head_dim, v_head_dim), splits)
         scratch = ctx.scratch(need) if need else None
         ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,
