@@ -19,6 +19,8 @@ import torch
 
 from .build import load_cuda_library
 
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
 ERROR_BITS = {1: "a token id outside the embedding table", 2: "a cache slot outside the pool",
@@ -41,8 +43,11 @@ def _code(t: torch.Tensor) -> int:
 def _cuda(*tensors: Optional[torch.Tensor]) -> None:
     """Checks that the operands are on the device.  Every wrapper that launches calls this first, so it is also
     where products that wait in the chain (see ``chain_linear``) are launched: whatever runs next may read them."""
-    flush_chain()
-    _cuda_only(*tensors)
+    if _held is not None or _chain is not None:
+        flush_chain()
+    for t in tensors:
+        if t is not None and not t.is_cuda:
+            raise KernelError("the kernels run on CUDA tensors only; there is no CPU path")
 
 
 def _cuda_only(*tensors: Optional[torch.Tensor]) -> None:
@@ -62,7 +67,9 @@ def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle.  (``torch.cuda.current_stream`` makes an object and looks the device up on its way: a
+    quarter of the host's time of an eager step.)"""
+    return ctypes.c_void_p(_raw_stream(_current_device()))
 
 
 # Launches of this package's kernels so far (library matrix products are not counted).
@@ -93,10 +100,13 @@ _error_words = {}
 
 def error_word(device: torch.device) -> torch.Tensor:
     """The device word into which kernels OR their error bits."""
-    key = torch.device(device).index or 0
-    if key not in _error_words:
-        _error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _error_words[key]
+    word = _error_words.get(device)
+    if word is None:
+        key = torch.device(device).index or 0
+        if key not in _error_words:
+            _error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        word = _error_words[device] = _error_words[key]
+    return word
 
 
 def check_errors(device: torch.device) -> None:
@@ -636,10 +646,10 @@ _sm_counts = {}
 
 
 def _sm_count(device) -> int:
-    key = torch.device(device).index or 0
-    if key not in _sm_counts:
-        _sm_counts[key] = torch.cuda.get_device_properties(device).multi_processor_count
-    return _sm_counts[key]
+    count = _sm_counts.get(device)
+    if count is None:
+        count = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return count
 
 
 # The gate's activation in a fused product: builds of their own, so that the dense models' stay as they are.
@@ -1109,6 +1119,8 @@ def few_row_takes(rows: int, weight: torch.Tensor, act_dtype: torch.dtype, mode:
     """Whether a product of ``rows`` rows runs on this package's few-row kernels (with the norm before it and the
     epilogue after it fused in) rather than as a library product with those as kernels of their own.  ``norm``: the
     product may come behind a norm (False: its input is a plain tensor)."""
+    if rows > SKINNY_MAX_ROWS and few_row_route != "chain":
+        return False                     # (asked of every product of a prompt portion)
     if few_row_route == "chain" and chain_takes(rows, weight, act_dtype, mode, head_dim):
         return True
     if few_row_route == "library":
@@ -1486,7 +1498,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     """
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32 and weight.dtype == torch.float32:
-        return cast(gemm_f32(x, weight), out_dtype)
+        return gemm_f32(x, weight) if out_dtype == torch.float32 else cast(gemm_f32(x, weight), out_dtype)
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16:
         if out_dtype in (torch.bfloat16, torch.float32) and x.dim() == 2 and x.is_contiguous() and x.is_cuda:
             mode = EPI_PLAIN_F32 if out_dtype == torch.float32 else EPI_PLAIN_BF16
