@@ -26,6 +26,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <initializer_list>
+
 #include "common.cuh"
 
 #ifndef HEAD_DIM
@@ -56,6 +58,10 @@ constexpr int N_BARS = 2 * K_STAGES + 2 * V_STAGES + 2 + 4;
 constexpr int TBL_ENTRIES = 2048;         // page numbers of a row that the copy warp keeps in shared memory (the rest it reads as before)
 constexpr int TBL_OFF = BAR_OFF + (N_BARS + 1) * 8;      // (one more slot holds the tensor-memory address)
 constexpr int SMEM_BYTES = TBL_OFF + TBL_ENTRIES * 4;
+constexpr int SHAPED_THREADS = THREADS + 128;             // two softmax threads a row
+constexpr int XCH_OFF = (SMEM_BYTES + 15) / 16 * 16;      // what they exchange: [4][2] flags, then [2][2][128] floats
+constexpr int SHAPED_SMEM_BYTES = XCH_OFF + 32 + 4 * BQ * 4;
+static_assert(1024 + SHAPED_SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
@@ -157,6 +163,10 @@ __device__ __forceinline__ void tmem_st32_raw(uint32_t taddr, const uint32_t (&v
                  "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
                : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
@@ -173,10 +183,13 @@ __device__ __forceinline__ int swz(int r, int c) { return (c >> 3) * HALF + r * 
 // ---------------------------------------------------------------------------------------------------------------
 // What the softmax threads of both kernels do.  A thread owns one query row: lane r of tensor memory.
 
-// The row's Q vector into its K-major tile in the 128-byte swizzle (zeros for a row that is not used).
-__device__ __forceinline__ void write_q_row(unsigned char* q_tile, const bf16* src, int r, bool used) {
+// The row's Q vector into its K-major tile in the 128-byte swizzle (zeros for a row that is not used), chunks
+// c_lo .. c_lo + CHUNKS - 1 of 16.
+template <int CHUNKS>
+__device__ __forceinline__ void write_q_row(unsigned char* q_tile, const bf16* src, int r, bool used, int c_lo) {
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
+  for (int i = 0; i < CHUNKS; ++i) {
+    const int c = c_lo + i;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (used) v = *reinterpret_cast<const uint4*>(src + c * 8);
     *reinterpret_cast<uint4*>(q_tile + swz(r, c)) = v;
@@ -184,11 +197,12 @@ __device__ __forceinline__ void write_q_row(unsigned char* q_tile, const bf16* s
   proxy_fence();
 }
 
-// Row r of an MN-major value tile (128 dims in two halves of 128 bytes), set to zero.
-__device__ __forceinline__ void zero_value_row(unsigned char* v_tile, int r) {
+// Row r of an MN-major value tile (128 dims in two halves of 128 bytes), chunks c_lo .. c_lo + CHUNKS - 1 of 16 set to zero.
+template <int CHUNKS>
+__device__ __forceinline__ void zero_value_row(unsigned char* v_tile, int r, int c_lo) {
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(v_tile + (c >> 3) * HALF + r * 128 + (c & 7) * 16) = zero;
+  for (int c = c_lo; c < c_lo + CHUNKS; ++c) *reinterpret_cast<uint4*>(v_tile + (c >> 3) * HALF + r * 128 + (c & 7) * 16) = zero;
 }
 
 struct RowState {
@@ -198,14 +212,14 @@ struct RowState {
 
 // One block of 128 keys for this thread's row.  The scores lie in the 128 columns from s_base on; the bfloat16
 // probabilities go back over the first 64 of them, two to a column (the A operand of P V), and are in tensor memory
-// when the function returns.  `block` counts the row's blocks from 0; P V of block - 1 commits to `pv_done`.  Every
+// when the function returns.  The row sees keys lo_key .. hi_key (none: hi_key -1).  `block` counts the row's blocks from 0; P V of block - 1 commits to `pv_done`.  Every
 // phase of that barrier is waited for here, in order: before the accumulator at o_base is rescaled (the row's
 // maximum grew by more than the step), else at the end, when that product has long finished.  A wait by parity
 // cannot tell "phase b - 1 is not finished" from "phase b - 2 is not finished": a waiter that skipped a phase
 // would pass at once.  Returns false when a wait ran out.
-__device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, int first_key, int qpos, int kv_end,
-                                              int window, bool masked, float scale_log2, int block, uint64_t* pv_done,
-                                              RowState& st, int* err) {
+__device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, int first_key, int lo_key, int hi_key,
+                                              bool masked, float scale_log2, int block, uint64_t* pv_done, RowState& st,
+                                              int* err) {
   tc_fence_after();
   // pass 1: the row's maximum over the block's visible keys (of the raw scores; the scale is positive)
   float mx = -INFINITY;
@@ -217,7 +231,7 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
 #pragma unroll
       for (int e = 0; e < 64; ++e) {
         const int key = first_key + c * 64 + e;
-        const bool vis = key <= qpos && key < kv_end && (window <= 0 || key > qpos - window);
+        const bool vis = key >= lo_key && key <= hi_key;
         mx = fmaxf(mx, vis ? v[e] : -INFINITY);
       }
     } else {
@@ -229,7 +243,7 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
       mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
     }
   }
-  mx = qpos >= 0 ? mx * scale_log2 : -INFINITY;
+  mx = hi_key >= 0 ? mx * scale_log2 : -INFINITY;
   // The reference follows the maximum when it grew by more than the step (or there was none yet).
   const bool raise = mx > st.m_ref + RESCALE_STEP || (st.m_ref == -INFINITY && mx > -INFINITY);
   const float m_new = raise ? mx : st.m_ref;
@@ -254,7 +268,7 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
   st.m_ref = m_new;
   // pass 2: probabilities relative to the reference and their sum; those of columns 64c .. 64c + 63 go back into
   // tensor memory over the scores that were just read (columns 32c .. 32c + 31)
-  const float neg_base = qpos >= 0 ? -base : -INFINITY;      // a row that is not used gets zeros
+  const float neg_base = hi_key >= 0 ? -base : -INFINITY;      // a row that is not used gets zeros
   float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
   for (int c = 0; c < 2; ++c) {
@@ -264,7 +278,7 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
 #pragma unroll
       for (int e = 0; e < 64; ++e) {
         const int key = first_key + c * 64 + e;
-        const bool vis = key <= qpos && key < kv_end && (window <= 0 || key > qpos - window);
+        const bool vis = key >= lo_key && key <= hi_key;
         v[e] = vis ? fast_exp2(fmaf(v[e], scale_log2, neg_base)) : 0.0f;
       }
     } else {
@@ -285,13 +299,137 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
   return pv_seen || mbar_wait_warp(pv_done, (block - 1) & 1, err);
 }
 
-// The finished row: the accumulator over the row's sum, as bfloat16.  (Every lane of the warp takes part in the
-// loads, also those whose row is not used.)
-__device__ __forceinline__ void store_output(uint32_t o_base, bf16* dst, float l_run, bool used) {
+// ---- The further forms of a score and of what is stored, for the builds of the one-tile kernel that know them (SHAPED):
+//   cap_log2 > 0       score <- cap tanh(score * scale / cap), in log2 units (tanh_in = scale / cap);
+//   split              a weight enters the product with the values as two bfloat16 terms, the rounded weight (in the first
+//                      64 columns of its score buffer) and what the rounding left (in the other 64): twice the P V;
+//   chunk C > 0        the query at position p also sees only keys from p - p % C on;
+//   sinks              exp(sinks[head]) joins the softmax's denominator;
+//   diff_* (DIFF)      query vectors are pairs, neighbouring rows 2j and 2j + 1 the two maps of one head: what is stored is
+//                      o / sqrt(mean(o^2) + eps) * gain, o = a_(2j) - lambda a_(2j + 1), in float until then.
+struct ScoreShape {
+  float cap_log2, tanh_in;
+  int split, chunk;
+  const float* sinks;
+  float diff_lambda, diff_gain, diff_eps;
+};
+// cap_log2 tanh(s tanh_in) + shift, with tanh(x) = 1 - 2 / (e^(2x) + 1): two special-function instructions.
+__device__ __forceinline__ float capped(const ScoreShape& f, float s, float shift) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(fast_exp2(s * (f.tanh_in * 2.8853900817779268f)) + 1.0f));
+  return fmaf(-2.0f * f.cap_log2, r, f.cap_log2 + shift);
+}
+
+// These forms cost several times the instructions of the plain one, so there a row has TWO threads: thread c = 0, 1 of a row
+// takes columns 64 c .. 64 c + 63 of its scores (one load; they stay in registers) and of its accumulator; the two warps
+// that hold the same 32 rows exchange their maxima and meet at a barrier of their own, behind which both have read their
+// scores, so that the weights' terms may overwrite all 128 columns.  `xch`: [2 parities][2 threads of a row][128 rows] floats,
+// `failed`: [2 parities] flags of this quarter.  A warp whose wait has run out still comes to the next barrier (ok: false);
+// behind that one both know and both leave, so that nobody is waited for in vain.  Meetings take turns with the parity: what
+// was written before one is read before the next, and written again only behind that.
+// (One thread a row, the scores read twice as in softmax_block: weights in two terms 104 us at 2,048 tokens x 16 heads,
+// 1,263 at 8,192; two threads 43 and 426.  The mma.sync kernel that served these forms: 139 and 1,363; soft-capped 152 and
+// 1,515 against 60 and 666; differences over a window of 1,024 159 and 716 against 72 and 309.)
+struct HalfRows {
+  float* xch;
+  volatile int* failed;
+  int c, r, quarter;
+  // Both warps of the quarter arrive; returns the partner's value.  `left`: one of the two had failed.
+  __device__ __forceinline__ float meet(float mine, int parity, bool ok, bool& left) const {
+    float* buf = xch + parity * 2 * BQ;
+    buf[c * BQ + r] = mine;
+    if (!ok) failed[parity] = 1;
+    tc_fence_before();
+    asm volatile("bar.sync %0, 64;\n" ::"r"(2 + quarter) : "memory");
+    tc_fence_after();
+    left = failed[parity] != 0;
+    return buf[(c ^ 1) * BQ + r];
+  }
+};
+
+// 2^exponent(score) of 64 scores, their sum added to sum4; the weights and (split) what their rounding left into tensor memory.
+template <typename F>
+__device__ __forceinline__ void store_weights(const float (&v)[64], uint32_t p_base, bool split, float (&sum4)[4], const F& exponent) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    uint32_t pr[8], rest[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = h * 16 + 2 * i;
+      const float a = fast_exp2(exponent(v[e])), b = fast_exp2(exponent(v[e + 1]));
+      sum4[i & 3] += a + b;
+      const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
+      pr[i] = *reinterpret_cast<const uint32_t*>(&two);
+      const __nv_bfloat162 rem = __floats2bfloat162_rn(a - __uint_as_float(pr[i] << 16), b - __uint_as_float(pr[i] & 0xffff0000u));
+      rest[i] = *reinterpret_cast<const uint32_t*>(&rem);
+    }
+    tmem_st8(p_base + h * 8, pr);
+    if (split) tmem_st8(p_base + 64 + h * 8, rest);
+  }
+}
+
+// As softmax_block, for this thread's 64 keys of the block; `ok` is what came before (a warp whose wait failed passes false),
+// `left` as in HalfRows.
+__device__ __forceinline__ bool softmax_half(bool ok, uint32_t s_base, uint32_t o_base, int first_key, int lo_key, int hi_key,
+                                             bool masked, float scale_log2, const ScoreShape& shape, int block,
+                                             uint64_t* pv_done, const HalfRows& rows, RowState& st, bool& left, int* err) {
+  tc_fence_after();
+  float v[64];
+  float mx = -INFINITY;
+  if (ok) {
+    tmem_ld64(s_base + rows.c * 64, v);
+    if (masked) {
+      const int lo = lo_key - first_key - rows.c * 64, hi = hi_key - first_key - rows.c * 64;
+#pragma unroll
+      for (int e = 0; e < 64; ++e) v[e] = e >= lo && e <= hi ? v[e] : -INFINITY;
+    }
+    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int e = 0; e < 64; ++e) m4[e & 3] = fmaxf(m4[e & 3], v[e]);
+    mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+  }
+  mx = fmaxf(mx, rows.meet(mx, block & 1, ok, left));
+  if (!ok || left) return false;
+  const bool cap = shape.cap_log2 > 0.0f;
+  if (hi_key < 0) mx = -INFINITY;
+  else if (cap) mx = mx > -INFINITY ? capped(shape, mx, 0.0f) : mx;      // (the cap rises with the score)
+  else mx *= scale_log2;
+  const bool raise = mx > st.m_ref + RESCALE_STEP || (st.m_ref == -INFINITY && mx > -INFINITY);
+  const float m_new = raise ? mx : st.m_ref;
+  const float corr = raise ? (st.m_ref == -INFINITY ? 0.0f : exp2f(st.m_ref - m_new)) : 1.0f;
+  bool pv_seen = block == 0;
+  if (block > 0 && __any_sync(0xffffffffu, raise ? 1 : 0)) {
+    if (!mbar_wait_warp(pv_done, (block - 1) & 1, err)) return false;
+    pv_seen = true;
+    tc_fence_after();
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      float o[32];
+      tmem_ld32(o_base + rows.c * 64 + h * 32, o);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) o[e] *= corr;
+      tmem_st32(o_base + rows.c * 64 + h * 32, o);
+    }
+  }
+  st.m_ref = m_new;
+  const float neg_base = hi_key < 0 ? -INFINITY : m_new == -INFINITY ? 0.0f : -m_new;      // a row that is not used gets zeros
+  float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const uint32_t p_base = s_base + rows.c * 32;
+  if (!cap) store_weights(v, p_base, shape.split, sum4, [&](float x) { return fmaf(x, scale_log2, neg_base); });
+  else if (!masked) store_weights(v, p_base, shape.split, sum4, [&](float x) { return capped(shape, x, neg_base); });
+  else store_weights(v, p_base, shape.split, sum4, [&](float x) { return x == -INFINITY ? x : capped(shape, x, neg_base); });
+  st.l_run = st.l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+  tmem_wait_st();                                      // P is in tensor memory
+  return pv_seen || mbar_wait_warp(pv_done, (block - 1) & 1, err);
+}
+
+// The finished row: the accumulator over the row's sum, as bfloat16, chunks c_lo .. c_hi - 1 of 32 columns.  (Every lane of the
+// warp takes part in the loads, also those whose row is not used.)
+__device__ __forceinline__ void store_output(uint32_t o_base, bf16* dst, float l_run, bool used, int c_lo, int c_hi) {
   tc_fence_after();
   const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
 #pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
+  for (int c = c_lo; c < c_hi; ++c) {
     float o[32];
     tmem_ld32(o_base + c * 32, o);
     if (used) {
@@ -307,12 +445,48 @@ __device__ __forceinline__ void store_output(uint32_t o_base, bf16* dst, float l
   tc_fence_before();
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+// The finished pair of rows 2j (even lanes) and 2j + 1: a head's two maps, their difference normed over its 128 values, this
+// thread's 64 columns of it (the even lane stores the first 16 of 32, the odd lane the others).  `dst`: the head's place.
+__device__ __forceinline__ void store_difference(uint32_t o_base, bf16* dst, float l_run, bool used, const ScoreShape& f,
+                                                 const HalfRows& rows, int parity) {
+  tc_fence_after();
+  const int odd = threadIdx.x & 1;
+  const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f, w = odd ? -f.diff_lambda * inv : inv;
+  float d[64];
+  tmem_ld64(o_base + rows.c * 64, d);
+  float ss = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 64; ++e) {
+    d[e] *= w;
+    d[e] += __shfl_xor_sync(0xffffffffu, d[e], 1);
+    ss = fmaf(d[e], d[e], ss);
+  }
+  bool left;
+  ss += rows.meet(ss, parity, true, left);
+  const float gain = f.diff_gain / sqrtf(ss / static_cast<float>(D) + f.diff_eps);
+  if (used) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      __align__(16) bf16 y[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) y[e] = __float2bfloat16_rn((odd ? d[c * 32 + 16 + e] : d[c * 32 + e]) * gain);
+      uint4* to = reinterpret_cast<uint4*>(dst + rows.c * 64 + c * 32 + odd * 16);
+      to[0] = reinterpret_cast<const uint4*>(y)[0];
+      to[1] = reinterpret_cast<const uint4*>(y)[1];
+    }
+  }
+  tc_fence_before();
+}
+
+// SHAPED: the forms of ScoreShape, with DIFF the difference of two maps, and two softmax threads a row (warps 2-9, the second
+// copy warp behind them); the plain build carries none of that code.
+template <bool SHAPED, bool DIFF>
+__global__ void __launch_bounds__(SHAPED ? SHAPED_THREADS : THREADS, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                        const bf16* __restrict__ q, bf16* __restrict__ out, const int* __restrict__ block_table,
                        int table_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                        const int* __restrict__ prefix_len, const int* __restrict__ rows, int nh, int nkv, int page_size,
-                       int box_rows, int window, float scale_log2, int* err) {
+                       int box_rows, int window, float scale_log2, const ScoreShape shape, int* err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* k_full = reinterpret_cast<uint64_t*>(sm + BAR_OFF);      // [3]
@@ -324,6 +498,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   uint64_t* p_full = q_full + 1;                                     // [2]: one per score buffer, so that a softmax that runs
   uint64_t* pv_done = p_full + 2;                                    //      a block ahead can never lap the MMA thread's wait
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
+  constexpr int SOFTMAX_WARPS = SHAPED ? 8 : 4;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -331,11 +506,13 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
     for (int s = 0; s < V_STAGES; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
     mbar_init(s_full, 1);
     mbar_init(s_full + 1, 1);
-    mbar_init(q_full, 4);
-    mbar_init(p_full, 4);
-    mbar_init(p_full + 1, 4);
+    mbar_init(q_full, SOFTMAX_WARPS);
+    mbar_init(p_full, SOFTMAX_WARPS);
+    mbar_init(p_full + 1, SOFTMAX_WARPS);
     mbar_init(pv_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    if (SHAPED)
+      for (int f = 0; f < 8; ++f) reinterpret_cast<int*>(sm + XCH_OFF)[f] = 0;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
@@ -363,11 +540,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   const int kv_end = active ? min(kv_len[row], prefix + tok0 + ntok) : 0;
   const int p_lo = prefix + tok0;
   int k_begin = window > 0 ? max(0, p_lo - window + 1) : 0;
+  if (SHAPED && shape.chunk > 0) k_begin = max(k_begin, p_lo - p_lo % shape.chunk);
   k_begin -= k_begin % BKV;
   const int nblk = active ? (kv_end - k_begin + BKV - 1) / BKV : 0;
   const int* table = block_table + static_cast<size_t>(row) * table_stride;
 
-  if (warp == 0 || warp >= 6) {
+  if (warp == 0 || warp >= 2 + SOFTMAX_WARPS) {
     // ---- copies: COPY_WARPS warps share a block's sub-blocks (box_rows keys each): warp c's lane l fetches the
     // sub-blocks c + COPY_WARPS l, ...  (One SM takes in more through boxes that several warps issue than through
     // as many from one warp: 34 to 37 against 23 GB/s in a probe that only copies pages of 16 keys; all copy warps
@@ -377,7 +555,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
     // while block i is still in the softmax.
     // The row's page numbers for this tile's keys come into shared memory first: a copy then does not begin with a
     // load from global memory whose answer it needs for its address.
-    const int cw = warp == 0 ? 0 : warp - 5;
+    const int cw = warp == 0 ? 0 : warp - 1 - SOFTMAX_WARPS;
     bool ok = true;
     int* tbl = reinterpret_cast<int*>(sm + TBL_OFF);
     const int first_page = k_begin / page_size;
@@ -448,6 +626,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
         for (int j = 0; j < BKV / 16; ++j)
           umma_a_tmem(tmem_o, tmem_base + (i & 1) * 128 + j * 8, desc_mn_major(v_addr + j * 16 * 128), kDescPV,
                       (i > 0 || j > 0) ? 1u : 0u);
+        if (SHAPED && shape.split) {                             // the weights' second terms
+#pragma unroll
+          for (int j = 0; j < BKV / 16; ++j)
+            umma_a_tmem(tmem_o, tmem_base + (i & 1) * 128 + 64 + j * 8, desc_mn_major(v_addr + j * 16 * 128), kDescPV, 1u);
+        }
         umma_commit(pv_done);
         umma_commit(v_empty + s);
         if (i + 2 < nblk) ok = issue_s(i + 2);
@@ -460,35 +643,63 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
     const int tok = r / group, head = head0 + r % group;
     const bool used = tok < ntok;
     const int qpos = used ? p_lo + tok : -1;
+    const int c = SHAPED ? (warp - 2) >> 2 : 0;      // which half of the row's columns (two threads a row)
+    constexpr int CHUNKS = SHAPED ? 8 : 16;
     if (nblk > 0) {
-      write_q_row(sm + Q_OFF, q + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D, r, used);
+      write_q_row<CHUNKS>(sm + Q_OFF, q + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D, r, used, 8 * c);
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
     }
+    int lo_key = window > 0 ? qpos - window + 1 : 0;
+    if (SHAPED && shape.chunk > 0) lo_key = max(lo_key, qpos - qpos % shape.chunk);
+    const int hi_key = min(qpos, kv_end - 1);
+    // the first key that the tile's last query sees
+    int all_see = window > 0 ? p_lo + ntok - window : 0;
+    if (SHAPED && shape.chunk > 0) all_see = max(all_see, (p_lo + ntok - 1) - (p_lo + ntok - 1) % shape.chunk);
     RowState st;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    bool ok = true;
-    for (int i = 0; i < nblk && ok; ++i) {
+    const HalfRows halves = {reinterpret_cast<float*>(sm + XCH_OFF) + 8, reinterpret_cast<volatile int*>(sm + XCH_OFF) + 2 * quarter, c, r, quarter};
+    bool ok = true, left = false;
+    for (int i = 0; i < nblk; ++i) {
       const int first_key = k_begin + i * BKV;
-      if (!mbar_wait_warp(s_full + (i & 1), (i >> 1) & 1, err)) { ok = false; break; }
-      const bool masked = first_key + BKV - 1 > p_lo || first_key + BKV > kv_end || (window > 0 && first_key <= p_lo + ntok - 1 - window);
-      ok = softmax_block(lane_base + (i & 1) * 128, lane_base + 256, first_key, qpos, kv_end, window, masked, scale_log2, i,
-                         pv_done, st, err);
+      if (ok) ok = mbar_wait_warp(s_full + (i & 1), (i >> 1) & 1, err);
+      const bool masked = first_key + BKV - 1 > p_lo || first_key + BKV > kv_end || first_key < all_see;
+      const uint32_t s_base = lane_base + (i & 1) * 128;
+      if (SHAPED)
+        ok = softmax_half(ok, s_base, lane_base + 256, first_key, lo_key, hi_key, masked, scale_log2, shape, i, pv_done, halves, st, left, err);
+      else if (ok)
+        ok = softmax_block(s_base, lane_base + 256, first_key, lo_key, hi_key, masked, scale_log2, i, pv_done, st, err);
       // value rows beyond what the tile may see must not reach P V, whatever the page or the stage held
       if (ok && first_key + BKV > kv_end) {
         const int s = i % V_STAGES;
         ok = mbar_wait_warp(v_full + s, (i / V_STAGES) & 1, err);      // the copies have landed
-        if (ok && first_key + r >= kv_end) zero_value_row(sm + V_OFF + s * TILE, r);
+        if (ok && first_key + r >= kv_end) zero_value_row<CHUNKS>(sm + V_OFF + s * TILE, r, 8 * c);
         proxy_fence();                                                 // the zeroed rows are visible to the tensor cores
       }
-      if (!ok) break;
+      if (!ok) {
+        if (!SHAPED || left) break;                                    // (two threads a row leave together, behind a barrier)
+        continue;
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full + (i & 1));
     }
     if (ok && nblk > 0) ok = mbar_wait_warp(pv_done, (nblk - 1) & 1, err);
-    if (ok && nblk > 0)
-      store_output(lane_base + 256, out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D, st.l_run, used);
+    if constexpr (SHAPED) {
+      if (nblk > 0 && !left) {
+        st.l_run += halves.meet(st.l_run, nblk & 1, ok, left);         // the row's other half
+        if (!left) {
+          if (shape.sinks != nullptr && st.l_run > 0.0f) st.l_run += exp2f(shape.sinks[head] * 1.4426950408889634f - st.m_ref);
+          if (DIFF)
+            store_difference(lane_base + 256, out + (static_cast<size_t>(q_begin + tok0 + tok) * (nh / 2) + head / 2) * D, st.l_run,
+                             used, shape, halves, (nblk + 1) & 1);
+          else
+            store_output(lane_base + 256, out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D, st.l_run, used, 2 * c, 2 * c + 2);
+        }
+      }
+    } else if (ok && nblk > 0) {
+      store_output(lane_base + 256, out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D, st.l_run, used, 0, 4);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -673,10 +884,11 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
     const int qpos = used ? my_p_lo + tok : -1;
     if (nblk_all > 0) {
       // (zeros for an unused row, and for all rows of a tile without tokens)
-      write_q_row(sm + PAIR_Q_OFF + t * TILE, q + (static_cast<size_t>(q_begin + my_tok0 + tok) * nh + head) * D, r, used);
+      write_q_row<16>(sm + PAIR_Q_OFF + t * TILE, q + (static_cast<size_t>(q_begin + my_tok0 + tok) * nh + head) * D, r, used, 0);
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
     }
+    const int lo_key = window > 0 ? qpos - window + 1 : 0, hi_key = min(qpos, my_kv_end - 1);
     RowState st;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t s_base = lane_base + t * 128, o_base = lane_base + 256 + t * 128;
@@ -686,13 +898,13 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
       if (!mbar_wait_warp(s_full + t, b & 1, err)) { ok = false; break; }
       const bool masked = first_key + BKV - 1 > my_p_lo || first_key + BKV > my_kv_end ||
                           (window > 0 && first_key <= my_p_lo + my_ntok - 1 - window);
-      ok = softmax_block(s_base, o_base, first_key, qpos, my_kv_end, window, masked, scale_log2, b, pv_done + t, st, err);
+      ok = softmax_block(s_base, o_base, first_key, lo_key, hi_key, masked, scale_log2, b, pv_done + t, st, err);
       // Value rows beyond what the CTA may see must not reach P V, whatever the page or the stage held.  Both tiles
       // write the same zeros, each before its own product.
       if (ok && first_key + BKV > kv_end_all) {
         const int s = b % VS;
         ok = mbar_wait_warp(v_full + s, (b / VS) & 1, err);
-        if (ok && first_key + r >= kv_end_all) zero_value_row(sm + PAIR_V_OFF + s * TILE, r);
+        if (ok && first_key + r >= kv_end_all) zero_value_row<16>(sm + PAIR_V_OFF + s * TILE, r, 0);
         proxy_fence();
       }
       if (!ok) break;
@@ -702,7 +914,7 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
     }
     if (ok && my_blocks > 0) ok = mbar_wait_warp(pv_done + t, (my_blocks - 1) & 1, err);
     if (ok && my_blocks > 0)
-      store_output(o_base, out + (static_cast<size_t>(q_begin + my_tok0 + tok) * nh + head) * D, st.l_run, used);
+      store_output(o_base, out + (static_cast<size_t>(q_begin + my_tok0 + tok) * nh + head) * D, st.l_run, used, 0, 4);
   }
   tc_fence_before();
   __syncthreads();
@@ -714,20 +926,24 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
 
 B200_EXPORT int b200_attention_tcgen05_head_dim() { return D; }
 
-// How many launches took the one-tile and the two-tile kernel so far (tests ask which path a model reached).
-static long long g_launches[2] = {0, 0};
-B200_EXPORT long long b200_attention_tcgen05_launches(int two_tiles) { return g_launches[two_tiles ? 1 : 0]; }
+// How many launches took the one-tile kernel (plain), the two-tile kernel and the one-tile kernel's further forms so far
+// (tests ask which path a model reached).
+static long long g_launches[3] = {0, 0, 0};
+B200_EXPORT long long b200_attention_tcgen05_launches(int kind) { return g_launches[kind < 0 || kind > 2 ? 0 : kind]; }
 
 // Portions of prompts over a bfloat16 cache, head size 128; the number of query heads per KV head must divide 128
 // and the page size must be a power of two.  `k_map`, `v_map`: descriptors of b200_kv_tensor_map (attention_mma.cu)
 // with box_rows = min(page_size, 32).  Other arguments as b200_prefill_attention of attention.cu.
 // `variant`: 1 = one tile of 128 query vectors per CTA, 2 = two tiles per CTA, 0 = two tiles when the longest
 // row then still gives every SM a CTA (pairs halve the traffic per query but also the number of CTAs).
+// `softcap` > 0, `split_p`, `chunk` > 0, `sinks` and `diff` (lambda, gain, eps; group even, no sinks): see ScoreShape; any of
+// them takes the one-tile kernel's further forms and needs scale > 0.
 B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map, const void* v_map, void* out,
                                                const int* block_table, int table_stride, const int* cu_q,
                                                const int* kv_len, const int* prefix_len, const int* rows, int n_rows,
                                                int max_q_len, int nh, int nkv, int page_size, int window, float scale,
-                                               int variant, int* err, cudaStream_t stream) {
+                                               int variant, float softcap, int split_p, int chunk, const float* sinks,
+                                               const float* diff, int* err, cudaStream_t stream) {
   if (n_rows <= 0 || max_q_len <= 0) return 0;
   if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || (page_size & (page_size - 1)) != 0) return B200_BAD_SIZE;
   if (variant < 0 || variant > 2) return B200_BAD_SIZE;
@@ -743,12 +959,16 @@ B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map,
     if (e != cudaSuccess) return static_cast<int>(e);
     sm_count = n;
   }
+  const bool shaped = softcap > 0.0f || split_p != 0 || chunk > 0 || sinks != nullptr || diff != nullptr;
+  if (shaped && (!(scale > 0.0f) || variant == 2 || (diff != nullptr && (group % 2 != 0 || sinks != nullptr)))) return B200_BAD_SIZE;
   const int n_pairs = (max_q_len + 2 * tile_tokens - 1) / (2 * tile_tokens);
-  const bool pairs = variant == 2 || (variant == 0 && static_cast<long long>(n_pairs) * nkv * n_rows >= sm_count);
-  const size_t smem = 1024 + (pairs ? PAIR_SMEM_BYTES : SMEM_BYTES);
+  const bool pairs = variant == 2 || (variant == 0 && !shaped && static_cast<long long>(n_pairs) * nkv * n_rows >= sm_count);
+  const size_t smem = 1024 + (pairs ? PAIR_SMEM_BYTES : shaped ? SHAPED_SMEM_BYTES : SMEM_BYTES);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + SMEM_BYTES);
+    cudaError_t e = cudaSuccess;
+    for (auto one : {prefill_tcgen05_kernel<false, false>, prefill_tcgen05_kernel<true, false>, prefill_tcgen05_kernel<true, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + SHAPED_SMEM_BYTES);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(prefill_tcgen05_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + PAIR_SMEM_BYTES);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -760,8 +980,20 @@ B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map,
   const int n_tiles = pairs ? n_pairs : (max_q_len + tile_tokens - 1) / tile_tokens;
   if (n_rows > 65535 || n_tiles > 65535) return B200_BAD_SIZE;      // the grid's y and z extents
   dim3 grid(nkv, n_rows, n_tiles);
-  ++g_launches[pairs ? 1 : 0];
-  return b200_launch(pairs ? prefill_tcgen05_pair_kernel : prefill_tcgen05_kernel, grid, dim3(pairs ? PAIR_THREADS : THREADS), smem, stream, 0, kmap,
-                     vmap, static_cast<const bf16*>(q), static_cast<bf16*>(out), block_table, table_stride, cu_q, kv_len,
-                     prefix_len, rows, nh, nkv, page_size, box_rows, window, scale * 1.4426950408889634f, err);
+  ++g_launches[shaped ? 2 : pairs ? 1 : 0];
+  const float scale_log2 = scale * 1.4426950408889634f;
+  if (pairs)
+    return b200_launch(prefill_tcgen05_pair_kernel, grid, dim3(PAIR_THREADS), smem, stream, 0, kmap, vmap, static_cast<const bf16*>(q),
+                       static_cast<bf16*>(out), block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size,
+                       box_rows, window, scale_log2, err);
+  ScoreShape shape = {};
+  if (softcap > 0.0f) { shape.cap_log2 = softcap * 1.4426950408889634f; shape.tanh_in = scale / softcap; }
+  shape.split = split_p;
+  shape.chunk = chunk;
+  shape.sinks = sinks;
+  if (diff != nullptr) { shape.diff_lambda = diff[0]; shape.diff_gain = diff[1]; shape.diff_eps = diff[2]; }
+  auto kernel = diff != nullptr ? prefill_tcgen05_kernel<true, true> : shaped ? prefill_tcgen05_kernel<true, false> : prefill_tcgen05_kernel<false, false>;
+  return b200_launch(kernel, grid, dim3(shaped ? SHAPED_THREADS : THREADS), smem, stream, 0, kmap, vmap, static_cast<const bf16*>(q),
+                     static_cast<bf16*>(out), block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size,
+                     box_rows, window, scale_log2, shape, err);
 }

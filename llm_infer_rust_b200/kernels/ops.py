@@ -329,6 +329,13 @@ def tcgen05_attention_launches() -> tuple:
     return int(lib.b200_attention_tcgen05_launches(0)), int(lib.b200_attention_tcgen05_launches(1))
 
 
+def tcgen05_shaped_launches() -> int:
+    """Launches of the tcgen05 prefill attention's further forms (soft-cap, weights in two terms, blocks, sinks, differences)."""
+    lib = load_cuda_library("attention_tcgen05.cu")
+    lib.b200_attention_tcgen05_launches.restype = ctypes.c_longlong
+    return int(lib.b200_attention_tcgen05_launches(2))
+
+
 def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefix_len, rows, n_rows,
                       max_q_len, num_heads, num_kv_heads, head_dim, page_size, window, scale,
                       tiles_per_cta: int = 0, v_head_dim: Optional[int] = None, softcap: float = 0.0,
@@ -339,14 +346,13 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
 
     ``v_head_dim``: the width of a value (and of an output) vector where it differs from a key's;
     ``softcap`` > 0: a score becomes cap * tanh(score / cap) before the mask; ``precise_weights``: the softmax
-    weights enter the product with the values as two bfloat16 terms (about 16 bits) instead of one.  A soft-cap, precise
-    weights and values of another width than keys take the mma.sync kernel (see ``decode_uses_tensor_cores``), not the
-    tcgen05 one (whose weights are single bfloat16 numbers in tensor memory); what that does not take goes to the
-    all-sizes kernel, whose weights are floats.
+    weights enter the product with the values as two bfloat16 terms (about 16 bits) instead of one.  Keys and values of 128
+    take the tcgen05 kernel from one or two tiles of 128 query vectors a KV head on, other sizes the mma.sync kernel (see
+    ``decode_uses_tensor_cores``); what that does not take goes to the all-sizes kernel, whose weights are floats.
 
     ``chunk`` C: a query at position p sees only keys from p - p % C on (its own block of C positions, counted from
-    the sequence's start); ``sinks`` (float32, one per query head): exp(sink) joins the softmax's denominator.  Both
-    are served by the mma.sync and the all-sizes kernels, not by the tcgen05 one.  ``shared_values``: one KV head
+    the sequence's start); ``sinks`` (float32, one per query head): exp(sink) joins the softmax's denominator.
+    ``shared_values``: one KV head
     whose values are the first ``v_head_dim`` columns of the key rows (``v_cache`` is not read and may be None): the
     mma.sync kernels fetch a block's rows once for both products and take the values in column tiles.
 
@@ -388,14 +394,17 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
         _check_difference(difference, q, out, num_heads, num_kv_heads, dv, sinks)
         box_rows = min(page_size, 32)
         group = num_heads // num_kv_heads
-        if head_dim == 128 and dv == 128 and difference is None and 128 % group == 0 and max_q_len * group >= 128 and not cap > 0.0 and not precise_weights \
-                and plain_mask:
-            # head size 128 and at least one full tile of 128 query vectors: the tcgen05 kernel
+        shaped = cap > 0.0 or precise_weights or not plain_mask or difference is not None
+        if head_dim == 128 and dv == 128 and 128 % group == 0 and max_q_len * group >= (256 if shaped else 128) \
+                and (not shaped or (scale > 0.0 and tiles_per_cta < 2)):
+            # heads of 128 and at least one full tile of 128 query vectors: the tcgen05 kernel.  Its further forms from two
+            # tiles on (16 query and 8 KV heads, weights in two terms, us on it and on the mma.sync kernel: 64 tokens 10.3 and
+            # 9.1, 128 tokens 10.4 and 12.6, 2,048 tokens 43 and 139; with a soft-cap 11.9 and 9.3, 11.8 and 12.6, 60 and 152)
             rc = load_cuda_library("attention_tcgen05.cu").b200_prefill_attention_tcgen05(
                 _p(q), kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), _p(out), _p(block_table),
                 block_table.shape[-1], _p(cu_q), _p(kv_len), _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads,
-                num_kv_heads, page_size, int(window or 0), ctypes.c_float(scale), int(tiles_per_cta),
-                _p(error_word(q.device)), _stream())
+                num_kv_heads, page_size, int(window or 0), ctypes.c_float(scale), int(tiles_per_cta), ctypes.c_float(cap),
+                int(bool(precise_weights)), int(chunk or 0), _p(sinks), _floats(difference), _p(error_word(q.device)), _stream())
             _ok(rc, "prefill_attention_tcgen05")
             return
         rc = _attention_mma(head_dim, dv, difference is not None).b200_prefill_attention_mma(

@@ -1,0 +1,77 @@
+"""The further forms of the tcgen05 prompt attention (keys and values of 128: soft-cap, weights in two terms, blocks of
+positions, sinks, windows, the difference of two maps) against the plain softmax in 64 bits, at the edges of its tiles of 128
+query vectors and blocks of 128 keys."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+D = 128
+
+
+def _plain(q, k, v, scale, cap, window, chunk, sinks, first):
+    """q [n, H, D] at positions first .., k and v [T, G, D]: float64 [n, H, D]."""
+    n, H = q.shape[:2]
+    rep = H // k.shape[1]
+    s = torch.einsum("ihd,jhd->hij", q.double(), k.double().repeat_interleave(rep, 1)) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    i, j = torch.arange(first, first + n)[:, None], torch.arange(k.shape[0])[None]
+    seen = j <= i
+    if window:
+        seen &= i - j < window
+    if chunk:
+        seen &= i // chunk == j // chunk
+    s = s.masked_fill(~seen, float("-inf"))
+    if sinks is not None:
+        s = torch.cat([s, sinks.double()[:, None, None].expand(H, n, 1)], 2)
+    return torch.einsum("hij,jhd->ihd", torch.softmax(s, 2)[:, :, :k.shape[0]], v.double().repeat_interleave(rep, 1))
+
+
+FORMS = [dict(cap=5.0), dict(), dict(cap=3.0, window=100), dict(window=17), dict(chunk=130), dict(chunk=48, sinks=True), dict(sinks=True),
+         dict(difference=(0.6, 0.65, 1e-5)), dict(difference=(0.6, 0.65, 1e-5), window=129)]
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: "-".join(f) or "split")
+@pytest.mark.parametrize("H,G,portions", [(4, 2, [128, 1, 130, 65]), (2, 2, [256, 257, 1]), (8, 1, [300]), (16, 1, [16, 17, 240]), (4, 1, [64, 3, 400])])
+def test_forms_against_the_plain_softmax(H, G, portions, form):
+    from llm_infer_rust_b200.kernels import ops
+    cap, window, chunk = form.get("cap", 0.0), form.get("window"), form.get("chunk")
+    difference = form.get("difference")
+    if difference and (H // G) % 2:
+        pytest.skip("a difference needs pairs of maps")
+    page, T, dev = 16, sum(portions), "cuda"
+    g = torch.Generator().manual_seed(T + H)
+    q, k, v = (torch.randn(T, n, D, generator=g).bfloat16() for n in (H, G, G))
+    for i in (T - 1, T // 2, 130 % T):                 # a key just outside the mask, one at its edge and the first fit best
+        lo = max(0, i - window + 1) if window else i - i % chunk if chunk else 0
+        for j, boost in ((max(0, lo - 1), 3.0), (lo, 2.0), (0, 2.5)):
+            k[j, 0] = (boost * q[i, 0].float() / q[i, 0].float().norm() * 4.0).bfloat16()
+    sinks = torch.linspace(-2.0, 4.0, H) if form.get("sinks") else None
+    pages = -(-T // page)
+    order = torch.randperm(pages, generator=g) + 1
+    caches = [torch.full((pages + 1, G, page, D), 77.0, dtype=torch.bfloat16) for _ in range(2)]     # stale values beyond
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    scale, at, heads = 0.3, 0, H // 2 if difference else H
+    for n in portions:
+        for cache, rows in zip(caches, (k, v)):
+            for p in range(at, at + n):
+                cache[order[p // page], :, p % page] = rows[p]
+        kc, vc = (c.to(dev) for c in caches)
+        out = torch.full((n, heads * D), float("nan"), dtype=torch.bfloat16, device=dev)
+        before = ops.tcgen05_shaped_launches()
+        ops.prefill_attention(q[at:at + n].reshape(n, -1).to(dev).contiguous(), kc, vc, out, order.to(torch.int32).reshape(1, -1).to(dev),
+                              i32([0, n]), i32([at + n]), i32([at]), i32([0]), 1, n, H, G, D, page, window, scale, v_head_dim=D,
+                              softcap=cap, precise_weights=True, chunk=chunk, sinks=None if sinks is None else sinks.to(dev),
+                              difference=difference)
+        ops.check_errors(torch.device(dev))
+        assert ops.tcgen05_shaped_launches() - before == (1 if n * (H // G) >= 256 else 0)
+        want = _plain(q[at:at + n], k[:at + n], v[:at + n], scale, cap, window, chunk, sinks, at)
+        slack = 2.0 ** -13 * v.float().abs().max().item()           # weights of 16 bits, sums and exponents in 32
+        if difference:
+            lam, gain, eps = difference
+            o = want[:, 0::2] - lam * want[:, 1::2]
+            f = gain / torch.sqrt((o * o).mean(-1, keepdim=True) + eps)
+            want, slack = o * f, 4 * slack * f                      # two maps, and the root that their error moves
+        got = out.cpu().double().reshape(n, heads, D)
+        assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()      # the stored value is rounded to 8 bits
+        at += n
