@@ -167,6 +167,20 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
                ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+               "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                 "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+               "tcgen05.wait::ld.sync.aligned;\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
@@ -297,6 +311,90 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
   st.l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
   tmem_wait_st();                                      // P is in tensor memory
   return pv_seen || mbar_wait_warp(pv_done, (block - 1) & 1, err);
+}
+
+// The two-tile kernel's block: all 128 scores in registers (one load of the row, where softmax_block waits for four), and the
+// products with the values begin when half of the weights stand: `half_done` is called behind the first 64 keys' weights.
+// S of a block is issued behind P V of the block before it, so whoever has seen these scores may touch the accumulator:
+// pv_done is not asked.  A tile walks a chain of its own latencies (measured with softmax_block, SM cycles a block at 8,192
+// tokens: 2,040 until the next scores stand, 2,700 in the softmax, 1,720 of those behind the maximum, for 1,024 of
+// special-function work), so what shortens the chain counts: 8,192 tokens x 16 heads 340 -> 302 us, 16,384 x 32 2,165 us
+// (1,015 TFLOP/s).  Two threads a row, which pay for the further forms below, were slower here (483 us: sixteen warps
+// leave 96 registers a thread, so the scores are read twice).
+__device__ __forceinline__ void tmem_ld32_begin(uint32_t taddr, float (&v)[32]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+               "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+                 "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+                 "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
+                 "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+               : "r"(taddr));
+}
+template <typename F>
+__device__ __forceinline__ void softmax_row(uint32_t s_base, uint32_t o_base, int first_key, int lo_key, int hi_key, bool masked,
+                                            float scale_log2, int block, RowState& st, const F& half_done) {
+  tc_fence_after();
+  float v[4][32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld32_begin(s_base + c * 32, v[c]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int e = 0; e < 32; ++e) asm volatile("" : "+f"(v[c][e]));      // (used only behind the wait)
+  if (masked) {
+    const int lo = lo_key - first_key, hi = hi_key - first_key;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int e = 0; e < 32; ++e) v[c][e] = c * 32 + e >= lo && c * 32 + e <= hi ? v[c][e] : -INFINITY;
+  }
+  float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int e = 0; e < 32; ++e) m4[e & 3] = fmaxf(m4[e & 3], v[c][e]);
+  const float raw = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+  const float mx = hi_key >= 0 ? raw * scale_log2 : -INFINITY;
+  const bool raise = mx > st.m_ref + RESCALE_STEP || (st.m_ref == -INFINITY && mx > -INFINITY);
+  const float m_new = raise ? mx : st.m_ref;
+  if (__any_sync(0xffffffffu, raise ? 1 : 0)) {
+    const float corr = raise ? (st.m_ref == -INFINITY ? 0.0f : exp2f(st.m_ref - m_new)) : 1.0f;
+    st.l_run *= corr;
+    if (block > 0) {
+#pragma unroll 1
+      for (int c = 0; c < 8; ++c) {
+        uint32_t o[16];
+        tmem_ld16(o_base + c * 16, o);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+        tmem_st16(o_base + c * 16, o);
+      }
+      tmem_wait_st();
+    }
+  }
+  st.m_ref = m_new;
+  const float neg_base = hi_key < 0 ? -INFINITY : m_new == -INFINITY ? 0.0f : -m_new;      // a row that is not used gets zeros
+  float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t pr[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float a = fast_exp2(fmaf(v[c][2 * i], scale_log2, neg_base)), b = fast_exp2(fmaf(v[c][2 * i + 1], scale_log2, neg_base));
+      sum4[i & 3] += a + b;
+      const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
+      pr[i] = *reinterpret_cast<const uint32_t*>(&two);
+    }
+    tmem_st16(s_base + c * 16, pr);
+    if (c == 1) {
+      tmem_wait_st();
+      half_done();
+    }
+  }
+  st.l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+  tmem_wait_st();                                      // P is in tensor memory
 }
 
 // ---- The further forms of a score and of what is stored, for the builds of the one-tile kernel that know them (SHAPED):
@@ -722,7 +820,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
 constexpr int PAIR_K_STAGES = 2, PAIR_V_STAGES = 2;      // (deeper rings were slower: more copies in flight, same traffic)
 constexpr int PAIR_V_OFF = 0, PAIR_K_OFF = PAIR_V_STAGES * TILE, PAIR_Q_OFF = PAIR_K_OFF + PAIR_K_STAGES * TILE;
 constexpr int PAIR_BAR_OFF = PAIR_Q_OFF + 2 * TILE;
-constexpr int PAIR_N_BARS = 2 * PAIR_K_STAGES + 2 * PAIR_V_STAGES + 2 + 2 + 2 + 1;
+constexpr int PAIR_N_BARS = 2 * PAIR_K_STAGES + 2 * PAIR_V_STAGES + 2 + 2 + 2 + 2 + 1;
 constexpr int PAIR_TBL_OFF = PAIR_BAR_OFF + (PAIR_N_BARS + 1) * 8;
 constexpr int PAIR_SMEM_BYTES = PAIR_TBL_OFF + TBL_ENTRIES * 4;
 
@@ -741,7 +839,8 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
   uint64_t* v_empty = v_full + VS;
   uint64_t* s_full = v_empty + VS;                                   // [2]: one per tile
   uint64_t* p_full = s_full + 2;                                     // [2]
-  uint64_t* pv_done = p_full + 2;                                    // [2]
+  uint64_t* p_half = p_full + 2;                                     // [2]: the weights of a block's first 64 keys
+  uint64_t* pv_done = p_half + 2;                                    // [2]
   uint64_t* q_full = pv_done + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 1);
 
@@ -749,7 +848,7 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
   if (threadIdx.x == 0) {
     for (int s = 0; s < KS; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); }
     for (int s = 0; s < VS; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
-    for (int t = 0; t < 2; ++t) { mbar_init(s_full + t, 1); mbar_init(p_full + t, 4); mbar_init(pv_done + t, 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(s_full + t, 1); mbar_init(p_full + t, 4); mbar_init(p_half + t, 4); mbar_init(pv_done + t, 1); }
     mbar_init(q_full, 8);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -859,14 +958,21 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || b >= nblk[t]) continue;
-          ok = mbar_wait(p_full + t, b & 1, err);            // P of block b lies where S of block b lay
+          ok = mbar_wait(p_half + t, b & 1, err);            // P of block b lies where S of block b lay
           if (ok) ok = mbar_wait(v_full + s, (b / VS) & 1, err);
           if (!ok) continue;
           tc_fence_after();
           const uint64_t v_step = static_cast<uint64_t>(s * (TILE >> 4));
 #pragma unroll
-          for (int j = 0; j < BKV / 16; ++j)
+          for (int j = 0; j < BKV / 16; ++j) {
+            if (j == BKV / 32) {                             // the weights of the other 64 keys
+              ok = mbar_wait(p_full + t, b & 1, err);
+              if (!ok) break;
+              tc_fence_after();
+            }
             umma_a_tmem(tmem_base + 256 + t * 128, tmem_base + t * 128 + j * 8, dv[j] + v_step, kDescPV, (b > 0 || j > 0) ? 1u : 0u);
+          }
+          if (!ok) continue;
           umma_commit(pv_done + t);
           if (t == 1 || b >= nblk[1]) umma_commit(v_empty + s);
           if (b + 1 < nblk[t]) ok = issue_s(t, b + 1);
@@ -898,20 +1004,25 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
       if (!mbar_wait_warp(s_full + t, b & 1, err)) { ok = false; break; }
       const bool masked = first_key + BKV - 1 > my_p_lo || first_key + BKV > my_kv_end ||
                           (window > 0 && first_key <= my_p_lo + my_ntok - 1 - window);
-      ok = softmax_block(s_base, o_base, first_key, lo_key, hi_key, masked, scale_log2, b, pv_done + t, st, err);
       // Value rows beyond what the CTA may see must not reach P V, whatever the page or the stage held.  Both tiles
       // write the same zeros, each before its own product.
-      if (ok && first_key + BKV > kv_end_all) {
+      if (first_key + BKV > kv_end_all) {
         const int s = b % VS;
         ok = mbar_wait_warp(v_full + s, (b / VS) & 1, err);
-        if (ok && first_key + r >= kv_end_all) zero_value_row<16>(sm + PAIR_V_OFF + s * TILE, r, 0);
+        if (!ok) break;
+        if (first_key + r >= kv_end_all) zero_value_row<16>(sm + PAIR_V_OFF + s * TILE, r, 0);
         proxy_fence();
       }
-      if (!ok) break;
+      softmax_row(s_base, o_base, first_key, lo_key, hi_key, masked, scale_log2, b, st, [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_half + t);
+      });
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full + t);
     }
+    // (S of the last block was issued behind P V of the one before it: only this phase can be the one that runs)
     if (ok && my_blocks > 0) ok = mbar_wait_warp(pv_done + t, (my_blocks - 1) & 1, err);
     if (ok && my_blocks > 0)
       store_output(o_base, out + (static_cast<size_t>(q_begin + my_tok0 + tok) * nh + head) * D, st.l_run, used, 0, 4);
