@@ -145,6 +145,27 @@ sigmoid_gate_mul_kernel(T* out, const T* a, const T* __restrict__ g, int g_strid
   }
 }
 
+// The same with one gate an element and eight elements a thread in 16-byte accesses (rows of whole 16-byte pieces).  Bound by
+// memory: one element a thread at a time, 1,500 rows of 2,048 bfloat16 took 23.5 us for 18 MB.
+template <typename T>
+__global__ void __launch_bounds__(256)
+sigmoid_gate_mul_vec_kernel(T* out, const T* a, const T* __restrict__ g, int g_stride, int width) {          // out may be a
+  pdl_launch_dependents();                          // the kernel after this one may be scheduled; it waits before it reads
+  pdl_wait();                                        // what this kernel reads belongs to the kernels before it
+  const size_t t = blockIdx.x;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= width) return;
+  float x[8], v[8];
+  load_floats<T, 8>(g + t * g_stride + c, x);
+  load_floats<T, 8>(a + t * width + c, v);
+  __align__(16) T y[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) y[i] = from_f32<T>(v[i] / (1.0f + expf(-x[i])));
+#pragma unroll
+  for (int i = 0; i < static_cast<int>(sizeof(y) / 16); ++i)
+    reinterpret_cast<uint4*>(out + t * width + c)[i] = reinterpret_cast<const uint4*>(y)[i];
+}
+
 B200_EXPORT int b200_poly_norm(void* out, const void* z, const float* coef, float eps, int tokens, int width,
                                int dtype, cudaStream_t stream) {
   if (tokens <= 0) return 0;
@@ -193,6 +214,15 @@ B200_EXPORT int b200_sigmoid_gate_mul(void* out, const void* a, const void* g, i
                                       int per, int dtype, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (width <= 0 || per <= 0 || width % per) return B200_BAD_SIZE;
+  if (per == 1 && width % 8 == 0 && g_stride % 8 == 0 && (dtype == B200_F32 || dtype == B200_BF16) &&
+      (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(g)) % 16 == 0) {
+    const dim3 grid(tokens, (width / 8 + 255) / 256), block(width / 8 < 256 ? (width / 8 + 31) / 32 * 32 : 256);
+    if (dtype == B200_F32)
+      return b200_launch(sigmoid_gate_mul_vec_kernel<float>, grid, block, 0, stream, 0, static_cast<float*>(out),
+                         static_cast<const float*>(a), static_cast<const float*>(g), g_stride, width);
+    return b200_launch(sigmoid_gate_mul_vec_kernel<__nv_bfloat16>, grid, block, 0, stream, 0, static_cast<__nv_bfloat16*>(out),
+                       static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(g), g_stride, width);
+  }
   if (dtype == B200_F32)
     return b200_launch(sigmoid_gate_mul_kernel<float>, dim3(tokens), dim3(256), 0, stream, 0, static_cast<float*>(out),
                        static_cast<const float*>(a), static_cast<const float*>(g), g_stride, width, per);

@@ -1,0 +1,89 @@
+"""Kernels and branches at the sizes where their split of the work changes, against the same operation in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rnd(*shape, dtype=torch.float32, seed=0, scale=1.0):
+    return (scale * torch.randn(*shape, generator=torch.Generator().manual_seed(seed))).to(DEV, dtype)
+
+
+# rows at the edge of the two kernels (16, 17), one column beyond a tile, K around chunks (128), spans (512), more spans than
+# warps (8), more than one span a block, odd K (no 16-byte loads)
+@pytest.mark.parametrize("m,n,k", [(1, 9, 127), (3, 8, 129), (16, 7, 513), (2, 24, 4500), (17, 65, 4100), (64, 64, 512), (65, 129, 1028),
+                                   (300, 1024, 2048), (33, 130, 515), (16, 40, 9001), (5, 3000, 1024), (16, 1030, 3072)])
+def test_32_bit_products(m, n, k):
+    from llm_infer_rust_b200.kernels import ops
+    a, w = _rnd(m, k), _rnd(n, k, seed=1)
+    got = ops.gemm_f32(a, w)
+    want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    # a chain of 128 sums, then 3, then K / 512: at most (131 + K / 512) roundings of 2^-24 of the terms' size
+    assert ((got.double() - want).abs() <= (131 + k / 512) * 2.0 ** -24 * size).all()
+    for r in {0, m // 2, m - 1}:                              # bit for bit what the row gives alone (the kernel for few rows)
+        assert torch.equal(ops.gemm_f32(a[r:r + 1].contiguous(), w)[0], got[r])
+
+
+def test_32_bit_products_of_a_head_each():
+    from llm_infer_rust_b200.kernels import ops
+    for rows in (3, 70):
+        x, w = _rnd(rows, 4 * 24 + 5), _rnd(4, 19, 24, seed=2)      # column ranges of wider rows, not 16-byte aligned
+        parts = x[:, 5:].reshape(rows, 4, 24).transpose(0, 1)
+        got = ops.head_products(parts, w)
+        want = torch.einsum("hrk,hnk->hrn", parts.double(), w.double())
+        assert ((got.double() - want).abs() <= 2.0 ** -20 * (1 + want.abs().max())).all()
+
+
+@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 1024), (torch.bfloat16, 1032), (torch.bfloat16, 4096), (torch.bfloat16, 16384),
+                                         (torch.bfloat16, 16392), (torch.float32, 512), (torch.float32, 516), (torch.float32, 8192)])
+def test_rms_norm_by_warps_by_blocks_and_beyond(dtype, width):
+    from llm_infer_rust_b200.kernels import ops
+    x, res, w = _rnd(5, width, dtype=dtype), _rnd(5, width, dtype=dtype, seed=1), _rnd(width, dtype=dtype, seed=2)
+    s = x.double() + res.double()
+    want = s / torch.sqrt((s * s).mean(-1, keepdim=True) + 1e-6) * w.double()
+    kept = res.clone()
+    got = ops.add_rms_norm(x, kept, w, 1e-6)
+    bound = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20          # one rounding of the result; float sums of squares
+    assert ((got.double() - want).abs() <= bound * want.abs() + 1e-6).all()
+    assert torch.equal(kept, (x.float() + res.float()).to(dtype))
+    rows = torch.tensor([4, 0, 4], dtype=torch.int32, device=DEV)
+    alone = ops.rms_norm(x, w, 1e-6, rows=rows)
+    xd = x.double()[[4, 0, 4]]
+    want = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((alone.double() - want).abs() <= bound * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,width,column", [(1, 8, 0), (3, 2048, 8), (2, 4104, 16), (5, 40, 3), (3, 12, 0)])
+def test_gates_in_whole_and_in_broken_vectors(tokens, width, column, dtype):
+    from llm_infer_rust_b200.kernels import ops
+    packed, a = _rnd(tokens, column + width + 8, dtype=dtype, scale=4.0), _rnd(tokens, width, dtype=dtype, seed=1)
+    want = a.double() * torch.sigmoid(packed[:, column:column + width].double())
+    got = ops.sigmoid_gate_mul(a.clone(), packed, column)
+    assert ((got.double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * want.abs() + 1e-9).all()
+
+
+@pytest.mark.parametrize("lengths", [[1 + (37 * i) % 200 for i in range(40)], [64] * 39 + [1], list(range(1, 75))])
+def test_decoded_rows_of_many_lengths_in_several_waves(lengths):
+    """More CTAs than SMs: the rows start longest first, whatever their order in the batch; every row is its own."""
+    from llm_infer_rust_b200.kernels import ops
+    H, G, D, page, n = 8, 4, 128, 16, len(lengths)
+    pages = [-(-x // page) for x in lengths]
+    first, width = [1 + sum(pages[:i]) for i in range(n)], max(pages)
+    kc, vc = (_rnd(1 + sum(pages), G, page, D, dtype=torch.bfloat16, seed=s) for s in (3, 4))
+    table = torch.zeros(n, width, dtype=torch.int32)
+    for i in range(n):
+        table[i, :pages[i]] = torch.arange(first[i], first[i] + pages[i])
+    q = _rnd(n, H * D, dtype=torch.bfloat16, seed=5)
+    out = torch.empty_like(q)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ops.decode_attention(q, kc, vc, out, None, table.to(DEV), i32(list(range(n + 1))), i32(lengths), i32(list(range(n))), n, H, G, D, page,
+                         None, D ** -0.5, 1)
+    ops.check_errors(torch.device(DEV))
+    for i in range(n):
+        k, v = (c[first[i]:first[i] + pages[i]].transpose(1, 2).reshape(-1, G, D)[:lengths[i]].double().repeat_interleave(H // G, 1) for c in (kc, vc))
+        s = torch.einsum("hd,jhd->hj", q[i].view(H, D).double(), k) * D ** -0.5
+        want = torch.einsum("hj,jhd->hd", torch.softmax(s, 1), v)
+        # a weight is rounded to 8 bits, and so is the result
+        assert ((out[i].view(H, D).double() - want).abs() <= 2.0 ** -8 * (want.abs() + v.abs().amax(0))).all(), i
