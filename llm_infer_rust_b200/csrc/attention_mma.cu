@@ -305,13 +305,15 @@ __device__ __forceinline__ void block_mma(const bf16* qs, const unsigned char* k
 // grid (splits, nkv, decode rows).  Partials: part_acc[((row * nh + head) * splits + split) * D + dim]
 // (unnormalised), part_ml[...][2] = (maximum in log2 units, sum).
 // Shared memory: [WARPS][STAGES] tiles (1024-byte aligned), the query tile [16][LD], the barriers.
-template <int WARPS, int STAGES, bool SHAPED>
+// SORTED: the rows with the most keys first (a build of its own: a step of one wave is a chain of short kernels and feels
+// every instruction in front of its first fetch, 0.5 % of a step of one row).
+template <int WARPS, int STAGES, bool SHAPED, bool SORTED>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                   const bf16* __restrict__ q, bf16* __restrict__ out, float* __restrict__ part_acc,
                   float* __restrict__ part_ml, const int* __restrict__ block_table, int table_stride,
                   const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ rows, int nh,
-                  int nkv, int page_size, int box_rows, int window, ScoreForm sf, int cluster_merge, int longest_first, int* err) {
+                  int nkv, int page_size, int box_rows, int window, ScoreForm sf, int cluster_merge, int* err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   bf16* qs = reinterpret_cast<bf16*>(tiles + static_cast<size_t>(WARPS) * STAGES * TILE_BYTES);   // [16][LD]
@@ -326,7 +328,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
   // both may be read while that kernel still runs.
   const int splits = gridDim.x, split = blockIdx.x, kvh = blockIdx.y;
   int pick = blockIdx.z;
-  if (longest_first) {
+  if constexpr (SORTED) {
     // More CTAs than SMs: they start in the grid's order, so the rows with the most keys come first and the short ones
     // fill the gaps behind them (45 rows of 100 to 2,000 keys x 8 KV heads, in the batch's order: 48 us for 30 us of bytes; now 42).
     // Every CTA ranks the rows by itself, a row a thread, under the kernel before.
@@ -863,12 +865,22 @@ B200_EXPORT int b200_decode_attention_mma(const void* q, const void* k_map, cons
   const int box_rows = page_size < KB ? page_size : KB;
   constexpr size_t smem = kFixedBytes + static_cast<size_t>(kWarps) * kStages * TILE_BYTES;
   const bool shaped = softcap > 0.0f || split_p != 0;
-  auto* kernel = shaped ? decode_mma_kernel<kWarps, kStages, true> : decode_mma_kernel<kWarps, kStages, false>;
-  static bool configured[2] = {false, false};
-  if (!configured[shaped]) {
+  static int sm_count = 0;
+  if (sm_count == 0) {
+    int dev = 0, n = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    sm_count = n;
+  }
+  const bool sorted = splits == 1 && static_cast<long long>(nkv) * n_rows > sm_count && n_rows <= kWarps * 32;
+  auto* kernel = shaped ? (sorted ? decode_mma_kernel<kWarps, kStages, true, true> : decode_mma_kernel<kWarps, kStages, true, false>)
+                        : (sorted ? decode_mma_kernel<kWarps, kStages, false, true> : decode_mma_kernel<kWarps, kStages, false, false>);
+  static bool configured[2][2] = {{false, false}, {false, false}};
+  if (!configured[shaped][sorted]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured[shaped] = true;
+    configured[shaped][sorted] = true;
   }
   CUtensorMap kmap, vmap;
   memcpy(&kmap, k_map, sizeof(kmap));
@@ -880,22 +892,13 @@ B200_EXPORT int b200_decode_attention_mma(const void* q, const void* k_map, cons
   // other counts leave them in `scratch` for a kernel of its own.
   // (Only while the grid is one wave: clusters must be placed whole, and with several waves of one CTA per SM that
   // costs more than the second kernel, 10.1 k against 10.7 k tokens a second at batch 64.)
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0, n = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    sm_count = n;
-  }
   const bool cluster_merge = (splits == 2 || splits == 4 || splits == 8) &&
                              static_cast<long long>(splits) * nkv * n_rows <= sm_count;
-  const bool longest_first = splits == 1 && static_cast<long long>(nkv) * n_rows > sm_count && n_rows <= kWarps * 32;
   int rc = b200_launch(kernel, grid, dim3(kWarps * 32), smem, stream, cluster_merge ? splits : 0,
                        kmap, vmap, static_cast<const bf16*>(q), static_cast<bf16*>(out), part_acc, part_ml, block_table,
                        table_stride, cu_q, kv_len, rows, nh, nkv, page_size, box_rows, window,
                        score_form(scale, softcap, split_p, chunk, sinks, v_col0, kShared ? out_width : DV, kShared ? out_col0 : 0, diff),
-                       cluster_merge ? 1 : 0, longest_first ? 1 : 0, err);
+                       cluster_merge ? 1 : 0, err);
   if (rc != 0 || splits == 1 || cluster_merge) return rc;
   if constexpr (kDiff) {
     return b200_launch(decode_mma_merge_diff_kernel, dim3(n_rows, nh / 2), dim3(DV >= 128 ? 128 : 64), 0, stream, 0,
