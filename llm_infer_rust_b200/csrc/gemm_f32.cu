@@ -353,6 +353,9 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const int spans = (p.k + SPAN - 1) / SPAN;
+  // Up to 16 rows one pass over W through shared memory beats a tile of 64 that is mostly padding (16 rows, weights of 4,096 x
+  // 1,024 / 1,024 x 2,048 / 1,024 x 3,072: 23 / 18 / 23 us against 47 / 47 / 47 on tiles); 17 to 32 rows are two passes or more
+  // (44 to 52 / 54 to 71 / 54 to 73 us) and tiles stay at 47.
   if (p.m <= 16) {
     const int sw = spans < 8 ? spans : 8, tiles = (p.n + FEW_WN - 1) / FEW_WN;
     int nt = 8 / sw;
