@@ -305,9 +305,11 @@ __device__ __forceinline__ void block_mma(const bf16* qs, const unsigned char* k
 // grid (splits, nkv, decode rows).  Partials: part_acc[((row * nh + head) * splits + split) * D + dim]
 // (unnormalised), part_ml[...][2] = (maximum in log2 units, sum).
 // Shared memory: [WARPS][STAGES] tiles (1024-byte aligned), the query tile [16][LD], the barriers.
-// SORTED: the rows with the most keys first (a build of its own: a step of one wave is a chain of short kernels and feels
-// every instruction in front of its first fetch, 0.5 % of a step of one row).
-template <int WARPS, int STAGES, bool SHAPED, bool SORTED>
+// CTAs start in the grid's order, so the caller lists the rows with the most keys first: in a grid of several waves the short
+// ones then fill the gaps behind them (45 rows of 100 to 2,000 keys x 8 KV heads, four query heads each: 45.9 us in the batch's
+// order, 41.3 by length).  Ranked by every CTA for itself the same rows took 42.5 us, and rows of one length paid for nothing
+// (64 of 512 keys, two query heads: 33.7 -> 35.1 us; 128 of 1,000: 101.6 -> 109.3).
+template <int WARPS, int STAGES, bool SHAPED>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                   const bf16* __restrict__ q, bf16* __restrict__ out, float* __restrict__ part_acc,
@@ -327,24 +329,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constan
   // step's index arrays were uploaded before the step's first kernel, and all other keys and values are older:
   // both may be read while that kernel still runs.
   const int splits = gridDim.x, split = blockIdx.x, kvh = blockIdx.y;
-  int pick = blockIdx.z;
-  if constexpr (SORTED) {
-    // More CTAs than SMs: they start in the grid's order, so the rows with the most keys come first and the short ones
-    // fill the gaps behind them (45 rows of 100 to 2,000 keys x 8 KV heads, in the batch's order: 48 us for 30 us of bytes; now 42).
-    // Every CTA ranks the rows by itself, a row a thread, under the kernel before.
-    __shared__ int lens[WARPS * 32];
-    __shared__ int chosen;
-    const int i = threadIdx.x, n = gridDim.z;
-    const int mine = i < n ? kv_len[rows[i]] : 0;
-    lens[i] = mine;
-    __syncthreads();
-    int rank = 0;
-    for (int j = 0; j < n; ++j) rank += lens[j] > mine || (lens[j] == mine && j < i);
-    if (i < n && rank == pick) chosen = i;
-    __syncthreads();
-    pick = chosen;
-  }
-  const int row = rows[pick];
+  const int row = rows[blockIdx.z];
   const int group = nh / nkv, head0 = kvh * group;
   const int tok = cu_q[row];
   const int kv_end = kv_len[row];
@@ -865,22 +850,12 @@ B200_EXPORT int b200_decode_attention_mma(const void* q, const void* k_map, cons
   const int box_rows = page_size < KB ? page_size : KB;
   constexpr size_t smem = kFixedBytes + static_cast<size_t>(kWarps) * kStages * TILE_BYTES;
   const bool shaped = softcap > 0.0f || split_p != 0;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0, n = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    sm_count = n;
-  }
-  const bool sorted = splits == 1 && static_cast<long long>(nkv) * n_rows > sm_count && n_rows <= kWarps * 32;
-  auto* kernel = shaped ? (sorted ? decode_mma_kernel<kWarps, kStages, true, true> : decode_mma_kernel<kWarps, kStages, true, false>)
-                        : (sorted ? decode_mma_kernel<kWarps, kStages, false, true> : decode_mma_kernel<kWarps, kStages, false, false>);
-  static bool configured[2][2] = {{false, false}, {false, false}};
-  if (!configured[shaped][sorted]) {
+  auto* kernel = shaped ? decode_mma_kernel<kWarps, kStages, true> : decode_mma_kernel<kWarps, kStages, false>;
+  static bool configured[2] = {false, false};
+  if (!configured[shaped]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured[shaped][sorted] = true;
+    configured[shaped] = true;
   }
   CUtensorMap kmap, vmap;
   memcpy(&kmap, k_map, sizeof(kmap));
@@ -892,6 +867,14 @@ B200_EXPORT int b200_decode_attention_mma(const void* q, const void* k_map, cons
   // other counts leave them in `scratch` for a kernel of its own.
   // (Only while the grid is one wave: clusters must be placed whole, and with several waves of one CTA per SM that
   // costs more than the second kernel, 10.1 k against 10.7 k tokens a second at batch 64.)
+  static int sm_count = 0;
+  if (sm_count == 0) {
+    int dev = 0, n = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    sm_count = n;
+  }
   const bool cluster_merge = (splits == 2 || splits == 4 || splits == 8) &&
                              static_cast<long long>(splits) * nkv * n_rows <= sm_count;
   int rc = b200_launch(kernel, grid, dim3(kWarps * 32), smem, stream, cluster_merge ? splits : 0,

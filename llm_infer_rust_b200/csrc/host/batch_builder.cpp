@@ -49,6 +49,7 @@ BatchLayout plan_batch(const CacheManager& cache, const BatchRequest& req) {
   L.off_prefix_len = take(L.num_rows);
   L.off_state_slot = take(L.num_rows);
   L.off_decode_rows = take(L.num_decode);
+  L.off_decode_order = take(L.num_decode);
   L.off_prefill_rows = take(L.num_prefill);
   L.off_logit_rows = take(L.num_logits);
   for (int g = 0; g < G; ++g) {
@@ -119,6 +120,12 @@ BatchLayout build_batch(const CacheManager& cache, const BatchRequest& req, int3
       }
     }
   }
+  // Decode attention starts its CTAs in the order of this list: in a grid of several waves the long rows then begin first and
+  // the short ones fill the gaps behind them.
+  int32_t* order = out + L.off_decode_order;
+  std::copy(out + L.off_decode_rows, out + L.off_decode_rows + n_dec, order);
+  const int32_t* kv_len = out + L.off_kv_len;
+  std::sort(order, order + n_dec, [kv_len](int32_t a, int32_t b) { return kv_len[a] != kv_len[b] ? kv_len[a] > kv_len[b] : a < b; });
   return L;
 }
 

@@ -28,6 +28,7 @@ struct BatchLayout {
   int off_tokens = 0, off_positions = 0, off_row_of_token = 0;
   int off_cu_q = 0, off_kv_len = 0, off_prefix_len = 0, off_state_slot = 0;
   int off_decode_rows = 0, off_prefill_rows = 0, off_logit_rows = 0;
+  int off_decode_order = 0;       // the decode rows again, those with the most keys first (equal ones in the batch's order)
   std::vector<int> off_slots;     // per group: write slot of every token
   std::vector<int> off_table;     // per group: block table [num_rows, table_width]
   std::vector<int> table_width;   // per group

@@ -141,6 +141,7 @@ PYBIND11_MODULE(_host_runtime, m) {
       .def_readonly("off_prefix_len", &BatchLayout::off_prefix_len)
       .def_readonly("off_state_slot", &BatchLayout::off_state_slot)
       .def_readonly("off_decode_rows", &BatchLayout::off_decode_rows)
+      .def_readonly("off_decode_order", &BatchLayout::off_decode_order)
       .def_readonly("off_prefill_rows", &BatchLayout::off_prefill_rows)
       .def_readonly("off_logit_rows", &BatchLayout::off_logit_rows)
       .def_readonly("off_slots", &BatchLayout::off_slots)

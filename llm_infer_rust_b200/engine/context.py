@@ -33,7 +33,7 @@ class StepContext:
     kv_len: torch.Tensor
     prefix_len: torch.Tensor
     state_slots: torch.Tensor
-    decode_rows: torch.Tensor
+    decode_rows: torch.Tensor            # those with the most keys first
     prefill_rows: torch.Tensor
     logit_rows: torch.Tensor
     slots: List[torch.Tensor]
@@ -67,7 +67,7 @@ def context_from_layout(layout, dev: torch.Tensor, host: Optional[torch.Tensor],
         row_of_token=view(layout.off_row_of_token, T), cu_q=view(layout.off_cu_q, R + 1),
         kv_len=view(layout.off_kv_len, R), prefix_len=view(layout.off_prefix_len, R),
         state_slots=view(layout.off_state_slot, R),
-        decode_rows=view(layout.off_decode_rows, layout.num_decode),
+        decode_rows=view(layout.off_decode_order, layout.num_decode),
         prefill_rows=view(layout.off_prefill_rows, layout.num_prefill),
         logit_rows=view(layout.off_logit_rows, layout.num_logits),
         slots=[view(layout.off_slots[g], T) for g in range(groups)],

@@ -543,7 +543,7 @@ def decode_attention(q, k_cache, v_cache, out, scratch, block_table, cu_q, kv_le
                      shared_values: bool = False, difference: Optional[Tuple[float, float, float]] = None) -> None:
     """Attention of single decoded tokens, the keys split over ``splits`` blocks per row (``v_head_dim``,
     ``softcap``, ``precise_weights``, ``chunk``, ``sinks``, ``shared_values``, ``difference``: see
-    ``prefill_attention``)."""
+    ``prefill_attention``).  Rows start in the order of ``rows``: list those with the most keys first."""
     _cuda(q, k_cache, v_cache, out, scratch, block_table, cu_q, kv_len, rows, sinks)
     _contig(q, k_cache, v_cache, out, block_table, scratch, sinks)
     _check_sinks(sinks, num_heads)

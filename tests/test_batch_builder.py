@@ -7,6 +7,7 @@ lengths, the last-token (or any wanted) logit rows and the block table.
 """
 import numpy as np
 import pytest
+import torch
 
 from llm_infer_rust_b200.kernels.build import load_host_runtime
 
@@ -190,3 +191,27 @@ def test_random_steps_against_a_recount(seed):
     for rid in live:
         m.release(rid)
     assert m.check() == "" and all(m.free_pages(g) == 200 for g in range(len(specs)))
+
+
+@pytest.mark.parametrize("lengths,pad,order", [([3, 9, 5, 9, 1], 0, [1, 3, 2, 0, 4]), ([2, 7], 4, [1, 0, 2, 3]), ([4, 4, 4], 0, [0, 1, 2]),
+                                               ([6], 0, [0])])
+def test_decode_attention_gets_the_rows_with_the_most_keys_first(lengths, pad, order):
+    """Decode attention starts its blocks in this order; equal rows keep the batch's, padding rows (one key) come last."""
+    from llm_infer_rust_b200.engine.context import context_from_layout
+    m = rt.CacheManager([rt.GroupSpec(2, 40, 0)], 6)
+    for i, n in enumerate(lengths):
+        grown(m, i + 1, n - 1, n)
+    grown(m, 99, 0, 3)
+    rows = [(i + 1, [i], [0]) for i in range(len(lengths))]
+    if not pad:                                           # a prompt's portion between them has no place in the list
+        rows.insert(1, (99, [7, 7, 7], [2]))
+        order = [r if r == 0 else r + 1 for r in order]
+    req = rt.BatchRequest()
+    req.ids, req.counts = [r[0] for r in rows], [len(r[1]) for r in rows]
+    req.tokens, req.want_counts, req.want_index = [t for r in rows for t in r[1]], [1] * len(rows), [r[2][0] for r in rows]
+    req.pad_rows_to, req.fixed_table_width = pad, [20]
+    buf = torch.full((rt.plan_batch(m, req).total_ints,), -7, dtype=torch.int32)
+    lay = rt.build_batch(m, req, buf.numpy())
+    ctx = context_from_layout(lay, buf, None, [2], torch.device("cpu"), torch.float32, 20)
+    assert ctx.decode_rows.tolist() == order
+    assert sorted(order) == buf[lay.off_decode_rows:lay.off_decode_rows + lay.num_decode].tolist()

@@ -66,7 +66,7 @@ def test_gates_in_whole_and_in_broken_vectors(tokens, width, column, dtype):
 
 @pytest.mark.parametrize("lengths", [[1 + (37 * i) % 200 for i in range(40)], [64] * 39 + [1], list(range(1, 75))])
 def test_decoded_rows_of_many_lengths_in_several_waves(lengths):
-    """More CTAs than SMs: the rows start longest first, whatever their order in the batch; every row is its own."""
+    """More CTAs than SMs, rows listed in any order: every row is its own."""
     from llm_infer_rust_b200.kernels import ops
     H, G, D, page, n = 8, 4, 128, 16, len(lengths)
     pages = [-(-x // page) for x in lengths]
