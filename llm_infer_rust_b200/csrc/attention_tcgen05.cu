@@ -1048,7 +1048,7 @@ B200_EXPORT long long b200_attention_tcgen05_launches(int kind) { return g_launc
 // `variant`: 1 = one tile of 128 query vectors per CTA, 2 = two tiles per CTA, 0 = two tiles when the longest
 // row then still gives every SM a CTA (pairs halve the traffic per query but also the number of CTAs).
 // `softcap` > 0, `split_p`, `chunk` > 0, `sinks` and `diff` (lambda, gain, eps; group even, no sinks): see ScoreShape; any of
-// them takes the one-tile kernel's further forms and needs scale > 0.
+// them takes the one-tile kernel's further forms.  `scale` > 0.
 B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map, const void* v_map, void* out,
                                                const int* block_table, int table_stride, const int* cu_q,
                                                const int* kv_len, const int* prefix_len, const int* rows, int n_rows,
@@ -1071,7 +1071,8 @@ B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map,
     sm_count = n;
   }
   const bool shaped = softcap > 0.0f || split_p != 0 || chunk > 0 || sinks != nullptr || diff != nullptr;
-  if (shaped && (!(scale > 0.0f) || variant == 2 || (diff != nullptr && (group % 2 != 0 || sinks != nullptr)))) return B200_BAD_SIZE;
+  if (!(scale > 0.0f)) return B200_BAD_SIZE;                         // maxima and masks are taken of the unscaled scores
+  if (shaped && (variant == 2 || (diff != nullptr && (group % 2 != 0 || sinks != nullptr)))) return B200_BAD_SIZE;
   const int n_pairs = (max_q_len + 2 * tile_tokens - 1) / (2 * tile_tokens);
   const bool pairs = variant == 2 || (variant == 0 && !shaped && static_cast<long long>(n_pairs) * nkv * n_rows >= sm_count);
   const size_t smem = 1024 + (pairs ? PAIR_SMEM_BYTES : shaped ? SHAPED_SMEM_BYTES : SMEM_BYTES);

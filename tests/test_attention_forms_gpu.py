@@ -75,3 +75,35 @@ def test_forms_against_the_plain_softmax(H, G, portions, form):
         got = out.cpu().double().reshape(n, heads, D)
         assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()      # the stored value is rounded to 8 bits
         at += n
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.2, 0.3])
+@pytest.mark.parametrize("H,G,rows", [(4, 4, 40), (16, 8, 1)])
+def test_a_scale_of_any_sign(H, G, rows, scale):
+    """Plain prompts at sizes where scale > 0 takes two tiles a CTA (40 rows) and one: with scale 0 every visible key weighs the
+    same, with scale < 0 the worst fitting one weighs most."""
+    from llm_infer_rust_b200.kernels import ops
+    page, n, dev = 16, 300, "cuda"
+    g = torch.Generator().manual_seed(rows)
+    q = torch.randn(rows * n, H, D, generator=g).bfloat16()
+    k, v = (torch.randn(rows, n, G, D, generator=g).bfloat16() for _ in range(2))
+    pages = -(-n // page)
+    caches = []
+    for x in (k, v):
+        c = torch.zeros(1 + rows * pages, G, page, D, dtype=torch.bfloat16)
+        c[1:] = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, pages * page - n)).reshape(rows * pages, page, G, D).transpose(1, 2)
+        caches.append(c.to(dev))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    out = torch.empty(rows * n, H * D, dtype=torch.bfloat16, device=dev)
+    before = ops.tcgen05_attention_launches()
+    ops.prefill_attention(q.reshape(rows * n, -1).to(dev), *caches, out, i32([[1 + r * pages + p for p in range(pages)] for r in range(rows)]),
+                          i32([r * n for r in range(rows + 1)]), i32([n] * rows), i32([0] * rows), i32(list(range(rows))), rows, n, H, G, D, page,
+                          None, scale)
+    ops.check_errors(torch.device(dev))
+    took = tuple(b - a for a, b in zip(before, ops.tcgen05_attention_launches()))
+    assert took == ((0, 0) if scale <= 0 else (0, 1) if rows > 1 else (1, 0))
+    for r in (0, rows - 1):
+        want = _plain(q[r * n:(r + 1) * n], k[r], v[r], scale, 0.0, None, None, None, 0)
+        got = out[r * n:(r + 1) * n].cpu().double().reshape(n, H, D)
+        # a weight is rounded to 8 bits, and so is the result
+        assert ((got - want).abs() <= 2.0 ** -8 * (want.abs() + v[r].float().abs().max().item())).all()
