@@ -1048,7 +1048,7 @@ B200_EXPORT long long b200_attention_tcgen05_launches(int kind) { return g_launc
 // `variant`: 1 = one tile of 128 query vectors per CTA, 2 = two tiles per CTA, 0 = two tiles when the longest
 // row then still gives every SM a CTA (pairs halve the traffic per query but also the number of CTAs).
 // `softcap` > 0, `split_p`, `chunk` > 0, `sinks` and `diff` (lambda, gain, eps; group even, no sinks): see ScoreShape; any of
-// them takes the one-tile kernel's further forms.  `scale` > 0.
+// them takes the one-tile kernel's further forms.  `scale` > 0; q and out on 16-byte boundaries.
 B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map, const void* v_map, void* out,
                                                const int* block_table, int table_stride, const int* cu_q,
                                                const int* kv_len, const int* prefix_len, const int* rows, int n_rows,
@@ -1058,6 +1058,7 @@ B200_EXPORT int b200_prefill_attention_tcgen05(const void* q, const void* k_map,
   if (n_rows <= 0 || max_q_len <= 0) return 0;
   if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || (page_size & (page_size - 1)) != 0) return B200_BAD_SIZE;
   if (variant < 0 || variant > 2) return B200_BAD_SIZE;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) % 16 != 0) return B200_BAD_ALIGN;
   const int group = nh / nkv;
   if (group > BQ || BQ % group != 0) return B200_BAD_SIZE;
   const int box_rows = page_size < 32 ? page_size : 32;

@@ -396,9 +396,10 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
         group = num_heads // num_kv_heads
         shaped = cap > 0.0 or precise_weights or not plain_mask or difference is not None
         if head_dim == 128 and dv == 128 and 128 % group == 0 and max_q_len * group >= (256 if shaped else 128) \
-                and scale > 0.0 and (not shaped or tiles_per_cta < 2):
-            # heads of 128, at least one full tile of 128 query vectors and scores that keep their order (the kernel takes a
-            # block's maximum, and masks, before it scales): the tcgen05 kernel.  Its further forms from two
+                and scale > 0.0 and out.data_ptr() % 16 == 0 and (not shaped or tiles_per_cta < 2):
+            # heads of 128, at least one full tile of 128 query vectors, scores that keep their order (the kernel takes a
+            # block's maximum, and masks, before it scales) and an output for 16-byte stores (the mma.sync kernel's are of 4
+            # bytes): the tcgen05 kernel.  Its further forms from two
             # tiles on (16 query and 8 KV heads, weights in two terms, us on it and on the mma.sync kernel: 64 tokens 10.3 and
             # 9.1, 128 tokens 10.4 and 12.6, 2,048 tokens 43 and 139; with a soft-cap 11.9 and 9.3, 11.8 and 12.6, 60 and 152)
             rc = load_cuda_library("attention_tcgen05.cu").b200_prefill_attention_tcgen05(

@@ -107,3 +107,28 @@ def test_a_scale_of_any_sign(H, G, rows, scale):
         got = out[r * n:(r + 1) * n].cpu().double().reshape(n, H, D)
         # a weight is rounded to 8 bits, and so is the result
         assert ((got - want).abs() <= 2.0 ** -8 * (want.abs() + v[r].float().abs().max().item())).all()
+
+
+@pytest.mark.parametrize("form", [dict(), dict(precise_weights=True, softcap=5.0), dict(precise_weights=True, difference=(0.6, 0.65, 1e-5))],
+                         ids=lambda f: "-".join(f) or "plain")
+def test_an_output_between_16_byte_boundaries(form):
+    """The output may be a view that begins 4 or 8 bytes into its storage: another kernel serves it, to the same result."""
+    from llm_infer_rust_b200.kernels import ops
+    H, G, page, n, dev = 4, 2, 16, 300, "cuda"
+    g = torch.Generator().manual_seed(3)
+    q = torch.randn(n, H * D, generator=g).bfloat16().to(dev)
+    kc, vc = (torch.randn(20, G, page, D, generator=g).bfloat16().to(dev) for _ in range(2))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    width = H * D // 2 if "difference" in form else H * D
+    outs = []
+    for skip in (0, 2, 4):                                # elements of two bytes
+        out = torch.full((n * width + 8,), float("nan"), dtype=torch.bfloat16, device=dev)[skip:skip + n * width].view(n, width)
+        before = sum(ops.tcgen05_attention_launches()) + ops.tcgen05_shaped_launches()
+        ops.prefill_attention(q, kc, vc, out, i32([list(range(1, 20))]), i32([0, n]), i32([n]), i32([0]), i32([0]), 1, n, H, G, D, page, None,
+                              0.2, v_head_dim=D, **form)
+        ops.check_errors(torch.device(dev))
+        assert sum(ops.tcgen05_attention_launches()) + ops.tcgen05_shaped_launches() - before == (0 if skip else 1)
+        outs.append(out.double())
+    assert torch.equal(outs[1], outs[2])
+    # two roundings to 8 bits apart, and (plain) weights of 8 bits on both sides; a difference's root moves with its maps' error
+    assert (outs[0] - outs[1]).abs().max() <= (2.0 ** -7 + (2.0 ** -8 if not form else 2.0 ** -10)) * vc.double().abs().max()
