@@ -502,16 +502,15 @@ static int launch_decode(const void* q, const void* kc, const void* vc, void* ou
   constexpr int DEC_WARPS = fixed4 + 4 * tile_bytes <= limit ? 4 : (fixed4 + 2 * tile_bytes <= limit ? 2 : 1);
   constexpr size_t fixed = (NV * D + DEC_WARPS * KB * NV) * sizeof(float);
   static_assert(fixed + DEC_WARPS * tile_bytes <= 220 * 1024, "one key block per warp must fit shared memory");
-  const int stages = fixed + DEC_WARPS * 2 * tile_bytes <= limit ? 2 : 1;
-  size_t smem = fixed + DEC_WARPS * stages * tile_bytes;
-  const size_t merge_bytes = DEC_WARPS * NV * (D + 2) * sizeof(float);
-  if (fixed + merge_bytes > smem) smem = fixed + merge_bytes;
-  static size_t configured = 0;
-  if (smem > configured) {
+  constexpr int stages = fixed + DEC_WARPS * 2 * tile_bytes <= limit ? 2 : 1;
+  constexpr size_t merge_bytes = DEC_WARPS * NV * (D + 2) * sizeof(float);
+  constexpr size_t smem = fixed + (merge_bytes > DEC_WARPS * stages * tile_bytes ? merge_bytes : DEC_WARPS * stages * tile_bytes);
+  static bool configured = false;
+  if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<T, DEC_WARPS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured = smem;
+    configured = true;
   }
   dim3 grid(splits, nkv * vec_groups, n_rows);
   decode_attention_kernel<T, DEC_WARPS><<<grid, DEC_WARPS * 32, smem, stream>>>(

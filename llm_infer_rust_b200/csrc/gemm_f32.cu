@@ -326,20 +326,23 @@ tiled_kernel(const Product p, int ksplit) {
 
 // ------------------------------------------------------------------ launchers
 constexpr size_t FEW_SMEM_LIMIT = 225 * 1024;
+constexpr int DEVICES = 16;                     // whose launch limits are remembered
 
 static size_t few_bytes(int mr, int sw, int nt) {
   return (static_cast<size_t>(mr) * 4 * sw * FEW_XCHUNK + 2 * sw * nt * FEW_WN * mr + sw * nt * FEW_STAGES * FEW_STAGE) * sizeof(float);
 }
 
 template <int MR, bool VEC>
-static int launch_few(const Product& p, int batch, int sw, int nt, int sms, cudaStream_t stream) {
+static int launch_few(const Product& p, int batch, int sw, int nt, int device, int sms, cudaStream_t stream) {
   const int warps = sw * nt;
   const size_t smem = few_bytes(MR, sw, nt);
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(few_rows_kernel<MR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  // Once a device, and the same size whoever comes first: a size that grew with the launches could be taken back by a thread
+  // whose smaller launch met a larger one.
+  static bool configured[DEVICES];
+  if (device >= DEVICES || !configured[device]) {
+    cudaError_t e = cudaFuncSetAttribute(few_rows_kernel<MR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(FEW_SMEM_LIMIT));
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured = smem;
+    if (device < DEVICES) configured[device] = true;
   }
   const int groups = (p.n + FEW_WN * nt - 1) / (FEW_WN * nt);
   const int resident = static_cast<int>((227 * 1024) / (smem + 1024));
@@ -351,7 +354,9 @@ static int launch_few(const Product& p, int batch, int sw, int nt, int sms, cuda
 
 static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   int device = 0, sms = 148;
-  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return static_cast<int>(e);
   const int spans = (p.k + SPAN - 1) / SPAN;
   // Up to 16 rows one pass over W through shared memory beats a tile of 64 that is mostly padding (16 rows, weights of 4,096 x
   // 1,024 / 1,024 x 2,048 / 1,024 x 3,072: 23 / 18 / 23 us against 47 / 47 / 47 on tiles); 17 to 32 rows are two passes or more
@@ -363,11 +368,11 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
     int mr = p.m > 8 ? 16 : p.m > 4 ? 8 : p.m > 2 ? 4 : p.m;
     while (mr > 1 && few_bytes(mr, sw, nt) > FEW_SMEM_LIMIT) mr /= 2;
     switch (mr) {
-      case 16: return vec ? launch_few<16, true>(p, batch, sw, nt, sms, stream) : launch_few<16, false>(p, batch, sw, nt, sms, stream);
-      case 8: return vec ? launch_few<8, true>(p, batch, sw, nt, sms, stream) : launch_few<8, false>(p, batch, sw, nt, sms, stream);
-      case 4: return vec ? launch_few<4, true>(p, batch, sw, nt, sms, stream) : launch_few<4, false>(p, batch, sw, nt, sms, stream);
-      case 2: return vec ? launch_few<2, true>(p, batch, sw, nt, sms, stream) : launch_few<2, false>(p, batch, sw, nt, sms, stream);
-      default: return vec ? launch_few<1, true>(p, batch, sw, nt, sms, stream) : launch_few<1, false>(p, batch, sw, nt, sms, stream);
+      case 16: return vec ? launch_few<16, true>(p, batch, sw, nt, device, sms, stream) : launch_few<16, false>(p, batch, sw, nt, device, sms, stream);
+      case 8: return vec ? launch_few<8, true>(p, batch, sw, nt, device, sms, stream) : launch_few<8, false>(p, batch, sw, nt, device, sms, stream);
+      case 4: return vec ? launch_few<4, true>(p, batch, sw, nt, device, sms, stream) : launch_few<4, false>(p, batch, sw, nt, device, sms, stream);
+      case 2: return vec ? launch_few<2, true>(p, batch, sw, nt, device, sms, stream) : launch_few<2, false>(p, batch, sw, nt, device, sms, stream);
+      default: return vec ? launch_few<1, true>(p, batch, sw, nt, device, sms, stream) : launch_few<1, false>(p, batch, sw, nt, device, sms, stream);
     }
   }
   const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + BM - 1) / BM;
@@ -390,7 +395,7 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   config.attrs = &attr;
   config.numAttrs = ksplit > 1 ? 1 : 0;
-  cudaError_t e = vec ? cudaLaunchKernelEx(&config, tiled_kernel<true>, p, ksplit) : cudaLaunchKernelEx(&config, tiled_kernel<false>, p, ksplit);
+  e = vec ? cudaLaunchKernelEx(&config, tiled_kernel<true>, p, ksplit) : cudaLaunchKernelEx(&config, tiled_kernel<false>, p, ksplit);
   return e == cudaSuccess ? b200_check_launch() : static_cast<int>(e);
 }
 

@@ -81,13 +81,14 @@ static int launch_step(float* streams, const float* start, const void* y, const 
                        const float* norm_w, float offset, float eps, const int* rows, void* out, int n, int width,
                        int store, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(width) * sizeof(float);
-  if (smem > 200 * 1024) return B200_BAD_SIZE;
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
+  constexpr size_t limit = 200 * 1024;
+  if (smem > limit) return B200_BAD_SIZE;
+  static bool configured = false;                     // (the same size whoever comes first: see gemm_f32.cu)
+  if (smem > 48 * 1024 && !configured) {
     cudaError_t e = cudaFuncSetAttribute(stream_step_kernel<S, TY, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+                                         static_cast<int>(limit));
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured = smem;
+    configured = true;
   }
   stream_step_kernel<S, TY, TO><<<n, 256, smem, stream>>>(streams, start, static_cast<const TY*>(y), before, read_in,
                                                           norm_w, offset, eps, rows, static_cast<TO*>(out), width,
