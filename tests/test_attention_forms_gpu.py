@@ -132,3 +132,54 @@ def test_an_output_between_16_byte_boundaries(form):
     assert torch.equal(outs[1], outs[2])
     # two roundings to 8 bits apart, and (plain) weights of 8 bits on both sides; a difference's root moves with its maps' error
     assert (outs[0] - outs[1]).abs().max() <= (2.0 ** -7 + (2.0 ** -8 if not form else 2.0 ** -10)) * vc.double().abs().max()
+
+
+SEVERAL = [dict(cap=5.0), dict(chunk=130, sinks=True), dict(window=129, difference=(0.6, 0.65, 1e-5)), dict(cap=5.0, sinks=True),
+           dict(window=100, sinks=True), dict(chunk=48)]
+
+
+@pytest.mark.parametrize("precise", [True, False], ids=["two-terms", "one-term"])
+@pytest.mark.parametrize("form", SEVERAL, ids="-".join)
+@pytest.mark.parametrize("H,G", [(4, 2), (16, 1)])
+def test_forms_over_rows_of_all_lengths(H, G, form, precise):
+    """Several rows in one launch, named in another order than the batch's, with cached tokens before them, among them rows with
+    nothing in most of the grid's tiles; weights in two bfloat16 terms and in one."""
+    from llm_infer_rust_b200.kernels import ops
+    cap, window, chunk, difference = form.get("cap", 0.0), form.get("window"), form.get("chunk"), form.get("difference")
+    rows, page, dev = [(0, 700), (300, 333), (5, 1), (0, 128)], 16, "cuda"
+    g = torch.Generator().manual_seed(H)
+    n = sum(r[1] for r in rows)
+    q = torch.randn(n, H, D, generator=g).bfloat16()
+    k, v = ([torch.randn(a + b, G, D, generator=g).bfloat16() for a, b in rows] for _ in range(2))
+    pages = [-(-(a + b) // page) for a, b in rows]
+    order = (torch.randperm(sum(pages), generator=g) + 1).tolist()
+    caches = [torch.full((sum(pages) + 1, G, page, D), 77.0, dtype=torch.bfloat16) for _ in range(2)]      # stale values beyond
+    table = torch.zeros(len(rows), max(pages), dtype=torch.int32)
+    for r, (a, b) in enumerate(rows):
+        mine = [order.pop() for _ in range(pages[r])]
+        table[r, :pages[r]] = torch.tensor(mine, dtype=torch.int32)
+        for cache, x in zip(caches, (k[r], v[r])):
+            for p in range(a + b):
+                cache[mine[p // page], :, p % page] = x[p]
+    sinks = torch.linspace(-2.0, 4.0, H) if form.get("sinks") else None
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    first, heads = [0, 700, 1033, 1034, 1162], H // 2 if difference else H
+    out = torch.full((n, heads * D), float("nan"), dtype=torch.bfloat16, device=dev)
+    before = ops.tcgen05_shaped_launches()
+    ops.prefill_attention(q.reshape(n, -1).to(dev), *(c.to(dev) for c in caches), out, table.to(dev), i32(first), i32([a + b for a, b in rows]),
+                          i32([a for a, _ in rows]), i32([2, 0, 3, 1]), 4, 700, H, G, D, page, window, 0.3, v_head_dim=D, softcap=cap,
+                          precise_weights=precise, chunk=chunk, sinks=None if sinks is None else sinks.to(dev), difference=difference)
+    ops.check_errors(torch.device(dev))
+    assert ops.tcgen05_shaped_launches() - before == 1
+    for r, (a, b) in enumerate(rows):
+        at = slice(first[r], first[r + 1])
+        want = _plain(q[at], k[r], v[r], 0.3, cap, window, chunk, sinks, a)
+        # weights of 16 bits or of 8, sums and exponents in 32
+        slack = 2.0 ** (-13 if precise else -8) * v[r].float().abs().max().item()
+        if difference:
+            lam, gain, eps = difference
+            o = want[:, 0::2] - lam * want[:, 1::2]
+            f = gain / torch.sqrt((o * o).mean(-1, keepdim=True) + eps)
+            want, slack = o * f, 4 * slack * f                      # two maps, and the root that their error moves
+        got = out[at].cpu().double().reshape(b, heads, D)
+        assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + slack).all(), r
