@@ -352,6 +352,24 @@ static int launch_few(const Product& p, int batch, int sw, int nt, int device, i
   return b200_check_launch();
 }
 
+// How many blocks (of one cluster) share a tile's spans: as many as give the fullest SM the least time (of equal times the
+// fewest rounds, then the fewest blocks).  An SM holds four blocks, and a block's two warps keep half of its schedulers busy, so a second block
+// costs nothing beside the first, a third and a fourth half as much again (one span, 1 to 4 blocks on an SM: 41, 43, 63, 66 us;
+// more come in waves of four).  Counted as if two blocks took an SM twice the time, 128 tiles of two spans stayed one block each:
+// N x K = 4,096 x 1,024 at 65 to 128 rows 84 us for 44, 6,144 x 1,024 at 17 to 64 rows 83 for 43, 1,024 x 2,048 at 500 176 for
+// 65 (the single chain of 64 x 64 tiles that came before: 69, 70, 124).
+static int blocks_a_tile(long long tiles, int spans, int sms) {
+  int best = 1;
+  long long best_cost = 0, best_rounds = 0;
+  for (int s = 1; s <= 8 && s <= spans; ++s) {
+    const long long blocks = (tiles * s + sms - 1) / sms, rounds = (spans + s - 1) / s;
+    const long long cost = rounds * (3 * (blocks / 4) + (blocks % 4 == 0 ? 0 : blocks % 4 <= 2 ? 2 : 3));
+    if (s == 1 || cost < best_cost || (cost == best_cost && rounds < best_rounds)) { best = s; best_cost = cost; best_rounds = rounds; }
+  }
+  return best;
+}
+B200_EXPORT int b200_gemm_f32_blocks_a_tile(long long tiles, int spans, int sms) { return blocks_a_tile(tiles, spans, sms); }
+
 static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   int device = 0, sms = 148;
   cudaError_t e = cudaGetDevice(&device);
@@ -377,13 +395,7 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   }
   const int n_tiles = (p.n + BN - 1) / BN, m_tiles = (p.m + BM - 1) / BM;
   const long long tiles = static_cast<long long>(n_tiles) * m_tiles * batch;
-  // How many blocks share a tile's spans: as few as give the fullest SM the least work (in spans).
-  int ksplit = 1;
-  long long best = (tiles + sms - 1) / sms * spans;
-  for (int s = 2; s <= 8 && s <= spans; ++s) {
-    const long long cost = (tiles * s + sms - 1) / sms * ((spans + s - 1) / s);
-    if (cost < best) { best = cost; ksplit = s; }
-  }
+  const int ksplit = blocks_a_tile(tiles, spans, sms);
   if (m_tiles > 65535) return B200_BAD_SIZE;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(n_tiles * ksplit, m_tiles, batch);

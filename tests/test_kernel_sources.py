@@ -1,4 +1,5 @@
 """What the kernels' sources promise and no single launch shows."""
+import ctypes
 import os
 import re
 
@@ -17,3 +18,17 @@ def test_launch_limits_do_not_follow_the_launches():
             grows = re.findall(r"\bstatic (?:size_t|int|unsigned|long long) configured\b.*", text)
             assert not grows, f"{name}: {grows}"
     assert seen > 5
+
+
+def test_blocks_that_share_a_tile_of_32_bit_products():
+    """Measured with every count of blocks (148 SMs): the fullest SM's time decides, two blocks on an SM cost as much as one."""
+    lib = build.load_cuda_library("gemm_f32.cu")
+
+    def shared(m, n, k):
+        tiles, spans = -(-m // 64) * -(-n // 64), -(-k // 512)
+        return lib.b200_gemm_f32_blocks_a_tile(ctypes.c_longlong(tiles), spans, 148)
+    for m, n, k, blocks in ((64, 4096, 1024, 2), (128, 4096, 1024, 2), (48, 6144, 1024, 2), (500, 1024, 2048, 4), (500, 1024, 3072, 6),
+                            (128, 4096, 2048, 4), (64, 4096, 4096, 8), (300, 24576, 4096, 8), (64, 4096, 12288, 8), (17, 64, 300, 1)):
+        assert shared(m, n, k) == blocks, (m, n, k)
+    # nine or ten spans take two rounds with five blocks or with eight: the three more would only add a round to nothing
+    assert shared(64, 64, 5000) == 5 and shared(64, 64, 4500) == 5 and shared(64, 64, 4096) == 8
