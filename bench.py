@@ -458,11 +458,11 @@ def kernel_table(size, peak):
                 q, k_cache, v_cache, o, c.table, c.cu_q, c.kv_len, c.prefix_len, c.rows, 1, T, nh, nkv, d, page, None,
                 d ** -0.5), flush), flops=fl, of="bf16")
         else:
-            from llm_infer_rust_b200.parts.attention import decode_splits
+            from llm_infer_rust_b200.parts.attention import attention_splits
             kvb = rows_dec * ctx_len * nkv * d * 2 * 2
             for name, kw in (("kefetar.attention_softcap", dict(v_head_dim=d, softcap=50.0, precise_weights=True)),
                              ("qwen3.attention", {})):
-                splits = decode_splits(ops.decode_ctas_per_split(bf, rows_dec, nh, nkv, d, page), ctx_len, 148)
+                splits = attention_splits(bf, rows_dec, nh, nkv, d, page, ctx_len, 148)
                 need = ops.decode_scratch_floats(rows_dec, nh, d, splits)
                 scratch = torch.empty(max(need, 1), device=dev)
                 put(f"decode.{name}", timed_alone(lambda: ops.decode_attention(
@@ -520,7 +520,7 @@ def mukenex_kernel_table(size, peak):
     import types
     import torch
     from llm_infer_rust_b200.kernels import ops
-    from llm_infer_rust_b200.parts.attention import decode_splits
+    from llm_infer_rust_b200.parts.attention import attention_splits
     z = DESIGN_SIZES[size]
     W, nh, nkv, d, I = z["width"], z["heads"], z["kv_heads"], z["head_dim"], z["inter"]
     rank, r, S, E, top, ffe, window = (256 if W <= 1024 else 384), 64, 4, 8, 2, z["inter"] // 2, 1024
@@ -619,10 +619,7 @@ def mukenex_kernel_table(size, peak):
                 d ** -0.5), flush), flops=4.0 * nh * d * T * (T + 1) / 2, of="bf16")
         else:
             def decode(name, qq, kk, vv, oo, heads, kvh, dk, dv_, bound, nbytes, **kw):
-                per_split = ops.decode_ctas_per_split(bf, rows_dec, heads, kvh, dk, page, dv_)
-                if kw.get("shared_values"):
-                    per_split = rows_dec * (heads // ops.latent_head_group(heads))
-                splits = decode_splits(per_split, bound, 148)
+                splits = attention_splits(bf, rows_dec, heads, kvh, dk, page, bound, 148, dv_, kw.get("shared_values", False))
                 need = ops.decode_scratch_floats(rows_dec, heads, max(dk, dv_), splits)
                 scratch = torch.empty(max(need, 1), device=dev)
                 win, scale = kw.pop("window_", None), kw.pop("scale_", dk ** -0.5)
@@ -719,7 +716,7 @@ def torinex_kernel_table(size, peak):
     import types
     import torch
     from llm_infer_rust_b200.kernels import ops
-    from llm_infer_rust_b200.parts.attention import decode_splits
+    from llm_infer_rust_b200.parts.attention import attention_splits
     z = DESIGN_SIZES[size]
     W, nh, nkv, d, I = z["width"], z["heads"], z["kv_heads"], z["head_dim"], z["inter"]
     r = TORINEX_EXPERTS
@@ -799,8 +796,7 @@ def torinex_kernel_table(size, peak):
                 d ** -0.5), flush), flops=4.0 * nh * d * T * (T + 1) / 2, of="bf16")
         else:
             def decode(name, bound, nbytes, **kw):
-                per_split = ops.decode_ctas_per_split(bf, rows_dec, nh, nkv, d, page)
-                splits = decode_splits(per_split, bound, 148)
+                splits = attention_splits(bf, rows_dec, nh, nkv, d, page, bound, 148)
                 need = ops.decode_scratch_floats(rows_dec, nh, d, splits)
                 scratch = torch.empty(max(need, 1), device=dev)
                 put(name, timed_alone(lambda: ops.decode_attention(
@@ -909,7 +905,7 @@ def lufizen_kernel_table(size, peak):
     import types
     import torch
     from llm_infer_rust_b200.kernels import ops
-    from llm_infer_rust_b200.parts.attention import decode_splits
+    from llm_infer_rust_b200.parts.attention import attention_splits
     z = DESIGN_SIZES[size]
     W, nh, nkv, d, I = z["width"], z["heads"], z["kv_heads"], z["head_dim"], z["inter"]
     rank, q_rank, r = lufizen_ranks(size)
@@ -1022,12 +1018,7 @@ def lufizen_kernel_table(size, peak):
                 flops=2.0 * nh * (2 * rank + r) * sum(min(p, window - 1) + 1 for p in range(T)), of="bf16")
         else:
             def decode(name, qq, kk, vv, oo, heads, kvh, dk, dv_, bound, nbytes, **kw):
-                per_split = ops.decode_ctas_per_split(bf, rows_dec, heads, kvh, dk, page, dv_)
-                keys = 512
-                if kw.get("shared_values"):
-                    per_split = rows_dec * (heads // ops.latent_head_group(heads))
-                    keys = 128                                     # the engine's rule for latent rows
-                splits = decode_splits(per_split, bound, 148, keys)
+                splits = attention_splits(bf, rows_dec, heads, kvh, dk, page, bound, 148, dv_, kw.get("shared_values", False))
                 need = ops.decode_scratch_floats(rows_dec, heads, max(dk, dv_), splits)
                 scratch = torch.empty(max(need, 1), device=dev)
                 win, scale = kw.pop("window_", None), kw.pop("scale_", dk ** -0.5)
@@ -1147,7 +1138,7 @@ def sigudra_kernel_table(size, peak):
     import types
     import torch
     from llm_infer_rust_b200.kernels import ops
-    from llm_infer_rust_b200.parts.attention import decode_splits
+    from llm_infer_rust_b200.parts.attention import attention_splits
     z, s, r = DESIGN_SIZES[size], sigudra_sizes(size), SIGUDRA_EXPERTS
     W, nh, nkv, d, I = z["width"], z["heads"], z["kv_heads"], z["head_dim"], z["inter"]
     E, top, ffe, window = r["experts"], r["top"], I // r["top"], s["window"]
@@ -1280,7 +1271,7 @@ def sigudra_kernel_table(size, peak):
                     q, k_cache, v_cache, o, c.table, c.cu_q, c.kv_len, c.prefix_len, c.rows, 1, T, nh, nkv, d, page, win,
                     d ** -0.5, **more), flush, repeats=few), flops=4.0 * nh * d * seen)
             else:
-                splits = decode_splits(ops.decode_ctas_per_split(bf, rows_dec, nh, nkv, d, page), window, 148)
+                splits = attention_splits(bf, rows_dec, nh, nkv, d, page, window, 148)
                 scratch = torch.empty(max(ops.decode_scratch_floats(rows_dec, nh, d, splits), 1), device=dev)
                 put(f"decode.{name}", timed_alone(lambda: ops.decode_attention(
                     q, k_cache, v_cache, o, scratch, c.table, c.cu_q, c.kv_len, c.rows, rows_dec, nh, nkv, d, page, win,
@@ -1353,7 +1344,7 @@ def bevuvik_kernel_table(size, peak):
     from llm_infer_rust_b200.config.spec import PartSpec
     from llm_infer_rust_b200.kernels import ops
     from llm_infer_rust_b200.parts import BuildEnv, build_part
-    from llm_infer_rust_b200.parts.attention import decode_splits
+    from llm_infer_rust_b200.parts.attention import attention_splits
     z = DESIGN_SIZES[size]
     W, nh, nkv, d, I = z["width"], z["heads"], z["kv_heads"], z["head_dim"], z["inter"]
     window, taps, rank, rkv = 1024, 4, z["head_dim"], z["heads"] // 2
@@ -1467,7 +1458,7 @@ def bevuvik_kernel_table(size, peak):
                     d ** -0.5, **more), flush, repeats=few), flops=per_pair * seen)
             else:
                 seen = min(win_ or ctx_len, ctx_len)
-                splits = decode_splits(ops.decode_ctas_per_split(bf, rows_dec, heads, nkv, d, page), seen, 148)
+                splits = attention_splits(bf, rows_dec, heads, nkv, d, page, seen, 148)
                 scratch = torch.empty(max(ops.decode_scratch_floats(rows_dec, heads, d, splits), 1), device=dev)
                 put(f"decode.{name}", timed_alone(lambda: ops.decode_attention(
                     qq, k_cache, v_cache, oo, scratch, c.table, c.cu_q, c.kv_len, c.rows, rows_dec, heads, nkv, d, page, win_,

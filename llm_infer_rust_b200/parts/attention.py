@@ -44,11 +44,18 @@ def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int,
     return cluster
 
 
-def _keys_per_cta(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim=None) -> int:
-    """The fewest keys worth a CTA: the all-sizes kernel's takes in 128 at a time, a tenth as fast as the tensor-core one."""
-    if ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim):
-        return _KEYS_PER_CTA_AT_LEAST
-    return _ALL_SIZES_KEYS_PER_CTA_AT_LEAST
+def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, kv_len_bound: int,
+                     sm_count: int, v_head_dim=None, shared_values: bool = False) -> int:
+    """Into how many splits decode attention cuts the keys of ``rows`` rows that hold up to ``kv_len_bound`` keys each (or see
+    no more), by the kernel that serves them (arguments as ``ops.decode_attention``)."""
+    if shared_values and ops.latent_uses_tensor_cores(dtype, num_heads, head_dim, v_head_dim, page_size):
+        return decode_splits(rows * (num_heads // ops.latent_head_group(num_heads)), kv_len_bound, sm_count,
+                             _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS)
+    # the all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one
+    on_tensor_cores = ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim)
+    return decode_splits(ops.decode_ctas_per_split(dtype, rows, num_heads, num_kv_heads, head_dim, page_size, v_head_dim),
+                         kv_len_bound, sm_count,
+                         _KEYS_PER_CTA_AT_LEAST if on_tensor_cores else _ALL_SIZES_KEYS_PER_CTA_AT_LEAST)
 
 
 class GQAttention(Part):
@@ -128,9 +135,7 @@ class GQAttention(Part):
                                   self.nh, self.nkv, self.d, page, self.window, self.scale)
         if ctx.num_decode:
             bound = min(ctx.kv_len_bound, self.window) if self.window else ctx.kv_len_bound
-            per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page)
-            splits = decode_splits(per_split, bound, ctx.sm_count,
-                                   _keys_per_cta(q.dtype, self.nh, self.nkv, self.d, page))
+            splits = attention_splits(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page, bound, ctx.sm_count)
             need = ops.decode_scratch_floats(ctx.num_decode, self.nh, self.d, splits)
             scratch = ctx.scratch(need) if need else None
             ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,
@@ -239,9 +244,7 @@ class GatedConvAttention(Part):
                                   v_head_dim=self.dv, softcap=self.softcap, precise_weights=True)
         if ctx.num_decode:
             bound = min(ctx.kv_len_bound, self.window) if self.window else ctx.kv_len_bound
-            per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page, self.dv)
-            splits = decode_splits(per_split, bound, ctx.sm_count,
-                                   _keys_per_cta(q.dtype, self.nh, self.nkv, self.d, page, self.dv))
+            splits = attention_splits(q.dtype, ctx.num_decode, self.nh, self.nkv, self.d, page, bound, ctx.sm_count, self.dv)
             need = ops.decode_scratch_floats(ctx.num_decode, self.nh, max(self.d, self.dv), splits)
             scratch = ctx.scratch(need) if need else None
             ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,
@@ -272,14 +275,8 @@ def _masked_attention(part, q, out, ctx, cache, num_heads, num_kv_heads, head_di
         for limit in (part.window, part.chunk):
             if limit:
                 bound = min(bound, limit)
-        keys_per_cta, keys_for_more = _KEYS_PER_CTA_AT_LEAST, _KEYS_FOR_MORE_SPLITS
-        if shared_values and ops.latent_uses_tensor_cores(q.dtype, num_heads, head_dim, v_head_dim, page):
-            per_split = ctx.num_decode * (num_heads // ops.latent_head_group(num_heads))
-            keys_per_cta, keys_for_more = _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS
-        else:
-            per_split = ops.decode_ctas_per_split(q.dtype, ctx.num_decode, num_heads, num_kv_heads, head_dim, page, v_head_dim)
-            keys_per_cta = _keys_per_cta(q.dtype, num_heads, num_kv_heads, head_dim, page, v_head_dim)
-        splits = decode_splits(per_split, bound, ctx.sm_count, keys_per_cta, keys_for_more)
+        splits = attention_splits(q.dtype, ctx.num_decode, num_heads, num_kv_heads, head_dim, page, bound, ctx.sm_count, v_head_dim,
+                                  shared_values)
         need = ops.decode_scratch_floats(ctx.num_decode, num_heads, max(head_dim, v_head_dim), splits)
         scratch = ctx.scratch(need) if need else None
         ops.decode_attention(q, cache.k, cache.v, out, scratch, ctx.block_tables[g], ctx.cu_q,

@@ -32,3 +32,18 @@ def test_a_bound_beyond_the_rows_does_not_leave_the_wave():
         for bound in (1, 511, 512, 4096, 131072):
             s = decode_splits(ctas, bound, 148)
             assert s == 1 or (s * ctas <= 148 and s * 512 <= bound)
+
+
+def test_the_benchmark_asks_for_the_splits_that_the_engine_takes():
+    """Latent rows (one KV head, values in the key rows) have a rule of their own: 8 rows x 16 heads of 320 columns, 2,048 keys,
+    sixteen splits; one row sixteen too.  The benchmark times the kernels it names with what the engine's parts ask for."""
+    import pathlib
+    import torch
+    from llm_infer_rust_b200.parts import attention as parts
+    latent = lambda rows, bound=2048: parts.attention_splits(torch.bfloat16, rows, 16, 1, 320, 16, bound, 148, 256, True)
+    assert latent(1) == latent(8) == 16 and latent(16) == 9
+    grouped = lambda rows, bound, dtype=torch.bfloat16: parts.attention_splits(dtype, rows, 16, 8, 128, 16, bound, 148)
+    assert grouped(8, 4096) == 2 and grouped(1, 4096) == 8 and grouped(64, 4096) == 1
+    assert grouped(4, 900, torch.float32) == 4           # the all-sizes kernel is split from 128 keys on
+    bench = (pathlib.Path(parts.__file__).parents[2] / "bench.py").read_text()
+    assert "decode_splits" not in bench and bench.count("attention_splits(") >= 6
