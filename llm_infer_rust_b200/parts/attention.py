@@ -18,20 +18,28 @@ _LATENT_KEYS_PER_CTA_AT_LEAST = 128
 _ALL_SIZES_KEYS_PER_CTA_AT_LEAST = 128
 # A cluster of n splits gives way to more splits where rows may hold n * n times as many keys (see decode_splits).
 _KEYS_FOR_MORE_SPLITS, _LATENT_KEYS_FOR_MORE_SPLITS = 256, 32
+# What the tensor-core kernel's grid costs beside its keys, in keys of one CTA's chain (8.7 ns each at 16 query and 8 KV heads of
+# 128): a kernel that combines the splits, and every wave of CTAs behind the first.  From this share of the SMs on it is memory
+# that bounds the CTAs, not their chains.  A row is taken to hold a quarter of what the rows may grow to.
+_MERGE_KEYS, _WAVE_KEYS = 200, 350
+_SMS_THAT_FILL_MEMORY = 0.8
+_KEPT = 4
 
 
-def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int,
-                  keys_per_cta: int = _KEYS_PER_CTA_AT_LEAST, keys_for_more: int = _KEYS_FOR_MORE_SPLITS) -> int:
-    """How many CTAs share one row's keys, ``ctas_per_split`` CTAs for each split.
+def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int, keys_per_cta: int = _KEYS_PER_CTA_AT_LEAST,
+                  keys_for_more: int = _KEYS_FOR_MORE_SPLITS, merge_keys: int = _MERGE_KEYS) -> int:
+    """How many CTAs share one row's keys, ``ctas_per_split`` CTAs for each split, in a grid of one wave of SMs.
 
-    The grid stays within one wave of SMs and every CTA keeps at least ``keys_per_cta`` keys.  Within a wave 2, 4 or 8
-    splits are the CTAs of one cluster, which combine their parts themselves; other counts need a kernel for it and are
-    taken where the cluster would leave half of the SMs idle and the rows may be long (``keys_for_more``).
-    (Measured at 16 query and 8 KV heads of 128, us at 300 / 1,000 / 4,096 / 8,192 keys a row: 8 rows 15 / 20 / 38 / 66 in
-    two splits, 24 / 27 / 47 / 70 in the nine that fill two and a half waves best; 4 rows 13 / 16 / 26 / 38 in four, 17 / 20
-    / 30 / 43 in nine; 12 rows 13 / 22 / 50 / 85 whole, 20 / 26 / 56 / 89 in three.  More than a cluster: 2 rows 21.5 / 29.7
-    / 83 us in four and 21.1 / 27.7 / 68 in seven or nine at 4,096 / 8,192 / 32,768 keys; 1 row 21.5 / 48 in eight and 21.5 /
-    42 in eighteen at 8,192 / 32,768.  ``kv_len_bound`` is what the rows may grow to when the step is captured, so the
+    Every CTA keeps at least ``keys_per_cta`` keys.  2, 4 or 8 splits are the CTAs of one cluster, which combine their parts
+    themselves; other counts need a kernel for it and are taken where the cluster would leave half of the SMs idle and the rows
+    may be long (``keys_for_more``), or where a row's time at a quarter of its bound falls by more than that kernel's
+    (``merge_keys``; 0: never).
+    (Steps of the 28 layers of Qwen3-0.6B, us at 300 / 1,000 / 4,096 / 8,192 / 32,768 keys a row.  1 row: eight splits 825 / 824 /
+    910 / 1,046 / 1,825, eighteen 920 / 923 / 949 / 1,017 / 1,467.  2 rows: four 799 / 818 / 1,028 / 1,296 / 2,808, nine 880 / 889 /
+    975 / 1,133 / 1,963.  3 rows: four 809 / 829 / 1,051 / 1,321 / 2,833, six 881 / 883 / 1,065 / 1,298 / 2,522.  5 rows: two 806 /
+    895 / 1,303 / 1,807 / 4,822, three 848 / 906 / 1,228 / 1,573 / 3,523.  6 rows: two 804 / 907 / 1,310 / 1,822 / 4,833, three 856 /
+    917 / 1,280 / 1,689 / 4,190.  8 rows: two 817 / 904 / 1,320 / 1,864 / 5,034, the nine that fill four waves best (576 CTAs on 148
+    SMs) 1,103 / 1,177 / 1,599 / 2,142 / 5,267.  ``kv_len_bound`` is what the rows may grow to when the step is captured, so the
     choice has to serve short rows too.)
     """
     ctas_per_split = max(1, ctas_per_split)
@@ -41,7 +49,32 @@ def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int,
     cluster = max(s for s in (1, 2, 4, 8) if s <= most and (s < 8 or 2 * ctas_per_split * s <= sm_count))
     if 2 * cluster * ctas_per_split <= sm_count and kv_len_bound >= cluster * cluster * keys_for_more:
         return 7 if most == 8 else most                   # (a cluster of eight was turned down above)
+    if merge_keys and most > cluster:
+        saved = 1 / cluster - max(1 / most, ctas_per_split / (_SMS_THAT_FILL_MEMORY * sm_count))      # of a row's keys
+        if saved * kv_len_bound / _KEPT >= merge_keys:
+            return 7 if most == 8 else most
     return cluster
+
+
+def _splits_over_waves(ctas_per_split: int, kv_len_bound: int, sm_count: int, splits: int) -> int:
+    """``splits``, a choice for one wave, or a count that takes several: a grid that leaves much of the SMs idle and cannot be split
+    within a wave (75 to 117 CTAs on 148 SMs) takes longer over long rows than two or three waves and a combining kernel.
+
+    (Qwen3-0.6B, us at 300 / 1,000 / 4,096 / 8,192 / 16,384 / 32,768 keys.  10 rows x 8 KV heads: whole 892 / 1,090 / 1,866 / 2,871 /
+    4,872 / 8,913, three splits 1,036 / 1,150 / 1,776 / 2,512 / 3,914 / 6,776, five 1,139 / 1,272 / 1,797 / 2,481 / 3,834 / 6,444.
+    12 rows: whole 893 / 1,088 / 1,870 / 2,878 / 4,885 / 8,899, three 1,065 / 1,190 / 1,847 / 2,635 / 4,230 / 7,534.  14 rows: whole
+    894 / 1,098 / 1,865 / 2,876 / 4,885 / 8,917, five 1,226 / 1,409 / 2,138 / 3,040 / 4,833 / 8,465.)"""
+    busy = _SMS_THAT_FILL_MEMORY * sm_count
+
+    def cost(s):
+        full, rest = divmod(ctas_per_split * s, sm_count)
+        waves = full + (rest > 0)
+        chains = full * sm_count / busy + (max(1.0, rest / busy) if rest else 0.0)
+        return chains * kv_len_bound / _KEPT / s + (_MERGE_KEYS if waves > 1 else 0) + _WAVE_KEYS * (waves - 1)
+    if ctas_per_split >= busy:
+        return splits                                     # memory bounds the grid as it is
+    most = min(64, kv_len_bound // _KEYS_PER_CTA_AT_LEAST, 4 * sm_count // max(1, ctas_per_split))
+    return min([splits] + [s for s in range(2, most + 1) if s * ctas_per_split > sm_count], key=cost)
 
 
 def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, kv_len_bound: int,
@@ -50,12 +83,12 @@ def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_d
     no more), by the kernel that serves them (arguments as ``ops.decode_attention``)."""
     if shared_values and ops.latent_uses_tensor_cores(dtype, num_heads, head_dim, v_head_dim, page_size):
         return decode_splits(rows * (num_heads // ops.latent_head_group(num_heads)), kv_len_bound, sm_count,
-                             _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS)
-    # the all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one
-    on_tensor_cores = ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim)
-    return decode_splits(ops.decode_ctas_per_split(dtype, rows, num_heads, num_kv_heads, head_dim, page_size, v_head_dim),
-                         kv_len_bound, sm_count,
-                         _KEYS_PER_CTA_AT_LEAST if on_tensor_cores else _ALL_SIZES_KEYS_PER_CTA_AT_LEAST)
+                             _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS, 0)
+    ctas = ops.decode_ctas_per_split(dtype, rows, num_heads, num_kv_heads, head_dim, page_size, v_head_dim)
+    if not ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim):
+        # the all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one
+        return decode_splits(ctas, kv_len_bound, sm_count, _ALL_SIZES_KEYS_PER_CTA_AT_LEAST, merge_keys=0)
+    return _splits_over_waves(ctas, kv_len_bound, sm_count, decode_splits(ctas, kv_len_bound, sm_count))
 
 
 class GQAttention(Part):

@@ -47,3 +47,23 @@ def test_the_benchmark_asks_for_the_splits_that_the_engine_takes():
     assert grouped(4, 900, torch.float32) == 4           # the all-sizes kernel is split from 128 keys on
     bench = (pathlib.Path(parts.__file__).parents[2] / "bench.py").read_text()
     assert "decode_splits" not in bench and bench.count("attention_splits(") >= 6
+
+
+def test_long_rows_on_few_sms_are_split_beyond_clusters_and_waves():
+    """At the shapes that were measured (16 query and 8 KV heads of 128): what is faster at a quarter of the bound and beyond, never
+    a count that short bounds would pay for."""
+    import torch
+    from llm_infer_rust_b200.parts.attention import attention_splits
+    splits = lambda rows, bound: attention_splits(torch.bfloat16, rows, 16, 8, 128, 16, bound, 148)
+    assert splits(3, 8192) == 4 and splits(3, 40960) == 6
+    assert splits(5, 4096) == 2 and splits(5, 8192) == splits(5, 40960) == 3          # two left 68 of 148 SMs idle
+    assert splits(6, 4096) == 2 and splits(6, 40960) == 3
+    assert splits(10, 8192) == 1 and splits(10, 12288) == 3 and splits(10, 40960) == 5          # whole left 68 idle
+    assert splits(12, 8192) == 1 and splits(12, 40960) == 3
+    for rows in (4, 7, 8, 9, 14, 15, 16, 17, 19, 32, 64):                             # nothing is to be had, or whole waves as they are
+        assert splits(rows, 40960) == (4 if rows == 4 else 2 if rows < 10 else 1)
+    for rows in range(1, 70):
+        for bound in (1, 300, 1024):
+            assert splits(rows, bound) <= max(1, bound // 512)
+        for bound in (4096, 8192, 40960, 131072):
+            assert 1 <= splits(rows, bound) <= 64 and splits(rows, bound) * rows * 8 <= max(4 * 148, rows * 8)
