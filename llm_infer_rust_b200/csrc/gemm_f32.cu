@@ -14,10 +14,10 @@
 //   wait in shared memory.
 // tiled_kernel (many rows): bound by the FFMA units.  64 x 64 tiles by two warps, 8 x 8 elements a thread: four 16-byte
 //   loads of shared memory for 64 FFMA (4 x 8 elements a thread as packed f32x2 pairs, with one operand stored twice, took
-//   half again as many loads and ran at half the rate).  The blocks of a cluster take different spans of one tile and add
+//   half again as many loads: 25 against 32 TFLOP/s at 1,000 rows).  The blocks of a cluster take different spans of one tile and add
 //   them up in order through distributed shared memory.
 // Measured in a step at the Qwen3-0.6B sizes, mean of a layer's four products, beside one 64 x 64 kernel that summed k in
-// one chain for both: 4 rows 126 -> 10.2 us (1.5 TB/s; the head alone 5 TB/s), 300 rows 150 -> 100 us (25 TFLOP/s).
+// one chain for both: 4 rows 122 -> 9.1 us (1.7 TB/s; the head alone 5 TB/s), 300 rows 145 -> 93 us (25 TFLOP/s).
 //
 // The batched form multiplies `batch` independent pairs whose rows may lie apart (leading dimensions lda, ldw, ldc
 // and a distance between consecutive matrices of each operand): per-head products of a mixer, where head h's rows are
@@ -376,16 +376,21 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int spans = (p.k + SPAN - 1) / SPAN;
-  // Up to 16 rows one pass over W through shared memory beats a tile of 64 that is mostly padding (16 rows, weights of 4,096 x
-  // 1,024 / 1,024 x 2,048 / 1,024 x 3,072: 23 / 18 / 23 us against 47 / 47 / 47 on tiles); 17 to 32 rows are two passes or more
-  // (44 to 52 / 54 to 71 / 54 to 73 us) and tiles stay at 47.
+  // Up to 16 rows the weights are streamed, in passes of `mr` rows: as many as fit shared memory beside the rings, 16 to K = 1,536
+  // (2,048 where N leaves a block one tile), 8 to 3,072, 4 beyond.  One pass is 2 to 9 times as fast as a tile of 64 that is
+  // mostly padding, and three passes or four still are where a span has a warp (16 rows of N x K = 4,096 x 1,024 / 1,024 x 3,072 /
+  // 8,192 x 3,072 / 24,576 x 4,096: 18 / 18 / 79 / 348 us against 42 / 41 / 122 / 363; four passes of 4,096 x 4,096 67 against 65).
+  // From nine spans on the warps go round, and three passes over many columns lose to tiles (9 rows of 4,096 x 5,120 / 8,192 x 8,192 /
+  // 4,096 x 12,288: 128 / 256 / 201 us against 124 / 245 / 185; 16 rows 164 / 341 / 259; 16 of 1,024 x 12,288 still 74 against 124).
+  // 17 to 32 rows are two passes or more everywhere (the first two sizes: 44 to 52 / 54 to 73 us) and stay on tiles.
   if (p.m <= 16) {
     const int sw = spans < 8 ? spans : 8, tiles = (p.n + FEW_WN - 1) / FEW_WN;
     int nt = 8 / sw;
     while (nt > 1 && (tiles + nt - 1) / nt < sms) --nt;              // small products: a block an SM before warps a block
     int mr = p.m > 8 ? 16 : p.m > 4 ? 8 : p.m > 2 ? 4 : p.m;
     while (mr > 1 && few_bytes(mr, sw, nt) > FEW_SMEM_LIMIT) mr /= 2;
-    switch (mr) {
+    const bool streams = spans <= 8 || (p.m + mr - 1) / mr <= 2 || p.n < 4096;
+    if (streams) switch (mr) {
       case 16: return vec ? launch_few<16, true>(p, batch, sw, nt, device, sms, stream) : launch_few<16, false>(p, batch, sw, nt, device, sms, stream);
       case 8: return vec ? launch_few<8, true>(p, batch, sw, nt, device, sms, stream) : launch_few<8, false>(p, batch, sw, nt, device, sms, stream);
       case 4: return vec ? launch_few<4, true>(p, batch, sw, nt, device, sms, stream) : launch_few<4, false>(p, batch, sw, nt, device, sms, stream);

@@ -11,9 +11,9 @@ def _rnd(*shape, dtype=torch.float32, seed=0, scale=1.0):
 
 
 # rows at the edge of the two kernels (16, 17), one column beyond a tile, K around chunks (128), spans (512), more spans than
-# warps (8), more than one span a block, odd K (no 16-byte loads)
+# warps (8), more than one span a block, odd K (no 16-byte loads), three passes over many columns (tiles) and two (streamed)
 @pytest.mark.parametrize("m,n,k", [(1, 9, 127), (3, 8, 129), (16, 7, 513), (2, 24, 4500), (17, 65, 4100), (64, 64, 512), (65, 129, 1028),
-                                   (300, 1024, 2048), (33, 130, 515), (16, 40, 9001), (5, 3000, 1024), (16, 1030, 3072)])
+                                   (300, 1024, 2048), (33, 130, 515), (16, 40, 9001), (5, 3000, 1024), (16, 1030, 3072), (9, 4100, 4500), (8, 4100, 4500)])
 def test_32_bit_products(m, n, k):
     from llm_infer_rust_b200.kernels import ops
     a, w = _rnd(m, k), _rnd(n, k, seed=1)
