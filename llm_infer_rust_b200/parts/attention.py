@@ -17,7 +17,7 @@ _LATENT_KEYS_PER_CTA_AT_LEAST = 128
 # (4 rows x 8 KV heads of up to 900 float32 keys: 100 us whole on 32 SMs, 21 us in four splits with their combination.)
 _ALL_SIZES_KEYS_PER_CTA_AT_LEAST = 128
 # A cluster of n splits gives way to more splits where rows may hold n * n times as many keys (see decode_splits).
-_KEYS_FOR_MORE_SPLITS, _LATENT_KEYS_FOR_MORE_SPLITS = 256, 32
+_KEYS_FOR_MORE_SPLITS = 256
 # What the tensor-core kernel's grid costs beside its keys, in keys of one CTA's chain (8.7 ns each at 16 query and 8 KV heads of
 # 128): a kernel that combines the splits, and every wave of CTAs behind the first.  From this share of the SMs on it is memory
 # that bounds the CTAs, not their chains.  A row is taken to hold a quarter of what the rows may grow to.
@@ -27,12 +27,12 @@ _KEPT = 4
 
 
 def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int, keys_per_cta: int = _KEYS_PER_CTA_AT_LEAST,
-                  keys_for_more: int = _KEYS_FOR_MORE_SPLITS, merge_keys: int = _MERGE_KEYS) -> int:
+                  merge_keys: int = _MERGE_KEYS) -> int:
     """How many CTAs share one row's keys, ``ctas_per_split`` CTAs for each split, in a grid of one wave of SMs.
 
     Every CTA keeps at least ``keys_per_cta`` keys.  2, 4 or 8 splits are the CTAs of one cluster, which combine their parts
     themselves; other counts need a kernel for it and are taken where the cluster would leave half of the SMs idle and the rows
-    may be long (``keys_for_more``), or where a row's time at a quarter of its bound falls by more than that kernel's
+    may be long, or where a row's time at a quarter of its bound falls by more than that kernel's
     (``merge_keys``; 0: never).
     (Steps of the 28 layers of Qwen3-0.6B, us at 300 / 1,000 / 4,096 / 8,192 / 32,768 keys a row.  1 row: eight splits 825 / 824 /
     910 / 1,046 / 1,825, eighteen 920 / 923 / 949 / 1,017 / 1,467.  2 rows: four 799 / 818 / 1,028 / 1,296 / 2,808, nine 880 / 889 /
@@ -47,7 +47,7 @@ def decode_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int, keys_pe
     # More than a handful of clusters of eight do not find room side by side: measured at 2 rows x 8 KV heads, 18.1 us
     # against 12.4 us with six splits (one row: 8 clusters of eight, 9.6 us, the best there).
     cluster = max(s for s in (1, 2, 4, 8) if s <= most and (s < 8 or 2 * ctas_per_split * s <= sm_count))
-    if 2 * cluster * ctas_per_split <= sm_count and kv_len_bound >= cluster * cluster * keys_for_more:
+    if 2 * cluster * ctas_per_split <= sm_count and kv_len_bound >= cluster * cluster * _KEYS_FOR_MORE_SPLITS:
         return 7 if most == 8 else most                   # (a cluster of eight was turned down above)
     if merge_keys and most > cluster:
         saved = 1 / cluster - max(1 / most, ctas_per_split / (_SMS_THAT_FILL_MEMORY * sm_count))      # of a row's keys
@@ -77,13 +77,33 @@ def _splits_over_waves(ctas_per_split: int, kv_len_bound: int, sm_count: int, sp
     return min([splits] + [s for s in range(2, most + 1) if s * ctas_per_split > sm_count], key=cost)
 
 
+def _filling_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int, keys_per_cta: int) -> int:
+    """The splits that fill whole waves of SMs as well as can be while every CTA keeps at least ``keys_per_cta`` keys: latent rows,
+    whose CTAs are long and whose clusters are dear (rows of 320 / 448 columns, 16 / 32 heads, 24 rows of 2,048 keys: 21.7 / 77 us
+    in the six and three splits that fill a wave, 37 / 141 in clusters of four and two; 16 rows of 448 columns: 90 us in nine splits
+    over two waves, 109 in four)."""
+    ctas_per_split = max(1, ctas_per_split)
+    if 8 * ctas_per_split >= 7 * sm_count:
+        return 1                                          # full without splits
+    most = max(1, min(64, kv_len_bound // max(1, keys_per_cta)))
+    best, best_fill = 1, 0.0
+    for splits in range(1, most + 1):
+        if splits == 8 and 2 * ctas_per_split * splits > sm_count:
+            continue                                      # (no room for so many clusters of eight side by side)
+        ctas = ctas_per_split * splits
+        fill = ctas / (sm_count * -(-ctas // sm_count))
+        if fill > best_fill * 1.05:
+            best, best_fill = splits, fill
+    return best
+
+
 def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, kv_len_bound: int,
                      sm_count: int, v_head_dim=None, shared_values: bool = False) -> int:
     """Into how many splits decode attention cuts the keys of ``rows`` rows that hold up to ``kv_len_bound`` keys each (or see
     no more), by the kernel that serves them (arguments as ``ops.decode_attention``)."""
     if shared_values and ops.latent_uses_tensor_cores(dtype, num_heads, head_dim, v_head_dim, page_size):
-        return decode_splits(rows * (num_heads // ops.latent_head_group(num_heads)), kv_len_bound, sm_count,
-                             _LATENT_KEYS_PER_CTA_AT_LEAST, _LATENT_KEYS_FOR_MORE_SPLITS, 0)
+        return _filling_splits(rows * (num_heads // ops.latent_head_group(num_heads)), kv_len_bound, sm_count,
+                               _LATENT_KEYS_PER_CTA_AT_LEAST)
     ctas = ops.decode_ctas_per_split(dtype, rows, num_heads, num_kv_heads, head_dim, page_size, v_head_dim)
     if not ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim):
         # the all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one
