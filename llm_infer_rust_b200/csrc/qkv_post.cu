@@ -94,12 +94,13 @@ __global__ void qkv_post_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_o
 }
 
 // The same work for heads whose size is 16 bytes times a power of two of at most 32 (64, 128 or 256 elements in bfloat16)
-// and a rotation over the whole head: `lanes` = head_dim / (elements of 16 bytes) lanes share up to four heads of one
+// and a rotation over the whole head: `lanes` = head_dim / (elements of 16 bytes) lanes share HG heads of one
 // token.  A lane holds 8 bytes of a head's first half and the 8 bytes that they are rotated with, so the rotation needs no
-// other lane; its angles and the token's position and slot are fetched once for the four heads (a head's angles are twice its
-// bytes), and all heads' loads are in flight together.  Bound by latency at few tokens and by memory at many.  One head a
-// lane group with its halves in different lanes, bfloat16, 32 + 2 x 8 heads of 128: 22.7 -> 16.7 us at 2,048 tokens, 84.6 ->
-// 75.9 at 8,192; float32, 16 + 2 x 8 heads: 23.3 -> 16.5 and 82.6 -> 58.9 us.
+// other lane; its angles and the token's position and slot are fetched once for the HG heads (a head's angles are twice its
+// bytes), and all heads' loads are in flight together.  Bound by memory at many tokens, where HG = 4 saves most (one head a
+// lane group with its halves in different lanes, bfloat16, 32 + 2 x 8 heads of 128: 22.7 -> 16.7 us at 2,048 tokens, 84.6 -> 75.9
+// at 8,192; float32, 16 + 2 x 8 heads: 23.3 -> 16.5 and 82.6 -> 58.9 us), and by the latency of a lane's chain at few, where one
+// head after the other is that chain (see heads_a_group).
 template <typename TA> struct Half16;                           // 8 bytes of a row as floats, and back
 template <> struct Half16<float> {
   static constexpr int N = 2;
@@ -128,16 +129,14 @@ __device__ __forceinline__ void load_few(const T* p, float (&v)[N]) {
   }
 }
 
-constexpr int HEADS_A_GROUP = 4;
-
-template <typename TA, typename TW>
+template <typename TA, typename TW, int HG>
 __global__ void __launch_bounds__(256)
 qkv_post_vec_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_out, TA* __restrict__ k_cache,
                     TA* __restrict__ v_cache, const TW* __restrict__ q_w, const TW* __restrict__ k_w, float eps,
                     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int max_pos,
                     const int* __restrict__ positions, const int* __restrict__ slots, int tokens, int nh, int nkv,
                     int d, int page_size, long long cache_slots, int lanes, int* err) {
-  constexpr int N = Half16<TA>::N, HG = HEADS_A_GROUP;
+  constexpr int N = Half16<TA>::N;
   const int heads = nh + 2 * nkv, head_groups = (heads + HG - 1) / HG;
   const int sub = threadIdx.x % lanes;                          // this lane's place inside its heads
   const long long work = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / lanes;
@@ -224,6 +223,16 @@ qkv_post_vec_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_out, TA* __re
   }
 }
 
+// How many heads a lane group takes, by the blocks of 256 threads that one head each would be: few blocks are all resident and
+// the shortest chain is fastest, many share the SMs and the fetches saved count.  Measured, us with 1 / 2 / 4 (bfloat16, 16 + 2 x 8
+// heads of 128): 64 tokens (128 blocks) 3.4 / 3.7 / 4.9, 200 (400) 3.5 / 4.1 / 4.9, 300 (600) 4.8 / 4.5 / 5.5, 500 (1,000) 5.5 / 5.1 /
+// 5.4, 777 (1,554) 7.4 / 6.4 / 6.0; float32: 64 (256) 3.6 / 3.6 / 4.1, 200 (800) 5.1 / 4.4 / 4.4, 300 (1,200) 6.0 / 5.1 / 5.0.
+static int heads_a_group(long long work, int lanes) {
+  const long long blocks = (work * lanes + 255) / 256;
+  return blocks <= 3 * 148 ? 1 : blocks <= 8 * 148 ? 2 : 4;
+}
+B200_EXPORT int b200_qkv_post_heads_a_group(long long work, int lanes) { return heads_a_group(work, lanes); }
+
 B200_EXPORT int b200_qkv_post(const void* qkv, void* q_out, void* k_cache, void* v_cache, const void* q_w,
                               const void* k_w, float eps, const float* cos_table, const float* sin_table,
                               int rot_dim, int max_pos, const int* positions, const int* slots, int tokens,
@@ -242,19 +251,23 @@ B200_EXPORT int b200_qkv_post(const void* qkv, void* q_out, void* k_cache, void*
                          reinterpret_cast<uintptr_t>(cos_table) % 16 == 0 && reinterpret_cast<uintptr_t>(sin_table) % 16 == 0;
     const bool whole_rotation = cos_table == nullptr || rot_dim == d;
     if (lanes >= 2 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && aligned && whole_rotation) {
-      const long long threads = static_cast<long long>(tokens) * ((nh + 2 * nkv + HEADS_A_GROUP - 1) / HEADS_A_GROUP) * lanes;
+      const int hg = heads_a_group(work, lanes);
+      const long long threads = static_cast<long long>(tokens) * ((nh + 2 * nkv + hg - 1) / hg) * lanes;
       const unsigned vblocks = static_cast<unsigned>((threads + 255) / 256);
-#define CALLV(TA, TW)                                                                                          \
-      qkv_post_vec_kernel<TA, TW><<<vblocks, 256, 0, stream>>>(                                                 \
+#define CALLG(TA, TW, HG)                                                                                      \
+      qkv_post_vec_kernel<TA, TW, HG><<<vblocks, 256, 0, stream>>>(                                             \
           static_cast<const TA*>(qkv), static_cast<TA*>(q_out), static_cast<TA*>(k_cache), static_cast<TA*>(v_cache), \
           static_cast<const TW*>(q_w), static_cast<const TW*>(k_w), eps, cos_table, sin_table, max_pos, positions, \
           slots, tokens, nh, nkv, d, page_size, cache_slots, lanes, err)
+#define CALLV(TA, TW)                                                                                          \
+      if (hg == 1) { CALLG(TA, TW, 1); } else if (hg == 2) { CALLG(TA, TW, 2); } else { CALLG(TA, TW, 4); }
       if (act_dtype == B200_F32 && w_dtype == B200_F32) { CALLV(float, float); }
       else if (act_dtype == B200_BF16 && w_dtype == B200_BF16) { CALLV(__nv_bfloat16, __nv_bfloat16); }
       else if (act_dtype == B200_BF16 && w_dtype == B200_F32) { CALLV(__nv_bfloat16, float); }
       else if (act_dtype == B200_F32 && w_dtype == B200_BF16) { CALLV(float, __nv_bfloat16); }
       else return B200_BAD_DTYPE;
 #undef CALLV
+#undef CALLG
       return b200_check_launch();
     }
   }

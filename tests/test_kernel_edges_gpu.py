@@ -87,3 +87,30 @@ def test_decoded_rows_of_many_lengths_in_several_waves(lengths):
         want = torch.einsum("hj,jhd->hd", torch.softmax(s, 1), v)
         # a weight is rounded to 8 bits, and so is the result
         assert ((out[i].view(H, D).double() - want).abs() <= 2.0 ** -8 * (want.abs() + v.abs().amax(0))).all(), i
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv", [(16, 8), (5, 1)])
+def test_a_token_between_projection_and_attention_is_the_same_in_every_batch(nh, nkv, dtype):
+    """Few tokens take one head a lane group, more two, many four (the head count no multiple of it): to the bit the same."""
+    from llm_infer_rust_b200.kernels import ops
+    d, page, n = 128, 16, 3000
+    x, pos = _rnd(n, (nh + 2 * nkv) * d, dtype=dtype), torch.arange(n, dtype=torch.int32, device=DEV)
+    qw, kw = _rnd(d, dtype=dtype, seed=1), _rnd(d, dtype=dtype, seed=2)
+    cos, sin = _rnd(n, d // 2, seed=3), _rnd(n, d // 2, seed=4)
+    got = []
+    for tokens in (n, 600, 300, 7):
+        q = torch.empty(tokens, nh * d, dtype=dtype, device=DEV)
+        kc, vc = (torch.zeros(n // page + 2, nkv, page, d, dtype=dtype, device=DEV) for _ in range(2))
+        ops.qkv_post(x[:tokens], q, kc, vc, qw, kw, 1e-6, cos, sin, d, pos[:tokens], pos[:tokens] + page, nh, nkv, d)
+        got.append((q[:7], kc[1, :, :7], vc[1, :, :7]))
+    ops.check_errors(torch.device(DEV))
+    assert all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other))
+    rows = x[:7].double().view(7, nh + 2 * nkv, d)
+    for h, (mine, w) in enumerate([(got[0][0].view(7, nh, d)[:, 0], qw), (got[0][1][0], kw)]):
+        t = rows[:, h * nh]
+        t = t / torch.sqrt((t * t).mean(-1, keepdim=True) + 1e-6) * w.double()
+        a, b, c, s = t[:, :64], t[:, 64:], cos[:7].double(), sin[:7].double()
+        want = torch.cat([a * c - b * s, b * c + a * s], 1)
+        # one rounding of the result; both products of a rotation carry a few of 2^-24
+        assert ((mine.double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * (want.abs() + 1)).all()

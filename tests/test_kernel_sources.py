@@ -32,3 +32,11 @@ def test_blocks_that_share_a_tile_of_32_bit_products():
         assert shared(m, n, k) == blocks, (m, n, k)
     # nine or ten spans take two rounds with five blocks or with eight: the three more would only add a round to nothing
     assert shared(64, 64, 5000) == 5 and shared(64, 64, 4500) == 5 and shared(64, 64, 4096) == 8
+
+
+def test_heads_that_a_lane_group_takes_between_projection_and_attention():
+    """A decode step's few tokens take the shortest chain, a prompt's many the fewest fetches (measured on both sides)."""
+    lib = build.load_cuda_library("qkv_post.cu")
+    taken = lambda tokens, heads, lanes: lib.b200_qkv_post_heads_a_group(ctypes.c_longlong(tokens * heads), lanes)
+    assert [taken(t, 32, 16) for t in (1, 27, 64, 200, 300, 500, 777, 8192)] == [1, 1, 1, 1, 2, 2, 4, 4]       # bfloat16, heads of 128
+    assert [taken(t, 32, 32) for t in (4, 64, 128, 200, 300, 2048)] == [1, 1, 2, 2, 4, 4]                      # float32
