@@ -146,7 +146,8 @@ sigmoid_gate_mul_kernel(T* out, const T* a, const T* __restrict__ g, int g_strid
 }
 
 // The same with one gate an element and eight elements a thread in 16-byte accesses (rows of whole 16-byte pieces).  Bound by
-// memory: one element a thread at a time, 1,500 rows of 2,048 bfloat16 took 23.5 us for 18 MB.
+// memory at many elements: one element a thread at a time, 1,500 rows of 2,048 bfloat16 took 12.5 us, here 9.7; at few by the
+// latency of a thread's eight exponentials and divisions, one behind the other.
 template <typename T>
 __global__ void __launch_bounds__(256)
 sigmoid_gate_mul_vec_kernel(T* out, const T* a, const T* __restrict__ g, int g_stride, int width) {          // out may be a
@@ -210,11 +211,19 @@ B200_EXPORT int b200_head_unit_norm_gate(void* out, const float* o, const void* 
   return b200_check_launch();
 }
 
+// Eight elements a thread where rows are wide (a thread of the other kernel then has four and more of its own, one after the
+// other) or the elements many.  Measured on both, us, one a thread / eight: 300 rows of 256 2.4 / 4.1, of 512 2.9 / 4.2, of 768 3.8 /
+// 4.1, of 1,024 4.2 / 4.2, of 2,048 6.2 / 4.7; one row of 256 2.3 / 3.1, of 2,048 4.4 / 3.6; 1,500 of 512 4.7 / 5.1, of 768 6.1 / 5.6;
+// 4,096 of 256 6.2 / 5.9 (bfloat16; float32 within 0.5 us of these).
+B200_EXPORT int b200_sigmoid_gate_mul_takes_eight(int tokens, int width) {
+  return width >= 1024 || static_cast<long long>(tokens) * width >= 1 << 20;
+}
+
 B200_EXPORT int b200_sigmoid_gate_mul(void* out, const void* a, const void* g, int g_stride, int tokens, int width,
                                       int per, int dtype, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (width <= 0 || per <= 0 || width % per) return B200_BAD_SIZE;
-  if (per == 1 && width % 8 == 0 && g_stride % 8 == 0 && (dtype == B200_F32 || dtype == B200_BF16) &&
+  if (per == 1 && b200_sigmoid_gate_mul_takes_eight(tokens, width) && width % 8 == 0 && g_stride % 8 == 0 && (dtype == B200_F32 || dtype == B200_BF16) &&
       (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(g)) % 16 == 0) {
     const dim3 grid(tokens, (width / 8 + 255) / 256), block(width / 8 < 256 ? (width / 8 + 31) / 32 * 32 : 256);
     if (dtype == B200_F32)

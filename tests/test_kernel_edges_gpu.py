@@ -64,6 +64,17 @@ def test_gates_in_whole_and_in_broken_vectors(tokens, width, column, dtype):
     assert ((got.double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * want.abs() + 1e-9).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_gated_row_is_the_same_in_every_batch(dtype):
+    """Few narrow rows take one element a thread, many take eight: to the bit the same."""
+    from llm_infer_rust_b200.kernels import ops
+    packed, a = _rnd(4200, 512, dtype=dtype, scale=4.0), _rnd(4200, 256, dtype=dtype, seed=1)
+    many, few = ops.sigmoid_gate_mul(a.clone(), packed, 256), ops.sigmoid_gate_mul(a[:9].clone(), packed[:9], 256)
+    assert torch.equal(many[:9], few)
+    want = a.double() * torch.sigmoid(packed[:, 256:].double())
+    assert ((many.double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) * want.abs() + 1e-9).all()
+
+
 @pytest.mark.parametrize("lengths", [[1 + (37 * i) % 200 for i in range(40)], [64] * 39 + [1], list(range(1, 75))])
 def test_decoded_rows_of_many_lengths_in_several_waves(lengths):
     """More CTAs than SMs, rows listed in any order: every row is its own."""

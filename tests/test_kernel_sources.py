@@ -40,3 +40,10 @@ def test_heads_that_a_lane_group_takes_between_projection_and_attention():
     taken = lambda tokens, heads, lanes: lib.b200_qkv_post_heads_a_group(ctypes.c_longlong(tokens * heads), lanes)
     assert [taken(t, 32, 16) for t in (1, 27, 64, 200, 300, 500, 777, 8192)] == [1, 1, 1, 1, 2, 2, 4, 4]       # bfloat16, heads of 128
     assert [taken(t, 32, 32) for t in (4, 64, 128, 200, 300, 2048)] == [1, 1, 2, 2, 4, 4]                      # float32
+
+
+def test_gates_take_eight_elements_a_thread_where_that_is_faster():
+    lib = build.load_cuda_library("gated.cu")
+    eight = lambda tokens, width: bool(lib.b200_sigmoid_gate_mul_takes_eight(tokens, width))
+    assert not any(eight(t, w) for t, w in ((1, 8), (300, 256), (300, 768), (64, 512), (1500, 512)))
+    assert all(eight(t, w) for t, w in ((1, 2048), (300, 1024), (1500, 768), (8192, 512)))
