@@ -22,6 +22,8 @@
 // instead, which streams every weight row once for the few rows that need it.
 #include <mma.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 constexpr int TM = 64, TN = 64;      // rows (sorted pairs) and columns of a tile
@@ -305,34 +307,37 @@ expert_gemm_bf16_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int*
 
 // ------------------------------------------------------------------ bfloat16 products of a step of few pairs
 // A decode step has a handful of rows an expert and must read all of that expert's weights: the tensor cores have
-// nothing to do, and the time is the weights' way out of memory.  So each warp takes FEW_COLS output columns of ONE
+// nothing to do, and the time is the weights' way out of memory.  So each warp takes COLS output columns of ONE
 // expert (their gate rows and up rows when GATED), streams the rows in 16-byte pieces (lane l takes columns
 // 8 l .. 8 l + 7, then 256 further on, in order; the lanes' sums meet in a butterfly) and multiplies them with up to
 // FEW_ROWS of the expert's rows at a time (more rows: another pass over the same weight rows, which the caches still
 // hold).  Two columns a warp and two pieces of all their rows on the way at once: the rows of x, read by every warp, cost as
-// many loads as the weights, and with one column and one piece a warp had 1 KB under way (8 rows x 2 of 8 experts,
-// width 1,024, ff 1,536: gate/up 19.9 -> 18.8 us, down 14.5 -> 13.5 us).  grid (ceil(N / (FEW_WARPS FEW_COLS)), experts); blocks of experts without rows return at once.  A row's result does
+// many loads as the weights, and with one column and one piece a warp had 1 KB under way.  `few_cols` says when: not where the
+// grid then leaves SMs idle, nor where experts have several rows each and the sums bound it.  Measured with weights from memory,
+// us a layer of experts (route, both products, combine), one column as it was / two: 1 row x 8 of 64 experts of 2,048 x 1,024 60.8 / 48.7, x 8 of
+// 128 of 2,048 x 768 76.3 / 57.4, 4 rows x 2 of 8 of 1,024 x 1,536 30.4 / 26.9; against it 4 rows of 4 experts of 512 x 256 8.3 / 9.3, 32 rows x 2 of 8
+// of 2,048 x 768 60.2 / 66.0.  grid (ceil(N / (FEW_WARPS COLS)), experts); blocks of experts without rows return at once.  A row's result does
 // not depend on what else the step holds.  K a multiple of 8.
-constexpr int FEW_PAIRS = 64, FEW_ROWS = 4, FEW_WARPS = 8, FEW_COLS = 2;
+constexpr int FEW_PAIRS = 64, FEW_ROWS = 4, FEW_WARPS = 8;
 
-template <bool GATED, typename TO>
+template <bool GATED, typename TO, int COLS>
 __global__ void __launch_bounds__(FEW_WARPS * 32)
 expert_rows_few_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __restrict__ sorted_token,
                        const __nv_bfloat16* __restrict__ W, long long w_stride, int ff, TO* __restrict__ C, int ldc,
                        int N, int K, const int* __restrict__ expert_start, const GluAct act) {
   pdl_launch_dependents();                          // the kernel after this one may be scheduled; it waits before it reads
   pdl_wait();                                        // what this kernel reads belongs to the kernels before it
-  constexpr int ROWS = GATED ? 2 * FEW_COLS : FEW_COLS;      // rows of W: the gate rows of the warp's columns, then their up rows
+  constexpr int ROWS = GATED ? 2 * COLS : COLS;      // rows of W: the gate rows of the warp's columns, then their up rows
   const int e = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n0 = (blockIdx.x * FEW_WARPS + warp) * FEW_COLS;
+  const int n0 = (blockIdx.x * FEW_WARPS + warp) * COLS;
   const int first = expert_start[e], last = expert_start[e + 1];
   if (first >= last || n0 >= N) return;
   const __nv_bfloat16* w[ROWS];
 #pragma unroll
-  for (int c = 0; c < FEW_COLS; ++c) {                 // (a column beyond the last reads the last one; it is not stored)
+  for (int c = 0; c < COLS; ++c) {                 // (a column beyond the last reads the last one; it is not stored)
     w[c] = W + static_cast<size_t>(e) * w_stride + static_cast<size_t>(min(n0 + c, N - 1)) * K;
-    if (GATED) w[FEW_COLS + c] = w[c] + static_cast<size_t>(ff) * K;
+    if (GATED) w[COLS + c] = w[c] + static_cast<size_t>(ff) * K;
   }
   for (int r0 = first; r0 < last; r0 += FEW_ROWS) {
     const int nr = min(FEW_ROWS, last - r0);
@@ -374,11 +379,11 @@ expert_rows_few_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* 
       }
     }
 #pragma unroll
-    for (int c = 0; c < FEW_COLS; ++c)
+    for (int c = 0; c < COLS; ++c)
 #pragma unroll
       for (int i = 0; i < FEW_ROWS; ++i) {
         const float s0 = warp_sum(acc[c][i]);
-        const float s1 = GATED ? warp_sum(acc[ROWS - FEW_COLS + c][i]) : 0.0f;
+        const float s1 = GATED ? warp_sum(acc[ROWS - COLS + c][i]) : 0.0f;
         if (lane == 0 && i < nr && n0 + c < N) {
           const float gain = GATED ? row_gain(act, r0 + i) : 1.0f;
           C[static_cast<size_t>(r0 + i) * ldc + n0 + c] = from_f32<TO>(GATED ? glu_f(gain * s0, gain * s1, act) : s0);
@@ -717,6 +722,14 @@ static int launch_combine(float* out, const float* y, const int* pos_of_pair, in
                      uniform, weight, static_cast<const float*>(c.add), c.add_scale);
 }
 
+// Columns a warp of expert_rows_few_kernel takes (see there): two while the blocks with rows fill the SMs and an expert has fewer
+// than four rows on average.
+static int few_cols(int cols, int pairs, int experts) {
+  const int blocks = (cols + 2 * FEW_WARPS - 1) / (2 * FEW_WARPS) * (pairs < experts ? pairs : experts);
+  return blocks >= 148 && pairs < 4 * experts ? 2 : 1;
+}
+B200_EXPORT int b200_experts_few_cols(int cols, int pairs, int experts) { return few_cols(cols, pairs, experts); }
+
 // x [tokens, width] -> out [tokens, width] float32.  `h` holds pairs * ff elements of x's dtype, `y` pairs * width
 // floats, `route` b200_expert_route_ints(...) ints.
 static int run_experts(const void* x, int dtype, const ExpertChoice& c, int top, int experts, const void* gate_up,
@@ -748,15 +761,18 @@ static int run_experts(const void* x, int dtype, const ExpertChoice& c, int top,
         static_cast<const float*>(h), ff, nullptr, static_cast<const float*>(down), dn_stride, 0, y, width, ff,
         expert_start, tile_expert, tile_first, num_tiles, act);
   } else if (dtype == B200_BF16 && pairs <= FEW_PAIRS && width % 8 == 0 && ff % 8 == 0) {
-    constexpr int per = FEW_WARPS * FEW_COLS;
-    const dim3 f1((ff + per - 1) / per, experts), f2((width + per - 1) / per, experts);
-    rc = b200_launch(expert_rows_few_kernel<true, __nv_bfloat16>, f1, dim3(FEW_WARPS * 32), 0, stream, 0,
-                     static_cast<const __nv_bfloat16*>(x), width, sorted_token, static_cast<const __nv_bfloat16*>(gate_up),
-                     gu_stride, ff, static_cast<__nv_bfloat16*>(h), ff, ff, width, expert_start, act);
+    auto product = [&](auto gated, int cols, auto... args) {
+      const int per = few_cols(cols, pairs, experts);
+      const dim3 grid((cols + FEW_WARPS * per - 1) / (FEW_WARPS * per), experts);
+      using TO = std::conditional_t<decltype(gated)::value, __nv_bfloat16, float>;
+      return b200_launch(per == 2 ? expert_rows_few_kernel<decltype(gated)::value, TO, 2> : expert_rows_few_kernel<decltype(gated)::value, TO, 1>,
+                         grid, dim3(FEW_WARPS * 32), 0, stream, 0, args...);
+    };
+    rc = product(std::true_type(), ff, static_cast<const __nv_bfloat16*>(x), width, sorted_token,
+                 static_cast<const __nv_bfloat16*>(gate_up), gu_stride, ff, static_cast<__nv_bfloat16*>(h), ff, ff, width, expert_start, act);
     if (rc != 0) return rc;
-    rc = b200_launch(expert_rows_few_kernel<false, float>, f2, dim3(FEW_WARPS * 32), 0, stream, 0,
-                     static_cast<const __nv_bfloat16*>(h), ff, static_cast<const int*>(nullptr),
-                     static_cast<const __nv_bfloat16*>(down), dn_stride, 0, y, width, width, ff, expert_start, act);
+    rc = product(std::false_type(), width, static_cast<const __nv_bfloat16*>(h), ff, static_cast<const int*>(nullptr),
+                 static_cast<const __nv_bfloat16*>(down), dn_stride, 0, y, width, width, ff, expert_start, act);
     if (rc != 0) return rc;
   } else if (dtype == B200_BF16) {
     expert_gemm_bf16_kernel<true, __nv_bfloat16><<<g1, 256, 0, stream>>>(

@@ -125,3 +125,23 @@ def test_a_token_between_projection_and_attention_is_the_same_in_every_batch(nh,
         want = torch.cat([a * c - b * s, b * c + a * s], 1)
         # one rounding of the result; both products of a rotation carry a few of 2^-24
         assert ((mine.double() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * (want.abs() + 1)).all()
+
+
+def test_a_row_of_few_rows_experts_is_the_same_in_every_step():
+    """Two rows take two columns a warp, 32 rows of two of eight experts one: to the bit the same (columns no multiple of a block's)."""
+    from llm_infer_rust_b200.kernels import ops
+    E, top, width, ff = 8, 2, 1032, 1544
+    gu, dn = _rnd(E, 2 * ff, width, dtype=torch.bfloat16, scale=width ** -0.5), _rnd(E, width, ff, dtype=torch.bfloat16, seed=1, scale=ff ** -0.5)
+    x, gains = _rnd(32, width, dtype=torch.bfloat16, seed=2), _rnd(32, top, seed=3).abs()
+    choice = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(i))[:top] for i in range(32)]).to(torch.int32).to(DEV)
+    many = ops.routed_experts(x, choice, gains, gu, dn)
+    for n in (1, 2, 5):
+        assert torch.equal(ops.routed_experts(x[:n], choice[:n], gains[:n], gu, dn), many[:n])
+    for t in (0, 31):
+        want = torch.zeros(width, dtype=torch.float64, device=DEV)
+        for k in range(top):
+            e = int(choice[t, k])
+            g, u = (gu[e].double() @ x[t].double()).split(ff)
+            want += gains[t, k].double() * (dn[e].double() @ (torch.nn.functional.silu(g) * u).bfloat16().double())
+        # the hidden row is rounded to 8 bits, where a sum in 32 bits may fall on the other side
+        assert ((many[t].double() - want).abs() <= 2.0 ** -8 * want.abs().max()).all()

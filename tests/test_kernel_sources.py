@@ -47,3 +47,11 @@ def test_gates_take_eight_elements_a_thread_where_that_is_faster():
     eight = lambda tokens, width: bool(lib.b200_sigmoid_gate_mul_takes_eight(tokens, width))
     assert not any(eight(t, w) for t, w in ((1, 8), (300, 256), (300, 768), (64, 512), (1500, 512)))
     assert all(eight(t, w) for t, w in ((1, 2048), (300, 1024), (1500, 768), (8192, 512)))
+
+
+def test_columns_that_a_warp_takes_of_few_rows_experts():
+    """Two while the grid fills the SMs and experts have few rows each (measured on both sides)."""
+    cols = build.load_cuda_library("experts.cu").b200_experts_few_cols
+    assert cols(1024, 8, 64) == cols(2048, 64, 64) == cols(1536, 8, 8) == cols(2048, 2, 8) == 2
+    assert cols(256, 4, 4) == cols(512, 32, 4) == 1                         # 64 and 128 blocks
+    assert cols(1536, 64, 8) == cols(768, 32, 8) == 1                       # four and eight rows an expert
