@@ -488,6 +488,23 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   return b200_check_launch();
 }
 
+// A decode CTA: four warps with two stages of keys and values each where that fits, else one stage, else fewer warps.
+template <typename T>
+struct DecodeShape {
+  static constexpr size_t TILE = 2 * KB * RowGeom<T>::STRIDE * sizeof(T), LIMIT = 200 * 1024;
+  static constexpr size_t FIXED4 = (NV * D + 4 * KB * NV) * sizeof(float);
+  static constexpr int WARPS = FIXED4 + 4 * TILE <= LIMIT ? 4 : (FIXED4 + 2 * TILE <= LIMIT ? 2 : 1);
+  static constexpr size_t FIXED = (NV * D + WARPS * KB * NV) * sizeof(float);
+  static_assert(FIXED + WARPS * TILE <= 220 * 1024, "one key block per warp must fit shared memory");
+  static constexpr int STAGES = FIXED + WARPS * 2 * TILE <= LIMIT ? 2 : 1;
+  static constexpr size_t MERGE = WARPS * NV * (D + 2) * sizeof(float);
+  static constexpr size_t SMEM = FIXED + (MERGE > WARPS * STAGES * TILE ? MERGE : WARPS * STAGES * TILE);
+};
+// Shared memory of a decode CTA in bytes: how many of them an SM holds.
+B200_EXPORT int b200_decode_attention_smem(int dtype) {
+  return static_cast<int>(dtype == B200_F32 ? DecodeShape<float>::SMEM : DecodeShape<__nv_bfloat16>::SMEM);
+}
+
 template <typename T>
 static int launch_decode(const void* q, const void* kc, const void* vc, void* out, float* part_acc, float* part_ml,
                          const int* block_table, int table_stride, const int* cu_q, const int* kv_len,
@@ -497,16 +514,8 @@ static int launch_decode(const void* q, const void* kc, const void* vc, void* ou
   using G = RowGeom<T>;
   const int group = nh / nkv;
   const int vec_groups = (group + NV - 1) / NV;
-  constexpr size_t tile_bytes = 2 * KB * G::STRIDE * sizeof(T);
-  constexpr size_t limit = 200 * 1024;
-  constexpr size_t fixed4 = (NV * D + 4 * KB * NV) * sizeof(float);
-  // Four warps with two stages where that fits, else one stage, else fewer warps.
-  constexpr int DEC_WARPS = fixed4 + 4 * tile_bytes <= limit ? 4 : (fixed4 + 2 * tile_bytes <= limit ? 2 : 1);
-  constexpr size_t fixed = (NV * D + DEC_WARPS * KB * NV) * sizeof(float);
-  static_assert(fixed + DEC_WARPS * tile_bytes <= 220 * 1024, "one key block per warp must fit shared memory");
-  constexpr int stages = fixed + DEC_WARPS * 2 * tile_bytes <= limit ? 2 : 1;
-  constexpr size_t merge_bytes = DEC_WARPS * NV * (D + 2) * sizeof(float);
-  constexpr size_t smem = fixed + (merge_bytes > DEC_WARPS * stages * tile_bytes ? merge_bytes : DEC_WARPS * stages * tile_bytes);
+  constexpr int DEC_WARPS = DecodeShape<T>::WARPS, stages = DecodeShape<T>::STAGES;
+  constexpr size_t smem = DecodeShape<T>::SMEM;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<T, DEC_WARPS>,

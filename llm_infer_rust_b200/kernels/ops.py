@@ -531,6 +531,12 @@ def decode_ctas_per_split(dtype: torch.dtype, n_rows: int, num_heads: int, num_k
     return n_rows * num_kv_heads * ((num_heads // num_kv_heads + 3) // 4)
 
 
+def all_sizes_decode_ctas_per_sm(dtype: torch.dtype, head_dim: int) -> int:
+    """How many of the all-sizes decode kernel's CTAs an SM holds (its shared memory decides)."""
+    code = F32 if dtype == torch.float32 else BF16
+    return max(1, 227 * 1024 // (_attention(head_dim).b200_decode_attention_smem(code) + 1024))
+
+
 def decode_scratch_floats(n_rows: int, num_heads: int, head_dim: int, splits: int) -> int:
     """Floats of scratch that decode attention needs (partial outputs are rows of the padded head size)."""
     return 0 if splits <= 1 else n_rows * num_heads * splits * (padded_head_dim(head_dim) + 2)

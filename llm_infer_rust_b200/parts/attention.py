@@ -1,6 +1,7 @@
 """Grouped-query attention over the paged cache."""
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
@@ -97,6 +98,7 @@ def _filling_splits(ctas_per_split: int, kv_len_bound: int, sm_count: int, keys_
     return best
 
 
+@functools.lru_cache(maxsize=1024)          # (every layer of a step asks for the same)
 def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, kv_len_bound: int,
                      sm_count: int, v_head_dim=None, shared_values: bool = False) -> int:
     """Into how many splits decode attention cuts the keys of ``rows`` rows that hold up to ``kv_len_bound`` keys each (or see
@@ -106,7 +108,12 @@ def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_d
                                _LATENT_KEYS_PER_CTA_AT_LEAST)
     ctas = ops.decode_ctas_per_split(dtype, rows, num_heads, num_kv_heads, head_dim, page_size, v_head_dim)
     if not ops.decode_uses_tensor_cores(dtype, num_heads, num_kv_heads, head_dim, page_size, v_head_dim):
-        # the all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one
+        # The all-sizes kernel takes in 128 keys at a time, a tenth as fast as the tensor-core one.  Of small heads an SM holds
+        # several CTAs, and a wave is as many more (heads of 32, float32, 4,096 keys, 40 query heads on one KV head: 8 rows 119 us
+        # whole, 51 in three splits, 45 in eight; 16 rows x 8 KV heads 118 whole, 55 in three).
+        per_sm = ops.all_sizes_decode_ctas_per_sm(dtype, max(head_dim, v_head_dim or head_dim))
+        if per_sm > 1:
+            return max(1, min(16, kv_len_bound // (2 * _ALL_SIZES_KEYS_PER_CTA_AT_LEAST), per_sm * sm_count // max(1, ctas)))
         return decode_splits(ctas, kv_len_bound, sm_count, _ALL_SIZES_KEYS_PER_CTA_AT_LEAST, merge_keys=0)
     return _splits_over_waves(ctas, kv_len_bound, sm_count, decode_splits(ctas, kv_len_bound, sm_count))
 

@@ -69,3 +69,16 @@ def test_long_rows_on_few_sms_are_split_beyond_clusters_and_waves():
             assert splits(rows, bound) <= max(1, bound // 512)
         for bound in (4096, 8192, 40960, 131072):
             assert 1 <= splits(rows, bound) <= 64 and splits(rows, bound) * rows * 8 <= max(4 * 148, rows * 8)
+
+
+def test_small_heads_of_the_all_sizes_kernel_fill_every_cta_that_an_sm_holds():
+    """Float32 heads of 32: three CTAs an SM (measured at 4,096 keys: 8 and 16 rows x 8 KV heads 32.5 and 55 us in six and three splits, whole
+    115 and 118); heads of 128 leave room for one."""
+    import torch
+    from llm_infer_rust_b200.kernels import ops
+    from llm_infer_rust_b200.parts.attention import attention_splits
+    assert ops.all_sizes_decode_ctas_per_sm(torch.float32, 32) == 3 and ops.all_sizes_decode_ctas_per_sm(torch.float32, 128) == 1
+    splits = lambda rows, nh, nkv, d, bound=4096: attention_splits(torch.float32, rows, nh, nkv, d, 16, bound, 148)
+    assert [splits(r, 16, 8, 32) for r in (1, 4, 8, 16, 32)] == [16, 13, 6, 3, 1]
+    assert splits(8, 40, 1, 32) == 5 and splits(4, 40, 1, 32) == 11 and splits(8, 16, 8, 32, 300) == 1
+    assert [splits(r, 16, 8, 128) for r in (1, 4, 8, 16)] == [8, 4, 2, 1]
