@@ -345,8 +345,8 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
     ``v_head_dim``: the width of a value (and of an output) vector where it differs from a key's;
     ``softcap`` > 0: a score becomes cap * tanh(score / cap) before the mask; ``precise_weights``: the softmax
     weights enter the product with the values as two bfloat16 terms (about 16 bits) instead of one.  Keys and values of 128
-    take the tcgen05 kernel from one or two tiles of 128 query vectors a KV head on, other sizes the mma.sync kernel (see
-    ``decode_uses_tensor_cores``); what that does not take goes to the all-sizes kernel, whose weights are floats.
+    take the tcgen05 kernel from one tile of 128 query vectors a KV head on (these further forms where
+    ``shaped_prompt_on_tcgen05`` says so), others the mma.sync kernel (see ``decode_uses_tensor_cores``); what that does not take goes to the all-sizes kernel, whose weights are floats.
 
     ``chunk`` C: a query at position p sees only keys from p - p % C on (its own block of C positions, counted from
     the sequence's start); ``sinks`` (float32, one per query head): exp(sink) joins the softmax's denominator.
@@ -393,13 +393,12 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
         box_rows = min(page_size, 32)
         group = num_heads // num_kv_heads
         shaped = cap > 0.0 or precise_weights or not plain_mask or difference is not None
-        if head_dim == 128 and dv == 128 and 128 % group == 0 and max_q_len * group >= (256 if shaped else 128) \
-                and scale > 0.0 and out.data_ptr() % 16 == 0 and (not shaped or tiles_per_cta < 2):
+        if head_dim == 128 and dv == 128 and 128 % group == 0 and max_q_len * group >= 128 and scale > 0.0 \
+                and out.data_ptr() % 16 == 0 and (not shaped or (tiles_per_cta < 2 and shaped_prompt_on_tcgen05(
+                    max_q_len, group, num_kv_heads, n_rows, block_table.shape[-1] * page_size, cap > 0.0, _sm_count(q.device)))):
             # heads of 128, at least one full tile of 128 query vectors, scores that keep their order (the kernel takes a
             # block's maximum, and masks, before it scales) and an output for 16-byte stores (the mma.sync kernel's are of 4
-            # bytes): the tcgen05 kernel.  Its further forms from two
-            # tiles on (16 query and 8 KV heads, weights in two terms, us on it and on the mma.sync kernel: 64 tokens 10.3 and
-            # 9.1, 128 tokens 10.4 and 12.6, 2,048 tokens 43 and 139; with a soft-cap 11.9 and 9.3, 11.8 and 12.6, 60 and 152)
+            # bytes): the tcgen05 kernel
             rc = load_cuda_library("attention_tcgen05.cu").b200_prefill_attention_tcgen05(
                 _p(q), kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), _p(out), _p(block_table),
                 block_table.shape[-1], _p(cu_q), _p(kv_len), _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads,
@@ -423,6 +422,24 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
         int(window or 0), ctypes.c_float(scale), _code(q), head_dim, dv, ctypes.c_float(cap), int(chunk or 0),
         _p(sinks), head_dim if shared_values else 0, _stream())
     _ok(rc, "prefill_attention")
+
+
+def shaped_prompt_on_tcgen05(max_q_len: int, group: int, num_kv_heads: int, n_rows: int, keys: int, capped: bool,
+                             sm_count: int) -> bool:
+    """Whether prompt attention's further forms (heads of 128) run on the tcgen05 kernel rather than the mma.sync one; ``keys``
+    bounds what a row holds.
+
+    A CTA of the tcgen05 kernel fills an SM and takes 9 us before its second block of 128 keys, so it wants two tiles of query
+    vectors a KV head, and the more keys the more waves there are.  (us on mma.sync / tcgen05, weights in two terms and, in brackets,
+    soft-capped; 16 query and 8 KV heads unless said.  One wave: 1 row of 128 tokens 11.5 / 10.8 (12.6 / 12.1), 64 tokens of 32 heads
+    9.4 / 11.3 alone and 115 / 37 behind 2,000 cached, 2,048 tokens 139 / 43 (152 / 60).  Two waves: 16 rows of 128 16.9 / 20.9 (17.0 /
+    23.0), 8 rows of 256 23.6 / 22.9 (25.1 / 26.2), 4 rows of 300 26.4 / 20.1 (28.0 / 22.5).  More: 16 rows of 200 33.1 / 40.8 (34.2 /
+    47.5), of 300 53.1 / 53.0 (56.8 / 62.1), of 400 82 / 78 (88 / 94), of 512 119 / 89 (127 / 109).)"""
+    tokens = 128 // group                                 # of a tile
+    if max_q_len < 2 * tokens or keys < 128:
+        return False
+    ctas = num_kv_heads * n_rows * -(-max_q_len // tokens)
+    return ctas <= sm_count or keys >= (512 if capped and ctas > 2 * sm_count else 256)
 
 
 def _check_cache(k_cache, v_cache, num_kv_heads, page_size, head_dim, v_head_dim) -> None:
