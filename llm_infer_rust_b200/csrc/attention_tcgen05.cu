@@ -8,7 +8,10 @@
 //   softmax        four warps, one thread per query row: two passes over the row of S in tensor memory
 //                  (tcgen05.ld): the row maximum, then exp2 and the row sum; the bfloat16 probabilities go back
 //                  into tensor memory (tcgen05.st), two to a column, over the first half of the scores they
-//                  came from;
+//                  came from.  The further forms (soft-cap, weights in two terms, blocks, sinks, differences) have
+//                  eight warps and two threads a row, each with its half of the scores in registers (softmax_half);
+//                  the two-tile kernel one thread a row, one score buffer a tile and the whole row in registers after
+//                  one pass, and its P V begins with the first 64 keys' weights (softmax_row);
 //   O += P V       tcgen05.mma with the A operand in tensor memory, M 128, N 128 (head dims), K 16 x 8,
 //                  accumulating in tensor memory over all blocks; V is used as it lies in the cache (keys x dims,
 //                  the dims contiguous: an MN-major B operand).  The tensor pipe runs the MMAs of one thread in

@@ -84,10 +84,11 @@ __global__ void rms_norm_kernel(TA* out, const TA* x, TA* residual, const TW* __
     dst[i] = from_f32<TA>(row_buf[i] * scale * to_f32<TW>(w[i]));
 }
 
-// Rows whose width is a multiple of the 16-byte vector and at most 32 * VPL vectors: one WARP per row, the row's
+// Rows whose width is a multiple of the 16-byte vector and at most 32 * WARP_VECTORS vectors: one WARP per row, the row's
 // values stay in registers between the sum of squares and the scaling, loads and stores are 16 bytes wide.
 // The sum runs over the lanes' partial sums in a fixed order, so a row's result does not depend on other rows.
-template <typename TA, typename TW, bool ADD, int VPL>
+constexpr int WARP_VECTORS = 4;                 // of a row that a lane holds
+template <typename TA, typename TW, bool ADD>
 __global__ void __launch_bounds__(256)
 rms_norm_warp_kernel(TA* out, const TA* x, TA* residual, const TW* __restrict__ w, const int* __restrict__ rows,
                      int n_rows, int width, float eps, int write_residual) {
@@ -97,10 +98,10 @@ rms_norm_warp_kernel(TA* out, const TA* x, TA* residual, const TW* __restrict__ 
   if (r >= n_rows) return;
   const size_t src = static_cast<size_t>(rows ? rows[r] : r) * width;
   const int vectors = width / N;
-  float v[VPL][N];
+  float v[WARP_VECTORS][N];
   float ss = 0.0f;
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
+  for (int i = 0; i < WARP_VECTORS; ++i) {
     const int c = (i * 32 + lane) * N;
     if (i * 32 + lane < vectors) {
       Vec16<TA>::load(x + src + c, v[i]);
@@ -120,7 +121,7 @@ rms_norm_warp_kernel(TA* out, const TA* x, TA* residual, const TW* __restrict__ 
   const float scale = rsqrtf(ss / static_cast<float>(width) + eps);
   TA* dst = out + static_cast<size_t>(r) * width;
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
+  for (int i = 0; i < WARP_VECTORS; ++i) {
     const int c = (i * 32 + lane) * N;
     if (i * 32 + lane < vectors) {
       __align__(16) TA y[N];
@@ -285,16 +286,16 @@ B200_EXPORT int b200_rms_norm(void* out, const void* x, void* residual, const vo
   if (n_rows <= 0) return 0;
   if (width <= 0) return B200_BAD_SIZE;
   {
-    // Rows of 16-byte vectors: a warp a row up to 32 * 4 of them, beyond that a block a row.
+    // Rows of 16-byte vectors: a warp a row up to 32 * WARP_VECTORS of them, beyond that a block a row.
     const int vec = act_dtype == B200_F32 ? 4 : 8;
     const bool aligned = reinterpret_cast<uintptr_t>(out) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(residual) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
     if (width % vec == 0 && width / vec <= 2 * 1024 && aligned) {
-      const bool small = width / vec <= 32 * 4;
+      const bool small = width / vec <= 32 * WARP_VECTORS;
       const int blocks = small ? (n_rows + 7) / 8 : n_rows;
       const int threads = small ? 256 : (width / vec + 63) / 64 * 32;
 #define LAUNCHW(TA, TW, ADD)                                                                                 \
-      if (small) rms_norm_warp_kernel<TA, TW, ADD, 4><<<blocks, threads, 0, stream>>>(static_cast<TA*>(out),  \
+      if (small) rms_norm_warp_kernel<TA, TW, ADD><<<blocks, threads, 0, stream>>>(static_cast<TA*>(out),  \
           static_cast<const TA*>(x), static_cast<TA*>(residual), static_cast<const TW*>(w), rows, n_rows, width, eps, \
           write_residual);                                                                                   \
       else rms_norm_block_kernel<TA, TW, ADD><<<blocks, threads, 0, stream>>>(static_cast<TA*>(out),          \
