@@ -201,10 +201,11 @@ __device__ __forceinline__ void load_key_block(T* dst, const T* __restrict__ cac
 // 32 hc ..): tile_tokens * heads <= 32 vectors.
 constexpr int PF_WARPS = 8;
 
-// (Three CTAs an SM where shared memory has room for them: with 88 registers instead of 80 heads of 16 had two, and 2,000 float32
-// tokens behind 1,000, 40 query heads, took 2,949 us for 2,383.)
+// (Heads of 16 are held to three CTAs an SM: with 88 registers instead of 80 they had two, and 2,000 float32 tokens behind 1,000, 40
+// query heads, took 2,949 us for 2,383.  0 leaves the others to the compiler, which stays at 80 or at what shared memory allows;
+// told that one CTA is enough it took all registers, and heads of 32 6,336 us for 2,546.)
 template <typename T>
-__global__ void __launch_bounds__(PF_WARPS * 32, D <= 16 ? 3 : 1)
+__global__ void __launch_bounds__(PF_WARPS * 32, D <= 16 ? 3 : 0)
 prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                          T* __restrict__ out, const int* __restrict__ block_table, int table_stride,
                          const int* __restrict__ cu_q, const int* __restrict__ kv_len,
@@ -458,6 +459,25 @@ __global__ void decode_merge_kernel(T* __restrict__ out, const float* __restrict
 }
 
 // ------------------------------------------------------------------ launchers
+// A prefill CTA: two blocks of keys and values where two CTAs of that size still share an SM, else one.
+template <typename T>
+struct PrefillShape {
+  static constexpr size_t FIXED = (32 * D + PF_WARPS * KB * NV) * sizeof(float), BLOCK = 2 * KB * RowGeom<T>::STRIDE * sizeof(T);
+  static constexpr int STAGES = FIXED + 2 * BLOCK <= 110 * 1024 ? 2 : 1;
+  static constexpr size_t SMEM = FIXED + STAGES * BLOCK;
+};
+// How many prefill CTAs an SM of the current device holds (tests: their registers decide how fast long prompts are).
+template <typename T>
+static int prefill_ctas_per_sm() {
+  int n = 0;
+  cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PrefillShape<T>::SMEM));
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, prefill_attention_kernel<T>, PF_WARPS * 32, PrefillShape<T>::SMEM);
+  return e == cudaSuccess ? n : -static_cast<int>(e);
+}
+B200_EXPORT int b200_prefill_attention_ctas_per_sm(int dtype) {
+  return dtype == B200_F32 ? prefill_ctas_per_sm<float>() : prefill_ctas_per_sm<__nv_bfloat16>();
+}
+
 template <typename T>
 static int launch_prefill(const void* q, const void* kc, const void* vc, void* out, const int* block_table,
                           int table_stride, const int* cu_q, const int* kv_len, const int* prefix_len,
@@ -468,10 +488,8 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   const int group = nh / nkv;
   const int head_chunks = (group + 31) / 32;                  // more than 32 query heads per KV head: several CTAs
   const int tile_tokens = group >= 32 ? 1 : 32 / group;
-  // Two blocks of keys where two CTAs of that size still share an SM, else one.
-  constexpr size_t fixed = (32 * D + PF_WARPS * KB * NV) * sizeof(float), block = 2 * KB * G::STRIDE * sizeof(T);
-  constexpr int stages = fixed + 2 * block <= 110 * 1024 ? 2 : 1;
-  constexpr size_t smem = fixed + stages * block;
+  constexpr int stages = PrefillShape<T>::STAGES;
+  constexpr size_t smem = PrefillShape<T>::SMEM;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -145,3 +145,11 @@ def test_a_row_of_few_rows_experts_is_the_same_in_every_step():
             want += gains[t, k].double() * (dn[e].double() @ (torch.nn.functional.silu(g) * u).bfloat16().double())
         # the hidden row is rounded to 8 bits, where a sum in 32 bits may fall on the other side
         assert ((many[t].double() - want).abs() <= 2.0 ** -8 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head_dim,ctas", [(16, 3), (32, 3), (48, 2), (64, 3), (128, 2)])
+def test_all_sizes_prompt_attention_keeps_its_blocks_on_an_sm(head_dim, ctas, dtype):
+    """A few registers more a thread and an SM holds a block less; long prompts then take up to twice the time."""
+    from llm_infer_rust_b200.kernels import ops
+    assert ops._attention(head_dim).b200_prefill_attention_ctas_per_sm(ops.F32 if dtype == torch.float32 else ops.BF16) >= ctas
