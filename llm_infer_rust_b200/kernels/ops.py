@@ -19,6 +19,9 @@ import torch
 
 from .build import load_cuda_library
 
+# (A torch built without CUDA has neither; the wrappers refuse its tensors before they would be called.)
+_raw_stream, _current_device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
 ERROR_BITS = {1: "a token id outside the embedding table", 2: "a cache slot outside the pool",
@@ -66,8 +69,8 @@ def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 def _stream() -> ctypes.c_void_p:
     """The current stream's handle.  (``torch.cuda.current_stream`` makes an object and looks the device up on its way: a
-    quarter of the host's time of an eager step.  Named here and not at import: a torch built without CUDA has neither.)"""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    quarter of the host's time of an eager step.)"""
+    return ctypes.c_void_p(_raw_stream(_current_device()))
 
 
 # Launches of this package's kernels so far (library matrix products are not counted).
