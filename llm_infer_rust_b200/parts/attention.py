@@ -113,7 +113,7 @@ def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_d
         # whole, 51 in three splits, 45 in eight; 16 rows x 8 KV heads 118 whole, 55 in three).
         per_sm = ops.all_sizes_decode_ctas_per_sm(dtype, max(head_dim, v_head_dim or head_dim))
         if per_sm > 1:
-            return max(1, min(16, kv_len_bound // (2 * _ALL_SIZES_KEYS_PER_CTA_AT_LEAST), per_sm * sm_count // max(1, ctas)))
+            return max(1, min(8, kv_len_bound // _ALL_SIZES_KEYS_PER_CTA_AT_LEAST, per_sm * sm_count // max(1, ctas)))
         return decode_splits(ctas, kv_len_bound, sm_count, _ALL_SIZES_KEYS_PER_CTA_AT_LEAST, merge_keys=0)
     return _splits_over_waves(ctas, kv_len_bound, sm_count, decode_splits(ctas, kv_len_bound, sm_count))
 

@@ -79,6 +79,6 @@ def test_small_heads_of_the_all_sizes_kernel_fill_every_cta_that_an_sm_holds():
     from llm_infer_rust_b200.parts.attention import attention_splits
     assert ops.all_sizes_decode_ctas_per_sm(torch.float32, 32) == 3 and ops.all_sizes_decode_ctas_per_sm(torch.float32, 128) == 1
     splits = lambda rows, nh, nkv, d, bound=4096: attention_splits(torch.float32, rows, nh, nkv, d, 16, bound, 148)
-    assert [splits(r, 16, 8, 32) for r in (1, 4, 8, 16, 32)] == [16, 13, 6, 3, 1]
-    assert splits(8, 40, 1, 32) == 5 and splits(4, 40, 1, 32) == 11 and splits(8, 16, 8, 32, 300) == 1
+    assert [splits(r, 16, 8, 32) for r in (1, 4, 8, 16, 32)] == [8, 8, 6, 3, 1]
+    assert splits(8, 40, 1, 32) == 5 and splits(4, 40, 1, 32) == 8 and splits(8, 16, 8, 32, 300) == 2
     assert [splits(r, 16, 8, 128) for r in (1, 4, 8, 16)] == [8, 4, 2, 1]
