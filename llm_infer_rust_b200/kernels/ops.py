@@ -396,7 +396,8 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
         box_rows = min(page_size, 32)
         group = num_heads // num_kv_heads
         shaped = cap > 0.0 or precise_weights or not plain_mask or difference is not None
-        limit = 0 if difference is not None else min((int(m) for m in (window, chunk) if m), default=0)      # (a difference: either way)
+        # (a difference was as fast on the tcgen05 kernel at every window)
+        limit = 0 if difference is not None else min(([int(window) + 128 // group] if window else []) + ([int(chunk)] if chunk else []), default=0)
         if head_dim == 128 and dv == 128 and 128 % group == 0 and max_q_len * group >= 128 and scale > 0.0 \
                 and out.data_ptr() % 16 == 0 and (not shaped or (tiles_per_cta < 2 and shaped_prompt_on_tcgen05(
                     max_q_len, group, num_kv_heads, n_rows, block_table.shape[-1] * page_size, cap > 0.0, _sm_count(q.device), limit))):
@@ -431,22 +432,24 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
 def shaped_prompt_on_tcgen05(max_q_len: int, group: int, num_kv_heads: int, n_rows: int, keys: int, capped: bool,
                              sm_count: int, limit: int = 0) -> bool:
     """Whether prompt attention's further forms (heads of 128) run on the tcgen05 kernel rather than the mma.sync one; ``keys``
-    bounds what a row holds, ``limit`` > 0 what a query sees of it (a window, a block of positions).
+    bounds what a row holds, ``limit`` > 0 what a tile's queries see of it (a window and a tile's tokens, a block of positions).
 
     A CTA of the tcgen05 kernel fills an SM and takes 9 us before its second block of 128 keys, so it wants two tiles of query
     vectors a KV head, and the more keys the more waves there are.  (us on mma.sync / tcgen05, weights in two terms and, in brackets,
     soft-capped; 16 query and 8 KV heads unless said.  One wave: 1 row of 128 tokens 11.5 / 10.8 (12.6 / 12.1), 100 tokens of 32 heads
     13.9 / 11.3, 64 of them 9.4 / 11.3 alone and 115 / 37 behind 2,000 cached, 2,048 tokens 139 / 43 (152 / 60).  Two waves: 16 rows of
     128 16.9 / 20.9 (17.0 / 23.0), 8 rows of 256 23.6 / 22.9 (25.1 / 26.2), 4 rows of 300 26.4 / 20.1 (28.0 / 22.5).  More: 16 rows of 200
-    33.1 / 40.8 (34.2 / 47.5), of 300 53.1 / 53.0 (56.8 / 62.1), of 400 82 / 78 (88 / 94; 32 heads 167 / 141 (178 / 169)), of 512 119 / 89
-    (127 / 109).  A window or blocks of 64: 1 row of 2,000 21.6 / 25.5, 8 of 1,000 60 / 83; of 128: 8 of 1,000 80 / 86, in blocks 60 / 72.)"""
+    33.1 / 40.8 (34.2 / 47.5; 8 rows, two waves, 22.2 / 22.3 (23.8 / 25.8), 4 rows of 32 heads 22.6 / 21.0 (24.2 / 23.9)), of 300 53.1 / 53.0 (56.8 / 62.1), of 400 82 / 78 (88 / 94; 32 heads 167 / 141 (178 / 169)), of 512 119 / 89
+    (127 / 109).  A window or blocks of 64: 1 row of 2,000 21.6 / 25.5, 8 of 1,000 60 / 83; of 128: 1 row of 2,000 29.4 / 25.1, 8 of
+    1,000 80 / 86, in blocks 60 / 72.)"""
     tokens = 128 // group                                 # of a tile
     seen = min(keys, limit) if limit > 0 else keys
     if max_q_len < 2 * tokens or keys < 96:
         return False
     ctas = num_kv_heads * n_rows * -(-max_q_len // tokens)
-    many = 256 if not capped or ctas <= 2 * sm_count else 512 if group < 4 else 384
-    return ctas <= sm_count or seen >= many
+    if ctas <= 2 * sm_count:
+        return ctas <= sm_count or seen >= (256 if capped and group < 4 else 192)
+    return seen >= (256 if not capped else 512 if group < 4 else 384)
 
 
 def _check_cache(k_cache, v_cache, num_kv_heads, page_size, head_dim, v_head_dim) -> None:

@@ -140,7 +140,7 @@ SEVERAL = [dict(cap=5.0), dict(chunk=130, sinks=True), dict(window=129, differen
 
 @pytest.mark.parametrize("precise", [True, False], ids=["two-terms", "one-term"])
 @pytest.mark.parametrize("form", SEVERAL, ids="-".join)
-@pytest.mark.parametrize("H,G", [(4, 2), (16, 1)])
+@pytest.mark.parametrize("H,G", [(4, 2), (4, 1)])
 def test_forms_over_rows_of_all_lengths(H, G, form, precise):
     """Several rows in one launch, named in another order than the batch's, with cached tokens before them, among them rows with
     nothing in most of the grid's tiles; weights in two bfloat16 terms and in one."""

@@ -35,5 +35,6 @@ def test_which_prompts_of_the_further_forms_take_the_tcgen05_kernel():
     assert taken(300, 16, 8, 16) and not taken(300, 16, 8, 16, capped=True)
     assert taken(100, 32, 8) and taken(400, 32, 8, 16, capped=True) and not taken(400, 16, 8, 16, capped=True)
     # windows and blocks: a query that sees few keys leaves a CTA little behind its first block
-    assert not taken(2000, 16, 8, limit=64) and not taken(1000, 16, 8, 8, limit=128)
+    assert not taken(2000, 16, 8, limit=64 + 64) and not taken(1000, 16, 8, 8, limit=128 + 64) and not taken(1000, 16, 8, 8, limit=128)
+    assert taken(2000, 16, 8, limit=128 + 64) and taken(200, 32, 8, 4, capped=True) and not taken(200, 16, 8, 8, capped=True)
     assert taken(500, 16, 8, limit=128) and taken(1000, 16, 8, 8, limit=512) and taken(2048, 16, 8, limit=1024)
