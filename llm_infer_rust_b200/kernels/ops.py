@@ -435,13 +435,15 @@ def shaped_prompt_on_tcgen05(max_q_len: int, group: int, num_kv_heads: int, n_ro
     bounds what a row holds, ``limit`` > 0 what a tile's queries see of it (a window and a tile's tokens, a block of positions).
 
     A CTA of the tcgen05 kernel fills an SM and takes 9 us before its second block of 128 keys, so it wants two tiles of query
-    vectors a KV head, and the more keys the more waves there are.  (us on mma.sync / tcgen05, weights in two terms and, in brackets,
-    soft-capped; 16 query and 8 KV heads unless said.  One wave: 1 row of 128 tokens 11.5 / 10.8 (12.6 / 12.1), 100 tokens of 32 heads
-    13.9 / 11.3, 64 of them 9.4 / 11.3 alone and 115 / 37 behind 2,000 cached, 2,048 tokens 139 / 43 (152 / 60).  Two waves: 16 rows of
-    128 16.9 / 20.9 (17.0 / 23.0), 8 rows of 256 23.6 / 22.9 (25.1 / 26.2), 4 rows of 300 26.4 / 20.1 (28.0 / 22.5).  More: 16 rows of 200
-    33.1 / 40.8 (34.2 / 47.5; 8 rows, two waves, 22.2 / 22.3 (23.8 / 25.8), 4 rows of 32 heads 22.6 / 21.0 (24.2 / 23.9)), of 300 53.1 / 53.0 (56.8 / 62.1), of 400 82 / 78 (88 / 94; 32 heads 167 / 141 (178 / 169)), of 512 119 / 89
-    (127 / 109).  A window or blocks of 64: 1 row of 2,000 21.6 / 25.5, 8 of 1,000 60 / 83; of 128: 1 row of 2,000 29.4 / 25.1, 8 of
-    1,000 80 / 86, in blocks 60 / 72.)"""
+    vectors a KV head, and the more keys the more waves there are.  Measured, us on mma.sync / tcgen05, weights in two terms and, in
+    brackets, soft-capped; 16 query and 8 KV heads unless said:
+      one wave: 1 row of 128 tokens 11.5 / 10.8 (12.6 / 12.1), of 2,048 139 / 43 (152 / 60); 32 heads, 100 tokens 13.9 / 11.3, 64 tokens
+      9.4 / 11.3 alone and 115 / 37 behind 2,000 cached;
+      two: 16 rows of 128 16.9 / 20.9 (17.0 / 23.0), 8 rows of 200 22.2 / 22.3 (23.8 / 25.8), of 256 23.6 / 22.9 (25.1 / 26.2), 4 rows of 300
+      26.4 / 20.1 (28.0 / 22.5); 32 heads, 4 rows of 200 22.6 / 21.0 (24.2 / 23.9);
+      more: 16 rows of 200 33.1 / 40.8 (34.2 / 47.5), of 300 53.1 / 53.0 (56.8 / 62.1), of 400 82 / 78 (88 / 94), of 512 119 / 89 (127 / 109);
+      32 heads, 16 rows of 400 167 / 141 (178 / 169);
+      a window of 64: 1 row of 2,000 21.6 / 25.5, 8 of 1,000 60 / 83; of 128: 29.4 / 25.1 and 80 / 86, in blocks of 128 60 / 72 for the second."""
     tokens = 128 // group                                 # of a tile
     seen = min(keys, limit) if limit > 0 else keys
     if max_q_len < 2 * tokens or keys < 96:
