@@ -1,0 +1,205 @@
+// How Python calls the C entry points of the kernel libraries: torch tensors go in as they are.
+//
+// A prompt of a length that does not come again is launched call by call (nine launches a layer), and small models wait
+// for the host then.  ctypes took 4 us for twenty arguments (an object an argument, a lock round every call) beside 1 to 2
+// for the checks of the tensors and 2 for an output tensor made through Python; here a call is a loop over its arguments.
+//
+// entry(address) gives a callable whose arguments say by their type what they are:
+//   a tensor, None, a ctypes structure or array     a pointer (to the tensor's data, null, to the object's memory)
+//   an int (a bool, an address)                     an integer of up to 64 bits
+//   a float                                         a 32-bit float
+// The entry points take these three kinds alone, return an int, and take at most MAX_INTS of the first two and MAX_FLOATS of
+// the third.  Under both calling conventions that a B200 host has (System V x86-64, AAPCS64) integers and floats are counted
+// apart: each kind fills its own registers in order, what integers do not fit follows on the stack in slots of eight bytes,
+// and what a callee does not ask for it does not look at.  So one call through one type with all of them reaches every such
+// function; the order between ints and floats of a signature does not matter, their order among themselves does.
+#include <torch/csrc/Device.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/torch.h>
+
+#include <cstdint>
+
+#if !defined(__x86_64__) && !defined(__aarch64__)
+#error "the calling convention of this host is not known to pass integers and floats apart"
+#endif
+#if defined(_WIN32) || defined(__APPLE__)
+#error "System V x86-64 or AAPCS64 with eight-byte stack slots"
+#endif
+
+namespace {
+
+constexpr int MAX_INTS = 48, FEW_INTS = 16, MAX_FLOATS = 8;
+using I = std::int64_t;
+
+#define I8(a, n) a[n], a[n + 1], a[n + 2], a[n + 3], a[n + 4], a[n + 5], a[n + 6], a[n + 7]
+#define F8(f) f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]
+#define T8 I, I, I, I, I, I, I, I
+#define TF float, float, float, float, float, float, float, float
+using FewFn = int (*)(T8, T8, TF);
+using MostFn = int (*)(T8, T8, T8, T8, T8, T8, TF);
+
+struct Entry {
+  PyObject_HEAD
+  vectorcallfunc call;
+  void* fn;
+};
+
+PyObject *structure_type, *array_type;      // of ctypes
+
+PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
+  HANDLE_TH_ERRORS
+  const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
+  if (kwnames != nullptr && PyTuple_GET_SIZE(kwnames) != 0) {
+    PyErr_SetString(PyExc_TypeError, "an entry point takes no keyword arguments");
+    return nullptr;
+  }
+  I ints[MAX_INTS] = {};
+  float floats[MAX_FLOATS] = {};
+  int ni = 0, nf = 0;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* a = args[i];
+    if (PyFloat_CheckExact(a)) {
+      if (nf == MAX_FLOATS) { PyErr_SetString(PyExc_TypeError, "too many floats for an entry point"); return nullptr; }
+      floats[nf++] = static_cast<float>(PyFloat_AS_DOUBLE(a));
+      continue;
+    }
+    I v = 0;
+    if (a == Py_None) {
+    } else if (PyLong_Check(a)) {
+      v = PyLong_AsLongLong(a);
+      if (v == -1 && PyErr_Occurred()) return nullptr;
+    } else if (THPVariable_Check(a)) {
+      v = reinterpret_cast<I>(THPVariable_Unpack(a).mutable_data_ptr());
+    } else if (PyObject_IsInstance(a, structure_type) == 1 || PyObject_IsInstance(a, array_type) == 1) {
+      // (the caller's argument holds the object, and with it its memory, until the call has returned)
+      Py_buffer view;
+      if (PyObject_GetBuffer(a, &view, PyBUF_SIMPLE) != 0) return nullptr;
+      v = reinterpret_cast<I>(view.buf);
+      PyBuffer_Release(&view);
+    } else {
+      PyErr_Format(PyExc_TypeError, "argument %zd of an entry point is a %s", i, Py_TYPE(a)->tp_name);
+      return nullptr;
+    }
+    if (ni == MAX_INTS) { PyErr_SetString(PyExc_TypeError, "too many arguments for an entry point"); return nullptr; }
+    ints[ni++] = v;
+  }
+  void* fn = reinterpret_cast<Entry*>(self)->fn;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  if (ni <= FEW_INTS)
+    rc = reinterpret_cast<FewFn>(fn)(I8(ints, 0), I8(ints, 8), F8(floats));
+  else
+    rc = reinterpret_cast<MostFn>(fn)(I8(ints, 0), I8(ints, 8), I8(ints, 16), I8(ints, 24), I8(ints, 32), I8(ints, 40), F8(floats));
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
+}
+
+PyTypeObject entry_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyObject* make_entry(PyObject*, PyObject* address) {
+  void* fn = PyLong_AsVoidPtr(address);
+  if (fn == nullptr) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "an entry point has an address");
+    return nullptr;
+  }
+  Entry* e = PyObject_New(Entry, &entry_type);
+  if (e == nullptr) return nullptr;
+  e->call = entry_call;
+  e->fn = fn;
+  return reinterpret_cast<PyObject*>(e);
+}
+
+// Whether every argument is None or a tensor for which `holds` is true.
+template <typename Holds>
+PyObject* all_of(PyObject* const* args, Py_ssize_t n, Holds holds) {
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    if (args[i] == Py_None) continue;
+    if (!THPVariable_Check(args[i])) {
+      PyErr_Format(PyExc_TypeError, "a tensor was expected, not a %s", Py_TYPE(args[i])->tp_name);
+      return nullptr;
+    }
+    if (!holds(THPVariable_Unpack(args[i]))) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
+}
+PyObject* all_cuda(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return all_of(args, n, [](const at::Tensor& t) { return t.is_cuda(); });
+  END_HANDLE_TH_ERRORS
+}
+PyObject* all_contiguous(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return all_of(args, n, [](const at::Tensor& t) { return t.is_contiguous(); });
+  END_HANDLE_TH_ERRORS
+}
+
+// empty(shape, dtype, device)
+PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 3 || !PyTuple_Check(args[0]) || !THPDtype_Check(args[1]) || !THPDevice_Check(args[2])) {
+    PyErr_SetString(PyExc_TypeError, "empty(shape, dtype, device)");
+    return nullptr;
+  }
+  c10::SmallVector<int64_t, 6> shape;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(args[0]); ++i) {
+    shape.push_back(PyLong_AsLongLong(PyTuple_GET_ITEM(args[0], i)));
+    if (shape.back() == -1 && PyErr_Occurred()) return nullptr;
+  }
+  const auto options = at::TensorOptions().dtype(reinterpret_cast<THPDtype*>(args[1])->scalar_type).device(reinterpret_cast<THPDevice*>(args[2])->device);
+  at::Tensor out;
+  {
+    pybind11::gil_scoped_release free;
+    out = at::empty(shape, options);
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// mm_t(x, w): x . w^T by the library
+PyObject* mm_t(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) {
+    PyErr_SetString(PyExc_TypeError, "mm_t(x, w)");
+    return nullptr;
+  }
+  const at::Tensor x = THPVariable_Unpack(args[0]), w = THPVariable_Unpack(args[1]);
+  at::Tensor out;
+  {
+    pybind11::gil_scoped_release free;
+    out = at::mm(x, w.t());
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"entry", make_entry, METH_O, "entry(address): the C entry point at an address as a callable"},
+    {"all_cuda", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(all_cuda)), METH_FASTCALL, "whether every tensor (None counts as one) is on a GPU"},
+    {"all_contiguous", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(all_contiguous)), METH_FASTCALL, "whether every tensor (None counts as one) is contiguous"},
+    {"empty", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(empty)), METH_FASTCALL, "empty(shape, dtype, device)"},
+    {"mm_t", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(mm_t)), METH_FASTCALL, "mm_t(x, w): x . w^T"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__calls() {
+  PyObject* ctypes = PyImport_ImportModule("ctypes");
+  if (ctypes == nullptr) return nullptr;
+  structure_type = PyObject_GetAttrString(ctypes, "Structure");
+  array_type = PyObject_GetAttrString(ctypes, "Array");
+  Py_DECREF(ctypes);
+  if (structure_type == nullptr || array_type == nullptr) return nullptr;
+  entry_type.tp_name = "_calls.Entry";
+  entry_type.tp_basicsize = sizeof(Entry);
+  entry_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
+  entry_type.tp_vectorcall_offset = offsetof(Entry, call);
+  entry_type.tp_call = PyVectorcall_Call;
+  entry_type.tp_dealloc = [](PyObject* o) { PyObject_Free(o); };
+  if (PyType_Ready(&entry_type) < 0) return nullptr;
+  return PyModule_Create(&module);
+}

@@ -6,8 +6,9 @@ Two kinds of libraries live under ``csrc/``:
   library per (source file, compile-time sizes) and loaded with ``ctypes``.  A
   model only ever asks for the sizes that it has, so a first call compiles just
   what that model needs;
-* the host runtime (``host/*.cpp``: cache manager, scheduler, batch builder),
-  compiled by the C++ compiler into a Python extension module.
+* the host runtime (``host/*.cpp``: cache manager, scheduler, batch builder) and
+  the binding of the kernels' entry points (``binding/calls.cpp``), compiled by the
+  C++ compiler into Python extension modules.
 
 Built files go to ``llm_infer_rust_b200/_build`` (or, if the package folder is
 read-only, to a folder under the temporary directory).  A library's file name
@@ -196,11 +197,101 @@ def load_cuda_library(source: str, defines: Optional[Dict[str, object]] = None) 
         return lib
 
 
+class EntryPoints:
+    """The C entry points of a kernel library as callables that take tensors, ints and floats as they are (see
+    csrc/binding/calls.cpp).  They return an int; ``library`` is the library itself, for those that return something else."""
+
+    def __init__(self, library: ctypes.CDLL):
+        self.library = library
+
+    def __getattr__(self, name: str):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        address = ctypes.cast(getattr(self.library, name), ctypes.c_void_p).value
+        fn = load_call_binding().entry(address)
+        setattr(self, name, fn)                       # (found without this function from now on)
+        return fn
+
+
+_entry_points: Dict[tuple, EntryPoints] = {}
+
+
+def load_entry_points(source: str, defines: Optional[Dict[str, object]] = None) -> EntryPoints:
+    """The entry points of ``load_cuda_library(source, defines)``."""
+    name = (source, tuple(sorted(defines.items())) if defines else ())
+    points = _entry_points.get(name)
+    if points is None:
+        points = _entry_points.setdefault(name, EntryPoints(load_cuda_library(source, defines)))
+    return points
+
+
 def all_cuda_libraries(head_dims: Iterable[int]) -> List[tuple]:
     """(source, defines) of every CUDA library that the package can ask for, attention for ``head_dims``."""
     per_head = ("attention.cu", "attention_mma.cu", "decode_attention_static.cu")
     libs = [(f, None) for f in sorted(os.listdir(CSRC)) if f.endswith(".cu") and f not in per_head]
     return libs + [(f, {"HEAD_DIM": int(d)}) for f in per_head for d in head_dims]
+
+
+def build_call_binding() -> str:
+    """Compile csrc/binding/calls.cpp, the extension module through which tensors reach the entry points; return its path."""
+    import torch
+    source = os.path.join(CSRC, "binding", "calls.cpp")
+    what = "the binding of the kernels' entry points"
+    cxx = _find_cxx(what)
+    flags = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _hash([source], [" ".join(flags), sys.version, torch.__version__])
+
+    def command(out: str) -> List[str]:
+        root = os.path.dirname(torch.__file__)
+        include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                   sysconfig.get_paths()["include"]]
+        lib = os.path.join(root, "lib")
+        return ([cxx] + flags + [f"-I{p}" for p in include] + [source, "-o", out, f"-L{lib}", f"-Wl,-rpath,{lib}"]
+                + ["-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    return _build_extension(os.path.join(build_dir(), f"calls_{digest}"), "_calls", command, what)
+
+
+def load_call_binding():
+    return _load_extension("calls", "_calls", build_call_binding)
+
+
+def _find_cxx(what: str) -> str:
+    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        raise BuildError(f"no C++ compiler was found for {what}")
+    return cxx
+
+
+def _build_extension(folder: str, module: str, command, what: str) -> str:
+    """Run ``command(output)`` unless ``folder`` holds the module already; return the module's path."""
+    path = os.path.join(folder, module + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    if os.path.isfile(path):
+        return path
+    os.makedirs(folder, exist_ok=True)
+    with open(os.path.join(folder, ".lock"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not os.path.isfile(path):
+                tmp = f"{path}.{os.getpid()}.tmp"
+                _run(command(tmp), what)
+                os.replace(tmp, path)
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+    return path
+
+
+def _load_extension(key: str, module: str, build):
+    mod = _loaded.get(key)
+    if mod is None:
+        with _lock:
+            mod = _loaded.get(key)
+            if mod is None:
+                spec = importlib.util.spec_from_file_location(module, build())
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                _loaded[key] = mod
+    return mod
 
 
 def _host_sources() -> List[str]:
@@ -211,37 +302,16 @@ def _host_sources() -> List[str]:
 def build_host_runtime() -> str:
     import pybind11
     sources = _host_sources()
-    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
-    if not cxx:
-        raise BuildError("no C++ compiler was found for the host runtime")
+    what = "the host runtime (cache manager, scheduler, batch builder)"
+    cxx = _find_cxx(what)
     flags = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
     digest = _hash(sources, [" ".join(flags), sys.version, pybind11.__version__])
-    folder = os.path.join(build_dir(), f"host_{digest}")
-    path = os.path.join(folder, "_host_runtime" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
-    if os.path.isfile(path):
-        return path
-    os.makedirs(folder, exist_ok=True)
-    with open(os.path.join(folder, ".lock"), "w") as lock:
-        fcntl.flock(lock, fcntl.LOCK_EX)
-        try:
-            if not os.path.isfile(path):
-                tmp = f"{path}.{os.getpid()}.tmp"
-                cmd = [cxx] + flags + ["-I", pybind11.get_include(), "-I", sysconfig.get_paths()["include"]]
-                cmd += [s for s in sources if s.endswith(".cpp")] + ["-o", tmp]
-                _run(cmd, "the host runtime (cache manager, scheduler, batch builder)")
-                os.replace(tmp, path)
-        finally:
-            fcntl.flock(lock, fcntl.LOCK_UN)
-    return path
+
+    def command(out: str) -> List[str]:
+        return ([cxx] + flags + ["-I", pybind11.get_include(), "-I", sysconfig.get_paths()["include"]]
+                + [s for s in sources if s.endswith(".cpp")] + ["-o", out])
+    return _build_extension(os.path.join(build_dir(), f"host_{digest}"), "_host_runtime", command, what)
 
 
 def load_host_runtime():
-    with _lock:
-        mod = _loaded.get("host")
-        if mod is None:
-            path = build_host_runtime()
-            spec = importlib.util.spec_from_file_location("_host_runtime", path)
-            mod = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(mod)
-            _loaded["host"] = mod
-        return mod
+    return _load_extension("host", "_host_runtime", build_host_runtime)

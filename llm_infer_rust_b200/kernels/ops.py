@@ -17,7 +17,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .build import load_cuda_library
+from .build import load_call_binding, load_cuda_library, load_entry_points
 
 # (A torch built without CUDA has neither; the wrappers refuse its tensors before they would be called.)
 _raw_stream, _current_device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
@@ -41,36 +41,42 @@ def _code(t: torch.Tensor) -> int:
         raise KernelError(f"dtype {t.dtype} is not supported (float32 and bfloat16 are)") from None
 
 
+# What the compiled binding does for the wrappers (csrc/binding/calls.cpp); loaded at the first use, so that importing needs
+# neither a compiler nor a GPU.
+def _bind(name: str):
+    def first(*args):
+        binding = load_call_binding()
+        for n in ("all_cuda", "all_contiguous", "empty", "mm_t"):
+            globals()["_" + n] = getattr(binding, n)
+        return getattr(binding, name)(*args)
+    return first
+
+
+_all_cuda, _all_contiguous, _empty, _mm_t = _bind("all_cuda"), _bind("all_contiguous"), _bind("empty"), _bind("mm_t")
+
+
 def _cuda(*tensors: Optional[torch.Tensor]) -> None:
     """Checks that the operands are on the device.  Every wrapper that launches calls this first, so it is also
     where products that wait in the chain (see ``chain_linear``) are launched: whatever runs next may read them."""
     if _held is not None or _chain is not None:
         flush_chain()
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise KernelError("the kernels run on CUDA tensors only; there is no CPU path")
+    _cuda_only(*tensors)
 
 
 def _cuda_only(*tensors: Optional[torch.Tensor]) -> None:
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise KernelError("the kernels run on CUDA tensors only; there is no CPU path")
+    if not _all_cuda(*tensors):
+        raise KernelError("the kernels run on CUDA tensors only; there is no CPU path")
 
 
 def _contig(*tensors: Optional[torch.Tensor]) -> None:
-    for t in tensors:
-        if t is not None and not t.is_contiguous():
-            raise KernelError("a kernel was given a non-contiguous tensor")
+    if not _all_contiguous(*tensors):
+        raise KernelError("a kernel was given a non-contiguous tensor")
 
 
-def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
-
-
-def _stream() -> ctypes.c_void_p:
+def _stream() -> int:
     """The current stream's handle.  (``torch.cuda.current_stream`` makes an object and looks the device up on its way: a
     quarter of the host's time of an eager step.)"""
-    return ctypes.c_void_p(_raw_stream(_current_device()))
+    return _raw_stream(_current_device())
 
 
 # Launches of this package's kernels so far (library matrix products are not counted).
@@ -167,7 +173,7 @@ def begin_read(ids: torch.Tensor) -> PendingRead:
 
 # --------------------------------------------------------------------------- libraries
 def _elementwise():
-    return load_cuda_library("elementwise.cu")
+    return load_entry_points("elementwise.cu")
 
 
 def padded_head_dim(head_dim: int) -> int:
@@ -179,7 +185,7 @@ def _attention(head_dim: int):
     """The all-sizes attention library for a real head size (any even number up to 512)."""
     if head_dim % 2 != 0 or not 2 <= head_dim <= 512:
         raise KernelError(f"head size {head_dim} is refused: the attention kernels take even head sizes up to 512")
-    return load_cuda_library("attention.cu", {"HEAD_DIM": padded_head_dim(head_dim)})
+    return load_entry_points("attention.cu", {"HEAD_DIM": padded_head_dim(head_dim)})
 
 
 # --------------------------------------------------------------------------- element-wise
@@ -189,10 +195,10 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, out_dtype: torch.dtype, sc
     _contig(ids, table)
     if ids.dtype != torch.int32:
         raise KernelError("token ids must be int32")
-    out = torch.empty((ids.numel(), table.shape[1]), dtype=out_dtype, device=table.device)
-    rc = _elementwise().b200_embedding(_p(out), _p(table), _p(ids), ids.numel(), table.shape[1],
-                                       table.shape[0], ctypes.c_float(scale), _code(out), _code(table),
-                                       _p(error_word(table.device)), _stream())
+    out = _empty((ids.numel(), table.shape[1]), out_dtype, table.device)
+    rc = _elementwise().b200_embedding(out, table, ids, ids.numel(), table.shape[1],
+                                       table.shape[0], float(scale), _code(out), _code(table),
+                                       error_word(table.device), _stream())
     _ok(rc, "embedding")
     return out
 
@@ -207,12 +213,12 @@ def pair_embedding(ids: torch.Tensor, table: torch.Tensor, pairs: torch.Tensor, 
     _i32(ids, last_token)
     if table.dtype != pairs.dtype or tuple(pairs.shape) != (buckets + 1, table.shape[1]) or last_token[0].numel() != 1:
         raise KernelError("pair_embedding: the second table must be [buckets + 1, width] in the first one's dtype")
-    out = torch.empty((ids.numel(), table.shape[1]), dtype=out_dtype, device=table.device)
+    out = _empty((ids.numel(), table.shape[1]), out_dtype, table.device)
     rc = _elementwise().b200_pair_embedding(
-        _p(out), _p(table), _p(pairs), _p(ids), _p(ctx.row_of_token), _p(ctx.cu_q), _p(ctx.prefix_len),
-        _p(ctx.state_slots), _p(last_token), ids.numel(), table.shape[1], table.shape[0], int(buckets),
-        ctypes.c_longlong(mul_prev), ctypes.c_longlong(mul_cur), _code(out), _code(table),
-        _p(error_word(table.device)), _stream())
+        out, table, pairs, ids, ctx.row_of_token, ctx.cu_q, ctx.prefix_len,
+        ctx.state_slots, last_token, ids.numel(), table.shape[1], table.shape[0], int(buckets),
+        int(mul_prev), int(mul_cur), _code(out), _code(table),
+        error_word(table.device), _stream())
     _ok(rc, "pair_embedding")
     return out
 
@@ -242,11 +248,11 @@ def _norm(x, residual, weight, eps, out, rows, write_residual):
     if rows is not None and rows.dtype != torch.int32:
         raise KernelError("row indices must be int32")
     if out is None:
-        out = torch.empty((n, width), dtype=x.dtype, device=x.device)
+        out = _empty((n, width), x.dtype, x.device)
     elif out.dtype != x.dtype or out.numel() != n * width:
         raise KernelError("norm output has the wrong dtype or size")
-    rc = _elementwise().b200_rms_norm(_p(out), _p(x), _p(residual), _p(weight), _p(rows), n, width,
-                                      ctypes.c_float(eps), int(bool(write_residual)), _code(x),
+    rc = _elementwise().b200_rms_norm(out, x, residual, weight, rows, n, width,
+                                      float(eps), int(bool(write_residual)), _code(x),
                                       _code(weight), _stream())
     _ok(rc, "rms_norm")
     return out
@@ -260,8 +266,8 @@ def silu_mul(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch
     if width2 % 2:
         raise KernelError("silu_mul needs an even width")
     if out is None:
-        out = torch.empty((tokens, width2 // 2), dtype=gate_up.dtype, device=gate_up.device)
-    rc = _elementwise().b200_silu_mul(_p(out), _p(gate_up), tokens, width2 // 2, _code(gate_up), _stream())
+        out = _empty((tokens, width2 // 2), gate_up.dtype, gate_up.device)
+    rc = _elementwise().b200_silu_mul(out, gate_up, tokens, width2 // 2, _code(gate_up), _stream())
     _ok(rc, "silu_mul")
     return out
 
@@ -271,8 +277,8 @@ def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     _contig(x)
     if x.dtype == dtype:
         return x
-    out = torch.empty(x.shape, dtype=dtype, device=x.device)
-    rc = _elementwise().b200_cast(_p(out), _p(x), ctypes.c_longlong(x.numel()), _code(out), _code(x), _stream())
+    out = _empty(x.shape, dtype, x.device)
+    rc = _elementwise().b200_cast(out, x, int(x.numel()), _code(out), _code(x), _stream())
     _ok(rc, "cast")
     return out
 
@@ -282,7 +288,7 @@ def scale_floats(z: torch.Tensor, scale: float) -> torch.Tensor:
     _cuda(z)
     _contig(z)
     _f32(z)
-    rc = _elementwise().b200_scale_floats(_p(z), ctypes.c_longlong(z.numel()), ctypes.c_float(scale), _stream())
+    rc = _elementwise().b200_scale_floats(z, int(z.numel()), float(scale), _stream())
     _ok(rc, "scale_floats")
     return z
 
@@ -314,11 +320,11 @@ def qkv_post(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: Optional[torch.Ten
     if k_cache is not None and (k_cache.shape[1] != num_kv_heads or k_cache.shape[3] != head_dim):
         raise KernelError("the cache must be [pages + 1, kv_heads, page_size, head_dim]")
     max_pos = 0 if cos is None else cos.shape[0]
-    lib = load_cuda_library("qkv_post.cu")
-    rc = lib.b200_qkv_post(_p(qkv), _p(q_out), _p(k_cache), _p(v_cache), _p(q_weight), _p(k_weight),
-                           ctypes.c_float(eps), _p(cos), _p(sin), rot_dim, max_pos, _p(positions), _p(slots),
-                           tokens, num_heads, num_kv_heads, head_dim, page_size, ctypes.c_longlong(cache_slots),
-                           _code(qkv), wcode, _p(error_word(qkv.device)), _stream())
+    lib = load_entry_points("qkv_post.cu")
+    rc = lib.b200_qkv_post(qkv, q_out, k_cache, v_cache, q_weight, k_weight,
+                           float(eps), cos, sin, rot_dim, max_pos, positions, slots,
+                           tokens, num_heads, num_kv_heads, head_dim, page_size, int(cache_slots),
+                           _code(qkv), wcode, error_word(qkv.device), _stream())
     _ok(rc, "qkv_post")
 
 
@@ -383,10 +389,10 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
             kmap = kv_tensor_map(k_cache, min(page_size, 32), lib)
             for col0 in range(0, dv, tile):
                 rc = lib.b200_prefill_attention_mma(
-                    _p(q), kmap, kmap, _p(out), _p(block_table), block_table.shape[-1], _p(cu_q), _p(kv_len),
-                    _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads, num_heads // group, page_size,
-                    int(window or 0), ctypes.c_float(scale), ctypes.c_float(cap), int(bool(precise_weights)),
-                    int(chunk or 0), _p(sinks), col0, dv, col0, None, _p(error_word(q.device)), _stream())
+                    q, kmap, kmap, out, block_table, block_table.shape[-1], cu_q, kv_len,
+                    prefix_len, rows, n_rows, max_q_len, num_heads, num_heads // group, page_size,
+                    int(window or 0), float(scale), float(cap), int(bool(precise_weights)),
+                    int(chunk or 0), sinks, col0, dv, col0, None, error_word(q.device), _stream())
                 _ok(rc, "prefill_attention_mma_shared")
             return
         v_cache = k_cache
@@ -404,28 +410,28 @@ def prefill_attention(q, k_cache, v_cache, out, block_table, cu_q, kv_len, prefi
             # heads of 128, at least one full tile of 128 query vectors, scores that keep their order (the kernel takes a
             # block's maximum, and masks, before it scales) and an output for 16-byte stores (the mma.sync kernel's are of 4
             # bytes): the tcgen05 kernel
-            rc = load_cuda_library("attention_tcgen05.cu").b200_prefill_attention_tcgen05(
-                _p(q), kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), _p(out), _p(block_table),
-                block_table.shape[-1], _p(cu_q), _p(kv_len), _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads,
-                num_kv_heads, page_size, int(window or 0), ctypes.c_float(scale), int(tiles_per_cta), ctypes.c_float(cap),
-                int(bool(precise_weights)), int(chunk or 0), _p(sinks), _floats(difference), _p(error_word(q.device)), _stream())
+            rc = load_entry_points("attention_tcgen05.cu").b200_prefill_attention_tcgen05(
+                q, kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), out, block_table,
+                block_table.shape[-1], cu_q, kv_len, prefix_len, rows, n_rows, max_q_len, num_heads,
+                num_kv_heads, page_size, int(window or 0), float(scale), int(tiles_per_cta), float(cap),
+                int(bool(precise_weights)), int(chunk or 0), sinks, _floats(difference), error_word(q.device), _stream())
             _ok(rc, "prefill_attention_tcgen05")
             return
         rc = _attention_mma(head_dim, dv, difference is not None).b200_prefill_attention_mma(
-            _p(q), kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), _p(out), _p(block_table),
-            block_table.shape[-1], _p(cu_q), _p(kv_len), _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads,
-            num_kv_heads, page_size, int(window or 0), ctypes.c_float(scale), ctypes.c_float(cap),
-            int(bool(precise_weights)), int(chunk or 0), _p(sinks), 0, 0, 0, _floats(difference),
-            _p(error_word(q.device)), _stream())
+            q, kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), out, block_table,
+            block_table.shape[-1], cu_q, kv_len, prefix_len, rows, n_rows, max_q_len, num_heads,
+            num_kv_heads, page_size, int(window or 0), float(scale), float(cap),
+            int(bool(precise_weights)), int(chunk or 0), sinks, 0, 0, 0, _floats(difference),
+            error_word(q.device), _stream())
         _ok(rc, "prefill_attention_mma")
         return
     if difference is not None:
         raise KernelError("the all-sizes attention kernel leaves the difference of two maps to head_difference")
     rc = _attention(max(head_dim, dv)).b200_prefill_attention(
-        _p(q), _p(k_cache), _p(v_cache), _p(out), _p(block_table), block_table.shape[-1], _p(cu_q),
-        _p(kv_len), _p(prefix_len), _p(rows), n_rows, max_q_len, num_heads, num_kv_heads, page_size,
-        int(window or 0), ctypes.c_float(scale), _code(q), head_dim, dv, ctypes.c_float(cap), int(chunk or 0),
-        _p(sinks), head_dim if shared_values else 0, _stream())
+        q, k_cache, v_cache, out, block_table, block_table.shape[-1], cu_q,
+        kv_len, prefix_len, rows, n_rows, max_q_len, num_heads, num_kv_heads, page_size,
+        int(window or 0), float(scale), _code(q), head_dim, dv, float(cap), int(chunk or 0),
+        sinks, head_dim if shared_values else 0, _stream())
     _ok(rc, "prefill_attention")
 
 
@@ -493,7 +499,7 @@ def _attention_mma(head_dim: int, v_head_dim: Optional[int] = None, difference: 
         defines["V_DIM"] = v_head_dim
     if difference:
         defines["DIFF"] = 1
-    return load_cuda_library("attention_mma.cu", defines)
+    return load_entry_points("attention_mma.cu", defines)
 
 
 def shared_value_tile(value_dim: int) -> int:
@@ -541,7 +547,7 @@ def kv_tensor_map(cache: torch.Tensor, box_rows: int, lib=None):
             raise KernelError("a TMA descriptor needs a contiguous bfloat16 cache [pages + 1, kv_heads, page_size, head_dim]")
         buf = ctypes.create_string_buffer(128)
         rows = cache.shape[0] * cache.shape[1] * cache.shape[2]
-        rc = (lib or _attention_mma(cache.shape[3])).b200_kv_tensor_map(buf, _p(cache), ctypes.c_longlong(rows),
+        rc = (lib or _attention_mma(cache.shape[3])).b200_kv_tensor_map(buf, cache, int(rows),
                                                                         cache.shape[3], box_rows)
         if rc != 0:
             raise KernelError(f"the TMA descriptor of a cache tensor could not be made (code {rc})")
@@ -601,10 +607,10 @@ def decode_attention(q, k_cache, v_cache, out, scratch, block_table, cu_q, kv_le
             in_kernel = splits == 1 or (splits in (2, 4, 8) and splits * groups * n_rows <= _sm_count(q.device))
             for col0 in range(0, dv, tile):
                 rc = lib.b200_decode_attention_mma(
-                    _p(q), kmap, kmap, _p(out), _p(scratch), _p(block_table), block_table.shape[-1], _p(cu_q),
-                    _p(kv_len), _p(rows), n_rows, num_heads, groups, page_size, int(window or 0),
-                    ctypes.c_float(scale), splits, ctypes.c_float(softcap or 0.0), int(bool(precise_weights)),
-                    int(chunk or 0), _p(sinks), col0, dv, col0, None, _p(error_word(q.device)), _stream())
+                    q, kmap, kmap, out, scratch, block_table, block_table.shape[-1], cu_q,
+                    kv_len, rows, n_rows, num_heads, groups, page_size, int(window or 0),
+                    float(scale), splits, float(softcap or 0.0), int(bool(precise_weights)),
+                    int(chunk or 0), sinks, col0, dv, col0, None, error_word(q.device), _stream())
                 _ok(rc, "decode_attention_mma_shared", 1 if in_kernel else 2)
             return
         v_cache = k_cache
@@ -613,20 +619,20 @@ def decode_attention(q, k_cache, v_cache, out, scratch, block_table, cu_q, kv_le
         _check_difference(difference, q, out, num_heads, num_kv_heads, dv, sinks)
         box_rows = min(page_size, 32)
         rc = _attention_mma(head_dim, dv, difference is not None).b200_decode_attention_mma(
-            _p(q), kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), _p(out), _p(scratch), _p(block_table), block_table.shape[-1],
-            _p(cu_q), _p(kv_len), _p(rows), n_rows, num_heads, num_kv_heads, page_size, int(window or 0),
-            ctypes.c_float(scale), splits, ctypes.c_float(softcap or 0.0), int(bool(precise_weights)),
-            int(chunk or 0), _p(sinks), 0, 0, 0, _floats(difference), _p(error_word(q.device)), _stream())
+            q, kv_tensor_map(k_cache, box_rows), kv_tensor_map(v_cache, box_rows), out, scratch, block_table, block_table.shape[-1],
+            cu_q, kv_len, rows, n_rows, num_heads, num_kv_heads, page_size, int(window or 0),
+            float(scale), splits, float(softcap or 0.0), int(bool(precise_weights)),
+            int(chunk or 0), sinks, 0, 0, 0, _floats(difference), error_word(q.device), _stream())
         in_kernel = splits == 1 or (splits in (2, 4, 8) and splits * num_kv_heads * n_rows <= _sm_count(q.device))
         _ok(rc, "decode_attention_mma", 1 if in_kernel else 2)      # (a cluster of 2, 4 or 8 splits combines them itself)
         return
     if difference is not None:
         raise KernelError("the all-sizes attention kernel leaves the difference of two maps to head_difference")
     rc = _attention(max(head_dim, dv)).b200_decode_attention(
-        _p(q), _p(k_cache), _p(v_cache), _p(out), _p(scratch), _p(block_table), block_table.shape[-1],
-        _p(cu_q), _p(kv_len), _p(rows), n_rows, num_heads, num_kv_heads, page_size, int(window or 0),
-        ctypes.c_float(scale), splits, _code(q), head_dim, dv, ctypes.c_float(softcap or 0.0), int(chunk or 0),
-        _p(sinks), head_dim if shared_values else 0, _stream())
+        q, k_cache, v_cache, out, scratch, block_table, block_table.shape[-1],
+        cu_q, kv_len, rows, n_rows, num_heads, num_kv_heads, page_size, int(window or 0),
+        float(scale), splits, _code(q), head_dim, dv, float(softcap or 0.0), int(chunk or 0),
+        sinks, head_dim if shared_values else 0, _stream())
     _ok(rc, "decode_attention", 2 if splits > 1 else 1)
 
 
@@ -709,7 +715,7 @@ def _skinny(qkv_forms: bool = False, glu: str = "silu"):
     if qkv_forms:
         defines["SKINNY_QKV_FORMS"] = 1
     defines.update(_GLU_DEFINES[glu])
-    lib = load_cuda_library("skinny_linear.cu", defines or None)
+    lib = load_entry_points("skinny_linear.cu", defines or None)
     if not getattr(lib, "_checked", False):
         if lib.b200_skinny_params_size() != ctypes.sizeof(_SkinnyParams):
             raise KernelError("the parameter block of skinny_linear.cu and its Python mirror differ")
@@ -722,8 +728,8 @@ def _weight_map(weight: torch.Tensor, box_rows: int):
     buf = _weight_maps.get(key)
     if buf is None:
         buf = ctypes.create_string_buffer(128)
-        rc = _skinny().b200_weight_tensor_map(buf, _p(weight), ctypes.c_longlong(weight.shape[0]),
-                                              ctypes.c_longlong(weight.shape[1]), box_rows)
+        rc = _skinny().b200_weight_tensor_map(buf, weight, int(weight.shape[0]),
+                                              int(weight.shape[1]), box_rows)
         if rc != 0:
             raise KernelError(f"the TMA descriptor of a weight matrix could not be made (code {rc})")
         if len(_weight_maps) > 8192:
@@ -868,15 +874,15 @@ def skinny_linear(x, weight: torch.Tensor, mode: int = EPI_PLAIN_BF16, x_rows: O
     P.out = out.data_ptr()
     sms = _sm_count(dev)
     box = lib.b200_skinny_box_rows(mode, head_dim, n, sms)
-    rc = lib.b200_skinny_linear(_weight_map(weight, box), ctypes.byref(P), head_dim, sms, _stream())
+    rc = lib.b200_skinny_linear(_weight_map(weight, box), P, head_dim, sms, _stream())
     _ok(rc, "skinny_linear")
     return out
 
 
 def _few_row_out(m: int, n: int, mode: int, device) -> torch.Tensor:
     if mode == EPI_SWIGLU:
-        return torch.empty((m, n // 2), dtype=torch.bfloat16, device=device)
-    return torch.empty((m, n), dtype=torch.float32 if mode == EPI_PLAIN_F32 else torch.bfloat16, device=device)
+        return _empty((m, n // 2), torch.bfloat16, device)
+    return _empty((m, n), torch.float32 if mode == EPI_PLAIN_F32 else torch.bfloat16, device)
 
 
 class _StreamParams(ctypes.Structure):
@@ -891,7 +897,7 @@ class _StreamParams(ctypes.Structure):
 
 
 def _stream_lib(glu: str = "silu"):
-    lib = load_cuda_library("stream_linear.cu", _GLU_DEFINES[glu] or None)
+    lib = load_entry_points("stream_linear.cu", _GLU_DEFINES[glu] or None)
     if not getattr(lib, "_checked", False):
         if lib.b200_stream_params_size() != ctypes.sizeof(_StreamParams):
             raise KernelError("the parameter block of stream_linear.cu and its Python mirror differ")
@@ -992,7 +998,7 @@ def stream_linear(x, weight: torch.Tensor, mode: int = EPI_PLAIN_BF16, x_rows: O
         P.post_residual, P.post_sum_out, P.post_stats = (t.data_ptr() for t in norm_after)
     P.out, P.rw, P.ks, P.xd = out.data_ptr(), rw, ks, xd
     P.pair = stream_pair if pair is None else pair
-    rc = _stream_lib(glu).b200_stream_linear(ctypes.byref(P), _sm_count(src.device), _stream())
+    rc = _stream_lib(glu).b200_stream_linear(P, _sm_count(src.device), _stream())
     _ok(rc, "stream_linear")
     return out
 
@@ -1043,7 +1049,7 @@ def _single_lazy(x, weight, mode, x_rows, qkv, lazy) -> torch.Tensor:
             cols = _skinny().b200_skinny_tile_rows(EPI_PLAIN_BF16, 0, n, _sm_count(h.out.device))
         if 0 < cols <= 128:
             tiles = -(-n // cols)
-            stat_t = torch.empty((tiles, SKINNY_MAX_ROWS), dtype=torch.float32, device=h.out.device)
+            stat_t = _empty((tiles, SKINNY_MAX_ROWS), torch.float32, h.out.device)
             sum_out = pending.residual_out if pending.residual_out is not None else torch.empty_like(pending.residual)
             _flush_held((pending.residual, sum_out, stat_t))
             stats = (stat_t, tiles)
@@ -1090,11 +1096,11 @@ class _ChainOp(ctypes.Structure):
 
 
 def _chain_lib():
-    lib = load_cuda_library("linear_chain.cu")
+    lib = load_entry_points("linear_chain.cu")
     if not getattr(lib, "_checked", False):
         if lib.b200_chain_op_size() != ctypes.sizeof(_ChainOp):
             raise KernelError("the product block of linear_chain.cu and its Python mirror differ")
-        lib.b200_chain_scratch_floats.restype = ctypes.c_longlong
+        lib.library.b200_chain_scratch_floats.restype = ctypes.c_longlong
         lib._checked = True
     return lib
 
@@ -1109,8 +1115,8 @@ def _chain_map(weight: torch.Tensor, box_rows: int):
     buf = _chain_maps.get(key)
     if buf is None:
         buf = ctypes.create_string_buffer(128)
-        rc = _chain_lib().b200_chain_weight_map(buf, _p(weight), ctypes.c_longlong(weight.shape[0]),
-                                                ctypes.c_longlong(weight.shape[1]), box_rows)
+        rc = _chain_lib().b200_chain_weight_map(buf, weight, int(weight.shape[0]),
+                                                int(weight.shape[1]), box_rows)
         if rc != 0:
             raise KernelError(f"the TMA descriptor of a weight matrix could not be made (code {rc})")
         if len(_chain_maps) > 8192:
@@ -1128,7 +1134,7 @@ def _chain_buffers(device):
         if torch.cuda.is_current_stream_capturing():
             raise KernelError("the chain kernel's buffers must exist before a graph is captured")
         floats = int(_chain_lib().b200_chain_scratch_floats(CHAIN_MAX_ROWS, _sm_count(device)))
-        st = _chain_state[key] = dict(scratch=torch.empty(floats, dtype=torch.float32, device=device),
+        st = _chain_state[key] = dict(scratch=_empty((floats,), torch.float32, device),
                                       tickets=torch.zeros(_CHAIN_TICKETS, dtype=torch.int32, device=device),
                                       sync=torch.zeros(_chain_lib().b200_chain_sync_words(), dtype=torch.int32,
                                                        device=device))
@@ -1264,7 +1270,7 @@ def _chain_append(pending, src, rows_t, m, weight, mode, qkv) -> torch.Tensor:
                 # rounded sum and leaves the rows' sums of squares, so nobody has to read whole rows again
                 prev = ch.ops[made[0]]
                 tiles = _chain_lib().b200_chain_tiles(EPI_PLAIN_BF16, prev.N, 1)      # (narrow tiles are the most)
-                stats = torch.empty(tiles * CHAIN_MAX_ROWS, dtype=torch.float32, device=dev)
+                stats = _empty((tiles * CHAIN_MAX_ROWS,), torch.float32, dev)
                 sum_out = pending.residual_out if pending.residual_out is not None else torch.empty_like(res)
                 prev.stats_out, prev.stats_res_in, prev.stats_res_out = stats.data_ptr(), res.data_ptr(), sum_out.data_ptr()
                 op.stats_in = stats.data_ptr()
@@ -1304,9 +1310,9 @@ def _chain_append(pending, src, rows_t, m, weight, mode, qkv) -> torch.Tensor:
         op.k_cache, op.v_cache = (0 if kc is None else kc.data_ptr()), (0 if vc is None else vc.data_ptr())
         ch.keep.append(qkv)
     elif mode == EPI_SWIGLU:
-        out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=dev)
+        out = _empty((m, n // 2), torch.bfloat16, dev)
     else:
-        out = torch.empty((m, n), dtype=torch.float32 if mode == EPI_PLAIN_F32 else torch.bfloat16, device=dev)
+        out = _empty((m, n), torch.float32 if mode == EPI_PLAIN_F32 else torch.bfloat16, dev)
     op.out = out.data_ptr()
     ch.ops.append(op)
     ch.weights.append(weight)
@@ -1337,7 +1343,7 @@ def flush_chain() -> None:
         rows = max(ch.ops[i].M for i in group)
         for i in group:
             op, w = ch.ops[i], ch.weights[i]
-            op.narrow = lib.b200_chain_narrow(op.mode, op.N, op.K, rows, ctypes.c_longlong(chain_narrow_bytes))
+            op.narrow = lib.b200_chain_narrow(op.mode, op.N, op.K, rows, int(chain_narrow_bytes))
             op.box_rows = lib.b200_chain_box_rows(op.mode, op.narrow)
     for i, source in ch.stats_from.items():
         ch.ops[i].stats_tiles = lib.b200_chain_tiles(ch.ops[source].mode, ch.ops[source].N, ch.ops[source].narrow)
@@ -1349,8 +1355,8 @@ def flush_chain() -> None:
             block = (_ChainOp * len(ops_now))(*ops_now)
             maps = ctypes.create_string_buffer(b"".join(_chain_map(ch.weights[i], ch.ops[i].box_rows).raw for i in group),
                                                128 * len(ops_now))
-            rc = lib.b200_linear_chain(block, maps, len(ops_now), _p(st["scratch"]), _p(st["tickets"]), _p(st["sync"]),
-                                       _p(error_word(ch.device)), _p(chain_trace), chain_stages, sms, _stream())
+            rc = lib.b200_linear_chain(block, maps, len(ops_now), st["scratch"], st["tickets"], st["sync"],
+                                       error_word(ch.device), chain_trace, chain_stages, sms, _stream())
             _ok(rc, "linear_chain")
 
 
@@ -1409,8 +1415,8 @@ def _gemm_map(t: torch.Tensor):
     buf = _gemm_maps.get(key)
     if buf is None:
         buf = ctypes.create_string_buffer(128)
-        rc = load_cuda_library("gemm_tcgen05.cu").b200_gemm_tensor_map(buf, _p(t), ctypes.c_longlong(t.shape[0]),
-                                                                       ctypes.c_longlong(t.shape[1]))
+        rc = load_entry_points("gemm_tcgen05.cu").b200_gemm_tensor_map(buf, t, int(t.shape[0]),
+                                                                       int(t.shape[1]))
         if rc != 0:
             raise KernelError(f"the TMA descriptor of a matrix could not be made (code {rc})")
         if len(_gemm_maps) > 8192:
@@ -1447,14 +1453,14 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, mode: int = GEMM_PLAIN, glu: 
         raise KernelError("the tcgen05 product takes contiguous bfloat16 [M, K] and [N, K] with K a multiple of 8")
     m, k = x.shape
     n = weight.shape[0]
-    out = torch.empty((m, n // 2 if mode == GEMM_SWIGLU else n), dtype=torch.bfloat16, device=x.device)
+    out = _empty((m, n // 2 if mode == GEMM_SWIGLU else n), torch.bfloat16, x.device)
     a_map = ctypes.create_string_buffer(128)          # activations move: their descriptor is made per call
-    lib = load_cuda_library("gemm_tcgen05.cu", _GLU_DEFINES[glu] or None)
-    rc = lib.b200_gemm_tensor_map(a_map, _p(x), ctypes.c_longlong(m), ctypes.c_longlong(k))
+    lib = load_entry_points("gemm_tcgen05.cu", _GLU_DEFINES[glu] or None)
+    rc = lib.b200_gemm_tensor_map(a_map, x, int(m), int(k))
     if rc != 0:
         raise KernelError(f"the TMA descriptor of the activations could not be made (code {rc})")
-    rc = lib.b200_gemm_tcgen05(a_map, _gemm_map(weight), _p(out), m, n, k, mode, ctypes.c_float(limit), ctypes.c_float(alpha),
-                               _p(error_word(x.device)), _stream())
+    rc = lib.b200_gemm_tcgen05(a_map, _gemm_map(weight), out, m, n, k, mode, float(limit), float(alpha),
+                               error_word(x.device), _stream())
     _ok(rc, "gemm_tcgen05")
     return out
 
@@ -1469,8 +1475,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     m, k = a.shape
     n = w.shape[0]
     if out is None:
-        out = torch.empty((m, n), dtype=torch.float32, device=a.device)
-    rc = load_cuda_library("gemm_f32.cu").b200_gemm_f32(_p(a), _p(w), _p(out), m, n, k, _stream())
+        out = _empty((m, n), torch.float32, a.device)
+    rc = load_entry_points("gemm_f32.cu").b200_gemm_f32(a, w, out, m, n, k, _stream())
     _ok(rc, "gemm_f32")
     return out
 
@@ -1487,13 +1493,13 @@ def head_products(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
             or x.dtype != weight.dtype:
         raise KernelError("head_products takes x [heads, rows, k] and contiguous weights [heads, n, k] of one dtype")
     if out is None:
-        out = torch.empty((heads, rows, n), dtype=x.dtype, device=x.device)
+        out = _empty((heads, rows, n), x.dtype, x.device)
     elif tuple(out.shape) != (heads, rows, n) or out.stride(2) != 1 or out.dtype != x.dtype:
         raise KernelError("head_products: the output must be [heads, rows, n] with a unit inner stride")
     if x.dtype == torch.float32:
-        rc = load_cuda_library("gemm_f32.cu").b200_gemm_f32_batched(
-            _p(x), _p(weight), _p(out), rows, n, k, heads, x.stride(1), k, out.stride(1),
-            ctypes.c_longlong(x.stride(0)), ctypes.c_longlong(n * k), ctypes.c_longlong(out.stride(0)), _stream())
+        rc = load_entry_points("gemm_f32.cu").b200_gemm_f32_batched(
+            x, weight, out, rows, n, k, heads, x.stride(1), k, out.stride(1),
+            int(x.stride(0)), int(n * k), int(out.stride(0)), _stream())
         _ok(rc, "gemm_f32_batched")
         return out
     if x.dtype != torch.bfloat16:
@@ -1515,7 +1521,7 @@ def linear_columns(packed: torch.Tensor, column: int, weight: torch.Tensor, out_
     if packed.dtype == torch.float32:
         return cast(head_products(x.unsqueeze(0), weight.unsqueeze(0))[0], out_dtype)
     flush_chain()
-    return torch.mm(x, weight.t(), out_dtype=out_dtype) if out_dtype != packed.dtype else torch.mm(x, weight.t())
+    return torch.mm(x, weight.t(), out_dtype=out_dtype) if out_dtype != packed.dtype else _mm_t(x, weight)
 
 
 def block_products(u: torch.Tensor, gates: torch.Tensor) -> torch.Tensor:
@@ -1550,7 +1556,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
                 return few_row_linear(x, weight, mode, lazy=lazy)
         _cuda(x, weight)
         if out_dtype == torch.bfloat16:
-            return torch.mm(x, weight.t())
+            return _mm_t(x, weight)
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
     if weight.dtype == torch.float32:
         return cast(gemm_f32(cast(x, torch.float32), weight), out_dtype)
@@ -1562,10 +1568,10 @@ def argmax(logits: torch.Tensor) -> torch.Tensor:
     _cuda(logits)
     if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
         raise KernelError("argmax takes float32 logits [rows, vocab] with unit inner stride")
-    out = torch.empty(logits.shape[0], dtype=torch.int32, device=logits.device)
-    rc = load_cuda_library("sampling.cu").b200_argmax(_p(logits), ctypes.c_longlong(logits.stride(0)),
-                                                      logits.shape[0], logits.shape[1], _p(out),
-                                                      _p(error_word(logits.device)), _stream())
+    out = _empty((logits.shape[0],), torch.int32, logits.device)
+    rc = load_entry_points("sampling.cu").b200_argmax(logits, int(logits.stride(0)),
+                                                      logits.shape[0], logits.shape[1], out,
+                                                      error_word(logits.device), _stream())
     _ok(rc, "argmax")
     return out
 
@@ -1577,17 +1583,17 @@ def sample(logits: torch.Tensor, params: torch.Tensor, uniforms: Optional[torch.
         raise KernelError("sample takes float32 logits [rows, vocab] with unit inner stride")
     if params.numel() * params.element_size() != logits.shape[0] * 32:
         raise KernelError("sampling parameters must hold 32 bytes per row")
-    out = torch.empty(logits.shape[0], dtype=torch.int32, device=logits.device)
-    rc = load_cuda_library("sampling.cu").b200_sample(_p(logits), ctypes.c_longlong(logits.stride(0)),
-                                                      logits.shape[0], logits.shape[1], _p(params), _p(out),
-                                                      _p(uniforms), _p(error_word(logits.device)), _stream())
+    out = _empty((logits.shape[0],), torch.int32, logits.device)
+    rc = load_entry_points("sampling.cu").b200_sample(logits, int(logits.stride(0)),
+                                                      logits.shape[0], logits.shape[1], params, out,
+                                                      uniforms, error_word(logits.device), _stream())
     _ok(rc, "sample")
     return out
 
 
 # --------------------------------------------------------------------------- float32 residual stream, one-gain norms
 def _token_conv():
-    return load_cuda_library("token_conv.cu")
+    return load_entry_points("token_conv.cu")
 
 
 def _f32(*tensors: Optional[torch.Tensor]) -> None:
@@ -1611,9 +1617,9 @@ def residual_scale(x: torch.Tensor, y: Optional[torch.Tensor], gain: torch.Tenso
     _f32(x, gain)
     if x.dim() != 2 or (y is not None and y.shape != x.shape) or gain.numel() != 1:
         raise KernelError("residual_scale takes x and y [tokens, width] and one gain")
-    scale = torch.empty(x.shape[0], dtype=torch.float32, device=x.device) if want_scale else None
-    rc = _token_conv().b200_residual_scale(_p(x), _p(y), _code(y) if y is not None else F32, _p(gain),
-                                           ctypes.c_float(eps), _p(scale), x.shape[0], x.shape[1], _stream())
+    scale = _empty((x.shape[0],), torch.float32, x.device) if want_scale else None
+    rc = _token_conv().b200_residual_scale(x, y, _code(y) if y is not None else F32, gain,
+                                           float(eps), scale, x.shape[0], x.shape[1], _stream())
     _ok(rc, "residual_scale")
     return scale
 
@@ -1625,8 +1631,8 @@ def scaled_rows(x: torch.Tensor, scale: torch.Tensor, rows: Optional[torch.Tenso
     _f32(x, scale)
     _i32(rows)
     n = x.shape[0] if rows is None else rows.numel()
-    out = torch.empty((n, x.shape[1]), dtype=out_dtype, device=x.device)
-    rc = _token_conv().b200_scaled_rows(_p(out), _code(out), _p(x), _p(scale), _p(rows), n, x.shape[1], _stream())
+    out = _empty((n, x.shape[1]), out_dtype, x.device)
+    rc = _token_conv().b200_scaled_rows(out, _code(out), x, scale, rows, n, x.shape[1], _stream())
     _ok(rc, "scaled_rows")
     return out
 
@@ -1661,12 +1667,12 @@ def causal_taps(x: torch.Tensor, weight: Optional[torch.Tensor], state: Optional
         raise KernelError("the taps must be [channels, taps]")
     if taps > 1 and (state is None or tuple(state.shape[1:]) != (taps - 1, c)):
         raise KernelError("the state of a convolution must be [slots + 1, taps - 1, channels]")
-    out = torch.empty((x.shape[0], c), dtype=out_dtype, device=x.device)
-    src = ctypes.c_void_p(x.data_ptr() + column * x.element_size())
+    out = _empty((x.shape[0], c), out_dtype, x.device)
+    src = int(x.data_ptr() + column * x.element_size())
     rc = _token_conv().b200_causal_taps(
-        src, _code(x), x.shape[1], _p(scale), _p(weight), taps, c, _p(state), _p(ctx.row_of_token), _p(ctx.cu_q),
-        _p(ctx.prefix_len), _p(ctx.state_slots), _p(out), _code(out), c, int(bool(identity)), x.shape[0],
-        ctx.num_rows, int(bool(update_state)), _all_single(ctx), _p(bias), _p(out_bias), _stream())
+        src, _code(x), x.shape[1], scale, weight, taps, c, state, ctx.row_of_token, ctx.cu_q,
+        ctx.prefix_len, ctx.state_slots, out, _code(out), c, int(bool(identity)), x.shape[0],
+        ctx.num_rows, int(bool(update_state)), _all_single(ctx), bias, out_bias, _stream())
     _ok(rc, "causal_taps", 2 if update_state and taps > 1 and not _all_single(ctx) else 1)
     return out
 
@@ -1685,11 +1691,11 @@ def add_norm_taps_single(x: torch.Tensor, y: Optional[torch.Tensor], gain: torch
     _f32(x, gain, weight, state)
     if weight.shape[0] != x.shape[1] or (taps > 1 and tuple(state.shape[1:]) != (taps - 1, x.shape[1])):
         raise KernelError("the taps must be [channels, taps] and the state [slots + 1, taps - 1, channels]")
-    scale = torch.empty(x.shape[0], dtype=torch.float32, device=x.device)
-    out = torch.empty(x.shape, dtype=out_dtype, device=x.device)
+    scale = _empty((x.shape[0],), torch.float32, x.device)
+    out = _empty(x.shape, out_dtype, x.device)
     rc = _token_conv().b200_add_norm_taps_single(
-        _p(x), _p(y), _code(y) if y is not None else F32, _p(gain), ctypes.c_float(eps), _p(scale), _p(weight), taps,
-        x.shape[1], _p(state), _p(ctx.row_of_token), _p(ctx.cu_q), _p(ctx.prefix_len), _p(ctx.state_slots), _p(out),
+        x, y, _code(y) if y is not None else F32, gain, float(eps), scale, weight, taps,
+        x.shape[1], state, ctx.row_of_token, ctx.cu_q, ctx.prefix_len, ctx.state_slots, out,
         _code(out), int(bool(identity)), x.shape[0], _stream())
     if rc in (-2, -3):
         return None
@@ -1704,9 +1710,9 @@ def taps_state_update(x: torch.Tensor, taps: int, channels: int, state: torch.Te
     _cuda(x, state)
     _contig(x, state)
     _f32(state)
-    at = ctypes.c_void_p(x.data_ptr() + column * x.element_size())
-    rc = _token_conv().b200_taps_state_update(at, _code(x), x.shape[1], None, taps, channels, _p(state),
-                                              _p(ctx.cu_q), _p(ctx.prefix_len), _p(ctx.state_slots), ctx.num_rows,
+    at = int(x.data_ptr() + column * x.element_size())
+    rc = _token_conv().b200_taps_state_update(at, _code(x), x.shape[1], None, taps, channels, state,
+                                              ctx.cu_q, ctx.prefix_len, ctx.state_slots, ctx.num_rows,
                                               0, _stream())
     _ok(rc, "taps_state_update")
 
@@ -1737,12 +1743,12 @@ def conv_qkv_post(x: torch.Tensor, conv_weight: Optional[torch.Tensor], state: O
     if inv_freq is not None and inv_freq.numel() * 2 != rot_dim:
         raise KernelError("one frequency for every rotated pair is needed")
     page_size = k_cache.shape[2]
-    rc = load_cuda_library("conv_qkv_post.cu").b200_conv_qkv_post(
-        _p(x), _code(x), x.shape[1], _p(conv_weight), taps, _p(state), _p(ctx.row_of_token), _p(ctx.cu_q),
-        _p(ctx.prefix_len), _p(ctx.state_slots), _p(q_out), _p(k_cache), _p(v_cache), _p(inv_freq),
-        int(rot_dim if inv_freq is not None else 0), _p(ctx.positions), _p(slots), num_heads, num_kv_heads, head_dim,
-        v_head_dim, page_size, ctypes.c_longlong(k_cache.shape[0] * page_size), _p(vmix), _p(v_first), int(v_mode),
-        x.shape[0], ctx.num_rows, _all_single(ctx), _p(error_word(x.device)), _stream())
+    rc = load_entry_points("conv_qkv_post.cu").b200_conv_qkv_post(
+        x, _code(x), x.shape[1], conv_weight, taps, state, ctx.row_of_token, ctx.cu_q,
+        ctx.prefix_len, ctx.state_slots, q_out, k_cache, v_cache, inv_freq,
+        int(rot_dim if inv_freq is not None else 0), ctx.positions, slots, num_heads, num_kv_heads, head_dim,
+        v_head_dim, page_size, int(k_cache.shape[0] * page_size), vmix, v_first, int(v_mode),
+        x.shape[0], ctx.num_rows, _all_single(ctx), error_word(x.device), _stream())
     _ok(rc, "conv_qkv_post", 2 if taps > 1 and not _all_single(ctx) else 1)
 
 
@@ -1764,28 +1770,28 @@ def retention(x: torch.Tensor, state: torch.Tensor, decay: torch.Tensor, inv_fre
     if x.shape[1] < heads * (2 * head_dim + v_head_dim) or tuple(state.shape[1:]) != (heads, head_dim, v_head_dim) \
             or decay.numel() != heads:
         raise KernelError("retention: sizes of the projection, the state or the decays do not fit")
-    o = torch.empty((x.shape[0], heads * v_head_dim), dtype=torch.float32, device=x.device)
-    lib = load_cuda_library("retention.cu")
+    o = _empty((x.shape[0], heads * v_head_dim), torch.float32, x.device)
+    lib = load_entry_points("retention.cu")
     tokens = x.shape[0]
     longest = int(getattr(ctx, "max_q_len", 0) or tokens)
     fits = head_dim <= 128 and v_head_dim <= 128 and head_dim % 4 == 0 and v_head_dim % 8 == 0 and x.shape[1] % 8 == 0
     if (chunked if chunked is not None else longest >= RETENTION_CHUNKED_FROM) and fits:
         # long rows: the state is carried chunk by chunk and every chunk's outputs are computed on their own
         max_chunks = tokens // 64 + ctx.num_rows
-        qf = torch.empty((2, tokens, heads * head_dim), dtype=torch.float32, device=x.device)
-        before = torch.empty((max_chunks, heads, head_dim, v_head_dim), dtype=torch.float32, device=x.device)
-        chunk_base = torch.empty(ctx.num_rows + 1, dtype=torch.int32, device=x.device)
+        qf = _empty((2, tokens, heads * head_dim), torch.float32, x.device)
+        before = _empty((max_chunks, heads, head_dim, v_head_dim), torch.float32, x.device)
+        chunk_base = _empty((ctx.num_rows + 1,), torch.int32, x.device)
         rc = lib.b200_retention_chunked(
-            _p(x), _code(x), x.shape[1], _p(o), _p(state), _p(decay), _p(inv_freq),
-            int(rot_dim if inv_freq is not None else 0), ctypes.c_float(k_scale), _p(ctx.positions), _p(ctx.cu_q),
-            _p(ctx.prefix_len), _p(ctx.state_slots), ctx.num_rows, heads, head_dim, v_head_dim, tokens, max_chunks,
-            _p(qf[0]), _p(qf[1]), _p(before), _p(chunk_base), _stream())
+            x, _code(x), x.shape[1], o, state, decay, inv_freq,
+            int(rot_dim if inv_freq is not None else 0), float(k_scale), ctx.positions, ctx.cu_q,
+            ctx.prefix_len, ctx.state_slots, ctx.num_rows, heads, head_dim, v_head_dim, tokens, max_chunks,
+            qf[0], qf[1], before, chunk_base, _stream())
         _ok(rc, "retention_chunked", 4)
         return o
     rc = lib.b200_retention(
-        _p(x), _code(x), x.shape[1], _p(o), _p(state), _p(decay), _p(inv_freq),
-        int(rot_dim if inv_freq is not None else 0), ctypes.c_float(k_scale), _p(ctx.positions), _p(ctx.cu_q),
-        _p(ctx.prefix_len), _p(ctx.state_slots), ctx.num_rows, heads, head_dim, v_head_dim, _stream())
+        x, _code(x), x.shape[1], o, state, decay, inv_freq,
+        int(rot_dim if inv_freq is not None else 0), float(k_scale), ctx.positions, ctx.cu_q,
+        ctx.prefix_len, ctx.state_slots, ctx.num_rows, heads, head_dim, v_head_dim, _stream())
     _ok(rc, "retention")
     return o
 
@@ -1815,11 +1821,11 @@ def state_head_blocks(head_dim: int) -> int:
 
 def _state_scan(form: "LinearStateForm"):
     """The scan of a form: the build for decays per key channel, or one per range of head sizes for one decay a head."""
-    return load_cuda_library("state_scan.cu", {"STATE_HEAD_BLOCKS": state_head_blocks(form.d)} if form.head_decay else None)
+    return load_entry_points("state_scan.cu", {"STATE_HEAD_BLOCKS": state_head_blocks(form.d)} if form.head_decay else None)
 
 
 def _linear_state():
-    lib = load_cuda_library("linear_state.cu")
+    lib = load_entry_points("linear_state.cu")
     if not getattr(lib, "_checked", False):
         if lib.b200_linear_state_shape_size() != ctypes.sizeof(_LinearStateShape) or \
                 lib.b200_state_decode_params_size() != ctypes.sizeof(_StateDecodeParams):
@@ -1898,16 +1904,16 @@ def state_decode(form: LinearStateForm, x: torch.Tensor, conv: Optional[torch.Te
             gate_column + (g2.shape[1] if g2 is not None else form.heads * form.dv) > width or \
             (a2 is not None and (a2.dtype != x.dtype or a2.shape[0] != form.heads * form.d or a_column + a2.shape[1] > width)):
         raise KernelError("state_decode: the low-rank products, the norm or the gate do not fit")
-    out = torch.empty((x.shape[0], form.heads * form.dv), dtype=x.dtype, device=x.device)
+    out = _empty((x.shape[0], form.heads * form.dv), x.dtype, x.device)
     own = form.heads == form.kv_heads
     params = _StateDecodeParams(a2.data_ptr() if a2 is not None else None, g2.data_ptr() if g2 is not None else None,
                                 int(a_column), a2.shape[1] if a2 is not None else 0,
                                 int(gate_column), g2.shape[1] if g2 is not None else 0, int(g2 is None), norm.data_ptr(),
                                 float(eps), int(own), 0)
-    at = ctypes.c_void_p(x.data_ptr() + column * x.element_size())
+    at = int(x.data_ptr() + column * x.element_size())
     rc = _linear_state().b200_state_decode(
-        at, _code(x), x.shape[1], _p(conv), taps, _p(conv_state), _p(ctx.row_of_token), _p(ctx.cu_q), _p(ctx.prefix_len),
-        _p(ctx.state_slots), ctypes.byref(form.shape), ctypes.byref(params), _p(out), _p(state), x.shape[0], _stream())
+        at, _code(x), x.shape[1], conv, taps, conv_state, ctx.row_of_token, ctx.cu_q, ctx.prefix_len,
+        ctx.state_slots, form.shape, params, out, state, x.shape[0], _stream())
     if rc == -2:
         return None
     _ok(rc, "state_decode")
@@ -1928,21 +1934,21 @@ def state_recurrence(form: LinearStateForm, x: torch.Tensor, z: Optional[torch.T
     tokens, dev = x.shape[0], x.device
     if (z is None) != form.head_decay or (z is not None and tuple(z.shape) != (tokens, form.heads * form.d)):
         raise KernelError("state_recurrence: one pre-activation for every head and key channel is needed")
-    qf = torch.empty((2, tokens, form.kv_heads * form.d), dtype=torch.float32, device=dev)
-    vf = torch.empty((tokens, form.heads * form.dv), dtype=torch.float32, device=dev)
-    gf = torch.empty((tokens, form.heads * (1 if form.head_decay else form.d)), dtype=torch.float32, device=dev)
-    beta = torch.empty((tokens, form.heads), dtype=torch.float32, device=dev) if form.delta else None
+    qf = _empty((2, tokens, form.kv_heads * form.d), torch.float32, dev)
+    vf = _empty((tokens, form.heads * form.dv), torch.float32, dev)
+    gf = _empty((tokens, form.heads * (1 if form.head_decay else form.d)), torch.float32, dev)
+    beta = _empty((tokens, form.heads), torch.float32, dev) if form.delta else None
     lib = _linear_state()
-    at = ctypes.c_void_p(x.data_ptr() + column * x.element_size())
+    at = int(x.data_ptr() + column * x.element_size())
     rc = lib.b200_state_prepare(
-        at, _code(x), x.shape[1], _p(conv), taps, _p(conv_state), _p(ctx.row_of_token), _p(ctx.cu_q), _p(ctx.prefix_len),
-        _p(ctx.state_slots), ctypes.byref(form.shape), _p(z), _p(qf[0]), _p(qf[1]), _p(vf), _p(gf), _p(beta), tokens, _stream())
+        at, _code(x), x.shape[1], conv, taps, conv_state, ctx.row_of_token, ctx.cu_q, ctx.prefix_len,
+        ctx.state_slots, form.shape, z, qf[0], qf[1], vf, gf, beta, tokens, _stream())
     _ok(rc, "state_prepare")
     if taps > 1:
         taps_state_update(x, taps, form.channels, conv_state, ctx, column)
-    o = torch.empty((tokens, form.heads * form.dv), dtype=torch.float32, device=dev)
-    rc = _state_scan(form).b200_state_scan(_p(qf[0]), _p(qf[1]), _p(vf), _p(gf), _p(beta), _p(o), _p(state), _p(ctx.cu_q),
-                             _p(ctx.prefix_len), _p(ctx.state_slots), ctx.num_rows, form.heads, form.kv_heads, form.d,
+    o = _empty((tokens, form.heads * form.dv), torch.float32, dev)
+    rc = _state_scan(form).b200_state_scan(qf[0], qf[1], vf, gf, beta, o, state, ctx.cu_q,
+                             ctx.prefix_len, ctx.state_slots, ctx.num_rows, form.heads, form.kv_heads, form.d,
                              form.dv, int(form.head_decay), _stream())
     _ok(rc, "state_scan")
     return o
@@ -1967,27 +1973,27 @@ def gated_lru(u: torch.Tensor, packed: torch.Tensor, y_column: int, gates: torch
             or any(t.numel() != width for t in (r_bias, i_bias, lam, y_bias)) or tuple(state.shape[1:]) != (width,) or \
             packed.shape[0] != tokens or y_column + width > packed.shape[1]:
         raise KernelError("gated_lru: sizes or dtypes do not fit")
-    lib = load_cuda_library("gated_lru.cu")
+    lib = load_entry_points("gated_lru.cu")
     out = torch.empty_like(u)
-    y = ctypes.c_void_p(packed.data_ptr() + y_column * packed.element_size())
+    y = int(packed.data_ptr() + y_column * packed.element_size())
     single = _all_single(ctx)
-    common = (_p(r_bias), _p(i_bias), _p(lam), _p(y_bias), width, blocks, _p(state))
+    common = (r_bias, i_bias, lam, y_bias, width, blocks, state)
     if single and tokens <= LRU_FEW_ROWS:
-        rc = lib.b200_lru_few(_p(u), y, _code(u), packed.shape[1], _p(gates), *common, _p(ctx.prefix_len),
-                              _p(ctx.state_slots), _p(out), tokens, _stream())
+        rc = lib.b200_lru_few(u, y, _code(u), packed.shape[1], gates, *common, ctx.prefix_len,
+                              ctx.state_slots, out, tokens, _stream())
         _ok(rc, "lru_few")
         return out
     pre = block_products(u, gates)
     if single:
-        rc = lib.b200_lru_rows(_p(u), y, _code(u), packed.shape[1], _p(pre), *common, _p(ctx.prefix_len),
-                               _p(ctx.state_slots), _p(out), tokens, _stream())
+        rc = lib.b200_lru_rows(u, y, _code(u), packed.shape[1], pre, *common, ctx.prefix_len,
+                               ctx.state_slots, out, tokens, _stream())
         _ok(rc, "lru_rows")
         return out
     windows = -(-tokens // int(lib.b200_lru_window()))
-    win = torch.empty((3, windows, width), dtype=torch.float32, device=u.device)
-    start = torch.empty((ctx.num_rows, width), dtype=torch.float32, device=u.device)
-    rc = lib.b200_lru_scan(_p(u), y, _code(u), packed.shape[1], _p(pre), *common, _p(ctx.row_of_token), _p(ctx.cu_q),
-                           _p(ctx.prefix_len), _p(ctx.state_slots), _p(win[0]), _p(win[1]), _p(win[2]), _p(start), _p(out),
+    win = _empty((3, windows, width), torch.float32, u.device)
+    start = _empty((ctx.num_rows, width), torch.float32, u.device)
+    rc = lib.b200_lru_scan(u, y, _code(u), packed.shape[1], pre, *common, ctx.row_of_token, ctx.cu_q,
+                           ctx.prefix_len, ctx.state_slots, win[0], win[1], win[2], start, out,
                            tokens, ctx.num_rows, _stream())
     _ok(rc, "lru_scan", 3)
     return out
@@ -1995,7 +2001,7 @@ def gated_lru(u: torch.Tensor, packed: torch.Tensor, y_column: int, gates: torch
 
 # --------------------------------------------------------------------------- gates and PolyNorm
 def _gated():
-    return load_cuda_library("gated.cu")
+    return load_entry_points("gated.cu")
 
 
 def poly_norm(z: torch.Tensor, coef: torch.Tensor, eps: float) -> torch.Tensor:
@@ -2006,7 +2012,7 @@ def poly_norm(z: torch.Tensor, coef: torch.Tensor, eps: float) -> torch.Tensor:
     if coef.numel() != 4 or z.dim() != 2:
         raise KernelError("poly_norm takes rows and four coefficients")
     out = torch.empty_like(z)
-    rc = _gated().b200_poly_norm(_p(out), _p(z), _p(coef), ctypes.c_float(eps), z.shape[0], z.shape[1], _code(z),
+    rc = _gated().b200_poly_norm(out, z, coef, float(eps), z.shape[0], z.shape[1], _code(z),
                                  _stream())
     _ok(rc, "poly_norm")
     return out
@@ -2024,10 +2030,10 @@ def head_unit_norm_gate(o: torch.Tensor, packed: torch.Tensor, gate_column: int,
         raise KernelError("head_unit_norm_gate: an unknown gate, or a weight that is not a head's size")
     if packed.shape[1] < gate_column + heads * v_head_dim or o.shape[1] != heads * v_head_dim:
         raise KernelError("head_unit_norm_gate: the gate's columns do not fit")
-    out = torch.empty((o.shape[0], o.shape[1]), dtype=packed.dtype, device=o.device)
-    at = ctypes.c_void_p(packed.data_ptr() + gate_column * packed.element_size())
-    rc = _gated().b200_head_unit_norm_gate(_p(out), _p(o), at, packed.shape[1], o.shape[0], heads, v_head_dim,
-                                           ctypes.c_float(eps), _p(weight), int(gate == "sigmoid"), _code(packed),
+    out = _empty((o.shape[0], o.shape[1]), packed.dtype, o.device)
+    at = int(packed.data_ptr() + gate_column * packed.element_size())
+    rc = _gated().b200_head_unit_norm_gate(out, o, at, packed.shape[1], o.shape[0], heads, v_head_dim,
+                                           float(eps), weight, int(gate == "sigmoid"), _code(packed),
                                            _stream())
     _ok(rc, "head_unit_norm_gate")
     return out
@@ -2041,7 +2047,7 @@ def sigmoid_gate_mul(a: torch.Tensor, packed: torch.Tensor, gate_column: int, pe
     if per <= 0 or a.shape[1] % per or a.dtype != packed.dtype or packed.shape[1] < gate_column + a.shape[1] // per:
         raise KernelError("sigmoid_gate_mul: dtype or columns do not fit")
     gate = packed.view(-1)[gate_column:]
-    rc = _gated().b200_sigmoid_gate_mul(_p(a), _p(a), ctypes.c_void_p(gate.data_ptr()), packed.shape[1], a.shape[0],
+    rc = _gated().b200_sigmoid_gate_mul(a, a, int(gate.data_ptr()), packed.shape[1], a.shape[0],
                                         a.shape[1], int(per), _code(a), _stream())
     _ok(rc, "sigmoid_gate_mul")
     return a
@@ -2059,8 +2065,8 @@ def activate(x: torch.Tensor, act: str, columns: Optional[int] = None, in_place:
     if act not in ACTIVATIONS or x.dim() != 2:
         raise KernelError(f"activation {act!r} is refused: {sorted(ACTIVATIONS)} on [tokens, width]")
     c = int(columns if columns is not None else x.shape[1])
-    out = x if in_place else torch.empty((x.shape[0], c), dtype=x.dtype, device=x.device)
-    rc = _gated().b200_activate_columns(_p(out), out.shape[1], _p(x), x.shape[1], x.shape[0], c, ACTIVATIONS[act],
+    out = x if in_place else _empty((x.shape[0], c), x.dtype, x.device)
+    rc = _gated().b200_activate_columns(out, out.shape[1], x, x.shape[1], x.shape[0], c, ACTIVATIONS[act],
                                         _code(x), _stream())
     _ok(rc, "activate_columns")
     return out
@@ -2074,10 +2080,10 @@ def row_norm_gate(o: torch.Tensor, weight: torch.Tensor, packed: torch.Tensor, g
     _f32(o, weight)
     if packed.shape[1] < gate_column + o.shape[1] or weight.numel() != o.shape[1]:
         raise KernelError("row_norm_gate: the gate's columns or the weight do not fit")
-    out = torch.empty(o.shape, dtype=packed.dtype, device=o.device)
+    out = _empty(o.shape, packed.dtype, o.device)
     gate = packed.view(-1)[gate_column:]
-    rc = _gated().b200_row_norm_gate(_p(out), _p(o), _p(weight), ctypes.c_void_p(gate.data_ptr()), packed.shape[1],
-                                     o.shape[0], o.shape[1], ctypes.c_float(eps), _code(packed), _stream())
+    rc = _gated().b200_row_norm_gate(out, o, weight, int(gate.data_ptr()), packed.shape[1],
+                                     o.shape[0], o.shape[1], float(eps), _code(packed), _stream())
     _ok(rc, "row_norm_gate")
     return out
 
@@ -2087,7 +2093,7 @@ def tanh_cap(z: torch.Tensor, cap: float) -> torch.Tensor:
     _cuda(z)
     _contig(z)
     _f32(z)
-    rc = _gated().b200_tanh_cap(_p(z), ctypes.c_longlong(z.numel()), ctypes.c_float(cap), _stream())
+    rc = _gated().b200_tanh_cap(z, int(z.numel()), float(cap), _stream())
     _ok(rc, "tanh_cap")
     return z
 
@@ -2121,10 +2127,10 @@ def stream_step(streams: torch.Tensor, norm_weight: torch.Tensor, offset: float,
     if read_in is not None and read_in.numel() != s:
         raise KernelError("stream_step: one read coefficient per stream")
     n = tokens if rows is None else rows.numel()
-    out = torch.empty((n, width), dtype=out_dtype, device=streams.device)
-    rc = load_cuda_library("residual_streams.cu").b200_stream_step(
-        _p(streams), s, _p(start), _p(y), _code(y) if y is not None else F32, _p(before), _p(read_in), _p(norm_weight),
-        ctypes.c_float(offset), ctypes.c_float(eps), _p(rows), _p(out), _code(out), n, width, int(bool(store)), _stream())
+    out = _empty((n, width), out_dtype, streams.device)
+    rc = load_entry_points("residual_streams.cu").b200_stream_step(
+        streams, s, start, y, _code(y) if y is not None else F32, before, read_in, norm_weight,
+        float(offset), float(eps), rows, out, _code(out), n, width, int(bool(store)), _stream())
     _ok(rc, "stream_step")
     return out
 
@@ -2170,12 +2176,12 @@ def heads_prepare(x: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor, v
     if inv_freq is not None and inv_freq.numel() * 2 != rot_dims:
         raise KernelError("one frequency for every rotated pair is needed")
     page_size = k_cache.shape[2]
-    rc = load_cuda_library("attention_prepare.cu").b200_heads_prepare(
-        _p(x), _code(x), x.shape[1], _p(bias), _p(q_weight), _p(k_weight), ctypes.c_float(eps), _p(inv_freq),
-        int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), _p(positions), _p(slots), x.shape[0],
-        num_heads, num_kv_heads, head_dim, v_head_dim, flags, maps, ctypes.c_float(rot_gain), page_size,
-        ctypes.c_longlong(k_cache.shape[0] * page_size), _p(q_out), _p(k_cache), _p(v_cache),
-        _p(error_word(x.device)), _stream())
+    rc = load_entry_points("attention_prepare.cu").b200_heads_prepare(
+        x, _code(x), x.shape[1], bias, q_weight, k_weight, float(eps), inv_freq,
+        int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), positions, slots, x.shape[0],
+        num_heads, num_kv_heads, head_dim, v_head_dim, flags, maps, float(rot_gain), page_size,
+        int(k_cache.shape[0] * page_size), q_out, k_cache, v_cache,
+        error_word(x.device), _stream())
     _ok(rc, "heads_prepare")
 
 
@@ -2208,12 +2214,12 @@ def joint_heads_prepare(x: torch.Tensor, q_out: torch.Tensor, k_cache: Optional[
         raise KernelError("joint_heads_prepare: bias or norm weights of the wrong size")
     if inv_freq is not None and inv_freq.numel() * 2 != rot_dims:
         raise KernelError("one frequency for every rotated pair is needed")
-    rc = load_cuda_library("attention_prepare.cu").b200_joint_heads_prepare(
-        _p(x), _code(x), x.shape[1], _p(bias), _p(q_weight), _p(k_weight if has_kv else None), ctypes.c_float(eps),
-        _p(inv_freq), int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), _p(positions),
-        _p(slots if has_kv else None), x.shape[0], num_heads, num_kv_heads, head_dim, v_head_dim, int(bool(has_kv)),
-        page_size, ctypes.c_longlong(cache_slots), _p(q_out), _p(k_cache if has_kv else None),
-        _p(v_cache if has_kv else None), _p(error_word(x.device)), _stream())
+    rc = load_entry_points("attention_prepare.cu").b200_joint_heads_prepare(
+        x, _code(x), x.shape[1], bias, q_weight, k_weight if has_kv else None, float(eps),
+        inv_freq, int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), positions,
+        slots if has_kv else None, x.shape[0], num_heads, num_kv_heads, head_dim, v_head_dim, int(bool(has_kv)),
+        page_size, int(cache_slots), q_out, k_cache if has_kv else None,
+        v_cache if has_kv else None, error_word(x.device), _stream())
     _ok(rc, "joint_heads_prepare")
 
 
@@ -2248,11 +2254,11 @@ def latent_prepare(x: torch.Tensor, q_lat: torch.Tensor, q_out: torch.Tensor, k_
     if inv_freq is not None and inv_freq.numel() * 2 != rot_dims:
         raise KernelError("one frequency for every rotated pair is needed")
     page_size = k_cache.shape[2]
-    rc = load_cuda_library("attention_prepare.cu").b200_latent_prepare(
-        _p(x), _code(x), x.shape[1], ctypes.c_void_p(down.data_ptr()), down.stride(0), _p(q_lat), _p(latent_weight), ctypes.c_float(eps), _p(inv_freq),
-        int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), _p(positions), _p(slots), tokens,
-        num_heads, head_dim, rot_dim, latent_dim, page_size, ctypes.c_longlong(k_cache.shape[0] * page_size),
-        _p(q_out), _p(k_cache), _p(v_cache), _p(error_word(x.device)), _stream())
+    rc = load_entry_points("attention_prepare.cu").b200_latent_prepare(
+        x, _code(x), x.shape[1], int(down.data_ptr()), down.stride(0), q_lat, latent_weight, float(eps), inv_freq,
+        int(rot_dims if inv_freq is not None else 0), int(bool(interleaved)), positions, slots, tokens,
+        num_heads, head_dim, rot_dim, latent_dim, page_size, int(k_cache.shape[0] * page_size),
+        q_out, k_cache, v_cache, error_word(x.device), _stream())
     _ok(rc, "latent_prepare")
 
 
@@ -2264,9 +2270,9 @@ def columns_rms_norm(x: torch.Tensor, width: int, weight: torch.Tensor, eps: flo
     _f32(weight)
     if x.dim() != 2 or x.shape[1] < width or weight.numel() != width:
         raise KernelError("columns_rms_norm: the rows are too narrow or the weight does not fit")
-    out = torch.empty((x.shape[0], width), dtype=x.dtype, device=x.device)
-    rc = load_cuda_library("attention_prepare.cu").b200_columns_rms_norm(
-        _p(x), _code(x), x.shape[1], _p(weight), ctypes.c_float(eps), x.shape[0], int(width), _p(out), _stream())
+    out = _empty((x.shape[0], width), x.dtype, x.device)
+    rc = load_entry_points("attention_prepare.cu").b200_columns_rms_norm(
+        x, _code(x), x.shape[1], weight, float(eps), x.shape[0], int(width), out, _stream())
     _ok(rc, "columns_rms_norm")
     return out
 
@@ -2284,13 +2290,13 @@ def _experts_buffers(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
     if gate_up.dtype != x.dtype or down.dtype != x.dtype or tuple(down.shape) != (experts, width, ff) \
             or gate_up.shape[2] != width:
         raise KernelError(f"{what}: sizes or dtypes do not fit")
-    lib = load_cuda_library("experts.cu")
-    lib.b200_expert_route_ints.restype = ctypes.c_longlong
+    lib = load_entry_points("experts.cu")
+    lib.library.b200_expert_route_ints.restype = ctypes.c_longlong
     pairs = tokens * top
-    route = torch.empty(int(lib.b200_expert_route_ints(tokens, top, experts)), dtype=torch.int32, device=x.device)
-    h = torch.empty((pairs, ff), dtype=x.dtype, device=x.device)
-    y = torch.empty((pairs, width), dtype=torch.float32, device=x.device)
-    out = torch.empty((tokens, width), dtype=torch.float32, device=x.device)
+    route = _empty((int(lib.library.b200_expert_route_ints(tokens, top, experts)),), torch.int32, x.device)
+    h = _empty((pairs, ff), x.dtype, x.device)
+    y = _empty((pairs, width), torch.float32, x.device)
+    out = _empty((tokens, width), torch.float32, x.device)
     return lib, experts, ff, pairs, route, h, y, out
 
 
@@ -2316,14 +2322,14 @@ def table_experts(x: torch.Tensor, token_ids: torch.Tensor, table: torch.Tensor,
         raise KernelError("table_experts: sizes or dtypes do not fit")
     lib, experts, ff, pairs, route, h, y, out = _experts_buffers(x, gate_up, down, top, "table_experts")
     if _experts_on_tcgen05(x, ff, pairs, tensor_memory):
-        xs = torch.empty((pairs, width), dtype=x.dtype, device=x.device)
-        rc = load_cuda_library("experts_tcgen05.cu").b200_table_experts_tcgen05(
-            _p(x), _p(token_ids), _p(table), vocab, top, experts, _p(gate_up), _p(down), tokens, width, ff, _p(xs),
-            _p(h), _p(y), _p(route), _p(out), _p(error_word(x.device)), _stream())
+        xs = _empty((pairs, width), x.dtype, x.device)
+        rc = load_entry_points("experts_tcgen05.cu").b200_table_experts_tcgen05(
+            x, token_ids, table, vocab, top, experts, gate_up, down, tokens, width, ff, xs,
+            h, y, route, out, error_word(x.device), _stream())
         _ok(rc, "table_experts_tcgen05", 5)
         return out
-    rc = lib.b200_table_experts(_p(x), _code(x), _p(token_ids), _p(table), vocab, top, experts, _p(gate_up), _p(down),
-                                tokens, width, ff, _p(h), _p(y), _p(route), _p(out), _p(error_word(x.device)), _stream())
+    rc = lib.b200_table_experts(x, _code(x), token_ids, table, vocab, top, experts, gate_up, down,
+                                tokens, width, ff, h, y, route, out, error_word(x.device), _stream())
     _ok(rc, "table_experts", 4)
     return out
 
@@ -2348,13 +2354,13 @@ def expert_router(x: torch.Tensor, weight: torch.Tensor, top: int, groups: int =
             (correction is not None and correction.numel() != experts) or \
             (gate is not None and (gate.numel() != width or gate.dtype != weight.dtype)):
         raise KernelError("expert_router: the router's matrix, correction or gate does not fit, or unknown scores")
-    choice = torch.empty((tokens, top), dtype=torch.int32, device=x.device)
-    gains = torch.empty((tokens, top), dtype=torch.float32, device=x.device)
-    gate_out = torch.empty((tokens,), dtype=torch.float32, device=x.device) if gate is not None else None
-    rc = load_cuda_library("experts.cu").b200_expert_router(
-        _p(x), _code(x), _p(weight), _code(weight), tokens, width, experts, int(groups), int(keep), int(top),
-        int(scores == "sigmoid"), int(bool(renormalize)), _p(correction), int(group_members),
-        ctypes.c_float(gain_scale), _p(gate), _p(gate_out), _p(choice), _p(gains), _stream())
+    choice = _empty((tokens, top), torch.int32, x.device)
+    gains = _empty((tokens, top), torch.float32, x.device)
+    gate_out = _empty((tokens,), torch.float32, x.device) if gate is not None else None
+    rc = load_entry_points("experts.cu").b200_expert_router(
+        x, _code(x), weight, _code(weight), tokens, width, experts, int(groups), int(keep), int(top),
+        int(scores == "sigmoid"), int(bool(renormalize)), correction, int(group_members),
+        float(gain_scale), gate, gate_out, choice, gains, _stream())
     _ok(rc, "expert_router")
     return (choice, gains) if gate is None else (choice, gains, gate_out)
 
@@ -2383,18 +2389,18 @@ def routed_experts(x: torch.Tensor, choice: torch.Tensor, gains: torch.Tensor, g
     lib, experts, ff, pairs, route, h, y, out = _experts_buffers(x, gate_up, down, top, "routed_experts")
     add_code = _code(add) if add is not None else F32
     if _experts_on_tcgen05(x, ff, pairs, tensor_memory):
-        xs = torch.empty((pairs, width), dtype=x.dtype, device=x.device)
-        rc = load_cuda_library("experts_tcgen05.cu").b200_routed_experts_tcgen05(
-            _p(x), _p(choice), _p(gains), top, experts, _p(gate_up), _p(down), tokens, width, ff, GLU_KINDS[glu],
-            ctypes.c_float(limit), ctypes.c_float(alpha), _p(add), add_code, _p(add_scale), int(bool(gains_on_input)), _p(xs),
-            _p(h), _p(y), _p(route), _p(out),
-            _p(error_word(x.device)), _stream())
+        xs = _empty((pairs, width), x.dtype, x.device)
+        rc = load_entry_points("experts_tcgen05.cu").b200_routed_experts_tcgen05(
+            x, choice, gains, top, experts, gate_up, down, tokens, width, ff, GLU_KINDS[glu],
+            float(limit), float(alpha), add, add_code, add_scale, int(bool(gains_on_input)), xs,
+            h, y, route, out,
+            error_word(x.device), _stream())
         _ok(rc, "routed_experts_tcgen05", 5)
         return out
-    rc = lib.b200_routed_experts(_p(x), _code(x), _p(choice), _p(gains), top, experts, _p(gate_up), _p(down), tokens,
-                                 width, ff, GLU_KINDS[glu], ctypes.c_float(limit), ctypes.c_float(alpha), _p(add),
-                                 add_code, _p(add_scale), int(bool(gains_on_input)), _p(h), _p(y), _p(route), _p(out),
-                                 _p(error_word(x.device)),
+    rc = lib.b200_routed_experts(x, _code(x), choice, gains, top, experts, gate_up, down, tokens,
+                                 width, ff, GLU_KINDS[glu], float(limit), float(alpha), add,
+                                 add_code, add_scale, int(bool(gains_on_input)), h, y, route, out,
+                                 error_word(x.device),
                                  _stream())
     _ok(rc, "routed_experts", 4)
     return out
@@ -2407,9 +2413,9 @@ def head_difference(a: torch.Tensor, heads: int, v_head_dim: int, lam: float, ga
     _contig(a)
     if a.shape[1] != heads * 2 * v_head_dim:
         raise KernelError("head_difference: two outputs a head are needed")
-    out = torch.empty((a.shape[0], heads * v_head_dim), dtype=a.dtype, device=a.device)
-    rc = _gated().b200_head_difference(_p(out), _p(a), ctypes.c_float(lam), ctypes.c_float(gain), ctypes.c_float(eps),
-                                       ctypes.c_longlong(a.shape[0] * heads), v_head_dim, _code(a), _stream())
+    out = _empty((a.shape[0], heads * v_head_dim), a.dtype, a.device)
+    rc = _gated().b200_head_difference(out, a, float(lam), float(gain), float(eps),
+                                       int(a.shape[0] * heads), v_head_dim, _code(a), _stream())
     _ok(rc, "head_difference")
     return out
 
@@ -2422,9 +2428,9 @@ def glu_columns(gate_up: torch.Tensor, glu: str = "silu", limit: float = 0.0, al
     tokens, width2 = gate_up.shape
     if width2 % 2 or glu not in GLU_COLUMN_KINDS:
         raise KernelError("glu_columns needs an even width and a known form")
-    out = torch.empty((tokens, width2 // 2), dtype=gate_up.dtype, device=gate_up.device)
-    rc = _gated().b200_glu_columns(_p(out), _p(gate_up), tokens, width2 // 2, GLU_COLUMN_KINDS[glu], ctypes.c_float(limit),
-                                   ctypes.c_float(alpha), _code(gate_up), _stream())
+    out = _empty((tokens, width2 // 2), gate_up.dtype, gate_up.device)
+    rc = _gated().b200_glu_columns(out, gate_up, tokens, width2 // 2, GLU_COLUMN_KINDS[glu], float(limit),
+                                   float(alpha), _code(gate_up), _stream())
     _ok(rc, "glu_columns")
     return out
 
@@ -2436,7 +2442,7 @@ def add_row_bias(y: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
     _f32(bias)
     if y.dim() != 2 or bias.numel() != y.shape[1]:
         raise KernelError("add_row_bias: one bias per column of y [tokens, width]")
-    rc = _gated().b200_add_row_bias(_p(y), _p(bias), y.shape[0], y.shape[1], _code(y), _stream())
+    rc = _gated().b200_add_row_bias(y, bias, y.shape[0], y.shape[1], _code(y), _stream())
     _ok(rc, "add_row_bias")
     return y
 
@@ -2450,8 +2456,8 @@ def act_table_mul(z: torch.Tensor, act: str, table: torch.Tensor, ids: torch.Ten
     if act not in ACTIVATIONS or table.dtype != z.dtype or ids.numel() != tokens or column + dim > table.shape[1]:
         raise KernelError("act_table_mul: sizes or dtypes do not fit")
     out = torch.empty_like(z)
-    rc = _gated().b200_act_table_mul(_p(out), _p(z), _p(table), _p(ids), tokens, table.shape[0], table.shape[1],
-                                     int(column), dim, ACTIVATIONS[act], _code(z), _p(error_word(z.device)), _stream())
+    rc = _gated().b200_act_table_mul(out, z, table, ids, tokens, table.shape[0], table.shape[1],
+                                     int(column), dim, ACTIVATIONS[act], _code(z), error_word(z.device), _stream())
     _ok(rc, "act_table_mul")
     return out
 
@@ -2479,10 +2485,10 @@ def token_side_few(stream: torch.Tensor, x: torch.Tensor, gate: torch.Tensor, ta
     if cast_to is not None and cast_to != torch.float32:
         if cast_to != x.dtype:
             raise KernelError("token_side_few: the rounded copy has the dtype of x")
-        out = torch.empty((tokens, width), dtype=cast_to, device=x.device)
+        out = _empty((tokens, width), cast_to, x.device)
     rc = _gated().b200_token_side_few(
-        _p(stream), _p(x), _p(gate), _p(table), _p(ids), _p(proj), _p(norm), ctypes.c_float(eps), _p(out), tokens,
-        table.shape[0], table.shape[1], int(column), dim, width, ACTIVATIONS[act], _code(x), _p(error_word(x.device)),
+        stream, x, gate, table, ids, proj, norm, float(eps), out, tokens,
+        table.shape[0], table.shape[1], int(column), dim, width, ACTIVATIONS[act], _code(x), error_word(x.device),
         _stream())
     _ok(rc, "token_side_few")
     if cast_to is None:
@@ -2504,9 +2510,9 @@ def norm_add(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float,
         raise KernelError("norm_add: y, the weight or the bias do not fit the stream")
     out = None
     if cast_to is not None and cast_to != torch.float32:
-        out = torch.empty((tokens, width), dtype=cast_to, device=x.device)
-    rc = load_cuda_library("post_norm.cu").b200_norm_add(
-        _p(x), _p(y), _code(y), _p(bias), _p(weight), ctypes.c_float(eps), int(bool(center)), _p(out),
+        out = _empty((tokens, width), cast_to, x.device)
+    rc = load_entry_points("post_norm.cu").b200_norm_add(
+        x, y, _code(y), bias, weight, float(eps), int(bool(center)), out,
         _code(out) if out is not None else F32, tokens, width, _stream())
     _ok(rc, "norm_add")
     if cast_to is None:
@@ -2536,10 +2542,10 @@ def norm_add_pair(x: torch.Tensor, pair: NormedPair, weight: torch.Tensor, eps: 
         raise KernelError("norm_add_pair: the branches, the weights or their eps do not fit")
     out = None
     if cast_to is not None and cast_to != torch.float32:
-        out = torch.empty((tokens, width), dtype=cast_to, device=x.device)
-    rc = load_cuda_library("post_norm.cu").b200_norm_add_pair(
-        _p(x), _p(a), _p(b), _code(a), _p(pair.a_weight), _p(pair.b_weight), _p(weight), ctypes.c_float(eps),
-        int(bool(center)), _p(out), _code(out) if out is not None else F32, tokens, width, _stream())
+        out = _empty((tokens, width), cast_to, x.device)
+    rc = load_entry_points("post_norm.cu").b200_norm_add_pair(
+        x, a, b, _code(a), pair.a_weight, pair.b_weight, weight, float(eps),
+        int(bool(center)), out, _code(out) if out is not None else F32, tokens, width, _stream())
     _ok(rc, "norm_add_pair")
     if cast_to is None:
         return None
@@ -2570,13 +2576,13 @@ def residual_sum(x: torch.Tensor, y=None, add: Optional[torch.Tensor] = None, bi
         raise KernelError("residual_sum: the terms, the weights or their eps do not fit the stream")
     n = tokens if rows is None else rows.numel()
     if out is None:
-        out = torch.empty((n, width), dtype=out_dtype, device=x.device)
+        out = _empty((n, width), out_dtype, x.device)
     elif out.shape[0] != n or column < 0 or column + width > out.shape[1]:
         raise KernelError("residual_sum: the result's columns do not fit")
-    rc = load_cuda_library("post_norm.cu").b200_residual_sum(
-        _p(x), _p(a), _p(b), _p(add), _code(terms[0]) if terms else F32, _p(bias), _p(wa), _p(wb), ctypes.c_float(mult),
-        _p(weight), ctypes.c_float(pair.eps if pair is not None else eps), _p(rows),
-        ctypes.c_void_p(out.data_ptr() + column * out.element_size()), _code(out), out.shape[1], int(bool(store)), n, width,
+    rc = load_entry_points("post_norm.cu").b200_residual_sum(
+        x, a, b, add, _code(terms[0]) if terms else F32, bias, wa, wb, float(mult),
+        weight, float(pair.eps if pair is not None else eps), rows,
+        int(out.data_ptr() + column * out.element_size()), _code(out), out.shape[1], int(bool(store)), n, width,
         _stream())
     _ok(rc, "residual_sum")
     return out
@@ -2594,8 +2600,8 @@ def norm_rows(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: torc
     if weight.numel() != width:
         raise KernelError("norm_rows: one weight per column is needed")
     n = x.shape[0] if rows is None else rows.numel()
-    out = torch.empty((n, width), dtype=out_dtype, device=x.device)
-    rc = load_cuda_library("post_norm.cu").b200_norm_rows(_p(out), _code(out), _p(x), _p(rows), _p(weight),
-                                                          ctypes.c_float(eps), int(bool(center)), n, width, _stream())
+    out = _empty((n, width), out_dtype, x.device)
+    rc = load_entry_points("post_norm.cu").b200_norm_rows(out, _code(out), x, rows, weight,
+                                                          float(eps), int(bool(center)), n, width, _stream())
     _ok(rc, "norm_rows")
     return out

@@ -1,0 +1,95 @@
+"""The binding through which tensors reach the kernels' C entry points (csrc/binding/calls.cpp), on functions compiled here."""
+import ctypes
+import subprocess
+import threading
+
+import pytest
+import torch
+
+import llm_infer_rust_b200.kernels.build as build
+
+_SOURCE = r"""
+#include <cstdint>
+#include <cstdio>
+// pointers, ints, 64-bit ints and floats in every order that a signature may have them; from the seventh on integers lie on the stack
+extern "C" int sum3(const float* a, float x, int n) { return static_cast<int>(a[0] + x) + n; }
+extern "C" int eight(float a, int i, float b, float c, long long l, float d, float e, float f, float g, float h, char* out) {
+  return std::snprintf(out, 200, "%g %g %g %g %g %g %g %g %d %lld", a, b, c, d, e, f, g, h, i, l);
+}
+extern "C" int many(int a, const void* b, float x, long long c, int d, int e, int f, int g, int h, float y, int i, int j, int k, int l,
+                    int m, int n, int o, long long p, void* q, int r, float z, int s, char* out) {
+  return std::snprintf(out, 400, "%d %d %g %lld %d %d %d %d %d %g %d %d %d %d %d %d %d %lld %d %d %g %d", a, b != nullptr, x, c, d, e, f,
+                       g, h, y, i, j, k, l, m, n, o, p, q != nullptr, r, z, s);
+}
+extern "C" int negative(int a, long long b) { return a == -3 && b == -(1ll << 40) ? -2 : 1; }
+"""
+
+
+@pytest.fixture(scope="module")
+def entries(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("entries")
+    source, library = folder / "entries.cpp", folder / "entries.so"
+    source.write_text(_SOURCE)
+    subprocess.run(["g++", "-O2", "-shared", "-fPIC", str(source), "-o", str(library)], check=True)
+    return build.EntryPoints(ctypes.CDLL(str(library)))
+
+
+def test_every_kind_of_argument_arrives(entries):
+    assert entries.sum3(torch.tensor([4.0, 9.0]), 2.5, 7) == 13
+    out = ctypes.create_string_buffer(400)
+    assert entries.eight(0.5, -7, 1.5, 2.5, 1 << 40, 3.5, 4.5, 5.5, 6.5, 7.5, out) > 0
+    assert out.value == b"0.5 1.5 2.5 3.5 4.5 5.5 6.5 7.5 -7 1099511627776"
+    args = [1, None, 0.25, -(1 << 33), 4, 5, 6, 7, 8, 1e-3, 9, 10, 11, 12, 13, -14, 15, 1 << 50, torch.zeros(1), True, -2.0, 17, out]
+    assert entries.many(*args) > 0
+    assert out.value == b"1 0 0.25 -8589934592 4 5 6 7 8 0.001 9 10 11 12 13 -14 15 1125899906842624 1 1 -2 17"
+    assert entries.negative(-3, -(1 << 40)) == -2
+
+
+def test_what_is_no_argument_is_refused(entries):
+    for bad in ("text", b"bytes", ctypes.c_void_p(8), ctypes.c_float(1.0), [1], object()):
+        with pytest.raises(TypeError):
+            entries.sum3(torch.zeros(1), bad, 1)
+    with pytest.raises(TypeError):
+        entries.sum3(*range(49))
+    with pytest.raises(TypeError):
+        entries.sum3(*[1.0] * 9)
+    with pytest.raises(TypeError):
+        entries.sum3(torch.zeros(1), 1.0, n=1)
+    with pytest.raises(OverflowError):
+        entries.sum3(1 << 70, 1.0, 1)
+    with pytest.raises(AttributeError):
+        entries.no_such_function
+
+
+def test_checks_and_outputs():
+    calls = build.load_call_binding()
+    a = torch.zeros(3, 4)
+    assert not calls.all_cuda(a) and calls.all_cuda(None) and calls.all_cuda()
+    assert calls.all_contiguous(a, None, a[1:]) and not calls.all_contiguous(a, a.t())
+    with pytest.raises(TypeError):
+        calls.all_cuda(None, 3)
+    for shape in ((5, 7), torch.Size([0, 3]), (4,), ()):
+        got = calls.empty(shape, torch.bfloat16, a.device)
+        assert got.shape == torch.Size(shape) and got.dtype == torch.bfloat16 and got.device == a.device and got.is_contiguous()
+    with pytest.raises(RuntimeError):
+        calls.empty((-1, 2), torch.float32, a.device)
+    x, w = torch.randn(3, 8), torch.randn(5, 8)
+    assert torch.equal(calls.mm_t(x, w), torch.mm(x, w.t()))
+    with pytest.raises(RuntimeError):
+        calls.mm_t(x, torch.randn(5, 9))
+
+
+def test_several_threads(entries):
+    got = []
+
+    def work(i):
+        out = ctypes.create_string_buffer(400)
+        for _ in range(200):
+            entries.eight(float(i), i, 1.5, 2.5, i, 3.5, 4.5, 5.5, 6.5, 7.5, out)
+            got.append(out.value == f"{i} 1.5 2.5 3.5 4.5 5.5 6.5 7.5 {i} {i}".encode())
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 800 and all(got)
