@@ -223,6 +223,121 @@ qkv_post_vec_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_out, TA* __re
   }
 }
 
+// Many tokens: the same lane groups (HG heads of one token a step) walk over the step's work, and what the next step reads
+// (its heads, its token's position and slot) is on its way while this one is normed, turned and stored.  A thread that comes
+// and goes with one group of heads has loads in flight for a part of its life only, and its index cost a 64-bit division.
+// Bound by latency still (four blocks an SM by registers).  bfloat16, 16 + 2 x 8 heads of 128, us in a graph before / now: 8,192
+// tokens 51.8 / 35.0 (134 MB: 3.8 TB/s), 2,919 20.2 / 14.1, 1,020 8.7 / 6.5; 32 + 2 x 8 heads, 2,048 tokens 20.3 / 14.6.  One head a
+// lane group: 44.0, 17.6, 7.2, 17.8.
+template <typename TA, typename TW, int HG>
+__global__ void __launch_bounds__(256, 4)
+qkv_post_walk_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_out, TA* __restrict__ k_cache,
+                     TA* __restrict__ v_cache, const TW* __restrict__ q_w, const TW* __restrict__ k_w, float eps,
+                     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int max_pos,
+                     const int* __restrict__ positions, const int* __restrict__ slots, int tokens, int nh, int nkv,
+                     int d, int page_size, long long cache_slots, int lanes, int* err) {
+  constexpr int N = Half16<TA>::N;
+  const int heads = nh + 2 * nkv, head_groups = (heads + HG - 1) / HG;
+  const int sub = threadIdx.x % lanes;
+  const int groups = gridDim.x * (blockDim.x / lanes), step_t = groups / head_groups, step_g = groups - step_t * head_groups;
+  const int first = blockIdx.x * (blockDim.x / lanes) + threadIdx.x / lanes;
+  int t = first / head_groups, g = first - t * head_groups;
+  const bool rotates = cos_table != nullptr, stores_any = slots != nullptr;
+  uint2 next_a[HG], next_b[HG];                                 // 8 bytes of a head's first half, and what they are rotated with
+  int next_pos = 0, next_slot = 0;
+  auto fetch = [&](int ft, int fg) {
+    if (ft >= tokens) return;
+    const int h0 = fg * HG;
+    const TA* src = qkv + (static_cast<size_t>(ft) * heads + h0) * d + sub * N;
+#pragma unroll
+    for (int i = 0; i < HG; ++i)
+      if (h0 + i < heads) {
+        next_a[i] = *reinterpret_cast<const uint2*>(src + i * d);
+        next_b[i] = *reinterpret_cast<const uint2*>(src + i * d + d / 2);
+      }
+    if (rotates) next_pos = positions[ft];
+    if (stores_any) next_slot = slots[ft];
+  };
+  fetch(t, g);
+  // (the lane groups of a warp leave together: those without work go on with the shuffles)
+  while (__any_sync(0xffffffffu, t < tokens)) {
+    const bool live = t < tokens;
+    const int h0 = g * HG, here = live ? min(HG, heads - h0) : 0;
+    float a[HG][N], b[HG][N];
+#pragma unroll
+    for (int i = 0; i < HG; ++i) {
+      Half16<TA>::load(reinterpret_cast<const TA*>(&next_a[i]), a[i]);
+      Half16<TA>::load(reinterpret_cast<const TA*>(&next_b[i]), b[i]);
+    }
+    const int pos = next_pos, slot = next_slot, now = t;
+    t += step_t;
+    g += step_g;
+    if (g >= head_groups) { g -= head_groups; ++t; }
+    fetch(t, g);
+    const bool turns = rotates && h0 < nh + nkv && here > 0, stores = stores_any && h0 + here > nh && here > 0;
+    const bool in_table = turns && pos >= 0 && pos < max_pos;
+    float c[N], sn[N];
+    if (in_table) {
+      load_few<float, N>(cos_table + static_cast<size_t>(pos) * (d / 2) + sub * N, c);
+      load_few<float, N>(sin_table + static_cast<size_t>(pos) * (d / 2) + sub * N, sn);
+    }
+    bool slot_ok = stores && slot != 0;
+    if (stores && (slot < 0 || slot >= cache_slots)) {
+      slot_ok = false;
+      if (sub == 0) atomicOr(err, B200_ERR_SLOT_RANGE);
+    }
+    if (turns && !in_table && sub == 0) atomicOr(err, B200_ERR_POSITION_RANGE);
+    float ss[HG];
+#pragma unroll
+    for (int i = 0; i < HG; ++i) {
+      ss[i] = 0.0f;
+#pragma unroll
+      for (int e = 0; e < N; ++e) ss[i] += a[i][e] * a[i][e] + b[i][e] * b[i][e];
+    }
+    if (q_w != nullptr)
+      for (int o = lanes >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < HG; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o, lanes);
+    const int page = slot_ok ? slot / page_size : 0, offset = slot_ok ? slot - page * page_size : 0;
+#pragma unroll
+    for (int i = 0; i < HG; ++i) {
+      if (i >= here) break;
+      const int h = h0 + i;
+      const bool is_q = h < nh, is_k = !is_q && h < nh + nkv;
+      if ((is_q || is_k) && q_w != nullptr) {
+        const TW* w = (is_q ? q_w : k_w) + sub * N;
+        const float scale = rsqrtf(ss[i] / static_cast<float>(d) + eps);
+        float wa[N], wb[N];
+        load_few<TW, N>(w, wa);
+        load_few<TW, N>(w + d / 2, wb);
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          a[i][e] = a[i][e] * scale * wa[e];
+          b[i][e] = b[i][e] * scale * wb[e];
+        }
+      }
+      if ((is_q || is_k) && in_table) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          const float x = a[i][e], y = b[i][e];
+          a[i][e] = x * c[e] - y * sn[e];
+          b[i][e] = y * c[e] + x * sn[e];
+        }
+      }
+      TA* dst;
+      if (is_q) {
+        dst = q_out + (static_cast<size_t>(now) * nh + h) * d;
+      } else {
+        if (!slot_ok) continue;
+        const int kvh = is_k ? h - nh : h - nh - nkv;
+        dst = (is_k ? k_cache : v_cache) + ((static_cast<size_t>(page) * nkv + kvh) * page_size + offset) * d;
+      }
+      Half16<TA>::store(dst + sub * N, a[i]);
+      Half16<TA>::store(dst + d / 2 + sub * N, b[i]);
+    }
+  }
+}
+
 // How many heads a lane group takes, by the blocks of 256 threads that one head each would be: few blocks are all resident and
 // the shortest chain is fastest, many share the SMs and the fetches saved count.  Measured, us with 1 / 2 / 4 (bfloat16, 16 + 2 x 8
 // heads of 128): 64 tokens (128 blocks) 3.4 / 3.7 / 4.9, 200 (400) 3.5 / 4.1 / 4.9, 300 (600) 4.8 / 4.5 / 5.5, 500 (1,000) 5.5 / 5.1 /
@@ -232,6 +347,13 @@ static int heads_a_group(long long work, int lanes) {
   return blocks <= 3 * 148 ? 1 : blocks <= 8 * 148 ? 2 : 4;
 }
 B200_EXPORT int b200_qkv_post_heads_a_group(long long work, int lanes) { return heads_a_group(work, lanes); }
+
+// The walking kernel takes bfloat16 steps of more than six blocks of 256 threads an SM: below, all of a step's threads are
+// resident at once (777 tokens x 32 heads 5.2 / 5.2, 500 4.1 / 4.3), and float32's two elements of 8 bytes leave a lane group of
+// 32 too little to have on its way (2,000 tokens 15.0 / 16.4).
+constexpr int WALK_HEADS = 2, WALK_BLOCKS = 8 * 148;
+static bool walk_takes(int act_dtype, long long threads) { return act_dtype == B200_BF16 && threads > 6ll * 148 * 256; }
+B200_EXPORT int b200_qkv_post_walks(int act_dtype, long long threads) { return walk_takes(act_dtype, threads); }
 
 B200_EXPORT int b200_qkv_post(const void* qkv, void* q_out, void* k_cache, void* v_cache, const void* q_w,
                               const void* k_w, float eps, const float* cos_table, const float* sin_table,
@@ -253,14 +375,21 @@ B200_EXPORT int b200_qkv_post(const void* qkv, void* q_out, void* k_cache, void*
     if (lanes >= 2 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && aligned && whole_rotation) {
       const int hg = heads_a_group(work, lanes);
       const long long threads = static_cast<long long>(tokens) * ((nh + 2 * nkv + hg - 1) / hg) * lanes;
+      const long long steps = static_cast<long long>(tokens) * ((nh + 2 * nkv + WALK_HEADS - 1) / WALK_HEADS);
+      const bool walks = walk_takes(act_dtype, steps * lanes);
       const unsigned vblocks = static_cast<unsigned>((threads + 255) / 256);
+#define CALLW(TA, TW)                                                                                          \
+      qkv_post_walk_kernel<TA, TW, WALK_HEADS><<<WALK_BLOCKS, 256, 0, stream>>>(                                          \
+          static_cast<const TA*>(qkv), static_cast<TA*>(q_out), static_cast<TA*>(k_cache), static_cast<TA*>(v_cache), \
+          static_cast<const TW*>(q_w), static_cast<const TW*>(k_w), eps, cos_table, sin_table, max_pos, positions, \
+          slots, tokens, nh, nkv, d, page_size, cache_slots, lanes, err)
 #define CALLG(TA, TW, HG)                                                                                      \
       qkv_post_vec_kernel<TA, TW, HG><<<vblocks, 256, 0, stream>>>(                                             \
           static_cast<const TA*>(qkv), static_cast<TA*>(q_out), static_cast<TA*>(k_cache), static_cast<TA*>(v_cache), \
           static_cast<const TW*>(q_w), static_cast<const TW*>(k_w), eps, cos_table, sin_table, max_pos, positions, \
           slots, tokens, nh, nkv, d, page_size, cache_slots, lanes, err)
 #define CALLV(TA, TW)                                                                                          \
-      if (hg == 1) { CALLG(TA, TW, 1); } else if (hg == 2) { CALLG(TA, TW, 2); } else { CALLG(TA, TW, 4); }
+      if (walks) { if constexpr (sizeof(TA) == 2) { CALLW(TA, TW); } } else if (hg == 1) { CALLG(TA, TW, 1); } else if (hg == 2) { CALLG(TA, TW, 2); } else { CALLG(TA, TW, 4); }
       if (act_dtype == B200_F32 && w_dtype == B200_F32) { CALLV(float, float); }
       else if (act_dtype == B200_BF16 && w_dtype == B200_BF16) { CALLV(__nv_bfloat16, __nv_bfloat16); }
       else if (act_dtype == B200_BF16 && w_dtype == B200_F32) { CALLV(__nv_bfloat16, float); }
@@ -268,6 +397,7 @@ B200_EXPORT int b200_qkv_post(const void* qkv, void* q_out, void* k_cache, void*
       else return B200_BAD_DTYPE;
 #undef CALLV
 #undef CALLG
+#undef CALLW
       return b200_check_launch();
     }
   }

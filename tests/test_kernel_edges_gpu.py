@@ -153,3 +153,50 @@ def test_all_sizes_prompt_attention_keeps_its_blocks_on_an_sm(head_dim, ctas, dt
     """A few registers more a thread and an SM holds a block less; long prompts then take up to twice the time."""
     from llm_infer_rust_b200.kernels import ops
     assert ops._attention(head_dim).b200_prefill_attention_ctas_per_sm(ops.F32 if dtype == torch.float32 else ops.BF16) >= ctas
+
+
+# more steps than the grid has lane groups, with a rest; an odd count of heads (the last step has one); heads of 64 and 256 (8 and 32
+# lanes); without norms, without tables, without a cache
+@pytest.mark.parametrize("tokens,nh,nkv,d,norm,turn,store", [(1020, 16, 8, 128, True, True, True), (2500, 32, 8, 128, True, True, True),
+                                                             (3001, 15, 5, 128, False, True, True), (6000, 9, 1, 64, True, True, False),
+                                                             (1300, 8, 4, 256, True, False, True)])
+def test_between_projection_and_attention_many_tokens_are_as_few(tokens, nh, nkv, d, norm, turn, store):
+    from llm_infer_rust_b200.kernels import ops
+    from llm_infer_rust_b200.kernels.build import load_entry_points
+    steps = tokens * -(-(nh + 2 * nkv) // 2) * d // 8
+    assert load_entry_points("qkv_post.cu").b200_qkv_post_walks(ops.BF16, steps)
+    qkv = _rnd(tokens, (nh + 2 * nkv) * d, dtype=torch.bfloat16)
+    w = [_rnd(d, dtype=torch.bfloat16, seed=s) for s in (1, 2)] if norm else [None, None]
+    cos, sin = (_rnd(700, d // 2, seed=s) for s in (3, 4)) if turn else (None, None)
+    gen = torch.Generator().manual_seed(5)
+    pos = torch.randint(0, 700, (tokens,), generator=gen).int().to(DEV)
+    slots = torch.randperm(tokens, generator=gen).int().to(DEV) + 16 if store else None
+    if store:
+        slots[::7] = 0                                          # padding rows
+    out = []
+    for cut in (tokens, 10):                                    # all at once, and ten tokens a call (the other kernel)
+        k = torch.zeros(tokens // 16 + 3, nkv, 16, d, dtype=torch.bfloat16, device=DEV) if store else None
+        v, q = torch.zeros_like(k) if store else None, torch.zeros(tokens, nh * d, dtype=torch.bfloat16, device=DEV)
+        for at in range(0, tokens, cut):
+            part = slice(at, at + cut)
+            ops.qkv_post(qkv[part], q[part], k, v, w[0], w[1], 1e-6, cos, sin, d if turn else 0, pos[part],
+                         slots[part] if store else None, nh, nkv, d)
+        out.append([q] + ([k, v] if store else []))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    ops.check_errors(qkv.device)
+
+
+def test_many_tokens_refuse_slots_and_positions_outside():
+    from llm_infer_rust_b200.kernels import ops
+    tokens, nh, nkv, d = 1200, 16, 8, 128
+    qkv, q = _rnd(tokens, (nh + 2 * nkv) * d, dtype=torch.bfloat16), torch.zeros(tokens, nh * d, dtype=torch.bfloat16, device=DEV)
+    k = torch.zeros(80, nkv, 16, d, dtype=torch.bfloat16, device=DEV)
+    v, cos, sin = torch.zeros_like(k), _rnd(1200, d // 2), _rnd(1200, d // 2)
+    pos, slots = torch.arange(tokens, dtype=torch.int32, device=DEV), torch.arange(tokens, dtype=torch.int32, device=DEV) + 16
+    for bad, where, what in ((1200, pos, "rotary"), (-1, pos, "rotary"), (80 * 16, slots, "slot"), (-5, slots, "slot")):
+        kept = where[777].clone()
+        where[777] = bad
+        ops.qkv_post(qkv, q, k, v, None, None, 1e-6, cos, sin, d, pos, slots, nh, nkv, d)
+        where[777] = kept
+        with pytest.raises(ops.KernelError, match=what):
+            ops.check_errors(qkv.device)

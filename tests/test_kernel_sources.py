@@ -55,3 +55,11 @@ def test_columns_that_a_warp_takes_of_few_rows_experts():
     assert cols(1024, 8, 64) == cols(2048, 64, 64) == cols(1536, 8, 8) == cols(2048, 2, 8) == 2
     assert cols(256, 4, 4) == cols(512, 32, 4) == 1                         # 64 and 128 blocks
     assert cols(1536, 64, 8) == cols(768, 32, 8) == 1                       # four and eight rows an expert
+
+
+def test_many_tokens_walk_between_projection_and_attention():
+    """bfloat16 from more than six blocks an SM on (measured on both sides), float32 never."""
+    walks = build.load_cuda_library("qkv_post.cu").b200_qkv_post_walks
+    threads = lambda tokens, heads: ctypes.c_longlong(tokens * (heads // 2) * 16)
+    assert all(walks(1, threads(t, h)) for t, h in ((1020, 32), (2048, 48), (8192, 32)))
+    assert not any(walks(1, threads(t, h)) for t, h in ((777, 32), (500, 32), (45, 48))) and not walks(0, threads(8192, 32))
