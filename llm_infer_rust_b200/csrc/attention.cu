@@ -33,7 +33,7 @@
 // Bound by instructions, not by bytes: a key's row is therefore looked up once a block (a lane a key) and handed to the
 // copying lanes by shuffles; a division and a table read for each 16 bytes took longer than the arithmetic (float32, 4 rows
 // of up to 900 keys in one split: 100 us, in four: 18 us; a prompt of 300 tokens with the next block's copies under the
-// arithmetic as well: 78.6 -> 60.9 us).
+// arithmetic as well: 78.6 -> 60.9 us; float32 prompts of heads up to 128 have a kernel on the tensor cores now, see below).
 #include <math.h>
 
 #include "common.cuh"
@@ -201,12 +201,9 @@ __device__ __forceinline__ void load_key_block(T* dst, const T* __restrict__ cac
 // 32 hc ..): tile_tokens * heads <= 32 vectors.
 constexpr int PF_WARPS = 8;
 
-// (Heads of 16 are held to three CTAs an SM: with 88 registers instead of 80 they had two, and 2,000 float32 tokens behind 1,000, 40
-// query heads, took 2,949 us for 2,383.  0 leaves the others to the compiler, which stays at 80 or at what shared memory allows;
-// told that one CTA is enough it took all registers, and heads of 32 6,336 us for 2,546.)
+// One tile of a portion, by CUDA cores (shared memory: PrefillShape<T>::SMEM).
 template <typename T>
-__global__ void __launch_bounds__(PF_WARPS * 32, D <= 16 ? 3 : 0)
-prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+__device__ __forceinline__ void prefill_tile(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                          T* __restrict__ out, const int* __restrict__ block_table, int table_stride,
                          const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                          const int* __restrict__ prefix_len, const int* __restrict__ rows, int nh, int nkv,
@@ -298,6 +295,271 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
     }
   }
 }
+
+// (Heads of 16 are held to three CTAs an SM: with 88 registers instead of 80 they had two, and 2,000 float32 tokens behind 1,000, 40
+// query heads, took 2,949 us for 2,383.  0 leaves the others to the compiler, which stays at 80 or at what shared memory allows;
+// told that one CTA is enough it took all registers, and heads of 32 6,336 us for 2,546.)
+template <typename T>
+__global__ void __launch_bounds__(PF_WARPS * 32, D <= 16 ? 3 : 0)
+prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+                         T* __restrict__ out, const int* __restrict__ block_table, int table_stride,
+                         const int* __restrict__ cu_q, const int* __restrict__ kv_len,
+                         const int* __restrict__ prefix_len, const int* __restrict__ rows, int nh, int nkv,
+                         int page_size, int window, float scale, int tile_tokens, int head_chunks, int hd,
+                         int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride, int stages) {
+  prefill_tile<T>(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window,
+                  scale, tile_tokens, head_chunks, hd, hd_v, softcap, chunk, sinks, v_stride, stages);
+}
+
+#if HEAD_DIM <= 128
+// ------------------------------------------------------------------ prompt portions in float, on the tensor cores
+// The same tiles (up to 32 query vectors of one KV head) with both products on mma.sync: a float is the exact sum of three
+// bfloat16 terms, and of the nine products of two such floats the six that reach 2^-24 are taken, the small ones first.
+// Every 16 columns (or keys) are summed from zero by the tensor cores and added to the rest in float by the thread, so that
+// what they cut off below a sum's last place stays that of sixteen terms.
+// Eight warps: two halves of the vectors (16 each) x four quarters of every block of 64 keys (16 keys each); each warp runs a
+// softmax of its own over its keys and the four parts of a vector are added up at the end in order.  Which keys a warp takes
+// depends on their positions alone, so a position's result has the same bits however the prompt was cut.
+// The query's terms stay in registers; keys and values are taken apart as they are read, since a block serves two warps only.
+// A tile whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term).
+// Bound by the instructions that take keys and values apart (two warps a scheduler, 22 for a thread's four numbers, six products).  us,
+// CUDA cores / this: 16 heads of 128, 8 KV heads, 300 tokens 59.3 / 30.7, 17 tokens 13.5 / 10.5, 2,000 tokens 991 / 598, 64 behind 2,000
+// cached 343 / 170, 16 rows of 5 behind 100 21.6 / 13.8; heads of 64, 300 tokens 42.3 / 18.7, of 16 37.6 / 11.5.  Error against 64 bits
+// 7.2e-7 -> 2.5e-7 (300 tokens).  Heads beyond 128 or of another width than their values stay with prefill_tile.
+constexpr int SPLIT_KEYS = 64;
+
+struct SplitPrefill {
+  static constexpr int K_ROW = D % 32 == 16 ? D : D + 16;      // floats of a row: 16-byte reads of two rows meet no bank twice
+  static constexpr int V_ROW = D + 4;                          // four rows, two apart, of a column each
+  static constexpr int STAGE = SPLIT_KEYS * (K_ROW + V_ROW);   // floats
+  static constexpr int MERGE = 4 * 32 * (D + 4);               // floats: the four parts of 32 vectors
+  static constexpr size_t TILES = sizeof(float) * (2 * STAGE > MERGE ? 2 * STAGE : MERGE);
+  static constexpr size_t SMEM = TILES + sizeof(float) * 4 * 32 * 2;
+};
+
+// Two floats as three bfloat16 terms each, packed (the first float in the low half): x = high + mid + low exactly, each term
+// the rest rounded to eight bits.
+__device__ __forceinline__ void terms_of(float x, float y, uint32_t& high, uint32_t& mid, uint32_t& low) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(high) : "f"(y), "f"(x));
+  x -= __uint_as_float(high << 16);
+  y -= __uint_as_float(high & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(mid) : "f"(y), "f"(x));
+  x -= __uint_as_float(mid << 16);
+  y -= __uint_as_float(mid & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(low) : "f"(y), "f"(x));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// sum[n] += a . b[n] over 16 columns, a and b in three terms; the tiles' chains of products side by side.
+template <int TILES>
+__device__ __forceinline__ void add_products(float (*sum)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[TILES][3], const uint32_t (&b1)[TILES][3]) {
+  constexpr int AI[6] = {2, 0, 1, 1, 0, 0}, BI[6] = {0, 2, 1, 0, 1, 0};
+  float t[TILES][4] = {};
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) mma_bf16(t[n], a[AI[i]], b0[n][BI[i]], b1[n][BI[i]]);
+#pragma unroll
+  for (int n = 0; n < TILES; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[n][i] += t[n][i];
+}
+
+__device__ __noinline__ void prefill_tile_again(const float* q, const float* k_cache, const float* v_cache, float* out,
+                                                const int* block_table, int table_stride, const int* cu_q, const int* kv_len,
+                                                const int* prefix_len, const int* rows, int nh, int nkv, int page_size, int window,
+                                                float scale, int tile_tokens, int head_chunks, float softcap, int chunk,
+                                                const float* sinks) {
+  prefill_tile<float>(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size,
+                      window, scale, tile_tokens, head_chunks, D, D, softcap, chunk, sinks, D, 1);
+}
+
+__global__ void __launch_bounds__(PF_WARPS * 32, 1)
+prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+                     float* __restrict__ out, const int* __restrict__ block_table, int table_stride,
+                     const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ prefix_len,
+                     const int* __restrict__ rows, int nh, int nkv, int page_size, int window, float scale, int tile_tokens,
+                     int head_chunks, float softcap, int chunk, const float* __restrict__ sinks) {
+  using S = SplitPrefill;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* tiles = reinterpret_cast<float*>(smem_raw);                     // [2][K rows, V rows]
+  float* parts_ml = reinterpret_cast<float*>(smem_raw + S::TILES);       // [4][32][2]
+  const int row = rows[blockIdx.z];
+  const int kvh = blockIdx.y / head_chunks, hc = blockIdx.y - kvh * head_chunks;
+  const int head_base = kvh * (nh / nkv) + hc * 32;
+  const int group = min(32, nh / nkv - hc * 32);
+  const int q_begin = cu_q[row], q_len = cu_q[row + 1] - q_begin;
+  const int tok0 = (gridDim.x - 1 - blockIdx.x) * tile_tokens;           // the tiles that see the most keys start first
+  if (tok0 >= q_len) return;
+  const int ntok = min(tile_tokens, q_len - tok0);
+  const int nvec = ntok * group;
+  const int p_lo = prefix_len[row] + tok0;
+  const int kv_end = min(kv_len[row], p_lo + ntok);
+  int k_begin = window > 0 ? max(0, p_lo - window + 1) : 0;
+  if (chunk > 0) k_begin = max(k_begin, p_lo - p_lo % chunk);
+  k_begin -= k_begin % SPLIT_KEYS;
+  const int* table = block_table + static_cast<size_t>(row) * table_stride;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int half = warp >> 2, quarter = warp & 3;
+  const int r = lane >> 2, c4 = lane & 3;                                // of a fragment: row (or column of B), place among four
+
+  auto fetch = [&](int first, int stage) {
+    float* ks = tiles + stage * S::STAGE;
+    float* vs = ks + SPLIT_KEYS * S::K_ROW;
+    const long long low = lane_row(table, page_size, nkv, kvh, first, kv_end), up = lane_row(table, page_size, nkv, kvh, first + 32, kv_end);
+    constexpr int PIECES = D / 4;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < SPLIT_KEYS * PIECES; i += PF_WARPS * 32) {
+      const int key = i / PIECES, part = i - key * PIECES;
+      const long long a = __shfl_sync(0xffffffffu, low, key & 31), b = __shfl_sync(0xffffffffu, up, key & 31);
+      const long long at = key < 32 ? a : b;
+      cp_async16(ks + key * S::K_ROW + part * 4, at >= 0 ? k_cache + at * D + part * 4 : k_cache, at >= 0);
+      cp_async16(vs + key * S::V_ROW + part * 4, at >= 0 ? v_cache + at * D + part * 4 : v_cache, at >= 0);
+    }
+  };
+  fetch(k_begin, 0);
+  cp_async_commit();
+
+  // The warp's 16 vectors, rows r and r + 8 of a fragment: their positions, and their terms (four columns 16 s + 4 c4 .. + 3 of
+  // a k-step s: the tensor cores sum over k, in whatever order both operands hold it).
+  int pos[2];
+  uint32_t qt[D / 16][3][4];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int vec = half * 16 + r + 8 * e;
+    const bool used = vec < nvec;
+    pos[e] = used ? p_lo + vec / group : -1;
+    const float* src = q + (static_cast<size_t>(q_begin + tok0 + (used ? vec / group : 0)) * nh + head_base + (used ? vec % group : 0)) * D;
+#pragma unroll
+    for (int s = 0; s < D / 16; ++s) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (used) v = *reinterpret_cast<const float4*>(src + 16 * s + 4 * c4);
+      terms_of(v.x * scale, v.y * scale, qt[s][0][e], qt[s][1][e], qt[s][2][e]);
+      terms_of(v.z * scale, v.w * scale, qt[s][0][2 + e], qt[s][1][2 + e], qt[s][2][2 + e]);
+    }
+  }
+  int p_max = max(pos[0], pos[1]), p_min = min(pos[0] < 0 ? 0x7fffffff : pos[0], pos[1] < 0 ? 0x7fffffff : pos[1]);
+  p_max = __reduce_max_sync(0xffffffffu, p_max);
+  p_min = __reduce_min_sync(0xffffffffu, p_min);
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, o[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[n][i] = 0.0f;
+
+  int stage = 0;
+  for (int kb = k_begin; kb < kv_end; kb += SPLIT_KEYS, stage ^= 1) {
+    if (kb + SPLIT_KEYS < kv_end) fetch(kb + SPLIT_KEYS, stage ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    const int first = kb + 16 * quarter;
+    if (p_max >= first && first < kv_end && (window <= 0 || first + 15 > p_min - window) && (chunk <= 0 || first + 15 >= p_min - p_min % chunk)) {
+      const float* ks = tiles + stage * S::STAGE + 16 * quarter * S::K_ROW;
+      const float* vs = tiles + stage * S::STAGE + SPLIT_KEYS * S::K_ROW + 16 * quarter * S::V_ROW;
+      float s[2][4] = {};                                                // scores: keys 8 t + 2 c4, + 1 of rows r and r + 8
+#pragma unroll
+      for (int step = 0; step < D / 16; ++step) {
+        uint32_t b0[2][3], b1[2][3];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float4 kv = *reinterpret_cast<const float4*>(ks + (8 * t + r) * S::K_ROW + 16 * step + 4 * c4);
+          terms_of(kv.x, kv.y, b0[t][0], b0[t][1], b0[t][2]);
+          terms_of(kv.z, kv.w, b1[t][0], b1[t][1], b1[t][2]);
+        }
+        add_products<2>(s, qt[step], b0, b1);
+      }
+      uint32_t pt[3][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float v[4], mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int key = first + 8 * (i >> 1) + 2 * c4 + (i & 1), p = pos[e];
+          float x = s[i >> 1][2 * e + (i & 1)];
+          if (softcap > 0.0f) x = softcap * tanhf(x * (1.0f / softcap));
+          const bool visible = p >= 0 && key <= p && key < kv_end && (window <= 0 || key > p - window) && (chunk <= 0 || key >= p - p % chunk);
+          v[i] = visible ? x : -INFINITY;
+          mx = fmaxf(mx, v[i]);
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float top = fmaxf(m[e], mx);
+        float sum = 0.0f, corr = 1.0f;
+        if (top != -INFINITY) {
+          corr = expf(m[e] - top);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { v[i] = expf(v[i] - top); sum += v[i]; }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[i] = v[i] != v[i] ? v[i] : 0.0f;   // (a NaN stays one: the tile is done again)
+        }
+        l[e] = l[e] * corr + sum;                                        // (this lane's keys; the four lanes are added up at the end)
+        m[e] = top;
+        terms_of(v[0], v[1], pt[0][e], pt[1][e], pt[2][e]);
+        terms_of(v[2], v[3], pt[0][2 + e], pt[1][2 + e], pt[2][2 + e]);
+        if (__any_sync(0xffffffffu, corr != 1.0f ? 1 : 0))
+#pragma unroll
+          for (int n = 0; n < D / 8; ++n) { o[n][2 * e] *= corr; o[n][2 * e + 1] *= corr; }
+      }
+#pragma unroll
+      for (int n = 0; n < D / 8; n += 2) {
+        uint32_t b0[2][3], b1[2][3];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float* col = vs + 8 * (n + t) + r + 2 * c4 * S::V_ROW;
+          terms_of(col[0], col[S::V_ROW], b0[t][0], b0[t][1], b0[t][2]);
+          terms_of(col[8 * S::V_ROW], col[9 * S::V_ROW], b1[t][0], b1[t][1], b1[t][2]);
+        }
+        add_products<2>(o + n, pt, b0, b1);
+      }
+    }
+    __syncthreads();                                                     // this block is read: the next copies may overwrite it
+  }
+  // The four parts of a vector.
+  float* parts = tiles;                                                  // [4][32][D + 4]
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int vec = half * 16 + r + 8 * e;
+    float sum = l[e] + __shfl_xor_sync(0xffffffffu, l[e], 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (c4 == 0) {
+      parts_ml[(quarter * 32 + vec) * 2] = m[e];
+      parts_ml[(quarter * 32 + vec) * 2 + 1] = sum;
+    }
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n)
+      *reinterpret_cast<float2*>(parts + (quarter * 32 + vec) * (D + 4) + 8 * n + 2 * c4) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
+  }
+  __syncthreads();
+  bool finite = true;
+  for (int i = threadIdx.x; i < nvec * (D / 4); i += PF_WARPS * 32) {
+    const int vec = i / (D / 4), at = i - vec * (D / 4);
+    float top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) top = fmaxf(top, parts_ml[(w * 32 + vec) * 2]);
+    float sum = 0.0f, acc[4] = {};
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float pm = parts_ml[(w * 32 + vec) * 2], f = top == -INFINITY ? 0.0f : expf(pm - top);
+      const float4 v = *reinterpret_cast<const float4*>(parts + (w * 32 + vec) * (D + 4) + 4 * at);
+      sum += parts_ml[(w * 32 + vec) * 2 + 1] * f;
+      acc[0] += v.x * f; acc[1] += v.y * f; acc[2] += v.z * f; acc[3] += v.w * f;
+    }
+    const int tok = vec / group, head = head_base + vec % group;
+    if (sinks != nullptr && sum > 0.0f) sum += expf(sinks[head] - top);
+    const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+    const float4 v = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+    finite = finite && fabsf(sum) < INFINITY && fabsf(acc[0]) < INFINITY && fabsf(acc[1]) < INFINITY && fabsf(acc[2]) < INFINITY && fabsf(acc[3]) < INFINITY;
+    *reinterpret_cast<float4*>(out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D + 4 * at) = v;
+  }
+  if (__syncthreads_or(finite ? 0 : 1))
+    prefill_tile_again(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window,
+                       scale, tile_tokens, head_chunks, softcap, chunk, sinks);
+}
+#endif
 
 // ------------------------------------------------------------------ decoded tokens, split over the keys
 // grid (splits, nkv * vector groups, decode rows); DEC_WARPS warps, each walking its own key blocks
@@ -499,6 +761,24 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   }
   if (static_cast<long long>(nkv) * head_chunks > 65535 || n_rows > 65535) return B200_BAD_SIZE;
   dim3 grid((max_q_len + tile_tokens - 1) / tile_tokens, nkv * head_chunks, n_rows);
+#if HEAD_DIM <= 128
+  if constexpr (sizeof(T) == 4) {
+    const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (hd == D && hd_v == D && (v_stride <= 0 || v_stride == D) && aligned(q) && aligned(kc) && aligned(vc) && aligned(out)) {
+      static_assert(SplitPrefill::SMEM >= PrefillShape<float>::FIXED + PrefillShape<float>::BLOCK, "a tile may be done again");
+      static bool split_configured = false;
+      if (!split_configured) {
+        cudaError_t e = cudaFuncSetAttribute(prefill_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SplitPrefill::SMEM));
+        if (e != cudaSuccess) return static_cast<int>(e);
+        split_configured = true;
+      }
+      prefill_split_kernel<<<grid, PF_WARPS * 32, SplitPrefill::SMEM, stream>>>(
+          static_cast<const float*>(q), static_cast<const float*>(kc), static_cast<const float*>(vc), static_cast<float*>(out), block_table,
+          table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window, scale, tile_tokens, head_chunks, softcap, chunk, sinks);
+      return b200_check_launch();
+    }
+  }
+#endif
   prefill_attention_kernel<T><<<grid, PF_WARPS * 32, smem, stream>>>(
       static_cast<const T*>(q), static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out),
       block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window, scale, tile_tokens,

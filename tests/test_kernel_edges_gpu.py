@@ -200,3 +200,99 @@ def test_many_tokens_refuse_slots_and_positions_outside():
         where[777] = kept
         with pytest.raises(ops.KernelError, match=what):
             ops.check_errors(qkv.device)
+
+
+def _paged(lens, cached, nkv, d, page, seed=0):
+    """Random pages of rows that hold ``cached`` + ``lens`` positions each: caches, block table, the rows' index arrays."""
+    gen = torch.Generator().manual_seed(seed)
+    total = [a + b for a, b in zip(lens, cached)]
+    pages = [-(-t // page) for t in total]
+    order, table, at = torch.randperm(sum(pages), generator=gen) + 1, torch.zeros(len(lens), max(pages), dtype=torch.int32), 0
+    for i, n in enumerate(pages):
+        table[i, :n] = order[at:at + n]
+        at += n
+    k, v = (torch.randn(sum(pages) + 1, nkv, page, d, generator=gen).to(DEV) for _ in range(2))
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    return k, v, table.to(DEV), ints(starts), ints(total), ints(cached), ints(list(range(len(lens))))
+
+
+def _attention_64(q, k, v, table, lens, cached, nh, nkv, d, page, scale, window=0, chunk=0, cap=0.0, sinks=None):
+    out, at = [], 0
+    for i, (n, p) in enumerate(zip(lens, cached)):
+        t = n + p
+        ks, vs = (c[table[i, :-(-t // page)].long()].double().permute(0, 2, 1, 3).reshape(-1, nkv, d)[:t].repeat_interleave(nh // nkv, 1)
+                  for c in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double().view(n, nh, d), ks) * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        pos, key = torch.arange(p, t, device=DEV)[:, None], torch.arange(t, device=DEV)[None]
+        hidden = (key > pos) | ((pos - key >= window) if window else False) | ((pos // chunk != key // chunk) if chunk else False)
+        s = s.masked_fill(hidden, float("-inf"))
+        if sinks is not None:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(-1, n, 1)], 2)
+        out.append(torch.einsum("hqk,khd->qhd", torch.softmax(s, -1)[:, :, :t], vs).reshape(n, -1))
+        at += n
+    return torch.cat(out)
+
+
+# float32 portions on mma.sync: one key more than a quarter of a block (16), than a block (64) and than two; tiles with a rest; groups of
+# 1, 2, 7, 16 and 40 (two chunks of heads); heads of 16, 48, 64, 96 and 128; page sizes of no power of two; windows and blocks inside
+# a block of keys; caps and sinks; heads that only the other kernel takes (24: no multiple of 16)
+@pytest.mark.parametrize("lens,cached,nh,nkv,d,page,form", [
+    ([17], [0], 16, 8, 128, 16, {}), ([65, 1, 40], [0, 130, 3], 16, 8, 128, 16, {}), ([33], [96], 8, 8, 64, 16, {}),
+    ([50], [10], 40, 1, 64, 4, {}), ([40], [0], 14, 2, 16, 16, {}), ([65], [3], 32, 2, 96, 3, {}), ([129], [0], 4, 4, 48, 16, {}),
+    ([100], [30], 16, 8, 128, 16, dict(window=17)), ([100], [30], 16, 8, 128, 16, dict(chunk=40)),
+    ([70], [30], 16, 8, 128, 16, dict(softcap=5.0)), ([64], [0], 16, 8, 64, 16, dict(sinks=True)), ([30], [20], 4, 2, 24, 16, {})])
+def test_32_bit_prompt_attention(lens, cached, nh, nkv, d, page, form):
+    from llm_infer_rust_b200.kernels import ops
+    k, v, table, cu, total, prefix, rows = _paged(lens, cached, nkv, d, page)
+    q, form = _rnd(sum(lens), nh * d, seed=3, scale=3.0), dict(form)
+    window, scale = form.pop("window", None), d ** -0.5
+    if form.pop("sinks", False):
+        form["sinks"] = _rnd(nh, seed=4)
+
+    def attend(q, lens, cu, total, prefix):
+        out = torch.empty_like(q)
+        ops.prefill_attention(q, k, v, out, table, cu, total, prefix, rows, len(lens), max(lens), nh, nkv, d, page, window, scale, **form)
+        return out
+    got = attend(q, lens, cu, total, prefix)
+    want = _attention_64(q, k, v, table, lens, cached, nh, nkv, d, page, scale, window or 0, form.get("chunk", 0), form.get("softcap", 0.0),
+                         form.get("sinks"))
+    # scores of up to 3 x 5 with sums of d terms in 32 bits: 2^-24 x 15 x (2 + log2 d) in the exponent, as much again in the sums
+    assert (got.double() - want).abs().max() <= 2.0 ** -24 * 400 * v.abs().max()
+    if len(lens) == 1:                                          # the same bits however the portion is cut
+        parts, ints = [], lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        cuts = [0, 1, lens[0] // 2, lens[0]]
+        for lo, hi in zip(cuts, cuts[1:]):
+            parts.append(attend(q[lo:hi].contiguous(), [hi - lo], ints(0, hi - lo), ints(cached[0] + hi), ints(cached[0] + lo)))
+        if not window and not form.get("chunk"):
+            assert torch.equal(torch.cat(parts), got)
+        else:                                                   # (a tile's first block follows its first query's window)
+            assert (torch.cat(parts) - got).abs().max() <= 2.0 ** -24 * 400 * v.abs().max()
+
+
+def test_32_bit_prompt_attention_of_infinities():
+    """Infinities and NaN of queries, keys and values come out where a plain softmax puts them."""
+    from llm_infer_rust_b200.kernels import ops
+    lens, cached, nh, nkv, d, page = [90], [0], 4, 2, 64, 16
+    k, v, table, cu, total, prefix, rows = _paged(lens, cached, nkv, d, page)
+    q = _rnd(90, nh * d, seed=3)
+    at = lambda position: (table[0, position // page].item(), position % page)
+    for what in ("value", "key", "query"):
+        kk, vv, qq = k.clone(), v.clone(), q.clone()
+        if what == "value":
+            vv[at(37)[0], 1, at(37)[1], 7] = float("inf")
+        elif what == "key":
+            kk[at(50)[0], 0, at(50)[1], 3] = float("nan")
+        else:
+            qq[66, 5] = float("-inf")
+        out = torch.empty_like(qq)
+        ops.prefill_attention(qq, kk, vv, out, table, cu, total, prefix, rows, 1, 90, nh, nkv, d, page, None, d ** -0.5)
+        want = _attention_64(qq, kk, vv, table, lens, cached, nh, nkv, d, page, d ** -0.5)
+        if what == "value":       # (a key that is not visible has the weight zero, and zero times infinity is a NaN in both kernels' blocks of keys)
+            seen = slice(37, 90)
+            assert torch.equal(out[seen].isinf(), want[seen].isinf()) and out[seen].isinf().sum() == 53 * 2
+            assert out[:32].isfinite().all()
+        else:
+            assert torch.equal(out.isnan(), want.isnan()) and out.isnan().any() and not out.isnan().all()
