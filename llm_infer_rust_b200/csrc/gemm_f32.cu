@@ -1,12 +1,22 @@
-// C[M, N] = A[M, K] . W[N, K]^T in true 32-bit: FFMA on CUDA cores only, no
-// tensor cores and no reduced-precision mode.  This is the matrix product of the
-// float32 engine (the reference's float path goes through libtorch matmul:
-// src/layers/linear.rs:5-7).
+// C[M, N] = A[M, K] . W[N, K]^T in true 32-bit: no reduced-precision mode.  This is the matrix product of the
+// float32 engine (the reference's float path goes through libtorch matmul: src/layers/linear.rs:5-7).
 //
-// The order of the additions depends on k alone: K is cut into chunks of 128 and spans of four chunks; a chunk is summed
-// over k in order, a span over its chunks in order, an element over its spans in order.  Both kernels below keep to it,
-// whatever M and N are, however many blocks share an element and wherever it sits in a tile, so a token's result is
-// bit-identical however the batch around it is cut.  (Short sums of short sums also round less than one long one.)
+// Products whose rows are whole 16-byte pieces run on the tensor cores in terms: a float is the exact sum of three bfloat16
+// numbers (8 + 8 + 8 bits), the product of two floats the sum of nine products of terms, each exact in float, and the six that
+// reach 2^-24 of it are taken.  32 k are summed by the tensor cores from zero, small products first (what an addition there cuts off
+// below a sum's last place stays that of 32 terms); those sums are added in float, an eighth of K (a span) in order, then the eight
+// spans in order.  That order depends on k alone and both kernels keep to it, split_kernel (tcgen05: many rows) and few_split_kernel
+// (mma.sync, which gives the same bits: the tests compare them), so a token's result is bit-identical however the batch around it
+// is cut.  Error against 64 bits 0.9e-7 of a product's norm (K = 1,024; FFMA in short sums 2.1e-7, in one chain 2.1e-6 for a model's
+// logits).  An element whose terms give no finite sum (an infinity has no second term) is summed again by FFMA; numbers below 2^-110
+// lose their third term to the smallest bfloat16.
+// Measured, us with FFMA tiles / in terms, layers of Qwen3-0.6B: QKV at 4, 32 and 300 rows 9.9 / 5.5, 41.7 / 11.0, 119 / 39 (65 of an
+// ideal 274 TFLOP/s: the terms are taken apart and the sums added up by CUDA cores), O 6.4 / 5.0, 40.8 / 9.7, 63 / 35, gate and up 11.0 / 7.3,
+// 43.2 / 15.6, 127 / 40, down 7.4 / 6.5, 40.8 / 13.6, 65 / 43; one row of large matrices is slower (151,936 x 1,024: 104 / 118).
+//
+// Other products (K or a distance between rows no multiple of four, unaligned pointers) and batched ones keep to FFMA on CUDA cores,
+// in an order of their own that depends on k alone as well: K is cut into chunks of 128 and spans of four chunks; a chunk is summed
+// over k in order, a span over its chunks in order, an element over its spans in order.
 //
 // few_rows_kernel (few rows): bound by reading W.  A warp takes 8 rows of W and one span: lane = (row of W, chunk), so
 //   the span's chunks are summed side by side and a product of 1,024 x 2,048 still has 512 warps at work.  W comes
@@ -23,6 +33,9 @@
 // and a distance between consecutive matrices of each operand): per-head products of a mixer, where head h's rows are
 // column ranges of wider matrices.
 #include <cooperative_groups.h>
+#include <cuda.h>
+
+#include <initializer_list>
 
 #include "common.cuh"
 
@@ -324,6 +337,486 @@ tiled_kernel(const Product p, int ksplit) {
   }
 }
 
+// ------------------------------------------------------------------ many rows, in terms
+constexpr int SP_BN = 128, SP_KS = 32, SP_SPANS = 8;                // rows of W a tile, k a stage, spans an element at most
+constexpr int SP_W_BYTES = SP_BN * SP_KS * 4;
+
+__device__ __forceinline__ void sp_init(uint64_t* bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void sp_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void sp_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void sp_load(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
+}
+template <bool ADDS>
+__device__ __forceinline__ void sp_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "n"(ADDS ? 1 : 0) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {                       // true in one lane of a whole warp
+  uint32_t is;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(is));
+  return is != 0;
+}
+__device__ __forceinline__ void sp_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void sp_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void sp_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void sp_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void sp_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void sp_st(uint32_t at, const uint32_t (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void sp_st(uint32_t at, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+               ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void sp_ld8(uint32_t at, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void sp_ld16(uint32_t at, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(at) : "memory");
+}
+
+// Two floats as three bfloat16 terms each, packed (the first float in the low half): x = high + mid + low exactly, each term
+// the rest rounded to eight bits.  (Rounded, not cut off: the products that are left out then have no common sign.  A value
+// that rounds to infinity gives no finite sum.)
+__device__ __forceinline__ void sp_split(float x, float y, uint32_t& high, uint32_t& mid, uint32_t& low) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(high) : "f"(y), "f"(x));
+  x -= __uint_as_float(high << 16);
+  y -= __uint_as_float(high & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(mid) : "f"(y), "f"(x));
+  x -= __uint_as_float(mid << 16);
+  y -= __uint_as_float(mid & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(low) : "f"(y), "f"(x));
+}
+
+// One element as plain FFMA: what stands where the terms gave no finite number (an infinity has no second term).
+__device__ __noinline__ float sp_plain(const float* __restrict__ a, const float* __restrict__ w, int k) {
+  float t = 0.0f;
+  for (int i = 0; i < k; ++i) t = fmaf(a[i], w[i], t);
+  return t;
+}
+__device__ __forceinline__ bool sp_finite(float t) { return fabsf(t) <= 3.402823466e38f; }
+
+template <int NT> struct SplitShape {
+  static constexpr int WARPS = 16;                                  // that take terms apart and add sums up
+  static constexpr int THREADS = (WARPS + 2) * 32;
+  static constexpr int GROUPS = WARPS / 4;                          // warps that share 32 rows of W
+  static constexpr int COLS = NT / GROUPS;                          // columns of the sums a thread
+  static constexpr int SLOTS = NT == 128 ? 2 : 4;                   // stages between their terms and their sums
+  static constexpr int TERMS = 3 * NT * SP_KS * 2;                  // bytes of a stage's terms of x
+  static constexpr int STAGE = SP_W_BYTES + NT * SP_KS * 4;
+  static constexpr int RING = NT == 128 ? 5 : 6;
+  static constexpr bool KEEPS = NT == 128;                          // (18 warps leave 96 registers a thread)
+  static constexpr int TMEM = 512;
+  static constexpr int W_TERMS = SLOTS * NT;                        // first column of the terms of W: 48 a slot
+  static constexpr int KEPT = W_TERMS + SLOTS * 48;
+  static_assert(KEPT + (KEEPS ? NT : 0) <= TMEM, "columns of tensor memory");
+  static constexpr int BYTES = 1024 + RING * STAGE + SLOTS * TERMS + (2 * RING + 2 * SLOTS) * 8 + 16;
+};
+
+struct SplitWork {
+  Product p;
+  int tokens;              // rows of x a tile: a multiple of 16 up to NT
+  int m_tiles, tiles, ksplit, spans_a_rank, span_stages, stages;
+  int* err;
+};
+
+// grid: tiles x ranks of a cluster, or (one rank) at most a block an SM, which walks over tiles.  Warp 16 issues the products, warp 17
+// the copies, the other sixteen take stages apart and add their sums up: of a stage's 1,800 cycles (112 rows of x) they need 900 and
+// 500, beside 1,600 of products, so neither side hides the other whole.
+template <int NT>
+__global__ void __launch_bounds__(SplitShape<NT>::THREADS, 1)
+split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const SplitWork job) {
+  using S = SplitShape<NT>;
+  constexpr int SLOTS = S::SLOTS, LAG = SLOTS - 1;
+  extern __shared__ unsigned char split_smem[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(split_smem) + 1023) & ~uintptr_t(1023));
+  unsigned char* terms = ring + S::RING * S::STAGE;
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(terms + SLOTS * S::TERMS);
+  uint64_t* raw_free = raw_full + S::RING;
+  uint64_t* terms_full = raw_free + S::RING;
+  uint64_t* done = terms_full + SLOTS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + SLOTS);
+  const Product& p = job.p;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = job.ksplit > 1 ? blockIdx.x % job.ksplit : 0;
+  const int first_tile = blockIdx.x / job.ksplit, tile_step = gridDim.x / job.ksplit;
+  const int k_lo = rank * job.spans_a_rank * job.span_stages;
+  const int k_hi = min(job.stages, k_lo + job.spans_a_rank * job.span_stages);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::RING; ++s) { sp_init(raw_full + s, 1); sp_init(raw_free + s, S::WARPS); }
+    for (int s = 0; s < SLOTS; ++s) { sp_init(terms_full + s, S::WARPS); sp_init(done + s, 1); }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == S::WARPS) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(S::TMEM) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  sp_fence_before();
+  __syncthreads();
+  sp_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  if (warp == S::WARPS + 1) {
+    if (lane == 0) {                                                // copies
+      pdl_wait();                                                   // (x, and where it was widened just now W, come from the kernel before)
+      const uint32_t bytes = SP_W_BYTES + job.tokens * SP_KS * 4;
+      int it = 0;
+      bool ok = true;
+      for (int tile = first_tile; tile < job.tiles && ok; tile += tile_step) {
+        const int n0 = tile / job.m_tiles * SP_BN, m0 = tile % job.m_tiles * job.tokens;
+        for (int kst = k_lo; kst < k_hi; ++kst, ++it) {
+          const int s = it % S::RING;
+          unsigned char* st = ring + s * S::STAGE;
+          if (it >= S::RING && !mbar_wait(raw_free + s, (it / S::RING - 1) & 1, job.err)) { ok = false; break; }
+          sp_expect(raw_full + s, bytes);
+          sp_load(st, &wmap, kst * SP_KS, n0, raw_full + s);
+          sp_load(st + SP_W_BYTES, &xmap, kst * SP_KS, m0, raw_full + s);
+        }
+      }
+      for (int j = it > S::RING ? it - S::RING : 0; j < it; ++j)    // no copy is left behind, whatever ran out
+        mbar_wait(raw_full + j % S::RING, (j / S::RING) & 1, job.err);
+    }
+    __syncwarp();
+  } else if (warp == S::WARPS) {
+    // products: the whole warp walks along, so that descriptors are made once a warp (in uniform registers); one lane issues
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(job.tokens >> 3) << 17) | ((SP_BN >> 4) << 24);
+    // terms of x: 8 rows x 16 bytes are contiguous, the next 8 rows follow, the next 8 k come NT x 16 bytes further on
+    const uint64_t layout = (static_cast<uint64_t>(NT * 16 >> 4) << 16) | (static_cast<uint64_t>(128 >> 4) << 32) | (1ull << 46);
+    const uint64_t first_b = layout | ((smem_u32(terms) >> 4) & 0x3FFFu);          // (the addresses' low bits never carry)
+    int it = 0;
+    bool ok = true;
+    for (int tile = first_tile; tile < job.tiles && ok; tile += tile_step)
+      for (int kst = k_lo; kst < k_hi; ++kst, ++it) {
+        const int s = it % SLOTS;
+        const bool mine = mbar_wait(terms_full + s, (it / SLOTS) & 1, job.err);
+        ok = __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
+        if (!ok) break;
+        sp_fence_after();
+        const uint32_t d = tmem + s * NT, a = tmem + S::W_TERMS + s * 48;
+        const uint64_t b = first_b + static_cast<uint32_t>(s * (S::TERMS >> 4));
+        if (elect_one()) {
+          // small products first: what they add is then not cut off below a large sum's last place
+          constexpr int WI[6] = {2, 0, 1, 1, 0, 0}, XI[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+          for (int q = 0; q < 12; ++q) {
+            const int half = q & 1, t = q >> 1;
+            if (q == 0) sp_mma<false>(d, a + WI[t] * 16 + half * 8, b + ((XI[t] * (NT * SP_KS * 2) + half * (2 * NT * 16)) >> 4), idesc);
+            else sp_mma<true>(d, a + WI[t] * 16 + half * 8, b + ((XI[t] * (NT * SP_KS * 2) + half * (2 * NT * 16)) >> 4), idesc);
+          }
+          sp_commit(done + s);
+        }
+        __syncwarp();
+      }
+    __syncwarp();
+  } else {
+    const int row = (warp & 3) * 32 + lane, group = warp >> 2;
+    const uint32_t lane_at = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    // a span's sums, and the element's so far: in registers, or (128 columns) beside the terms in tensor memory
+    float sum[S::COLS], held[S::KEEPS ? 1 : S::COLS];
+    const uint32_t kept = tmem + lane_at + S::KEPT + group * S::COLS;
+    constexpr int CHUNKS = 8 / S::GROUPS;                           // 16-byte pieces of a row's 32 k
+    int it = 0;
+    bool ok = true;
+
+    // the sums of stage `of` go to the span's
+    auto add_up = [&](int of, bool first) {
+      const int s = of % SLOTS;
+      const bool mine = mbar_wait(done + s, (of / SLOTS) & 1, job.err);
+      if (!__all_sync(0xffffffffu, mine ? 1 : 0)) return false;
+      sp_fence_after();
+      const uint32_t at = tmem + lane_at + s * NT + group * S::COLS;
+      constexpr int STEP = S::COLS < 16 ? S::COLS : 16;
+#pragma unroll
+      for (int c = 0; c < S::COLS; c += STEP) {
+        uint32_t v[STEP];
+        if constexpr (STEP == 8) sp_ld8(at + c, v); else sp_ld16(at + c, v);
+        sp_wait_ld();
+#pragma unroll
+        for (int e = 0; e < STEP; ++e) sum[c + e] = first ? __uint_as_float(v[e]) : sum[c + e] + __uint_as_float(v[e]);
+      }
+      sp_fence_before();
+      return true;
+    };
+    auto span_ends = [&](int kst) {                                 // after stage kst of the rank's
+      const int at = kst - k_lo;
+      if (kst + 1 != k_hi && (at + 1) % job.span_stages != 0) return;
+      if (job.ksplit > 1 && kst + 1 == k_hi && at >= job.span_stages) return;      // (two spans a rank: the second stays in sum)
+      const bool first = at < job.span_stages;
+      if constexpr (S::KEEPS) {
+#pragma unroll
+        for (int c = 0; c < S::COLS; c += 8) {
+          uint32_t v[8];
+          if (!first) {
+            sp_ld8(kept + c, v);
+            sp_wait_ld();
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(first ? sum[c + e] : __uint_as_float(v[e]) + sum[c + e]);
+          sp_st(kept + c, v);
+        }
+        sp_wait_st();
+      } else {
+#pragma unroll
+        for (int c = 0; c < S::COLS; ++c) held[c] = first ? sum[c] : held[c] + sum[c];
+      }
+    };
+    // calls f(column, its total) for the thread's columns
+    auto totals = [&](auto f) {
+      if constexpr (S::KEEPS) {
+#pragma unroll
+        for (int c = 0; c < S::COLS; c += 8) {
+          uint32_t v[8];
+          sp_ld8(kept + c, v);
+          sp_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f(c + e, __uint_as_float(v[e]));
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < S::COLS; ++c) f(c, held[c]);
+      }
+    };
+
+    pdl_wait();
+    for (int tile = first_tile; tile < job.tiles && ok; tile += tile_step) {
+      const int n0 = tile / job.m_tiles * SP_BN, m0 = tile % job.m_tiles * job.tokens;
+      const int it0 = it - k_lo;
+      for (int kst = k_lo; kst < k_hi + LAG; ++kst) {
+        if (kst < k_hi) {
+          const int slot = it % S::RING, s = it % SLOTS;
+          const bool mine = mbar_wait(raw_full + slot, (it / S::RING) & 1, job.err);
+          ok = __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
+          if (!ok) break;
+          const unsigned char* w_raw = ring + slot * S::STAGE + row * 128;
+          const unsigned char* x_raw = w_raw + SP_W_BYTES;
+          uint32_t high[2 * CHUNKS], mid[2 * CHUNKS], low[2 * CHUNKS];
+#pragma unroll
+          for (int c = 0; c < CHUNKS; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(w_raw + (((group * CHUNKS + c) ^ (row & 7)) << 4));
+            sp_split(v.x, v.y, high[2 * c], mid[2 * c], low[2 * c]);
+            sp_split(v.z, v.w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
+          }
+          const uint32_t at = tmem + lane_at + S::W_TERMS + s * 48 + group * 2 * CHUNKS;
+          sp_st(at, high);
+          sp_st(at + 16, mid);
+          sp_st(at + 32, low);
+          if (row < job.tokens) {
+#pragma unroll
+            for (int c = 0; c < CHUNKS; ++c) {
+              const float4 v = *reinterpret_cast<const float4*>(x_raw + (((group * CHUNKS + c) ^ (row & 7)) << 4));
+              sp_split(v.x, v.y, high[2 * c], mid[2 * c], low[2 * c]);
+              sp_split(v.z, v.w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
+            }
+            unsigned char* to = terms + s * S::TERMS + (row >> 3) * 128 + (row & 7) * 16;
+#pragma unroll
+            for (int c = 0; c < CHUNKS; c += 2) {
+              unsigned char* q = to + (group * CHUNKS + c) / 2 * (NT * 16);
+              *reinterpret_cast<uint4*>(q) = make_uint4(high[2 * c], high[2 * c + 1], high[2 * c + 2], high[2 * c + 3]);
+              *reinterpret_cast<uint4*>(q + NT * SP_KS * 2) = make_uint4(mid[2 * c], mid[2 * c + 1], mid[2 * c + 2], mid[2 * c + 3]);
+              *reinterpret_cast<uint4*>(q + 2 * NT * SP_KS * 2) = make_uint4(low[2 * c], low[2 * c + 1], low[2 * c + 2], low[2 * c + 3]);
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+          sp_wait_st();
+          sp_fence_before();
+          __syncwarp();
+          if (lane == 0) { sp_arrive(raw_free + slot); sp_arrive(terms_full + s); }
+          ++it;
+        }
+        const int past = kst - LAG;                                 // the stage whose sums are added up meanwhile
+        if (past >= k_lo) {
+          ok = add_up(it0 + past, (past - k_lo) % job.span_stages == 0);
+          if (!ok) break;
+          span_ends(past);
+        }
+      }
+      if (!ok || job.ksplit > 1) break;
+      const int n = n0 + row;
+      totals([&](int c, float v) {
+        const int t = group * S::COLS + c, m = m0 + t;
+        if (t < job.tokens && m < p.m && n < p.n) {
+          if (!sp_finite(v)) v = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
+          p.c[static_cast<size_t>(m) * p.ldc + n] = v;
+        }
+      });
+    }
+    if (job.ksplit > 1) {
+      // (every copy has landed and every product has ended: the ring holds the spans' sums from here on)
+      float* parts = reinterpret_cast<float*>(ring);                // [spans a rank][NT][128]
+      asm volatile("bar.sync 1, %0;\n" ::"n"(S::WARPS * 32) : "memory");
+      totals([&](int c, float v) { parts[(group * S::COLS + c) * SP_BN + row] = v; });
+      if (job.spans_a_rank > 1)
+#pragma unroll
+        for (int c = 0; c < S::COLS; ++c) parts[(NT + group * S::COLS + c) * SP_BN + row] = sum[c];
+    }
+    __syncwarp();
+  }
+  if (job.ksplit > 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const int n0 = first_tile / job.m_tiles * SP_BN, m0 = first_tile % job.m_tiles * job.tokens;
+    const int spans = (job.stages + job.span_stages - 1) / job.span_stages;
+    const float* parts = reinterpret_cast<const float*>(ring);
+    for (int i = rank * S::THREADS + threadIdx.x; i < job.tokens * SP_BN; i += job.ksplit * S::THREADS) {
+      const int m = m0 + i / SP_BN, n = n0 + i % SP_BN;
+      float v[SP_SPANS], t = 0.0f;
+#pragma unroll
+      for (int s = 0; s < SP_SPANS; ++s)
+        if (s < spans) v[s] = cluster.map_shared_rank(parts, s / job.spans_a_rank)[s % job.spans_a_rank * NT * SP_BN + i];
+#pragma unroll
+      for (int s = 0; s < SP_SPANS; ++s)
+        if (s < spans) t = s == 0 ? v[s] : t + v[s];
+      if (m < p.m && n < p.n) {
+        if (!sp_finite(t)) t = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
+        p.c[static_cast<size_t>(m) * p.ldc + n] = t;
+      }
+    }
+    cluster.sync();                                                 // the sums are read: the block may end
+  }
+  sp_fence_before();
+  __syncthreads();
+  if (warp == S::WARPS) {
+    sp_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::TMEM) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ few rows, in the same terms
+// The same products in the same order through mma.sync, whose sums have the bits of tcgen05's (the tests compare them): what a
+// warp needs of W (16 rows, one span) comes through a ring of cp.async stages that only this warp reads, is taken apart in
+// registers and multiplied there, without the way through tensor memory and its barriers.  The eight warps of a block take the
+// eight spans of a tile and their sums meet in shared memory.
+template <int MR, int WN> struct FewSplit {                         // rows of x a block, rows of W a tile
+  static constexpr int WARPS = SP_SPANS;
+  static constexpr int RING = WN == 16 ? (MR == 8 ? 4 : 3) : (MR == 8 ? 10 : 6);
+  static constexpr int STAGE = (WN + MR) * SP_KS;                   // floats
+  static constexpr int RED = WARPS * WN * MR;                       // floats of a tile's spans
+  static constexpr int BYTES = (WARPS * RING * STAGE + 2 * RED) * 4;
+};
+
+__device__ __forceinline__ void sp_mma_sync(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// grid (blocks, groups of MR rows of x).  WN = 8 leaves half of an instruction's rows empty: for products whose tiles of 16 would
+// not reach every SM.
+template <int MR, int WN>
+__global__ void __launch_bounds__(256, MR == 8 && WN == 16 ? 2 : 1)
+few_split_kernel(const Product p, int tiles, int stages, int span_stages) {
+  using F = FewSplit<MR, WN>;
+  extern __shared__ __align__(128) float few_split_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c4 = lane & 3;
+  const int m0 = blockIdx.y * MR;
+  float* ring = few_split_smem + warp * F::RING * F::STAGE;
+  float* red = few_split_smem + F::WARPS * F::RING * F::STAGE;      // [2][8 spans][16][MR]
+  const int k_lo = min(stages, warp * span_stages), mine = min(stages, k_lo + span_stages) - k_lo;      // this warp's stages of a tile
+  const int spans = (stages + span_stages - 1) / span_stages;
+  const int my_tiles = static_cast<int>(blockIdx.x) < tiles ? (tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0, steps = my_tiles * mine;
+
+  // Stage `step` of this warp: 16 rows of W and the rows of x, 32 k each; a row's 16-byte pieces are exchanged by twice its number
+  // mod 4, so that the four rows of a half warp's reads lie in different banks.
+  int f_tile = blockIdx.x, f_at = 0;
+  auto fetch = [&](int step) {
+    if (step < steps) {
+      float* st = ring + step % F::RING * F::STAGE;
+      const int k0 = (k_lo + f_at) * SP_KS;
+#pragma unroll
+      for (int j = 0; j < (WN + MR) / 4; ++j) {
+        const int line = j * 4 + (lane >> 3), piece = lane & 7, kk = k0 + piece * 4;
+        const bool of_w = line < WN;
+        const int row = of_w ? f_tile * WN + line : m0 + line - WN;
+        const bool valid = row < (of_w ? p.n : p.m) && kk < p.k;
+        const float* src = of_w ? p.w + static_cast<size_t>(row) * p.ldw + kk : p.a + static_cast<size_t>(row) * p.lda + kk;
+        cp_async16(st + line * SP_KS + ((piece ^ (2 * (line & 3))) << 2), valid ? src : p.w, valid);
+      }
+      if (++f_at == mine) { f_at = 0; f_tile += gridDim.x; }
+    }
+    cp_async_commit();
+  };
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < F::RING - 1; ++s) fetch(s);
+
+  int step = 0, parity = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, parity ^= 1) {
+    float sum[MR / 8][4];
+    for (int at = 0; at < mine; ++at, ++step) {
+      fetch(step + F::RING - 1);
+      cp_async_wait<F::RING - 1>();
+      __syncwarp();
+      const float* st = ring + step % F::RING * F::STAGE;
+      float t[MR / 8][4] = {};
+      uint32_t a[2][3][4], b[MR / 8][2][3][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                                 // sixteen k each
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (WN == 8 && (e & 1)) {
+            a[h][0][e] = a[h][1][e] = a[h][2][e] = 0;
+            continue;
+          }
+          const int line = r + (e & 1) * 8, piece = h * 4 + (e >> 1) * 2 + (c4 >> 1);
+          const float2 v = *reinterpret_cast<const float2*>(st + line * SP_KS + ((piece ^ (2 * (line & 3))) << 2) + (c4 & 1) * 2);
+          sp_split(v.x, v.y, a[h][0][e], a[h][1][e], a[h][2][e]);
+        }
+#pragma unroll
+        for (int x = 0; x < MR / 8; ++x)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int line = WN + x * 8 + r, piece = h * 4 + e * 2 + (c4 >> 1);
+            const float2 v = *reinterpret_cast<const float2*>(st + line * SP_KS + ((piece ^ (2 * (line & 3))) << 2) + (c4 & 1) * 2);
+            sp_split(v.x, v.y, b[x][h][0][e], b[x][h][1][e], b[x][h][2][e]);
+          }
+      }
+      constexpr int WI[6] = {2, 0, 1, 1, 0, 0}, XI[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+      for (int q = 0; q < 12; ++q)
+#pragma unroll
+        for (int x = 0; x < MR / 8; ++x) sp_mma_sync(t[x], a[q & 1][WI[q >> 1]], b[x][q & 1][XI[q >> 1]]);
+#pragma unroll
+      for (int x = 0; x < MR / 8; ++x)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[x][i] = at == 0 ? t[x][i] : sum[x][i] + t[x][i];
+      __syncwarp();                                                 // the stage is read
+    }
+    float* to = red + (parity * F::WARPS + warp) * WN * MR;
+    if (mine > 0)
+#pragma unroll
+      for (int x = 0; x < MR / 8; ++x)
+#pragma unroll
+        for (int i = 0; i < WN / 4; ++i) to[(x * 8 + 2 * c4 + (i & 1)) * WN + r + (i >> 1) * 8] = sum[x][i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < WN * MR; i += 256) {           // the element: its spans in order
+      const int m = m0 + i / WN, n = tile * WN + i % WN;
+      if (m >= p.m || n >= p.n) continue;
+      const float* from = red + parity * F::WARPS * WN * MR + i;
+      float v = from[0];
+      for (int s = 1; s < spans; ++s) v += from[s * WN * MR];
+      if (!sp_finite(v)) v = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
+      p.c[static_cast<size_t>(m) * p.ldc + n] = v;
+    }
+  }
+  cp_async_wait<0>();
+}
+
 // ------------------------------------------------------------------ launchers
 constexpr size_t FEW_SMEM_LIMIT = 225 * 1024;
 constexpr int DEVICES = 16;                     // whose launch limits are remembered
@@ -370,11 +863,135 @@ static int blocks_a_tile(long long tiles, int spans, int sms) {
 }
 B200_EXPORT int b200_gemm_f32_blocks_a_tile(long long tiles, int spans, int sms) { return blocks_a_tile(tiles, spans, sms); }
 
-static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
+// What a product costs split_kernel, in stages of one block: rounds of blocks over the SMs, each its stages and what begins and ends a
+// block (a cluster's placement and its exchange of sums take as long as eleven stages).  `ranks`: how many blocks share a tile's k,
+// one or two spans each.  (Measured with one, four and eight: 4,096 x 1,024 at 64 rows 31 / 21 / 38 us, 6,144 x 1,024 at 64 31 / 41 /
+// 50, 1,024 x 3,072 at 300 99 / 43 / 48.)
+static long long split_cost(int tiles, int spans, int stages, int sms, int& ranks) {
+  ranks = 1;
+  long long least = static_cast<long long>((tiles + sms - 1) / sms) * (stages + 3);
+  for (int r : {(spans + 1) / 2, spans}) {
+    const long long cost = (static_cast<long long>(tiles) * r + sms - 1) / sms * ((stages + r - 1) / r + 11);
+    if (spans >= 3 && cost < least) { ranks = r; least = cost; }
+  }
+  return least;
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// Boxes of `box_rows` rows x 32 floats, 128-byte swizzle; what lies outside reads as zeros.
+static int encode_rows(CUtensorMap* map, const float* base, int rows, int cols, int ld, int box_rows) {
+  static EncodeTiledFn encode = nullptr;
+  if (encode == nullptr) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (fn == nullptr || found != cudaDriverEntryPointSuccess) return static_cast<int>(cudaErrorNotSupported);
+    encode = reinterpret_cast<EncodeTiledFn>(fn);
+  }
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * sizeof(float)};
+  const cuuint32_t box[2] = {SP_KS, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t elem_strides[2] = {1u, 1u};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, elem_strides,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 1000 + static_cast<int>(r);
+}
+
+static SplitWork split_work(const Product& p, int nt, int sms, int* err, long long& cost) {
+  SplitWork job = {};
+  job.p = p;
+  job.err = err;
+  job.m_tiles = (p.m + nt - 1) / nt;
+  job.tokens = ((p.m + job.m_tiles - 1) / job.m_tiles + 15) / 16 * 16;
+  job.m_tiles = (p.m + job.tokens - 1) / job.tokens;
+  const long long tiles = static_cast<long long>((p.n + SP_BN - 1) / SP_BN) * job.m_tiles;
+  job.tiles = tiles > (1 << 28) ? 0 : static_cast<int>(tiles);
+  job.stages = (p.k + SP_KS - 1) / SP_KS;
+  job.span_stages = (job.stages + SP_SPANS - 1) / SP_SPANS;
+  const int spans = (job.stages + job.span_stages - 1) / job.span_stages;
+  cost = split_cost(job.tiles, spans, job.stages, sms, job.ksplit);
+  job.spans_a_rank = job.ksplit > 1 ? (spans + job.ksplit - 1) / job.ksplit : spans;
+  return job;
+}
+
+template <int NT>
+static int launch_split(const SplitWork& job, int device, int sms, cudaStream_t stream) {
+  using S = SplitShape<NT>;
+  static bool configured[DEVICES];
+  if (device >= DEVICES || !configured[device]) {
+    cudaError_t e = cudaFuncSetAttribute(split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (device < DEVICES) configured[device] = true;
+  }
+  const Product& p = job.p;
+  if (job.tiles <= 0) return B200_BAD_SIZE;
+  CUtensorMap wmap, xmap;
+  int rc = encode_rows(&wmap, p.w, p.n, p.k, p.ldw, SP_BN);
+  if (rc == 0) rc = encode_rows(&xmap, p.a, p.m, p.k, p.lda, job.tokens);
+  if (rc != 0) return rc;
+  const int grid = job.ksplit > 1 ? job.tiles * job.ksplit : job.tiles < sms ? job.tiles : sms;
+  return b200_launch(split_kernel<NT>, dim3(grid), dim3(S::THREADS), S::BYTES, stream, job.ksplit > 1 ? job.ksplit : 0, wmap, xmap, job);
+}
+
+template <int MR, int WN>
+static int launch_few_split(const Product& p, int device, int sms, cudaStream_t stream) {
+  using F = FewSplit<MR, WN>;
+  static bool configured[DEVICES];
+  if (device >= DEVICES || !configured[device]) {
+    cudaError_t e = cudaFuncSetAttribute(few_split_kernel<MR, WN>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::BYTES);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (device < DEVICES) configured[device] = true;
+  }
+  const int tiles = (p.n + WN - 1) / WN, stages = (p.k + SP_KS - 1) / SP_KS, span_stages = (stages + SP_SPANS - 1) / SP_SPANS;
+  const int places = sms * (MR == 8 && WN == 16 ? 2 : 1);
+  const dim3 grid(tiles < places ? tiles : places, (p.m + MR - 1) / MR);
+  return b200_launch(few_split_kernel<MR, WN>, grid, dim3(256), F::BYTES, stream, 0, p, tiles, stages, span_stages);
+}
+
+// Which kernel takes a product in terms: few_split_kernel up to 16 rows, and up to 128 in groups of 32 where that is the shorter way.
+// Its groups cost a tile of 16 rows of W 0.135 us a stage, a block an SM at a time (and 2.7 us to begin), split_kernel's stage costs 0.88
+// us with up to 64 rows of x and 1.1 with 128.  (us on few_split / split, 32 rows: 4,096 x 1,024 11.0 / 17.3, 4,096 x 12,288 95 / 88; 64
+// rows: 1,024 x 2,048 9.9 / 16.3, 4,096 x 4,096 67 / 42, 151,936 x 1,024 593 / 252; 96: 1,024 x 2,048 18.6 / 20.3, 6,144 x 1,024 39.4 / 38.8.)
+// Tiles of eight rows of W where those of sixteen leave SMs without a block (1,024 x 2,048, one row: 5.6 -> 4.9 us).
+static bool few_split_takes(const Product& p, int sms, long long split_stages, int nt) {
+  if (p.m <= 16) return true;
+  if (p.m > 128) return false;
+  const long long tiles = static_cast<long long>((p.n + 15) / 16) * ((p.m + 31) / 32), stages = (p.k + SP_KS - 1) / SP_KS;
+  return 20 + (tiles + sms - 1) / sms * stages <= split_stages * (nt == 64 ? 13 : 16) / 2;
+}
+
+static int launch_terms(const Product& p, int* err, int device, int sms, cudaStream_t stream) {
+  const int nt = p.m <= 64 ? 64 : 128;
+  long long cost = 0;
+  const SplitWork job = split_work(p, nt, sms, err, cost);
+  if (few_split_takes(p, sms, cost, nt)) {
+    const bool narrow = (p.n + 15) / 16 < sms;
+    if (p.m <= 8) return narrow ? launch_few_split<8, 8>(p, device, sms, stream) : launch_few_split<8, 16>(p, device, sms, stream);
+    if (p.m <= 16) return narrow ? launch_few_split<16, 8>(p, device, sms, stream) : launch_few_split<16, 16>(p, device, sms, stream);
+    return launch_few_split<32, 16>(p, device, sms, stream);
+  }
+  return nt == 64 ? launch_split<64>(job, device, sms, stream) : launch_split<128>(job, device, sms, stream);
+}
+// (0: few_split_kernel, 1: split_kernel)
+B200_EXPORT int b200_gemm_f32_route(int m, int n, int k, int sms) {
+  Product p = {};
+  p.m = m; p.n = n; p.k = k;
+  long long cost = 0;
+  split_work(p, m <= 64 ? 64 : 128, sms, nullptr, cost);
+  return few_split_takes(p, sms, cost, m <= 64 ? 64 : 128) ? 0 : 1;
+}
+
+static int launch(const Product& p, int batch, bool vec, int* err, cudaStream_t stream) {
   int device = 0, sms = 148;
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return static_cast<int>(e);
+  if (vec && batch == 1) return launch_terms(p, err, device, sms, stream);
   const int spans = (p.k + SPAN - 1) / SPAN;
   // Up to 16 rows the weights are streamed, in passes of `mr` rows: as many as fit shared memory beside the rings, 16 to K = 1,536
   // (2,048 where N leaves a block one tile), 8 to 3,072, 4 beyond.  One pass is 2 to 9 times as fast as a tile of 64 that is
@@ -418,20 +1035,20 @@ static int launch(const Product& p, int batch, bool vec, cudaStream_t stream) {
 
 static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
-B200_EXPORT int b200_gemm_f32(const float* a, const float* w, float* c, int m, int n, int k, cudaStream_t stream) {
+B200_EXPORT int b200_gemm_f32(const float* a, const float* w, float* c, int m, int n, int k, int* err, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (k <= 0) return B200_BAD_SIZE;
   const Product p = {a, w, c, m, n, k, k, k, n, 0, 0, 0};
-  return launch(p, 1, k % 4 == 0 && aligned16(a) && aligned16(w), stream);
+  return launch(p, 1, k % 4 == 0 && aligned16(a) && aligned16(w), err, stream);
 }
 
 // c[b] (m x n, rows ldc apart) = a[b] (m x k, rows lda apart) . w[b] (n x k, rows ldw apart)^T for b < batch; matrix b
 // of an operand starts step_* floats behind matrix b - 1.
 B200_EXPORT int b200_gemm_f32_batched(const float* a, const float* w, float* c, int m, int n, int k, int batch, int lda,
                                       int ldw, int ldc, long long step_a, long long step_w, long long step_c,
-                                      cudaStream_t stream) {
+                                      int* err, cudaStream_t stream) {
   if (m <= 0 || n <= 0 || batch <= 0) return 0;
   if (k <= 0 || lda < k || ldw < k || ldc < n || batch > 65535) return B200_BAD_SIZE;
   const Product p = {a, w, c, m, n, k, lda, ldw, ldc, step_a, step_w, step_c};
-  return launch(p, batch, k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && step_a % 4 == 0 && step_w % 4 == 0 && aligned16(a) && aligned16(w), stream);
+  return launch(p, batch, k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && step_a % 4 == 0 && step_w % 4 == 0 && aligned16(a) && aligned16(w), err, stream);
 }

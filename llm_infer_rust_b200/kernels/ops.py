@@ -1467,7 +1467,7 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, mode: int = GEMM_PLAIN, glu: 
 
 # --------------------------------------------------------------------------- matrix products
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """a[M, K] . w[N, K]^T in true 32-bit on CUDA cores."""
+    """a[M, K] . w[N, K]^T in true 32-bit; a row's result has the same bits whatever the other rows."""
     _cuda(a, w, out)
     _contig(a, w, out)
     if a.dtype != torch.float32 or w.dtype != torch.float32 or a.shape[1] != w.shape[1]:
@@ -1476,7 +1476,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     n = w.shape[0]
     if out is None:
         out = _empty((m, n), torch.float32, a.device)
-    rc = load_entry_points("gemm_f32.cu").b200_gemm_f32(a, w, out, m, n, k, _stream())
+    rc = load_entry_points("gemm_f32.cu").b200_gemm_f32(a, w, out, m, n, k, error_word(a.device), _stream())
     _ok(rc, "gemm_f32")
     return out
 
@@ -1499,7 +1499,8 @@ def head_products(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
     if x.dtype == torch.float32:
         rc = load_entry_points("gemm_f32.cu").b200_gemm_f32_batched(
             x, weight, out, rows, n, k, heads, x.stride(1), k, out.stride(1),
-            int(x.stride(0)), int(n * k), int(out.stride(0)), _stream())
+            int(x.stride(0)), int(n * k), int(out.stride(0)),
+            error_word(x.device), _stream())
         _ok(rc, "gemm_f32_batched")
         return out
     if x.dtype != torch.bfloat16:

@@ -25,6 +25,57 @@ def test_32_bit_products(m, n, k):
         assert torch.equal(ops.gemm_f32(a[r:r + 1].contiguous(), w)[0], got[r])
 
 
+# groups of 8, 16 and 32 rows of x and tiles of 64 and 128, each with a rest; one row of W beyond a tile; K of one stage (32), of spans of
+# one stage and of several, with a rest; one, three, four and eight blocks a tile; few columns and many
+@pytest.mark.parametrize("m,n,k", [(1, 127, 4), (9, 129, 32), (16, 2500, 36), (17, 128, 36), (32, 1024, 3072), (33, 257, 256), (64, 300, 260),
+                                   (40, 20000, 1056), (65, 1024, 2048), (100, 30000, 256), (128, 130, 1056), (129, 640, 96), (257, 128, 8000),
+                                   (300, 2500, 1024), (300, 1030, 3072), (4, 20000, 1024), (8, 4100, 12288)])
+def test_32_bit_products_in_three_terms(m, n, k):
+    from llm_infer_rust_b200.kernels import ops
+    for offset in (0.0, 1.0):                                   # sums that cancel, and sums that grow
+        a, w = _rnd(m, k) + offset, _rnd(n, k, seed=1) + offset
+        got = ops.gemm_f32(a, w)
+        want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+        # 32 k: twelve sums on the tensor cores, which may cut off a last place (2^-23) each; then K / 256 + 2 stages a span and
+        # eight spans, roundings of 2^-24; what three of the nine products leave out is 2^-24 at most
+        assert ((got.double() - want).abs() <= (24 + 1 + k / 256 + 10) * 2.0 ** -24 * size).all()
+        # bit for bit what rows give alone and in the other kernels' counts
+        for rows in (slice(0, 1), slice(m // 2, m // 2 + 1), slice(m - 1, m), slice(0, 8), slice(0, 16), slice(0, 50), slice(0, 130)):
+            assert torch.equal(ops.gemm_f32(a[rows].contiguous(), w), got[rows])
+        ops.check_errors(a.device)
+
+
+@pytest.mark.parametrize("spread", [3.0, 8.0, None])
+def test_32_bit_products_of_few_and_many_rows_have_the_same_bits(spread):
+    """mma.sync and tcgen05 cut off what does not fit their sums at the same place, whatever the numbers: wide spreads, cancelling pairs."""
+    from llm_infer_rust_b200.kernels import ops
+    a, w = _rnd(140, 512), _rnd(20000, 512, seed=1)
+    if spread is not None:
+        a, w = a * torch.exp(spread * _rnd(140, 512, seed=2)), w * torch.exp(spread * _rnd(20000, 512, seed=3))
+    else:
+        a[:, 1::2], w[:, 1::2] = a[:, 0::2], -w[:, 0::2] * (1 + 1e-6 * _rnd(20000, 256, seed=4))
+    whole = ops.gemm_f32(a, w)
+    for rows in (8, 16, 32):
+        assert torch.equal(torch.cat([ops.gemm_f32(a[i:i + rows].contiguous(), w) for i in range(0, 140, rows)]), whole)
+
+
+def test_32_bit_products_of_infinities_and_the_largest_numbers():
+    """A value without three finite terms: an infinity, a NaN, a number that rounds to a bfloat16 infinity."""
+    from llm_infer_rust_b200.kernels import ops
+    for m, n, k in ((3, 200, 256), (40, 130, 2048), (200, 300, 1024), (150, 20000, 64)):
+        a, w = _rnd(m, k), _rnd(n, k, seed=1)
+        a[0, 5], a[1, 9], a[2, 1], w[11, 4], w[5, 5] = float("inf"), float("nan"), 3.4e38, float("-inf"), 0.0
+        w[:, 1] *= 0.1
+        got, want = ops.gemm_f32(a, w), a.double() @ w.double().t()
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        assert torch.equal(got[got.isinf()].double(), want[want.isinf()])
+        fine = want.isfinite()
+        assert fine[2].any() and ((got.double() - want).abs()[fine] <= 1e-5 * want.abs().clamp_min(10.0)[fine]).all()
+    small, w = _rnd(5, 64) * 1e-30, _rnd(130, 64, seed=1)
+    want, size = small.double() @ w.double().t(), small.double().abs() @ w.double().abs().t()
+    assert ((ops.gemm_f32(small, w).double() - want).abs() <= 40 * 2.0 ** -24 * size).all()
+
+
 def test_32_bit_products_of_a_head_each():
     from llm_infer_rust_b200.kernels import ops
     for rows in (3, 70):
