@@ -116,6 +116,15 @@ __device__ __forceinline__ void umma_a_tmem(uint32_t tmem_c, uint32_t tmem_a, ui
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
+// True in one lane of a whole warp.  The warp that issues products walks along as a whole and only the instruction itself is one
+// lane's: what comes before it is then the same in every lane for all the compiler knows, and descriptors are made in uniform
+// registers, where the instruction takes them.  (From one lane's own registers every product waited for eight moves.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(is));
+  return is != 0;
+}
+__device__ __forceinline__ int same_in_warp(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -601,7 +610,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
   constexpr int SOFTMAX_WARPS = SHAPED ? 8 : 4;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = same_in_warp(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < K_STAGES; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); }
     for (int s = 0; s < V_STAGES; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
@@ -622,7 +631,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = same_in_warp(*tmem_slot);
   pdl_launch_dependents();
   pdl_wait();                                  // q, the step's index arrays and the newest keys and values come from earlier kernels
 
@@ -643,7 +652,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   int k_begin = window > 0 ? max(0, p_lo - window + 1) : 0;
   if (SHAPED && shape.chunk > 0) k_begin = max(k_begin, p_lo - p_lo % shape.chunk);
   k_begin -= k_begin % BKV;
-  const int nblk = active ? (kv_end - k_begin + BKV - 1) / BKV : 0;
+  const int nblk = same_in_warp(active ? (kv_end - k_begin + BKV - 1) / BKV : 0);
   const int* table = block_table + static_cast<size_t>(row) * table_stride;
 
   if (warp == 0 || warp >= 2 + SOFTMAX_WARPS) {
@@ -694,46 +703,51 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
       if (ok) fetch(&vmap, sm + V_OFF + s * TILE, v_full + s, k_begin + i * BKV);
     }
   } else if (warp == 1) {
-    // ---- MMA issue (one lane): S_0, S_1; then for every block: O += P V of block i, S of block i + 2
-    if (lane == 0 && nblk > 0) {
-      bool ok = mbar_wait(q_full, 0, err);
-      const uint32_t q_addr = smem_u32(sm + Q_OFF);
+    // ---- MMA issue: S_0, S_1; then for every block: O += P V of block i, S of block i + 2
+    if (nblk > 0) {
+      bool ok = mbar_wait_warp(q_full, 0, err);
       const uint32_t tmem_o = tmem_base + 256;
+      // (descriptors differ in their start address only, the low 14 bits in units of 16 bytes, which never carry here)
+      const uint64_t dq = desc_k_major(smem_u32(sm + Q_OFF)), dk = desc_k_major(smem_u32(sm + K_OFF)), dv = desc_mn_major(smem_u32(sm + V_OFF));
       auto issue_s = [&](int i) {
         const int s = i % K_STAGES;
-        if (!mbar_wait(k_full + s, (i / K_STAGES) & 1, err)) return false;
+        if (!mbar_wait_warp(k_full + s, (i / K_STAGES) & 1, err)) return false;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sm + K_OFF + s * TILE);
+        const uint64_t k0 = dk + static_cast<uint32_t>(s * (TILE >> 4));
         const uint32_t tmem_s = tmem_base + (i & 1) * 128;
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < D / 16; ++j) {
-          const uint32_t off = (j >> 2) * HALF + (j & 3) * 32;
-          umma(tmem_s, desc_k_major(q_addr + off), desc_k_major(k_addr + off), kDescQK, j > 0 ? 1u : 0u);
+          for (int j = 0; j < D / 16; ++j) {
+            const uint32_t off = ((j >> 2) * HALF + (j & 3) * 32) >> 4;
+            umma(tmem_s, dq + off, k0 + off, kDescQK, j > 0 ? 1u : 0u);
+          }
+          umma_commit(s_full + (i & 1));
+          umma_commit(k_empty + s);
         }
-        umma_commit(s_full + (i & 1));
-        umma_commit(k_empty + s);
+        __syncwarp();
         return true;
       };
       if (ok) ok = issue_s(0);
       if (ok && nblk > 1) ok = issue_s(1);
       for (int i = 0; i < nblk && ok; ++i) {
         const int s = i % V_STAGES;
-        ok = mbar_wait(p_full + (i & 1), (i >> 1) & 1, err);      // P of block i lies where S of block i lay
-        if (ok) ok = mbar_wait(v_full + s, (i / V_STAGES) & 1, err);
+        ok = mbar_wait_warp(p_full + (i & 1), (i >> 1) & 1, err);      // P of block i lies where S of block i lay
+        if (ok) ok = mbar_wait_warp(v_full + s, (i / V_STAGES) & 1, err);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sm + V_OFF + s * TILE);
+        const uint64_t v0 = dv + static_cast<uint32_t>(s * (TILE >> 4));
+        const uint32_t tmem_p = tmem_base + (i & 1) * 128, more = i > 0 ? 1u : 0u;
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < BKV / 16; ++j)
-          umma_a_tmem(tmem_o, tmem_base + (i & 1) * 128 + j * 8, desc_mn_major(v_addr + j * 16 * 128), kDescPV,
-                      (i > 0 || j > 0) ? 1u : 0u);
-        if (SHAPED && shape.split) {                             // the weights' second terms
+          for (int j = 0; j < BKV / 16; ++j) umma_a_tmem(tmem_o, tmem_p + j * 8, v0 + j * 128, kDescPV, j > 0 ? 1u : more);
+          if (SHAPED && shape.split) {                             // the weights' second terms
 #pragma unroll
-          for (int j = 0; j < BKV / 16; ++j)
-            umma_a_tmem(tmem_o, tmem_base + (i & 1) * 128 + 64 + j * 8, desc_mn_major(v_addr + j * 16 * 128), kDescPV, 1u);
+            for (int j = 0; j < BKV / 16; ++j) umma_a_tmem(tmem_o, tmem_p + 64 + j * 8, v0 + j * 128, kDescPV, 1u);
+          }
+          umma_commit(pv_done);
+          umma_commit(v_empty + s);
         }
-        umma_commit(pv_done);
-        umma_commit(v_empty + s);
+        __syncwarp();
         if (i + 2 < nblk) ok = issue_s(i + 2);
       }
     }
@@ -847,7 +861,7 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
   uint64_t* q_full = pv_done + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = same_in_warp(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < KS; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); }
     for (int s = 0; s < VS; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
@@ -862,7 +876,7 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;        // columns: S of tile A 0..127, S of tile B 128..255, O of A 256..383, O of B 384..511
+  const uint32_t tmem_base = same_in_warp(*tmem_slot);        // columns: S of tile A 0..127, S of tile B 128..255, O of A 256..383, O of B 384..511
   pdl_launch_dependents();
   pdl_wait();
 
@@ -887,7 +901,7 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
   int k_begin = window > 0 ? max(0, p_lo[0] - window + 1) : 0;
   k_begin -= k_begin % BKV;
 #pragma unroll
-  for (int t = 0; t < 2; ++t) nblk[t] = ntok[t] > 0 ? (kv_end[t] - k_begin + BKV - 1) / BKV : 0;
+  for (int t = 0; t < 2; ++t) nblk[t] = same_in_warp(ntok[t] > 0 ? (kv_end[t] - k_begin + BKV - 1) / BKV : 0);
   const int nblk_all = max(nblk[0], nblk[1]);
   const int kv_end_all = max(kv_end[0], kv_end[1]);
   const int* table = block_table + static_cast<size_t>(row) * table_stride;
@@ -928,30 +942,28 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
       if (ok) fetch(&vmap, sm + PAIR_V_OFF + s * TILE, v_full + s, k_begin + i * BKV);
     }
   } else if (warp == 1) {
-    // ---- MMA issue (one lane)
-    if (lane == 0 && nblk_all > 0) {
-      bool ok = mbar_wait(q_full, 0, err);
-      // The operand descriptors differ only in their start address (the low 14 bits, in units of 16 bytes, which never
-      // carry here): built once, then a stage or a tile is an addition.
-      uint64_t dq[D / 16], dk[D / 16], dv[BKV / 16];
-#pragma unroll
-      for (int j = 0; j < D / 16; ++j) {
-        const uint32_t off = (j >> 2) * HALF + (j & 3) * 32;
-        dq[j] = desc_k_major(smem_u32(sm + PAIR_Q_OFF) + off);
-        dk[j] = desc_k_major(smem_u32(sm + PAIR_K_OFF) + off);
-      }
-#pragma unroll
-      for (int j = 0; j < BKV / 16; ++j) dv[j] = desc_mn_major(smem_u32(sm + PAIR_V_OFF) + j * 16 * 128);
+    // ---- MMA issue
+    if (nblk_all > 0) {
+      bool ok = mbar_wait_warp(q_full, 0, err);
+      // (descriptors differ in their start address only, the low 14 bits in units of 16 bytes, which never carry here)
+      const uint64_t dq = desc_k_major(smem_u32(sm + PAIR_Q_OFF)), dk = desc_k_major(smem_u32(sm + PAIR_K_OFF)), dv = desc_mn_major(smem_u32(sm + PAIR_V_OFF));
       // S of tile t over key block b; the block's last user gives the stage back
       auto issue_s = [&](int t, int b) {                         // (t is a constant at every call)
         const int s = b % KS;
-        if (!mbar_wait(k_full + s, (b / KS) & 1, err)) return false;
+        if (!mbar_wait_warp(k_full + s, (b / KS) & 1, err)) return false;
         tc_fence_after();
-        const uint64_t q_step = static_cast<uint64_t>(t * (TILE >> 4)), k_step = static_cast<uint64_t>(s * (TILE >> 4));
+        const uint64_t q0 = dq + static_cast<uint32_t>(t * (TILE >> 4)), k0 = dk + static_cast<uint32_t>(s * (TILE >> 4));
+        const bool last = t == 1 || b >= nblk[1];
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < D / 16; ++j) umma(tmem_base + t * 128, dq[j] + q_step, dk[j] + k_step, kDescQK, j > 0 ? 1u : 0u);
-        umma_commit(s_full + t);
-        if (t == 1 || b >= nblk[1]) umma_commit(k_empty + s);
+          for (int j = 0; j < D / 16; ++j) {
+            const uint32_t off = ((j >> 2) * HALF + (j & 3) * 32) >> 4;
+            umma(tmem_base + t * 128, q0 + off, k0 + off, kDescQK, j > 0 ? 1u : 0u);
+          }
+          umma_commit(s_full + t);
+          if (last) umma_commit(k_empty + s);
+        }
+        __syncwarp();
         return true;
       };
       if (ok && nblk[0] > 0) ok = issue_s(0, 0);
@@ -961,23 +973,28 @@ prefill_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap kmap, const __gr
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || b >= nblk[t]) continue;
-          ok = mbar_wait(p_half + t, b & 1, err);            // P of block b lies where S of block b lay
-          if (ok) ok = mbar_wait(v_full + s, (b / VS) & 1, err);
+          ok = mbar_wait_warp(p_half + t, b & 1, err);            // P of block b lies where S of block b lay
+          if (ok) ok = mbar_wait_warp(v_full + s, (b / VS) & 1, err);
           if (!ok) continue;
           tc_fence_after();
-          const uint64_t v_step = static_cast<uint64_t>(s * (TILE >> 4));
+          const uint64_t v0 = dv + static_cast<uint32_t>(s * (TILE >> 4));
+          const uint32_t tmem_o = tmem_base + 256 + t * 128, tmem_p = tmem_base + t * 128, more = b > 0 ? 1u : 0u;
+          const bool last = t == 1 || b >= nblk[1];
+          if (elect_one()) {
 #pragma unroll
-          for (int j = 0; j < BKV / 16; ++j) {
-            if (j == BKV / 32) {                             // the weights of the other 64 keys
-              ok = mbar_wait(p_full + t, b & 1, err);
-              if (!ok) break;
-              tc_fence_after();
-            }
-            umma_a_tmem(tmem_base + 256 + t * 128, tmem_base + t * 128 + j * 8, dv[j] + v_step, kDescPV, (b > 0 || j > 0) ? 1u : 0u);
+            for (int j = 0; j < BKV / 32; ++j) umma_a_tmem(tmem_o, tmem_p + j * 8, v0 + j * 128, kDescPV, j > 0 ? 1u : more);
           }
+          __syncwarp();
+          ok = mbar_wait_warp(p_full + t, b & 1, err);            // the weights of the other 64 keys
           if (!ok) continue;
-          umma_commit(pv_done + t);
-          if (t == 1 || b >= nblk[1]) umma_commit(v_empty + s);
+          tc_fence_after();
+          if (elect_one()) {
+#pragma unroll
+            for (int j = BKV / 32; j < BKV / 16; ++j) umma_a_tmem(tmem_o, tmem_p + j * 8, v0 + j * 128, kDescPV, 1u);
+            umma_commit(pv_done + t);
+            if (last) umma_commit(v_empty + s);
+          }
+          __syncwarp();
           if (b + 1 < nblk[t]) ok = issue_s(t, b + 1);
         }
       }
