@@ -13,13 +13,20 @@
 // apart: each kind fills its own registers in order, what integers do not fit follows on the stack in slots of eight bytes,
 // and what a callee does not ask for it does not look at.  So one call through one type with all of them reaches every such
 // function; the order between ints and floats of a signature does not matter, their order among themselves does.
+//
+// record() ... finish(slots): the calls that this thread makes in between are kept beside being made, and replay(values) makes them
+// again with other tensors in the places of `slots` (a layer's weights and cache, its input and its output).  A step's layers
+// that are alike make the same calls on the same sizes: one goes through Python, the others are issued by one loop here (a
+// layer of a prompt took the host 108 us, nine launches of 5).  A recording lives as long as its step.
 #include <torch/csrc/Device.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <vector>
 
 #if !defined(__x86_64__) && !defined(__aarch64__)
 #error "the calling convention of this host is not known to pass integers and floats apart"
@@ -48,6 +55,32 @@ struct Entry {
 
 PyObject *structure_type, *array_type;      // of ctypes
 
+// A call as it was made: an entry point with its arguments (of the integers, which are pointers and, behind finish(), which
+// slot's), or a product of the library.
+struct Call {
+  void* fn = nullptr;                       // null: out = x . w^T
+  int ni = 0, nf = 0;
+  I ints[MAX_INTS];
+  float floats[MAX_FLOATS];
+  bool pointer[MAX_INTS];
+  int slot[MAX_INTS];
+  at::Tensor x, w, out;
+  int x_slot = -1, w_slot = -1, out_slot = -1;
+};
+struct Recording {
+  std::vector<Call> calls;
+  std::vector<PyObject*> held;              // whose memory the calls' pointers lead to
+  struct Slot { at::Tensor tensor; bool aligned; };
+  std::vector<Slot> slots;                  // as they were recorded (no tensor: a ctypes object)
+  ~Recording() { for (PyObject* o : held) Py_DECREF(o); }
+};
+thread_local Recording* recording = nullptr;
+
+int invoke(void* fn, const I* ints, int ni, const float* floats) {
+  if (ni <= FEW_INTS) return reinterpret_cast<FewFn>(fn)(I8(ints, 0), I8(ints, 8), F8(floats));
+  return reinterpret_cast<MostFn>(fn)(I8(ints, 0), I8(ints, 8), I8(ints, 16), I8(ints, 24), I8(ints, 32), I8(ints, 40), F8(floats));
+}
+
 PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   HANDLE_TH_ERRORS
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
@@ -57,6 +90,7 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
   }
   I ints[MAX_INTS] = {};
   float floats[MAX_FLOATS] = {};
+  bool pointer[MAX_INTS] = {};
   int ni = 0, nf = 0;
   for (Py_ssize_t i = 0; i < n; ++i) {
     PyObject* a = args[i];
@@ -83,16 +117,27 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
       return nullptr;
     }
     if (ni == MAX_INTS) { PyErr_SetString(PyExc_TypeError, "too many arguments for an entry point"); return nullptr; }
+    pointer[ni] = a != Py_None && !PyLong_Check(a);
+    if (recording != nullptr && pointer[ni]) {
+      Py_INCREF(a);
+      recording->held.push_back(a);
+    }
     ints[ni++] = v;
   }
   void* fn = reinterpret_cast<Entry*>(self)->fn;
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  if (ni <= FEW_INTS)
-    rc = reinterpret_cast<FewFn>(fn)(I8(ints, 0), I8(ints, 8), F8(floats));
-  else
-    rc = reinterpret_cast<MostFn>(fn)(I8(ints, 0), I8(ints, 8), I8(ints, 16), I8(ints, 24), I8(ints, 32), I8(ints, 40), F8(floats));
+  rc = invoke(fn, ints, ni, floats);
   Py_END_ALLOW_THREADS
+  if (recording != nullptr) {
+    Call& c = recording->calls.emplace_back();
+    c.fn = fn;
+    c.ni = ni;
+    c.nf = nf;
+    std::copy(ints, ints + MAX_INTS, c.ints);
+    std::copy(floats, floats + MAX_FLOATS, c.floats);
+    std::copy(pointer, pointer + MAX_INTS, c.pointer);
+  }
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
 }
@@ -171,11 +216,138 @@ PyObject* mm_t(PyObject*, PyObject* const* args, Py_ssize_t n) {
     pybind11::gil_scoped_release free;
     out = at::mm(x, w.t());
   }
+  if (recording != nullptr) {
+    Call& c = recording->calls.emplace_back();
+    c.x = x;
+    c.w = w;
+    c.out = out;
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
 
+// ---- recordings
+struct RecordingObject {
+  PyObject_HEAD
+  Recording* r;
+};
+PyTypeObject recording_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+// The address of a tensor's data or a ctypes object's memory; -1 (with an error set) for anything else.
+I address_of(PyObject* o) {
+  if (THPVariable_Check(o)) return reinterpret_cast<I>(THPVariable_Unpack(o).mutable_data_ptr());
+  if (PyObject_IsInstance(o, structure_type) == 1 || PyObject_IsInstance(o, array_type) == 1) {
+    Py_buffer view;
+    if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) return -1;
+    const I at = reinterpret_cast<I>(view.buf);
+    PyBuffer_Release(&view);
+    return at;
+  }
+  PyErr_Format(PyExc_TypeError, "a recording's slots are tensors and ctypes objects, not a %s", Py_TYPE(o)->tp_name);
+  return -1;
+}
+
+PyObject* record(PyObject*, PyObject*) {
+  if (recording != nullptr) {
+    PyErr_SetString(PyExc_RuntimeError, "this thread records already");
+    return nullptr;
+  }
+  recording = new Recording;
+  Py_RETURN_NONE;
+}
+PyObject* discard(PyObject*, PyObject*) {
+  delete recording;
+  recording = nullptr;
+  Py_RETURN_NONE;
+}
+// finish(slots) -> the recording.  An argument that leads to a slot's memory is the slot's; a tensor of a product likewise.
+PyObject* finish(PyObject*, PyObject* slots) {
+  HANDLE_TH_ERRORS
+  if (recording == nullptr || !PyTuple_Check(slots)) {
+    PyErr_SetString(PyExc_RuntimeError, "finish(slots), a tuple, behind record()");
+    return nullptr;
+  }
+  const int n = static_cast<int>(PyTuple_GET_SIZE(slots));
+  std::vector<I> at(n);
+  recording->slots.clear();
+  for (int i = 0; i < n; ++i) {
+    PyObject* o = PyTuple_GET_ITEM(slots, i);
+    at[i] = address_of(o);
+    if (PyErr_Occurred()) return nullptr;
+    recording->slots.push_back({THPVariable_Check(o) ? THPVariable_Unpack(o) : at::Tensor(), at[i] % 16 == 0});
+  }
+  auto slot_of = [&](I address) {
+    for (int i = 0; i < n; ++i)
+      if (at[i] == address) return i;
+    return -1;
+  };
+  for (Call& c : recording->calls) {
+    for (int i = 0; i < c.ni; ++i) c.slot[i] = c.pointer[i] ? slot_of(c.ints[i]) : -1;
+    if (c.fn == nullptr) {
+      c.x_slot = slot_of(reinterpret_cast<I>(c.x.mutable_data_ptr()));
+      c.w_slot = slot_of(reinterpret_cast<I>(c.w.mutable_data_ptr()));
+      c.out_slot = slot_of(reinterpret_cast<I>(c.out.mutable_data_ptr()));
+    }
+  }
+  RecordingObject* o = PyObject_New(RecordingObject, &recording_type);
+  if (o == nullptr) return nullptr;
+  o->r = recording;
+  recording = nullptr;
+  return reinterpret_cast<PyObject*>(o);
+  END_HANDLE_TH_ERRORS
+}
+// replay(recording, values) -> 0, or the first code that is not; None, and nothing done, where a value is not like its slot (an
+// entry point chooses its kernel by sizes, types and alignment, the wrappers choose entry points by them).
+PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2 || Py_TYPE(args[0]) != &recording_type || !PyTuple_Check(args[1])) {
+    PyErr_SetString(PyExc_TypeError, "replay(recording, values)");
+    return nullptr;
+  }
+  const Recording& r = *reinterpret_cast<RecordingObject*>(args[0])->r;
+  const int n = static_cast<int>(PyTuple_GET_SIZE(args[1]));
+  if (n != static_cast<int>(r.slots.size())) Py_RETURN_NONE;
+  std::vector<I> at(n);
+  std::vector<at::Tensor> tensors(n);
+  for (int i = 0; i < n; ++i) {
+    PyObject* o = PyTuple_GET_ITEM(args[1], i);
+    at[i] = address_of(o);
+    if (PyErr_Occurred()) return nullptr;
+    const at::Tensor& was = r.slots[i].tensor;
+    if (THPVariable_Check(o) != was.defined() || (at[i] % 16 == 0) != r.slots[i].aligned) Py_RETURN_NONE;
+    if (!was.defined()) continue;
+    tensors[i] = THPVariable_Unpack(o);
+    if (tensors[i].scalar_type() != was.scalar_type() || tensors[i].device() != was.device() || tensors[i].sizes() != was.sizes() ||
+        tensors[i].strides() != was.strides())
+      Py_RETURN_NONE;
+  }
+  int rc = 0;
+  {
+    pybind11::gil_scoped_release free;
+    at::NoGradGuard no_grad;
+    for (const Call& c : r.calls) {
+      if (c.fn != nullptr) {
+        I ints[MAX_INTS];
+        std::copy(c.ints, c.ints + MAX_INTS, ints);
+        for (int i = 0; i < c.ni; ++i)
+          if (c.slot[i] >= 0) ints[i] = at[c.slot[i]];
+        rc = invoke(c.fn, ints, c.ni, c.floats);
+        if (rc != 0) break;
+      } else {
+        at::Tensor out = c.out_slot >= 0 ? tensors[c.out_slot] : c.out;
+        at::mm_out(out, c.x_slot >= 0 ? tensors[c.x_slot] : c.x, (c.w_slot >= 0 ? tensors[c.w_slot] : c.w).t());
+      }
+    }
+  }
+  return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"record", record, METH_NOARGS, "keep the calls that this thread makes from now on"},
+    {"discard", discard, METH_NOARGS, "forget what record() has kept"},
+    {"finish", finish, METH_O, "finish(slots): the recording since record()"},
+    {"replay", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(replay)), METH_FASTCALL, "replay(recording, values): its calls with values in the slots' places"},
     {"entry", make_entry, METH_O, "entry(address): the C entry point at an address as a callable"},
     {"all_cuda", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(all_cuda)), METH_FASTCALL, "whether every tensor (None counts as one) is on a GPU"},
     {"all_contiguous", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(all_contiguous)), METH_FASTCALL, "whether every tensor (None counts as one) is contiguous"},
@@ -200,6 +372,13 @@ PyMODINIT_FUNC PyInit__calls() {
   entry_type.tp_vectorcall_offset = offsetof(Entry, call);
   entry_type.tp_call = PyVectorcall_Call;
   entry_type.tp_dealloc = [](PyObject* o) { PyObject_Free(o); };
-  if (PyType_Ready(&entry_type) < 0) return nullptr;
+  recording_type.tp_name = "_calls.Recording";
+  recording_type.tp_basicsize = sizeof(RecordingObject);
+  recording_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  recording_type.tp_dealloc = [](PyObject* o) {
+    delete reinterpret_cast<RecordingObject*>(o)->r;
+    PyObject_Free(o);
+  };
+  if (PyType_Ready(&entry_type) < 0 || PyType_Ready(&recording_type) < 0) return nullptr;
   return PyModule_Create(&module);
 }

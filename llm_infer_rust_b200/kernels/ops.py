@@ -92,6 +92,36 @@ def add_launches(n: int) -> None:
     _launches[0] += n
 
 
+class LayerCalls:
+    """The calls that a layer makes through this module, kept while ``run`` makes them, and made again for layers like it.
+
+    ``slots``: the tensors (and TMA descriptors) that are another layer's own in its place, in one order for all; everything
+    else that the calls lead to (the step's index arrays, what the layer makes on its way) is the same memory again."""
+
+    def __init__(self, run, slots):
+        binding = self._binding = load_call_binding()
+        before = launch_count()
+        binding.record()
+        try:
+            self.result = run()
+            self._recording = binding.finish(tuple(slots(self.result)))
+        except BaseException:
+            binding.discard()
+            raise
+        self._launches = launch_count() - before
+
+    def again(self, values) -> bool:
+        """Make the calls with ``values`` in the places of the slots; False, and nothing done, when one of them is not like its
+        slot (another shape, dtype or alignment)."""
+        rc = self._binding.replay(self._recording, tuple(values))
+        if rc is None:
+            return False
+        if rc == 0:
+            add_launches(self._launches)
+            return True
+        raise KernelError(f"a layer's call: {_RC.get(rc) or f'CUDA error {rc} at launch'}")
+
+
 def _ok(rc: int, name: str, kernels: int = 1) -> None:
     if rc == 0:
         _launches[0] += kernels
@@ -1410,7 +1440,8 @@ GEMM_PLAIN, GEMM_SWIGLU = 0, 1
 _gemm_maps = {}
 
 
-def _gemm_map(t: torch.Tensor):
+def gemm_map(t: torch.Tensor):
+    """The TMA descriptor of a weight matrix for ``gemm_tc`` (made once)."""
     key = (t.data_ptr(), tuple(t.shape))
     buf = _gemm_maps.get(key)
     if buf is None:
@@ -1459,7 +1490,7 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, mode: int = GEMM_PLAIN, glu: 
     rc = lib.b200_gemm_tensor_map(a_map, x, int(m), int(k))
     if rc != 0:
         raise KernelError(f"the TMA descriptor of the activations could not be made (code {rc})")
-    rc = lib.b200_gemm_tcgen05(a_map, _gemm_map(weight), out, m, n, k, mode, float(limit), float(alpha),
+    rc = lib.b200_gemm_tcgen05(a_map, gemm_map(weight), out, m, n, k, mode, float(limit), float(alpha),
                                error_word(x.device), _stream())
     _ok(rc, "gemm_tcgen05")
     return out

@@ -162,6 +162,20 @@ class GQAttention(Part):
     def state_spec(self):
         return None
 
+    def repeat_slots(self, tokens, cache):
+        """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
+        p = self.params
+        if type(self) is not GQAttention or cache.k is None or ops.few_row_takes(tokens, p["qkv_proj"], self.env.dtype, ops.EPI_QKV, self.d) \
+                or ops.few_row_takes(tokens, p["o_proj"], self.env.dtype, norm=False):
+            return None
+        slots = [p["qkv_proj"], p["o_proj"], cache.k, cache.v]
+        if self.qk_eps is not None:
+            slots += [p["q_norm"], p["k_norm"]]
+        page = cache.k.shape[2]
+        if ops.decode_uses_tensor_cores(cache.k.dtype, self.nh, self.nkv, self.d, page):
+            slots += [ops.kv_tensor_map(cache.k, min(page, 32)), ops.kv_tensor_map(cache.v, min(page, 32))]
+        return slots
+
     def takes_pending(self, tokens: int) -> bool:
         """Whether a step of ``tokens`` tokens runs the input norm as the prologue of the QKV product."""
         return ops.few_row_takes(tokens, self.params["qkv_proj"], self.env.dtype, ops.EPI_QKV, self.d)

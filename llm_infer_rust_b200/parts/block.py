@@ -5,7 +5,7 @@ import torch
 
 from ..kernels import ops
 from .base import ParamDecl, Part
-from .norm import OwedRMSNorm, OwedSum
+from .norm import OwedRMSNorm, OwedSum, RMSNorm
 from .registry import build_part, register_part
 
 
@@ -44,6 +44,19 @@ class PreNormDeferredAdd:
         other part runs, everything that waits is launched."""
         if not getattr(part, "chainable", False):
             ops.flush_chain()
+
+    def repeat_slots(self, h, cache):
+        """What is this layer's own in the calls that ``forward`` makes for a step of these tokens, for ``ops.LayerCalls``;
+        None where a step of a layer like it might make others (few tokens, whose products wait for one another; parts that do not
+        say, or that add to what these do)."""
+        if type(self) is not PreNormDeferredAdd or type(self.input_norm) is not RMSNorm or type(self.post_mixer_norm) is not RMSNorm:
+            return None
+        mixer, feed = getattr(self.mixer, "repeat_slots", None), getattr(self.feed_forward, "repeat_slots", None)
+        mixer = mixer(h.shape[0], cache) if mixer is not None else None
+        feed = feed(h) if feed is not None else None
+        if mixer is None or feed is None:
+            return None
+        return [self.input_norm.params["weight"], self.post_mixer_norm.params["weight"]] + mixer + feed
 
     def forward(self, h, residual, ctx, cache):
         tokens = h.shape[0]

@@ -26,6 +26,14 @@ class SwiGLU(Part):
         return {"gate_up_proj": ParamDecl((2 * self.inter, self.hidden)),
                 "down_proj": ParamDecl((self.hidden, self.inter))}
 
+    def repeat_slots(self, x):
+        """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
+        gate_up, down = self.params["gate_up_proj"], self.params["down_proj"]
+        if type(self) is not SwiGLU or ops.few_row_takes(x.shape[0], gate_up, self.env.dtype, ops.EPI_SWIGLU) \
+                or ops.few_row_takes(x.shape[0], down, self.env.dtype, norm=False):
+            return None
+        return [gate_up, down] + ([ops.gemm_map(gate_up)] if ops.gemm_tc_pays(x, gate_up, ops.GEMM_SWIGLU) else [])
+
     def takes_pending(self, tokens: int) -> bool:
         """Whether a step of ``tokens`` tokens runs the norm before it as the prologue of the gate/up product."""
         return ops.few_row_takes(tokens, self.params["gate_up_proj"], self.env.dtype, ops.EPI_SWIGLU)

@@ -41,6 +41,14 @@ class DecoderModel:
                 if mine != theirs:
                     raise ValueError(f"run list entry {e} reads the cache of entry {entry.reads}, "
                                      f"whose keys and values have another shape or window")
+        # where the stretch of entries with the same parts in a row that entry e is in ends: their steps make the same calls
+        self._alike_until = list(range(1, len(self.run_list) + 1))
+        for e in range(len(self.run_list) - 2, -1, -1):
+            mine, following = self.run_list[e], self.run_list[e + 1]
+            if mine.reads is None and following.reads is None and following.input is None \
+                    and spec.layers[mine.layer] == spec.layers[following.layer]:
+                self._alike_until[e] = self._alike_until[e + 1]
+        self.repeats_layers = True         # False: every layer of a step goes through Python
 
     # ------------------------------------------------------------------ parameters
     def _owners(self) -> Dict[str, Part]:
@@ -87,6 +95,37 @@ class DecoderModel:
         return total
 
     # ------------------------------------------------------------------ one step
+    def _repeated(self, first, h, residual, caches):
+        """The end of a stretch of entries from ``first`` on whose steps make the same calls (None: a stretch of one)."""
+        end = self._alike_until[first]
+        if not self.repeats_layers or residual is None or end - first < 2:
+            return None
+        slots_of = getattr(self.blocks[self.run_list[first].layer], "repeat_slots", None)
+        if slots_of is None or slots_of(h, caches[first]) is None:
+            return None
+        mine = caches[first]
+        for e in range(first + 1, end):
+            if caches[e].group != mine.group or caches[e].writes != mine.writes:
+                end = e
+                break
+        return end if end - first >= 2 else None
+
+    def _repeat(self, first, end, h, residual, ctx, caches):
+        """The entries ``first`` .. ``end`` - 1: the first one's calls are kept and made again with the others' weights and caches.
+        Two buffers take turns: a layer leaves its output where the layer before found its input (which it normed in place)."""
+        own = lambda e, h: self.blocks[self.run_list[e].layer].repeat_slots(h, caches[e])
+        slots = own(first, h)
+        calls = ops.LayerCalls(lambda: self.blocks[self.run_list[first].layer].forward(h, residual, ctx, caches[first]),
+                               lambda result: [h, result[0]] + slots)
+        (out, residual), spare = calls.result, h
+        for e in range(first + 1, end):
+            values = own(e, out)
+            if values is not None and calls.again([out, spare] + values):
+                out, spare = spare, out
+            else:
+                out, residual = self.blocks[self.run_list[e].layer].forward(out, residual, ctx, caches[e])
+        return out, residual
+
     def forward(self, ctx, caches, embedding_cache=None) -> torch.Tensor:
         """Run the step's tokens; float32 logits [ctx.num_logits, vocab] at ``ctx.logit_rows``.  ``embedding_cache``:
         the states of an embedding that keeps some."""
@@ -97,10 +136,18 @@ class DecoderModel:
         residual = None
         # what the stream inputs keep of the embedding's output, before a layer changes it
         kept = {name: part.begin(h) for name, part in self.stream_inputs.items()}
-        for e, entry in enumerate(self.run_list):
+        e = 0
+        while e < len(self.run_list):
+            entry = self.run_list[e]
             if entry.input is not None:
                 h, residual = self.stream_inputs[entry.input].forward(h, residual, kept[entry.input])
-            h, residual = self.blocks[entry.layer].forward(h, residual, ctx, caches[e])
+            end = self._repeated(e, h, residual, caches)
+            if end is None:
+                h, residual = self.blocks[entry.layer].forward(h, residual, ctx, caches[e])
+                e += 1
+            else:
+                h, residual = self._repeat(e, end, h, residual, ctx, caches)
+                e = end
         takes = getattr(self.lm_head, "takes_pending", None)
         if not (getattr(self.final_norm, "chainable", False) and getattr(self.lm_head, "chainable", False)):
             ops.flush_chain()

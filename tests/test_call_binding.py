@@ -93,3 +93,86 @@ def test_several_threads(entries):
     for t in threads:
         t.join()
     assert len(got) == 800 and all(got)
+
+
+_ADD = r"""
+extern "C" int add(float* out, const float* a, const float* b, float scale, int n) {
+  for (int i = 0; i < n; ++i) out[i] = a[i] + scale * b[i];
+  return n > 100 ? -2 : 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def adding(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("adding")
+    (folder / "add.cpp").write_text(_ADD)
+    subprocess.run(["g++", "-O2", "-shared", "-fPIC", str(folder / "add.cpp"), "-o", str(folder / "add.so")], check=True)
+    return build.EntryPoints(ctypes.CDLL(str(folder / "add.so")))
+
+
+def _layer(adding, calls, h, w, b, scale=2.0):
+    """h <- h + scale b in place; the product with w^T, to which an inner buffer adds b again."""
+    n = h.numel()
+    assert adding.add(h, h, b, scale, n) == 0
+    inner = torch.empty_like(h)
+    assert adding.add(inner, h, b, 1.0, n) == 0
+    return calls.mm_t(inner, w)
+
+
+def test_a_layers_calls_are_made_again_with_anothers_weights(adding):
+    calls = build.load_call_binding()
+    ws, bs = [torch.randn(4, 4) for _ in range(5)], [torch.randn(3, 4) for _ in range(5)]
+    want = start = torch.randn(3, 4)
+    for w, b in zip(ws, bs):
+        want = _layer(adding, calls, want.clone(), w, b)
+    h = start.clone()
+    calls.record()
+    out = _layer(adding, calls, h, ws[0], bs[0])
+    kept = calls.finish((h, out, ws[0], bs[0]))
+    spare = h
+    for w, b in zip(ws[1:], bs[1:]):
+        assert calls.replay(kept, (out, spare, w, b)) == 0
+        out, spare = spare, out
+    assert torch.equal(out, want)
+
+
+def test_values_that_are_not_like_their_slots_are_left_to_the_caller(adding):
+    calls = build.load_call_binding()
+    h, w, b = torch.randn(3, 4), torch.randn(4, 4), torch.randn(3, 4)
+    calls.record()
+    with pytest.raises(RuntimeError):
+        calls.record()                                          # one at a time
+    out = _layer(adding, calls, h, w, b)
+    kept = calls.finish((h, out, w, b))
+    odd = torch.randn(17)[1:].reshape(4, 4)                     # not on the boundary that w was on
+    before = h.clone()
+    for bad in ((h, out, w), (h, out, w.double(), b), (h, out, torch.randn(4, 5), b), (h, out, w.t(), b), (h, out, odd, b),
+                (h, out, ctypes.create_string_buffer(64), b)):
+        assert calls.replay(kept, bad) is None and torch.equal(h, before)
+    with pytest.raises(TypeError):
+        calls.replay(kept, (h, out, w, 3))
+    with pytest.raises(RuntimeError):
+        calls.finish((h,))                                      # nothing is recorded
+    calls.record()
+    calls.discard()
+    calls.record()
+    big = torch.zeros(128)
+    assert adding.add(big, big, big, 1.0, 100) == 0
+    kept = calls.finish((big,))
+    assert calls.replay(kept, (torch.zeros(128),)) == 0
+    calls.record()
+    adding.add(big, big, big, 1.0, 101)
+    assert calls.replay(calls.finish((big,)), (big,)) == -2     # an entry point's code comes back
+
+
+def test_recordings_are_a_threads_own(adding):
+    calls = build.load_call_binding()
+    h, b = torch.zeros(3, 4), torch.ones(3, 4)
+    calls.record()
+    other = threading.Thread(target=lambda: adding.add(torch.zeros(3, 4), b, b, 1.0, 12))
+    other.start()
+    other.join()
+    adding.add(h, h, b, 1.0, 12)
+    kept = calls.finish((h, b))
+    assert calls.replay(kept, (h, b)) == 0 and torch.equal(h, 2 * b)
