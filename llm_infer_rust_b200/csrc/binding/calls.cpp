@@ -276,6 +276,9 @@ PyObject* finish(PyObject*, PyObject* slots) {
     if (PyErr_Occurred()) return nullptr;
     recording->slots.push_back({THPVariable_Check(o) ? THPVariable_Unpack(o) : at::Tensor(), at[i] % 16 == 0});
   }
+  // (two slots of one address: an argument does not say whose it is, and no other layer is like this one)
+  for (int i = 0; i < n; ++i)
+    if (std::count(at.begin(), at.end(), at[i]) > 1) { recording->slots.clear(); break; }
   auto slot_of = [&](I address) {
     for (int i = 0; i < n; ++i)
       if (at[i] == address) return i;

@@ -164,6 +164,10 @@ def test_values_that_are_not_like_their_slots_are_left_to_the_caller(adding):
     calls.record()
     adding.add(big, big, big, 1.0, 101)
     assert calls.replay(calls.finish((big,)), (big,)) == -2     # an entry point's code comes back
+    calls.record()
+    adding.add(big, big, big, 1.0, 100)
+    kept = calls.finish((big, big))                             # which of the two an argument leads to is not known
+    assert calls.replay(kept, (torch.zeros(128), torch.zeros(128))) is None
 
 
 def test_recordings_are_a_threads_own(adding):
