@@ -32,6 +32,7 @@
 #include <initializer_list>
 
 #include "common.cuh"
+#include "pairs.cuh"
 
 #ifndef HEAD_DIM
 #define HEAD_DIM 128
@@ -331,7 +332,8 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
 // pv_done is not asked.  A tile walks a chain of its own latencies (measured with softmax_block, SM cycles a block at 8,192
 // tokens: 2,040 until the next scores stand, 2,700 in the softmax, 1,720 of those behind the maximum, for 1,024 of
 // special-function work), so what shortens the chain counts: 8,192 tokens x 16 heads 340 -> 302 us, 16,384 x 32 2,165 us
-// (1,015 TFLOP/s).  Two threads a row, which pay for the further forms below, were slower here (483 us: sixteen warps
+// (1,015 TFLOP/s).  Behind the maximum the thread's issue slots are the chain, so scale and sum take two scores an instruction
+// (with the MMAs issued by a whole warp: 275 -> 263 us, 3,000 tokens 58.6 -> 56.2, 16,384 x 32 1,998 -> 1,909).  Two threads a row, which pay for the further forms below, were slower here (483 us: sixteen warps
 // leave 96 registers a thread, so the scores are read twice).
 __device__ __forceinline__ void tmem_ld32_begin(uint32_t taddr, float (&v)[32]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -388,14 +390,18 @@ __device__ __forceinline__ void softmax_row(uint32_t s_base, uint32_t o_base, in
   }
   st.m_ref = m_new;
   const float neg_base = hi_key < 0 ? -INFINITY : m_new == -INFINITY ? 0.0f : -m_new;      // a row that is not used gets zeros
-  float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  f32x2 sums[2] = {0, 0};
+  const f32x2 scale2 = twice(scale_log2), base2 = twice(neg_base);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     uint32_t pr[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float a = fast_exp2(fmaf(v[c][2 * i], scale_log2, neg_base)), b = fast_exp2(fmaf(v[c][2 * i + 1], scale_log2, neg_base));
-      sum4[i & 3] += a + b;
+      float a, b;
+      unpack2(fma2(pack2(v[c][2 * i], v[c][2 * i + 1]), scale2, base2), a, b);
+      a = fast_exp2(a);
+      b = fast_exp2(b);
+      sums[i & 1] = add2(sums[i & 1], pack2(a, b));
       const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
       pr[i] = *reinterpret_cast<const uint32_t*>(&two);
     }
@@ -405,6 +411,9 @@ __device__ __forceinline__ void softmax_row(uint32_t s_base, uint32_t o_base, in
       half_done();
     }
   }
+  float sum4[4];
+  unpack2(sums[0], sum4[0], sum4[1]);
+  unpack2(sums[1], sum4[2], sum4[3]);
   st.l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
   tmem_wait_st();                                      // P is in tensor memory
 }
