@@ -674,19 +674,26 @@ split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
     const int n0 = first_tile / job.m_tiles * SP_BN, m0 = first_tile % job.m_tiles * job.tokens;
     const int spans = (job.stages + job.span_stages - 1) / job.span_stages;
     const float* parts = reinterpret_cast<const float*>(ring);
-    for (int i = rank * S::THREADS + threadIdx.x; i < job.tokens * SP_BN; i += job.ksplit * S::THREADS) {
-      const int m = m0 + i / SP_BN, n = n0 + i % SP_BN;
-      float v[SP_SPANS], t = 0.0f;
+    // Four rows of W a turn: the other ranks' memory is far, and its requests, not its bytes, take the time (300 rows of 1,024 x
+    // 2,048 one float a turn 34.6 us, four 28.0; 1,024 x 3,072 42.5 -> 35.7).
+    for (int i = rank * S::THREADS + threadIdx.x; i < job.tokens * SP_BN / 4; i += job.ksplit * S::THREADS) {
+      const int m = m0 + i / (SP_BN / 4), n = n0 + i % (SP_BN / 4) * 4;
+      float4 v[SP_SPANS];
 #pragma unroll
       for (int s = 0; s < SP_SPANS; ++s)
-        if (s < spans) v[s] = cluster.map_shared_rank(parts, s / job.spans_a_rank)[s % job.spans_a_rank * NT * SP_BN + i];
+        if (s < spans)
+          v[s] = reinterpret_cast<const float4*>(cluster.map_shared_rank(parts, s / job.spans_a_rank) + s % job.spans_a_rank * NT * SP_BN)[i];
+      float t[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
 #pragma unroll
-      for (int s = 0; s < SP_SPANS; ++s)
-        if (s < spans) t = s == 0 ? v[s] : t + v[s];
-      if (m < p.m && n < p.n) {
-        if (!sp_finite(t)) t = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
-        p.c[static_cast<size_t>(m) * p.ldc + n] = t;
-      }
+      for (int s = 1; s < SP_SPANS; ++s)
+        if (s < spans) { t[0] += v[s].x; t[1] += v[s].y; t[2] += v[s].z; t[3] += v[s].w; }
+      if (m >= p.m) continue;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n + e < p.n) {
+          if (!sp_finite(t[e])) t[e] = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n + e) * p.ldw, p.k);
+          p.c[static_cast<size_t>(m) * p.ldc + n + e] = t[e];
+        }
     }
     cluster.sync();                                                 // the sums are read: the block may end
   }
@@ -864,9 +871,9 @@ static int blocks_a_tile(long long tiles, int spans, int sms) {
 B200_EXPORT int b200_gemm_f32_blocks_a_tile(long long tiles, int spans, int sms) { return blocks_a_tile(tiles, spans, sms); }
 
 // What a product costs split_kernel, in stages of one block: rounds of blocks over the SMs, each its stages and what begins and ends a
-// block (a cluster's placement and its exchange of sums take as long as eleven stages).  `ranks`: how many blocks share a tile's k,
-// one or two spans each.  (Measured with one, four and eight: 4,096 x 1,024 at 64 rows 31 / 21 / 38 us, 6,144 x 1,024 at 64 31 / 41 /
-// 50, 1,024 x 3,072 at 300 99 / 43 / 48.)
+// block (a cluster's placement and its exchange of sums take as long as nine to eleven stages).  `ranks`: how many blocks share a
+// tile's k, one or two spans each.  (Measured with one, four and eight, the sums exchanged one float a turn: 4,096 x 1,024 at 64 rows
+// 31 / 21 / 38 us, 6,144 x 1,024 at 64 31 / 41 / 50, 1,024 x 3,072 at 300 99 / 43 / 48.)
 static long long split_cost(int tiles, int spans, int stages, int sms, int& ranks) {
   ranks = 1;
   long long least = static_cast<long long>((tiles + sms - 1) / sms) * (stages + 3);
