@@ -219,18 +219,19 @@ __global__ void retention_chunk_base_kernel(const int* __restrict__ cu_q, int nu
   }
 }
 
-// (2a) A block owns a 32 x 64 tile of one chunk's own contribution U = sum over j < L of decay^(L-1-j) k_j v_j^T;
-// a thread 4 rows (4 ty ..) of 2 columns (2 tx, 2 tx + 1).  k is multiplied by its power of the decay as it is
-// staged, so a token costs a thread one 16-byte load of k that the whole warp shares, one 8-byte load of v and
-// 8 FMAs.  U goes where the state before the chunk will stand (`before`); (2b) folds the chunks together.
-constexpr int RS_I = 32, RS_J = 64;
+// (2a) A block owns a 64 x 64 tile of one chunk's own contribution U = sum over j < L of decay^(L-1-j) k_j v_j^T;
+// a thread 4 rows (4 ty ..) of 4 columns (4 tx ..).  k is multiplied by its power of the decay as it is staged, so a token
+// costs a thread two 16-byte loads and 16 FMAs: three passes of shared memory a warp (tiles of 32 x 64 with 8 FMAs a thread
+// took as many for half the work, and shared memory bound them).  U goes where the state before the chunk will stand
+// (`before`); (2b) folds the chunks together.
+constexpr int RS_I = 64, RS_J = 64;
 template <typename T>
 __global__ void __launch_bounds__(256)
 retention_chunk_sum_kernel(const T* __restrict__ x, int in_stride, const float* __restrict__ kf,
                            float* __restrict__ before, const float* __restrict__ decay, const int* __restrict__ cu_q,
                            const int* __restrict__ chunk_base, int num_rows, int heads, int d, int dv) {
-  __shared__ __align__(16) float ks[RC][RS_I + 4];
-  __shared__ __align__(16) float vs[RC][RS_J + 2];
+  __shared__ __align__(16) float ks[RC][RS_I];
+  __shared__ __align__(16) float vs[RC][RS_J];
   const int slot = blockIdx.x, h = blockIdx.y;
   if (slot >= chunk_base[num_rows]) return;
   int r = 0;
@@ -240,38 +241,49 @@ retention_chunk_sum_kernel(const T* __restrict__ x, int in_stride, const float* 
   const int L = min(RC, n - base);
   const int tiles_v = (dv + RS_J - 1) / RS_J;
   const int ti = blockIdx.z / tiles_v, tj = blockIdx.z - ti * tiles_v;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int col = tj * RS_J + 2 * tx, row0 = ti * RS_I + 4 * ty;
   const float lg = log2f(decay[h]);
-  const int voff = 2 * heads * d + h * dv;
-  const bool k_ok = ti * RS_I + tx < d, v0_ok = tj * RS_J + tx < dv, v1_ok = tj * RS_J + 32 + tx < dv;
-  const float* kcol = kf + static_cast<size_t>(h) * d + ti * RS_I + tx;
-  const T* vcol = x + voff + tj * RS_J + tx;
+  const float* krow = kf + static_cast<size_t>(first + base) * heads * d + h * d + ti * RS_I;
+  const T* vrow = x + static_cast<size_t>(first + base) * in_stride + 2 * heads * d + h * dv + tj * RS_J;
+  float4 kv[4];
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const int j = ty + 8 * m;
-    const size_t t = static_cast<size_t>(first + base + j);
-    const float w = L - 1 - j == 0 ? 1.0f : exp2f(static_cast<float>(L - 1 - j) * lg);
-    ks[j][tx] = (j < L && k_ok) ? kcol[t * heads * d] * w : 0.0f;
-    vs[j][tx] = (j < L && v0_ok) ? to_f32<T>(vcol[t * in_stride]) : 0.0f;
-    vs[j][tx + 32] = (j < L && v1_ok) ? to_f32<T>(vcol[t * in_stride + 32]) : 0.0f;
+  for (int m = 0; m < 4; ++m) {
+    const int j = (threadIdx.x >> 4) + 16 * m, e = (threadIdx.x & 15) * 4;
+    kv[m] = j < L && ti * RS_I + e < d ? *reinterpret_cast<const float4*>(krow + static_cast<size_t>(j) * heads * d + e)
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const int j = (threadIdx.x >> 3) + 32 * m, col = (threadIdx.x & 7) * 8;
+    float v[8] = {};
+    if (j < L && tj * RS_J + col < dv) load_floats<T, 8>(vrow + static_cast<size_t>(j) * in_stride + col, v);
+    *reinterpret_cast<float4*>(&vs[j][col]) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(&vs[j][col + 4]) = make_float4(v[4], v[5], v[6], v[7]);
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int j = (threadIdx.x >> 4) + 16 * m, e = (threadIdx.x & 15) * 4;
+    const float w = L - 1 - j <= 0 ? 1.0f : exp2f(static_cast<float>(L - 1 - j) * lg);      // (rows beyond L hold zeros)
+    *reinterpret_cast<float4*>(&ks[j][e]) = make_float4(kv[m].x * w, kv[m].y * w, kv[m].z * w, kv[m].w * w);
   }
   __syncthreads();
-  float U[4][2] = {};
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float U[4][4] = {};
 #pragma unroll 8
-  for (int j = 0; j < RC; ++j) {                    // rows beyond L hold zeros
+  for (int j = 0; j < RC; ++j) {
     const float4 k4 = *reinterpret_cast<const float4*>(&ks[j][4 * ty]);
-    const float2 v2 = *reinterpret_cast<const float2*>(&vs[j][2 * tx]);
-    U[0][0] = fmaf(k4.x, v2.x, U[0][0]); U[0][1] = fmaf(k4.x, v2.y, U[0][1]);
-    U[1][0] = fmaf(k4.y, v2.x, U[1][0]); U[1][1] = fmaf(k4.y, v2.y, U[1][1]);
-    U[2][0] = fmaf(k4.z, v2.x, U[2][0]); U[2][1] = fmaf(k4.z, v2.y, U[2][1]);
-    U[3][0] = fmaf(k4.w, v2.x, U[3][0]); U[3][1] = fmaf(k4.w, v2.y, U[3][1]);
+    const float4 v4 = *reinterpret_cast<const float4*>(&vs[j][4 * tx]);
+    const float k[4] = {k4.x, k4.y, k4.z, k4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) U[a][b] = fmaf(k[a], v[b], U[a][b]);
   }
+  const int col = tj * RS_J + 4 * tx, row0 = ti * RS_I + 4 * ty;
   float* dst = before + (static_cast<size_t>(slot) * heads + h) * d * dv;
 #pragma unroll
   for (int m = 0; m < 4; ++m)
     if (row0 + m < d && col < dv)
-      *reinterpret_cast<float2*>(dst + static_cast<size_t>(row0 + m) * dv + col) = make_float2(U[m][0], U[m][1]);
+      *reinterpret_cast<float4*>(dst + static_cast<size_t>(row0 + m) * dv + col) = make_float4(U[m][0], U[m][1], U[m][2], U[m][3]);
 }
 
 // (2b) grid (rows, heads, pieces of 256 elements): S = the row's state (zeros at a sequence's start); chunk by
@@ -395,24 +407,28 @@ retention_chunk_kernel(const T* __restrict__ x, int in_stride, const float* __re
   const int voff = 2 * heads * d + h * dv;
 
   {
-    // q and k: a thread fetches 16-byte pieces (4 consecutive e of one token), four pieces in flight
-    const int pieces = d / 4, total = RC * pieces;
+    // q and k: a thread fetches 16-byte pieces (4 consecutive e of one token), four pieces in flight.  Two pieces of a token
+    // are neighbouring lanes' and a warp has sixteen tokens, so that its transposed stores go to 32 banks (the pieces of one
+    // token beside one another met in two banks, sixteen to a bank).  With the larger tiles of (2a) and, below, the products with
+    // V only up to a warp's own tokens: 2,048 tokens x 16 heads of 128, all five kernels, 167 -> 136 us; 64 tokens 43.7 -> 37.4.
+    const int pieces = d / 4, total = RC * 2 * ((pieces + 1) / 2);
     for (int idx0 = threadIdx.x; idx0 < total; idx0 += 4 * blockDim.x) {
       float4 qv[4], kv[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int idx = idx0 + u * blockDim.x;
-        const int i = idx / pieces, e = (idx - i * pieces) * 4;
-        const bool ok = idx < total && i < L;
-        const size_t at_ = static_cast<size_t>(t0 + (ok ? i : 0)) * hd + h * d + e;
+        const int i = (idx >> 1) % RC, p = 2 * (idx / (2 * RC)) + (idx & 1);
+        const bool ok = p < pieces && i < L;
+        const size_t at_ = static_cast<size_t>(t0 + (ok ? i : 0)) * hd + h * d + (ok ? 4 * p : 0);
         qv[u] = ok ? *reinterpret_cast<const float4*>(qf + at_) : make_float4(0.f, 0.f, 0.f, 0.f);
         kv[u] = ok ? *reinterpret_cast<const float4*>(kf + at_) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int idx = idx0 + u * blockDim.x;
-        if (idx >= total) continue;
-        const int i = idx / pieces, e = (idx - i * pieces) * 4;
+        const int i = (idx >> 1) % RC, p = 2 * (idx / (2 * RC)) + (idx & 1);
+        if (p >= pieces) continue;
+        const int e = 4 * p;
         qt[(e + 0) * RC_LD + i] = qv[u].x; qt[(e + 1) * RC_LD + i] = qv[u].y;
         qt[(e + 2) * RC_LD + i] = qv[u].z; qt[(e + 3) * RC_LD + i] = qv[u].w;
         kt[(e + 0) * RC_LD + i] = kv[u].x; kt[(e + 1) * RC_LD + i] = kv[u].y;
@@ -488,7 +504,7 @@ retention_chunk_kernel(const T* __restrict__ x, int in_stride, const float* __re
   fetch_slab(0);
   // o[i][col] for i in 4 ty .., col in 4 tx .. and 64 + 4 tx ..: A V first, then decay^(i+1) q_i^T S_before
   float out[4][8] = {};
-  tile_product_split<4>(at, RC_LD, vb, RV_LD, RC, ty * 4, tx * 4, out);
+  tile_product_split<4>(at, RC_LD, vb, RV_LD, (threadIdx.x >> 5) * 8 + 8, ty * 4, tx * 4, out);      // (a warp's eight rows see no later token)
   float inter[4][8] = {};
   for (int e0 = 0; e0 < d; e0 += RC) {
     __syncthreads();                                            // vb is free
