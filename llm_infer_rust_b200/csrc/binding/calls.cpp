@@ -129,7 +129,7 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
   Py_BEGIN_ALLOW_THREADS
   rc = invoke(fn, ints, ni, floats);
   Py_END_ALLOW_THREADS
-  if (recording != nullptr) {
+  if (recording != nullptr && rc == 0) {      // (another result is a question's answer, which the wrapper has gone by, or an error)
     Call& c = recording->calls.emplace_back();
     c.fn = fn;
     c.ni = ni;

@@ -98,7 +98,7 @@ def test_several_threads(entries):
 _ADD = r"""
 extern "C" int add(float* out, const float* a, const float* b, float scale, int n) {
   for (int i = 0; i < n; ++i) out[i] = a[i] + scale * b[i];
-  return n > 100 ? -2 : 0;
+  return n > 100 || out[0] > 1e30f ? -2 : 0;
 }
 """
 
@@ -161,9 +161,11 @@ def test_values_that_are_not_like_their_slots_are_left_to_the_caller(adding):
     assert adding.add(big, big, big, 1.0, 100) == 0
     kept = calls.finish((big,))
     assert calls.replay(kept, (torch.zeros(128),)) == 0
+    assert calls.replay(kept, (torch.full((128,), 1e30),)) == -2     # an entry point's code comes back
     calls.record()
-    adding.add(big, big, big, 1.0, 101)
-    assert calls.replay(calls.finish((big,)), (big,)) == -2     # an entry point's code comes back
+    assert adding.add(big, big, big, 1.0, 101) == -2            # as an answer that is no code: asked once, not made again
+    other = torch.ones(128)
+    assert calls.replay(calls.finish((big,)), (other,)) == 0 and torch.equal(other, torch.ones(128))
     calls.record()
     adding.add(big, big, big, 1.0, 100)
     kept = calls.finish((big, big))                             # which of the two an argument leads to is not known
