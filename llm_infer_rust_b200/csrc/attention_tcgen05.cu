@@ -438,6 +438,20 @@ __device__ __forceinline__ float capped(const ScoreShape& f, float s, float shif
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(fast_exp2(s * (f.tanh_in * 2.8853900817779268f)) + 1.0f));
   return fmaf(-2.0f * f.cap_log2, r, f.cap_log2 + shift);
 }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The same of two scores; NaN stays NaN, a masked score (-inf) does not stay masked.
+__device__ __forceinline__ f32x2 capped2(const ScoreShape& f, f32x2 s, float shift) {
+  float a, b;
+  unpack2(mul2(s, twice(f.tanh_in * 2.8853900817779268f)), a, b);
+  unpack2(add2(pack2(fast_exp2(a), fast_exp2(b)), twice(1.0f)), a, b);
+  asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(a));
+  asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(b));
+  return fma2(twice(-2.0f * f.cap_log2), pack2(a, b), twice(f.cap_log2 + shift));
+}
 
 // These forms cost several times the instructions of the plain one, so there a row has TWO threads: thread c = 0, 1 of a row
 // takes columns 64 c .. 64 c + 63 of its scores (one load; they stay in registers) and of its accumulator; the two warps
@@ -466,20 +480,26 @@ struct HalfRows {
   }
 };
 
-// 2^exponent(score) of 64 scores, their sum added to sum4; the weights and (split) what their rounding left into tensor memory.
+// 2^exponent(scores) of 64 scores, two at a time, their sum added to sums; the weights and (split) what their rounding left into
+// tensor memory.  Multiply-adds and sums take two an instruction.
 template <typename F>
-__device__ __forceinline__ void store_weights(const float (&v)[64], uint32_t p_base, bool split, float (&sum4)[4], const F& exponent) {
+__device__ __forceinline__ void store_weights(const float (&v)[64], uint32_t p_base, bool split, f32x2 (&sums)[2], const F& exponent) {
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     uint32_t pr[8], rest[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int e = h * 16 + 2 * i;
-      const float a = fast_exp2(exponent(v[e])), b = fast_exp2(exponent(v[e + 1]));
-      sum4[i & 3] += a + b;
+      float a, b;
+      unpack2(exponent(v[e], v[e + 1]), a, b);
+      a = fast_exp2(a);
+      b = fast_exp2(b);
+      const f32x2 both = pack2(a, b);
+      sums[i & 1] = add2(sums[i & 1], both);
       const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
       pr[i] = *reinterpret_cast<const uint32_t*>(&two);
-      const __nv_bfloat162 rem = __floats2bfloat162_rn(a - __uint_as_float(pr[i] << 16), b - __uint_as_float(pr[i] & 0xffff0000u));
+      unpack2(fma2(pack2(__uint_as_float(pr[i] << 16), __uint_as_float(pr[i] & 0xffff0000u)), twice(-1.0f), both), a, b);
+      const __nv_bfloat162 rem = __floats2bfloat162_rn(a, b);
       rest[i] = *reinterpret_cast<const uint32_t*>(&rem);
     }
     tmem_st8(p_base + h * 8, pr);
@@ -532,11 +552,21 @@ __device__ __forceinline__ bool softmax_half(bool ok, uint32_t s_base, uint32_t 
   }
   st.m_ref = m_new;
   const float neg_base = hi_key < 0 ? -INFINITY : m_new == -INFINITY ? 0.0f : -m_new;      // a row that is not used gets zeros
-  float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  f32x2 sums[2] = {0, 0};
   const uint32_t p_base = s_base + rows.c * 32;
-  if (!cap) store_weights(v, p_base, shape.split, sum4, [&](float x) { return fmaf(x, scale_log2, neg_base); });
-  else if (!masked) store_weights(v, p_base, shape.split, sum4, [&](float x) { return capped(shape, x, neg_base); });
-  else store_weights(v, p_base, shape.split, sum4, [&](float x) { return x == -INFINITY ? x : capped(shape, x, neg_base); });
+  if (!cap)
+    store_weights(v, p_base, shape.split, sums, [&](float x, float y) { return fma2(pack2(x, y), twice(scale_log2), twice(neg_base)); });
+  else if (!masked)
+    store_weights(v, p_base, shape.split, sums, [&](float x, float y) { return capped2(shape, pack2(x, y), neg_base); });
+  else
+    store_weights(v, p_base, shape.split, sums, [&](float x, float y) {
+      float a, b;
+      unpack2(capped2(shape, pack2(x, y), neg_base), a, b);
+      return pack2(x == -INFINITY ? x : a, y == -INFINITY ? y : b);
+    });
+  float sum4[4];
+  unpack2(sums[0], sum4[0], sum4[1]);
+  unpack2(sums[1], sum4[2], sum4[3]);
   st.l_run = st.l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
   tmem_wait_st();                                      // P is in tensor memory
   return pv_seen || mbar_wait_warp(pv_done, (block - 1) & 1, err);
