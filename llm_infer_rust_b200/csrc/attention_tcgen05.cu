@@ -333,8 +333,11 @@ __device__ __forceinline__ bool softmax_block(uint32_t s_base, uint32_t o_base, 
 // tokens: 2,040 until the next scores stand, 2,700 in the softmax, 1,720 of those behind the maximum, for 1,024 of
 // special-function work), so what shortens the chain counts: 8,192 tokens x 16 heads 340 -> 302 us, 16,384 x 32 2,165 us
 // (1,015 TFLOP/s).  Behind the maximum the thread's issue slots are the chain, so scale and sum take two scores an instruction
-// (with the MMAs issued by a whole warp: 275 -> 263 us, 3,000 tokens 58.6 -> 56.2, 16,384 x 32 1,998 -> 1,909).  Two threads a row, which pay for the further forms below, were slower here (483 us: sixteen warps
-// leave 96 registers a thread, so the scores are read twice).
+// (with the MMAs issued by a whole warp: 275 -> 265 us, 3,000 tokens 58.6 -> 56.8; from the two before both, 16,384 x 32 2,283 -> 2,171).
+// The weights are added up as softmax_block adds them, a pair's two and then pairs into four sums, so that both kernels give the
+// same bits: which of them runs follows from the other rows of the step.  (Every weight into a sum of its own place, one addition less
+// in the chain, was 264 us.)  Two threads a row, which pay for the further forms below, were slower here (483 us: sixteen warps leave
+// 96 registers a thread, so the scores are read twice).
 __device__ __forceinline__ void tmem_ld32_begin(uint32_t taddr, float (&v)[32]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -396,14 +399,18 @@ __device__ __forceinline__ void softmax_row(uint32_t s_base, uint32_t o_base, in
   for (int c = 0; c < 4; ++c) {
     uint32_t pr[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float a, b;
-      unpack2(fma2(pack2(v[c][2 * i], v[c][2 * i + 1]), scale2, base2), a, b);
-      a = fast_exp2(a);
-      b = fast_exp2(b);
-      sums[i & 1] = add2(sums[i & 1], pack2(a, b));
-      const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
-      pr[i] = *reinterpret_cast<const uint32_t*>(&two);
+    for (int i = 0; i < 16; i += 2) {                  // two pairs of weights a turn: (a0, b0), (a1, b1)
+      float a0, b0, a1, b1;
+      unpack2(fma2(pack2(v[c][2 * i], v[c][2 * i + 1]), scale2, base2), a0, b0);
+      unpack2(fma2(pack2(v[c][2 * i + 2], v[c][2 * i + 3]), scale2, base2), a1, b1);
+      a0 = fast_exp2(a0);
+      b0 = fast_exp2(b0);
+      a1 = fast_exp2(a1);
+      b1 = fast_exp2(b1);
+      sums[(i >> 1) & 1] = add2(sums[(i >> 1) & 1], add2(pack2(a0, a1), pack2(b0, b1)));
+      const __nv_bfloat162 p0 = __floats2bfloat162_rn(a0, b0), p1 = __floats2bfloat162_rn(a1, b1);
+      pr[i] = *reinterpret_cast<const uint32_t*>(&p0);
+      pr[i + 1] = *reinterpret_cast<const uint32_t*>(&p1);
     }
     tmem_st16(s_base + c * 16, pr);
     if (c == 1) {
@@ -480,7 +487,7 @@ struct HalfRows {
   }
 };
 
-// 2^exponent(scores) of 64 scores, two at a time, their sum added to sums; the weights and (split) what their rounding left into
+// 2^exponent(scores) of 64 scores, two at a time, their sum added to sums (a pair's two weights first, then pairs into four sums); the weights and (split) what their rounding left into
 // tensor memory.  Multiply-adds and sums take two an instruction.
 template <typename F>
 __device__ __forceinline__ void store_weights(const float (&v)[64], uint32_t p_base, bool split, f32x2 (&sums)[2], const F& exponent) {
@@ -488,19 +495,23 @@ __device__ __forceinline__ void store_weights(const float (&v)[64], uint32_t p_b
   for (int h = 0; h < 4; ++h) {
     uint32_t pr[8], rest[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 8; i += 2) {                   // two pairs of weights a turn: (a0, b0), (a1, b1)
       const int e = h * 16 + 2 * i;
-      float a, b;
-      unpack2(exponent(v[e], v[e + 1]), a, b);
-      a = fast_exp2(a);
-      b = fast_exp2(b);
-      const f32x2 both = pack2(a, b);
-      sums[i & 1] = add2(sums[i & 1], both);
-      const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
-      pr[i] = *reinterpret_cast<const uint32_t*>(&two);
-      unpack2(fma2(pack2(__uint_as_float(pr[i] << 16), __uint_as_float(pr[i] & 0xffff0000u)), twice(-1.0f), both), a, b);
-      const __nv_bfloat162 rem = __floats2bfloat162_rn(a, b);
-      rest[i] = *reinterpret_cast<const uint32_t*>(&rem);
+      float a0, b0, a1, b1;
+      unpack2(exponent(v[e], v[e + 1]), a0, b0);
+      unpack2(exponent(v[e + 2], v[e + 3]), a1, b1);
+      const f32x2 a = pack2(fast_exp2(a0), fast_exp2(a1)), b = pack2(fast_exp2(b0), fast_exp2(b1));
+      sums[(i >> 1) & 1] = add2(sums[(i >> 1) & 1], add2(a, b));
+      unpack2(a, a0, a1);
+      unpack2(b, b0, b1);
+      const __nv_bfloat162 p0 = __floats2bfloat162_rn(a0, b0), p1 = __floats2bfloat162_rn(a1, b1);
+      pr[i] = *reinterpret_cast<const uint32_t*>(&p0);
+      pr[i + 1] = *reinterpret_cast<const uint32_t*>(&p1);
+      unpack2(fma2(pack2(__uint_as_float(pr[i] << 16), __uint_as_float(pr[i + 1] << 16)), twice(-1.0f), a), a0, a1);
+      unpack2(fma2(pack2(__uint_as_float(pr[i] & 0xffff0000u), __uint_as_float(pr[i + 1] & 0xffff0000u)), twice(-1.0f), b), b0, b1);
+      const __nv_bfloat162 r0 = __floats2bfloat162_rn(a0, b0), r1 = __floats2bfloat162_rn(a1, b1);
+      rest[i] = *reinterpret_cast<const uint32_t*>(&r0);
+      rest[i + 1] = *reinterpret_cast<const uint32_t*>(&r1);
     }
     tmem_st8(p_base + h * 8, pr);
     if (split) tmem_st8(p_base + 64 + h * 8, rest);

@@ -513,6 +513,23 @@ def test_prefill_attention_over_many_key_blocks(nh, nkv, window, page, tiles_per
     close(out, want, torch.bfloat16, bf16_atol=attention_atol(c))
 
 
+@pytest.mark.parametrize("nh,nkv,window", [(16, 8, None), (8, 1, None), (4, 4, 200), (32, 8, 77), (4, 4, None)])
+def test_prompt_attention_does_not_depend_on_the_tiles_a_cta(nh, nkv, window):
+    """One and two tiles of 128 query vectors per CTA give the same bits: which of the two kernels runs follows from the size of
+    the grid, that is from the other rows of the step, and a row's result does not."""
+    o = ops()
+    d, page = 128, 16
+    c = paged_case([(0, 700), (300, 333), (1000, 130), (0, 1500)], nh, nkv, d, page, torch.bfloat16, seed=11)
+    serve = torch.tensor([2, 0, 3, 1], dtype=torch.int32, device=DEV)
+    outs = []
+    for tiles in (1, 2):
+        outs.append(torch.full_like(c["q"], 9.0))
+        o.prefill_attention(c["q"], c["kc"], c["vc"], outs[-1], c["table"], c["cu"], c["kv_len"], c["prefix"], serve, 4,
+                            1500, nh, nkv, d, page, window, 1.5 / math.sqrt(d), tiles_per_cta=tiles)
+    o.check_errors(torch.device(DEV))
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_attention_finds_one_far_key_among_a_thousand():
     """One key far back scores high: whoever skips or misplaces it changes the result."""
     o = ops()
