@@ -17,12 +17,16 @@
 // record() ... finish(slots): the calls that this thread makes in between are kept beside being made, and replay(values) makes them
 // again with other tensors in the places of `slots` (a layer's weights and cache, its input and its output).  A step's layers
 // that are alike make the same calls on the same sizes: one goes through Python, the others are issued by one loop here (a
-// layer of a prompt took the host 108 us, nine launches of 5).  A recording lives as long as its step.
+// layer of a prompt took the host 108 us, nine launches of 5).  A recording lives as long as its step.  It is of use only where every
+// place that another layer's memory could stand in is known: an argument that leads into a slot's memory behind its start, a plain
+// address of it, a block of parameters or a descriptor that is no slot (addresses may stand in it), or a product of another view
+// than the slot's make replay() leave the layers to Python.
 #include <torch/csrc/Device.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
+#include <ATen/EmptyTensor.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -55,14 +59,17 @@ struct Entry {
 
 PyObject *structure_type, *array_type;      // of ctypes
 
-// A call as it was made: an entry point with its arguments (of the integers, which are pointers and, behind finish(), which
-// slot's), or a product of the library.
+// What an integer argument was.
+enum : unsigned char { NUMBER, TENSOR, OBJECT };      // (OBJECT: a ctypes structure or array)
+
+// A call as it was made: an entry point with its arguments (and, behind finish(), which of them are a slot's), or a product of
+// the library.
 struct Call {
   void* fn = nullptr;                       // null: out = x . w^T
   int ni = 0, nf = 0;
   I ints[MAX_INTS];
   float floats[MAX_FLOATS];
-  bool pointer[MAX_INTS];
+  unsigned char kind[MAX_INTS];
   int slot[MAX_INTS];
   at::Tensor x, w, out;
   int x_slot = -1, w_slot = -1, out_slot = -1;
@@ -90,7 +97,7 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
   }
   I ints[MAX_INTS] = {};
   float floats[MAX_FLOATS] = {};
-  bool pointer[MAX_INTS] = {};
+  unsigned char kind[MAX_INTS] = {};
   int ni = 0, nf = 0;
   for (Py_ssize_t i = 0; i < n; ++i) {
     PyObject* a = args[i];
@@ -100,16 +107,19 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
       continue;
     }
     I v = 0;
+    unsigned char is = NUMBER;
     if (a == Py_None) {
     } else if (PyLong_Check(a)) {
       v = PyLong_AsLongLong(a);
       if (v == -1 && PyErr_Occurred()) return nullptr;
     } else if (THPVariable_Check(a)) {
+      is = TENSOR;
       v = reinterpret_cast<I>(THPVariable_Unpack(a).mutable_data_ptr());
     } else if (PyObject_IsInstance(a, structure_type) == 1 || PyObject_IsInstance(a, array_type) == 1) {
       // (the caller's argument holds the object, and with it its memory, until the call has returned)
       Py_buffer view;
       if (PyObject_GetBuffer(a, &view, PyBUF_SIMPLE) != 0) return nullptr;
+      is = OBJECT;
       v = reinterpret_cast<I>(view.buf);
       PyBuffer_Release(&view);
     } else {
@@ -117,8 +127,8 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
       return nullptr;
     }
     if (ni == MAX_INTS) { PyErr_SetString(PyExc_TypeError, "too many arguments for an entry point"); return nullptr; }
-    pointer[ni] = a != Py_None && !PyLong_Check(a);
-    if (recording != nullptr && pointer[ni]) {
+    kind[ni] = is;
+    if (recording != nullptr && is != NUMBER) {
       Py_INCREF(a);
       recording->held.push_back(a);
     }
@@ -136,7 +146,7 @@ PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObj
     c.nf = nf;
     std::copy(ints, ints + MAX_INTS, c.ints);
     std::copy(floats, floats + MAX_FLOATS, c.floats);
-    std::copy(pointer, pointer + MAX_INTS, c.pointer);
+    std::copy(kind, kind + MAX_INTS, c.kind);
   }
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
@@ -260,7 +270,8 @@ PyObject* discard(PyObject*, PyObject*) {
   recording = nullptr;
   Py_RETURN_NONE;
 }
-// finish(slots) -> the recording.  An argument that leads to a slot's memory is the slot's; a tensor of a product likewise.
+// finish(slots) -> the recording.  An argument that leads to the start of a slot's memory is the slot's; a tensor of a product
+// likewise.  Where an argument might lead to a slot's memory in another way the recording keeps no slots and replay() does nothing.
 PyObject* finish(PyObject*, PyObject* slots) {
   HANDLE_TH_ERRORS
   if (recording == nullptr || !PyTuple_Check(slots)) {
@@ -268,30 +279,51 @@ PyObject* finish(PyObject*, PyObject* slots) {
     return nullptr;
   }
   const int n = static_cast<int>(PyTuple_GET_SIZE(slots));
-  std::vector<I> at(n);
+  std::vector<I> at(n), bytes(n, 1);
   recording->slots.clear();
   for (int i = 0; i < n; ++i) {
     PyObject* o = PyTuple_GET_ITEM(slots, i);
     at[i] = address_of(o);
     if (PyErr_Occurred()) return nullptr;
     recording->slots.push_back({THPVariable_Check(o) ? THPVariable_Unpack(o) : at::Tensor(), at[i] % 16 == 0});
+    const at::Tensor& t = recording->slots.back().tensor;
+    if (t.defined()) bytes[i] = static_cast<I>(at::detail::computeStorageNbytes(t.sizes(), t.strides(), t.element_size()));
   }
   // (two slots of one address: an argument does not say whose it is, and no other layer is like this one)
-  for (int i = 0; i < n; ++i)
-    if (std::count(at.begin(), at.end(), at[i]) > 1) { recording->slots.clear(); break; }
+  bool known = true;
+  for (int i = 0; i < n; ++i) known = known && std::count(at.begin(), at.end(), at[i]) == 1;
   auto slot_of = [&](I address) {
     for (int i = 0; i < n; ++i)
       if (at[i] == address) return i;
     return -1;
   };
+  auto inside = [&](I address) {
+    for (int i = 0; i < n; ++i)
+      if (address >= at[i] && address - at[i] < bytes[i]) return true;
+    return false;
+  };
+  // a tensor of a product: the slot's own view of its memory, or none of it
+  auto product_slot = [&](const at::Tensor& t) {
+    const I address = reinterpret_cast<I>(t.mutable_data_ptr());
+    const int s = slot_of(address);
+    if (s < 0) known = known && !inside(address);
+    else known = known && recording->slots[s].tensor.defined() && t.sizes() == recording->slots[s].tensor.sizes() &&
+                 t.strides() == recording->slots[s].tensor.strides();
+    return s;
+  };
   for (Call& c : recording->calls) {
-    for (int i = 0; i < c.ni; ++i) c.slot[i] = c.pointer[i] ? slot_of(c.ints[i]) : -1;
+    for (int i = 0; i < c.ni; ++i) {
+      c.slot[i] = c.kind[i] == NUMBER ? -1 : slot_of(c.ints[i]);
+      if (c.slot[i] >= 0) known = known && (c.kind[i] == TENSOR) == recording->slots[c.slot[i]].tensor.defined();
+      else known = known && c.kind[i] != OBJECT && !inside(c.ints[i]);
+    }
     if (c.fn == nullptr) {
-      c.x_slot = slot_of(reinterpret_cast<I>(c.x.mutable_data_ptr()));
-      c.w_slot = slot_of(reinterpret_cast<I>(c.w.mutable_data_ptr()));
-      c.out_slot = slot_of(reinterpret_cast<I>(c.out.mutable_data_ptr()));
+      c.x_slot = product_slot(c.x);
+      c.w_slot = product_slot(c.w);
+      c.out_slot = product_slot(c.out);
     }
   }
+  if (!known) recording->slots.clear();
   RecordingObject* o = PyObject_New(RecordingObject, &recording_type);
   if (o == nullptr) return nullptr;
   o->r = recording;

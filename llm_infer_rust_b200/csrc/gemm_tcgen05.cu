@@ -273,8 +273,8 @@ B200_EXPORT int b200_gemm_tensor_map(void* out_map, const void* matrix, long lon
 
 // out = a . w^T (mode 0: [m, n]) or silu(a . gate^T) * (a . up^T) (mode 1: w = [gate; up], out [m, n / 2]; in a build with
 // another gate, see glu_product, that one).
-// `a_map`, `w_map`: descriptors of b200_gemm_tensor_map for a [m, k] and w [n, k].
-B200_EXPORT int b200_gemm_tcgen05(const void* a_map, const void* w_map, void* out, int m, int n, int k, int mode,
+// `w_map`: the descriptor of b200_gemm_tensor_map for w [n, k]; activations move, so the one of a [m, k] is made here.
+B200_EXPORT int b200_gemm_tcgen05(const void* a, const void* w_map, void* out, int m, int n, int k, int mode,
                                   float glu_limit, float glu_alpha, int* err, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (k <= 0 || k % 8 != 0 || (mode != GEMM_PLAIN && mode != GEMM_SWIGLU)) return B200_BAD_SIZE;
@@ -288,7 +288,8 @@ B200_EXPORT int b200_gemm_tcgen05(const void* a_map, const void* w_map, void* ou
     configured = true;
   }
   CUtensorMap amap, wmap;
-  memcpy(&amap, a_map, sizeof(amap));
+  const int rc = b200_gemm_tensor_map(&amap, a, m, k);
+  if (rc != 0) return rc;
   memcpy(&wmap, w_map, sizeof(wmap));
   const int m_tiles = (m + BM - 1) / BM;
   const int cols = mode == GEMM_SWIGLU ? n / 2 : n;

@@ -112,7 +112,7 @@ class LayerCalls:
 
     def again(self, values) -> bool:
         """Make the calls with ``values`` in the places of the slots; False, and nothing done, when one of them is not like its
-        slot (another shape, dtype or alignment)."""
+        slot (another shape, dtype or alignment) or a call led to a slot's memory by other ways than the slot itself."""
         rc = self._binding.replay(self._recording, tuple(values))
         if rc is None:
             return False
@@ -1485,12 +1485,8 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, mode: int = GEMM_PLAIN, glu: 
     m, k = x.shape
     n = weight.shape[0]
     out = _empty((m, n // 2 if mode == GEMM_SWIGLU else n), torch.bfloat16, x.device)
-    a_map = ctypes.create_string_buffer(128)          # activations move: their descriptor is made per call
     lib = load_entry_points("gemm_tcgen05.cu", _GLU_DEFINES[glu] or None)
-    rc = lib.b200_gemm_tensor_map(a_map, x, int(m), int(k))
-    if rc != 0:
-        raise KernelError(f"the TMA descriptor of the activations could not be made (code {rc})")
-    rc = lib.b200_gemm_tcgen05(a_map, gemm_map(weight), out, m, n, k, mode, float(limit), float(alpha),
+    rc = lib.b200_gemm_tcgen05(x, gemm_map(weight), out, m, n, k, mode, float(limit), float(alpha),
                                error_word(x.device), _stream())
     _ok(rc, "gemm_tcgen05")
     return out

@@ -166,7 +166,7 @@ class GQAttention(Part):
         """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
         p = self.params
         if type(self) is not GQAttention or cache.k is None or ops.few_row_takes(tokens, p["qkv_proj"], self.env.dtype, ops.EPI_QKV, self.d) \
-                or ops.few_row_takes(tokens, p["o_proj"], self.env.dtype, norm=False):
+                or any(ops.few_row_takes(tokens, p[name], self.env.dtype, norm=False) for name in ("qkv_proj", "o_proj")):
             return None
         slots = [p["qkv_proj"], p["o_proj"], cache.k, cache.v]
         if self.qk_eps is not None:

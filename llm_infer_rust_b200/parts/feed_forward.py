@@ -30,7 +30,7 @@ class SwiGLU(Part):
         """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
         gate_up, down = self.params["gate_up_proj"], self.params["down_proj"]
         if type(self) is not SwiGLU or ops.few_row_takes(x.shape[0], gate_up, self.env.dtype, ops.EPI_SWIGLU) \
-                or ops.few_row_takes(x.shape[0], down, self.env.dtype, norm=False):
+                or any(ops.few_row_takes(x.shape[0], w, self.env.dtype, norm=False) for w in (gate_up, down)):
             return None
         return [gate_up, down] + ([ops.gemm_map(gate_up)] if ops.gemm_tc_pays(x, gate_up, ops.GEMM_SWIGLU) else [])
 

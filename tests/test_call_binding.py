@@ -172,6 +172,27 @@ def test_values_that_are_not_like_their_slots_are_left_to_the_caller(adding):
     assert calls.replay(kept, (torch.zeros(128), torch.zeros(128))) is None
 
 
+class _Block(ctypes.Structure):
+    _fields_ = [("address", ctypes.c_void_p)]
+
+
+@pytest.mark.parametrize("way", ["start", "inside", "address", "address inside", "block", "array", "product of a part", "product behind it"])
+def test_a_slots_memory_reached_by_other_ways(adding, way):
+    """Whatever leads into a slot's memory other than by its start is not exchanged, so such a layer is left to Python."""
+    calls = build.load_call_binding()
+    h, b, w = torch.zeros(4, 4), torch.arange(16.0).view(4, 4), torch.randn(4, 4)
+    block = _Block(b.data_ptr())
+    array = (ctypes.c_float * 16)()
+    reach = {"start": b, "inside": b[1:], "address": b.data_ptr(), "address inside": b.data_ptr() + 16, "block": block, "array": array}
+    calls.record()
+    if way in reach:
+        assert adding.add(h, h, reach[way], 0.0 if way == "block" else 1.0, 1) == 0
+    else:
+        calls.mm_t(b[:2] if way == "product of a part" else b[1:], w)
+    kept = calls.finish((h, b, w))
+    assert calls.replay(kept, (torch.zeros(4, 4), b.clone(), w)) == (0 if way == "start" else None)
+
+
 def test_recordings_are_a_threads_own(adding):
     calls = build.load_call_binding()
     h, b = torch.zeros(3, 4), torch.ones(3, 4)

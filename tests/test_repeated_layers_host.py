@@ -1,0 +1,40 @@
+"""Which layers' calls may be made again with another layer's memory (parts/block.py, parts/model.py), decided without a GPU."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from llm_infer_rust_b200.config.spec import PartSpec
+from llm_infer_rust_b200.kernels import ops
+from llm_infer_rust_b200.parts.attention import GQAttention
+from llm_infer_rust_b200.parts.base import BuildEnv
+from llm_infer_rust_b200.parts.feed_forward import SwiGLU
+
+ENV = BuildEnv(torch.float32, torch.device("cpu"), {})
+CACHE = SimpleNamespace(k=torch.zeros(3, 2, 16, 32), v=torch.zeros(3, 2, 16, 32))
+
+
+def _bound(part):
+    for name, decl in part.param_decls().items():
+        part.bind(name, torch.zeros(decl.shape))
+    return part
+
+
+def _attention(**spec):
+    return _bound(GQAttention(PartSpec("gq_attention", dict(dict(hidden_size=64, num_heads=4, num_kv_heads=2, head_dim=32, qk_norm_eps=1e-6), **spec)), ENV))
+
+
+def _feed_forward():
+    return _bound(SwiGLU(PartSpec("swiglu", dict(hidden_size=64, intermediate_size=96)), ENV))
+
+
+@pytest.mark.parametrize("takes", ["qkv_proj", "o_proj", "gate_up_proj", "down_proj", None])
+def test_a_product_on_the_few_row_kernels_is_not_made_again(monkeypatch, takes):
+    """Those take their operands' addresses in a block of parameters.  Whichever of a part's products goes there, and also when only
+    the plain form of it does, behind a fused form that is refused, the layer goes through Python."""
+    mixer, feed = _attention(), _feed_forward()
+    on_few = {**mixer.params, **feed.params}.get(takes)
+    monkeypatch.setattr(ops, "few_row_takes", lambda rows, weight, dtype, mode=ops.EPI_PLAIN_BF16, head_dim=0, norm=True:
+                        weight is on_few and mode == ops.EPI_PLAIN_BF16 and not norm)
+    assert (mixer.repeat_slots(9, CACHE) is None) == (takes in ("qkv_proj", "o_proj"))
+    assert (feed.repeat_slots(torch.zeros(9, 64)) is None) == (takes in ("gate_up_proj", "down_proj"))
