@@ -163,7 +163,8 @@ class GQAttention(Part):
         return None
 
     def repeat_slots(self, tokens, cache):
-        """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
+        """The numbers that go into the calls of a step of many tokens, and the tensors of them that are this part's own (None: the
+        step goes another way)."""
         p = self.params
         if type(self) is not GQAttention or cache.k is None or ops.few_row_takes(tokens, p["qkv_proj"], self.env.dtype, ops.EPI_QKV, self.d) \
                 or any(ops.few_row_takes(tokens, p[name], self.env.dtype, norm=False) for name in ("qkv_proj", "o_proj")):
@@ -174,7 +175,7 @@ class GQAttention(Part):
         page = cache.k.shape[2]
         if ops.decode_uses_tensor_cores(cache.k.dtype, self.nh, self.nkv, self.d, page):
             slots += [ops.kv_tensor_map(cache.k, min(page, 32)), ops.kv_tensor_map(cache.v, min(page, 32))]
-        return slots
+        return (self.nh, self.nkv, self.d, self.qk_eps, self.window, self.scale, id(self.rope)), slots
 
     def takes_pending(self, tokens: int) -> bool:
         """Whether a step of ``tokens`` tokens runs the input norm as the prologue of the QKV product."""

@@ -46,17 +46,22 @@ class PreNormDeferredAdd:
             ops.flush_chain()
 
     def repeat_slots(self, h, cache):
-        """What is this layer's own in the calls that ``forward`` makes for a step of these tokens, for ``ops.LayerCalls``;
-        None where a step of a layer like it might make others (few tokens, whose products wait for one another; parts that do not
-        say, or that add to what these do)."""
-        if type(self) is not PreNormDeferredAdd or type(self.input_norm) is not RMSNorm or type(self.post_mixer_norm) is not RMSNorm:
+        """For ``ops.LayerCalls``: the numbers that go into the calls that ``forward`` makes for a step of these tokens (only
+        layers with the same ones make the same calls), and the tensors of them that are this layer's own.  None where a step of a
+        layer like it might make others: few tokens, whose products wait for one another; parts that do not say, that add to
+        what these do, or whose ``forward`` was replaced on the object."""
+        before, after, mixer, feed = self.input_norm, self.post_mixer_norm, self.mixer, self.feed_forward
+        if type(self) is not PreNormDeferredAdd or type(before) is not RMSNorm or type(after) is not RMSNorm \
+                or "forward" in self.__dict__ or "forward_add" in before.__dict__ or "forward_add" in after.__dict__ \
+                or "forward" in mixer.__dict__ or "forward" in feed.__dict__:
             return None
-        mixer, feed = getattr(self.mixer, "repeat_slots", None), getattr(self.feed_forward, "repeat_slots", None)
-        mixer = mixer(h.shape[0], cache) if mixer is not None else None
-        feed = feed(h) if feed is not None else None
-        if mixer is None or feed is None:
+        of_mixer, of_feed = getattr(mixer, "repeat_slots", None), getattr(feed, "repeat_slots", None)
+        of_mixer = of_mixer(h.shape[0], cache) if of_mixer is not None else None
+        of_feed = of_feed(h) if of_feed is not None else None
+        if of_mixer is None or of_feed is None:
             return None
-        return [self.input_norm.params["weight"], self.post_mixer_norm.params["weight"]] + mixer + feed
+        numbers, slots = of_mixer
+        return (before.eps, after.eps) + numbers, [before.params["weight"], after.params["weight"]] + slots + of_feed
 
     def forward(self, h, residual, ctx, cache):
         tokens = h.shape[0]

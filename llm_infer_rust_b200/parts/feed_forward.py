@@ -27,7 +27,7 @@ class SwiGLU(Part):
                 "down_proj": ParamDecl((self.hidden, self.inter))}
 
     def repeat_slots(self, x):
-        """What is this part's own in the calls of a step of many tokens (None: the step goes another way)."""
+        """The tensors that are this part's own in the calls of a step of many tokens (None: the step goes another way)."""
         gate_up, down = self.params["gate_up_proj"], self.params["down_proj"]
         if type(self) is not SwiGLU or ops.few_row_takes(x.shape[0], gate_up, self.env.dtype, ops.EPI_SWIGLU) \
                 or any(ops.few_row_takes(x.shape[0], w, self.env.dtype, norm=False) for w in (gate_up, down)):

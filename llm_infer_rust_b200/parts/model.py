@@ -111,16 +111,17 @@ class DecoderModel:
         return end if end - first >= 2 else None
 
     def _repeat(self, first, end, h, residual, ctx, caches):
-        """The entries ``first`` .. ``end`` - 1: the first one's calls are kept and made again with the others' weights and caches.
+        """The entries ``first`` .. ``end`` - 1: the first one's calls are kept and made again with the others' weights and caches
+        (what a layer's parts say now counts: one whose numbers were changed since it was built goes through Python).
         Two buffers take turns: a layer leaves its output where the layer before found its input (which it normed in place)."""
         own = lambda e, h: self.blocks[self.run_list[e].layer].repeat_slots(h, caches[e])
-        slots = own(first, h)
+        numbers, slots = own(first, h)
         calls = ops.LayerCalls(lambda: self.blocks[self.run_list[first].layer].forward(h, residual, ctx, caches[first]),
                                lambda result: [h, result[0]] + slots)
         (out, residual), spare = calls.result, h
         for e in range(first + 1, end):
             values = own(e, out)
-            if values is not None and calls.again([out, spare] + values):
+            if values is not None and values[0] == numbers and calls.again([out, spare] + values[1]):
                 out, spare = spare, out
             else:
                 out, residual = self.blocks[self.run_list[e].layer].forward(out, residual, ctx, caches[e])

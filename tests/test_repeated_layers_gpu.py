@@ -70,6 +70,22 @@ def test_a_layer_whose_weights_are_of_another_kind_goes_through_python():
     assert all(torch.equal(a, b) for a, b in zip(got, plain)) and all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+def test_a_layer_that_was_changed_goes_through_python():
+    """A wrapper round one layer sees every step of many tokens, a scale and a window set on another layer's attention count."""
+    engine = _engine("bfloat16")
+    seen, block = [], engine.model.blocks[3]
+    inner = block.forward
+    block.forward = lambda h, residual, ctx, cache: seen.append(h.shape[0]) or inner(h, residual, ctx, cache)
+    before = _steps(engine)
+    assert seen == [300, 107, sum(range(22, 40)), 20, 56, 3]
+    engine.model.blocks[2].mixer.scale *= 2.0
+    engine.model.blocks[4].mixer.window = 50
+    got = _steps(engine)
+    engine.model.repeats_layers = False
+    want = _steps(engine)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and not any(torch.equal(a, b) for a, b in zip(got, before))
+
+
 def test_repeated_layers_inside_a_captured_prompt():
     """A shape that comes a second time is captured: what is kept are launches, and the graph gives what the step gave."""
     from llm_infer_rust_b200 import StepEntry

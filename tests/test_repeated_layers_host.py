@@ -8,7 +8,9 @@ from llm_infer_rust_b200.config.spec import PartSpec
 from llm_infer_rust_b200.kernels import ops
 from llm_infer_rust_b200.parts.attention import GQAttention
 from llm_infer_rust_b200.parts.base import BuildEnv
+from llm_infer_rust_b200.parts.block import PreNormDeferredAdd
 from llm_infer_rust_b200.parts.feed_forward import SwiGLU
+from llm_infer_rust_b200.parts.norm import RMSNorm
 
 ENV = BuildEnv(torch.float32, torch.device("cpu"), {})
 CACHE = SimpleNamespace(k=torch.zeros(3, 2, 16, 32), v=torch.zeros(3, 2, 16, 32))
@@ -38,3 +40,31 @@ def test_a_product_on_the_few_row_kernels_is_not_made_again(monkeypatch, takes):
                         weight is on_few and mode == ops.EPI_PLAIN_BF16 and not norm)
     assert (mixer.repeat_slots(9, CACHE) is None) == (takes in ("qkv_proj", "o_proj"))
     assert (feed.repeat_slots(torch.zeros(9, 64)) is None) == (takes in ("gate_up_proj", "down_proj"))
+
+
+def _block():
+    block = PreNormDeferredAdd.__new__(PreNormDeferredAdd)
+    block.input_norm, block.post_mixer_norm = (_bound(RMSNorm(PartSpec("rms_norm", dict(width=64, eps=1e-6)), ENV)) for _ in range(2))
+    block.mixer, block.feed_forward = _attention(), _feed_forward()
+    return block
+
+
+@pytest.mark.parametrize("where", ["block", "input_norm", "post_mixer_norm", "mixer", "feed_forward"])
+def test_a_layer_whose_forward_was_replaced_says_so(where):
+    """A wrapper put on one object, as one does to look at what a layer gives: its calls are not made past it."""
+    block, h = _block(), torch.zeros(9, 64)
+    assert block.repeat_slots(h, CACHE) is not None
+    part = block if where == "block" else getattr(block, where)
+    name = "forward_add" if where.endswith("norm") else "forward"
+    setattr(part, name, getattr(part, name))
+    assert block.repeat_slots(h, CACHE) is None
+
+
+@pytest.mark.parametrize("where,name,value", [("input_norm", "eps", 1e-3), ("post_mixer_norm", "eps", 1e-3), ("mixer", "scale", 0.5),
+                                              ("mixer", "window", 5), ("mixer", "qk_eps", 1e-3), ("mixer", "nkv", 1),
+                                              ("mixer", "rope", SimpleNamespace())])
+def test_a_layer_with_other_numbers_is_not_like_the_others(where, name, value):
+    block, other, h = _block(), _block(), torch.zeros(9, 64)
+    assert block.repeat_slots(h, CACHE)[0] == other.repeat_slots(h, CACHE)[0]
+    setattr(getattr(block, where), name, value)
+    assert block.repeat_slots(h, CACHE)[0] != other.repeat_slots(h, CACHE)[0]
