@@ -1163,7 +1163,7 @@ def _chain_buffers(device):
     if st is None:
         if torch.cuda.is_current_stream_capturing():
             raise KernelError("the chain kernel's buffers must exist before a graph is captured")
-        floats = int(_chain_lib().b200_chain_scratch_floats(CHAIN_MAX_ROWS, _sm_count(device)))
+        floats = int(_chain_lib().library.b200_chain_scratch_floats(CHAIN_MAX_ROWS, _sm_count(device)))
         st = _chain_state[key] = dict(scratch=_empty((floats,), torch.float32, device),
                                       tickets=torch.zeros(_CHAIN_TICKETS, dtype=torch.int32, device=device),
                                       sync=torch.zeros(_chain_lib().b200_chain_sync_words(), dtype=torch.int32,

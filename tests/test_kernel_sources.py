@@ -20,6 +20,28 @@ def test_launch_limits_do_not_follow_the_launches():
     assert seen > 5
 
 
+def test_results_that_are_no_int_are_not_asked_for_through_the_binding():
+    """The binding calls every entry point as one that returns an int; a wider result has to come through the library itself."""
+    wide = set()
+    for name in sorted(os.listdir(build.CSRC)):
+        if name.endswith(".cu"):
+            with open(os.path.join(build.CSRC, name)) as f:
+                wide.update(re.findall(r"^B200_EXPORT (?!int )[\w ]+?[ *](b200_\w+)\(", f.read(), re.M))
+    assert len(wide) > 3
+    package, asked = os.path.dirname(build.CSRC), 0
+    for folder, _, files in os.walk(package):
+        for name in (n for n in files if n.endswith(".py")):
+            with open(os.path.join(folder, name)) as f:
+                lines = f.read().splitlines()
+            for i, line in enumerate(lines):
+                for receiver, entry in re.findall(r"((?:\w|\.|\(\))+)\.(b200_\w+)\b(?=\()", line):
+                    if entry in wide:
+                        asked += 1
+                        itself = receiver.endswith(".library") or any(f"{receiver} = load_cuda_library(" in p for p in lines[max(0, i - 5):i])
+                        assert itself, f"{name}:{i + 1}: {line.strip()}"
+    assert asked > 2
+
+
 def test_blocks_that_share_a_tile_of_32_bit_products():
     """Measured with every count of blocks (148 SMs): the fullest SM's time decides, two blocks on an SM cost as much as one."""
     lib = build.load_cuda_library("gemm_f32.cu")
