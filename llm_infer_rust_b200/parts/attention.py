@@ -118,6 +118,13 @@ def attention_splits(dtype, rows: int, num_heads: int, num_kv_heads: int, head_d
     return _splits_over_waves(ctas, kv_len_bound, sm_count, decode_splits(ctas, kv_len_bound, sm_count))
 
 
+# Kept calls hold a layer's intermediates until its stretch of layers ends: what attention made then stays beside the feed-forward's
+# (224 MiB more at the peak of 8,192 tokens at the 8B sizes).  Steps of so many tokens that the host is ahead of the GPU anyway gain
+# nothing by it.  Through Python / kept, us a step: 0.6B sizes, 777 tokens (12 MiB held) 3,112 / 2,496, 1,500 (23 MiB) 3,240 / 3,264,
+# 2,048 3,987 / 3,991; 8B sizes, eight layers, 500 tokens (14 MiB) 1,790 / 1,832, 8,192 (224 MiB) 26,799 / 26,910.
+_REPEAT_HOLDS_AT_MOST = 24 << 20
+
+
 class GQAttention(Part):
     """q, k, v = x W_qkv^T; per-head RMSNorm of q and k; rotary encoding; keys and
     values go to the cache; causal (optionally windowed) attention over the cache;
@@ -168,6 +175,8 @@ class GQAttention(Part):
         p = self.params
         if type(self) is not GQAttention or cache.k is None or ops.few_row_takes(tokens, p["qkv_proj"], self.env.dtype, ops.EPI_QKV, self.d) \
                 or any(ops.few_row_takes(tokens, p[name], self.env.dtype, norm=False) for name in ("qkv_proj", "o_proj")):
+            return None
+        if tokens * (3 * self.nh + 2 * self.nkv) * self.d * self.env.dtype.itemsize > _REPEAT_HOLDS_AT_MOST:      # (QKV, q, the heads' outputs)
             return None
         slots = [p["qkv_proj"], p["o_proj"], cache.k, cache.v]
         if self.qk_eps is not None:

@@ -98,3 +98,22 @@ def test_repeated_layers_inside_a_captured_prompt():
         out.append(engine.step([StepEntry(1, prompt, [199])]).clone())
         engine.close_request(1)
     assert len(engine._shape_graphs) == 1 and all(torch.equal(o, out[0]) for o in out)
+
+
+def test_kept_layers_hold_little():
+    """The peak of a step of many tokens is what it is without kept calls."""
+    from llm_infer_rust_b200 import StepEntry
+    config = dict(CONFIG, num_attention_heads=16, num_key_value_heads=8, head_dim=128)
+    engine = _engine("bfloat16", config)
+    peaks = []
+    for engine.model.repeats_layers in (False, True):
+        for r in range(1, 6):
+            engine.open_request(r)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        engine.step([StepEntry(r, list(range(2, 290)) * 2, [575]) for r in range(1, 6)])
+        peaks.append(torch.cuda.max_memory_allocated() - before)
+        for r in range(1, 6):
+            engine.close_request(r)
+    assert peaks[1] <= peaks[0] + (1 << 20)

@@ -68,3 +68,10 @@ def test_a_layer_with_other_numbers_is_not_like_the_others(where, name, value):
     assert block.repeat_slots(h, CACHE)[0] == other.repeat_slots(h, CACHE)[0]
     setattr(getattr(block, where), name, value)
     assert block.repeat_slots(h, CACHE)[0] != other.repeat_slots(h, CACHE)[0]
+
+
+def test_a_step_whose_intermediates_are_many_is_not_kept():
+    """A kept layer's QKV, q and heads' outputs stay beside what the feed-forward makes: 24 MiB of them at most."""
+    mixer, bytes_a_token = _attention(), (3 * 4 + 2 * 2) * 32 * 4
+    assert mixer.repeat_slots((24 << 20) // bytes_a_token, CACHE) is not None
+    assert mixer.repeat_slots((24 << 20) // bytes_a_token + 1, CACHE) is None
