@@ -404,13 +404,57 @@ __device__ __forceinline__ void sp_split(float x, float y, uint32_t& high, uint3
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(low) : "f"(y), "f"(x));
 }
 
-// One element as plain FFMA: what stands where the terms gave no finite number (an infinity has no second term).
-__device__ __noinline__ float sp_plain(const float* __restrict__ a, const float* __restrict__ w, int k) {
-  float t = 0.0f;
-  for (int i = 0; i < k; ++i) t = fmaf(a[i], w[i], t);
+// Elements for which the terms give no number (an infinity has no second term) are summed again in FFMA, by whole warps: a lane
+// takes every 32nd piece of four k, the 32 sums meet by halves.  Lane `l` of the warp that calls this has element (m, n) of C and
+// its sum t; it gets t back, or the new sum where `again`.  A row of x that holds a NaN has NaN everywhere and is found in one pass over it: behind
+// the first NaN of a prompt's rows every element of theirs comes here.  (One thread an element, down its row of W alone, would
+// hold a tile of 128 x 128 up for tens of milliseconds at K = 12,288.)
+__device__ __forceinline__ bool sp_settled(float t) { return fabsf(t) <= 3.402823466e38f; }
+__device__ __noinline__ float sp_again(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, int k, int m, int n, float t, bool again) {
+  const int lane = threadIdx.x & 31;
+  unsigned todo = __ballot_sync(0xffffffffu, again);
+  int looked_at = -1;
+  while (todo != 0) {
+    const int j = __ffs(todo) - 1, jm = __shfl_sync(0xffffffffu, m, j), jn = __shfl_sync(0xffffffffu, n, j);
+    const float4* x = reinterpret_cast<const float4*>(a + static_cast<size_t>(jm) * lda);
+    if (jm != looked_at) {
+      looked_at = jm;
+      bool nan = false;
+#pragma unroll 4
+      for (int i = lane; i < k / 4; i += 32) {
+        const float4 v = x[i];
+        nan = nan || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+      }
+      if (__any_sync(0xffffffffu, nan)) {
+        if (again && m == jm) t = __int_as_float(0x7fffffff);
+        todo &= ~__ballot_sync(0xffffffffu, m == jm);
+        continue;
+      }
+    }
+    const float4* y = reinterpret_cast<const float4*>(w + static_cast<size_t>(jn) * ldw);
+    float sum = 0.0f;
+#pragma unroll 4
+    for (int i = lane; i < k / 4; i += 32) {
+      const float4 u = x[i], v = y[i];
+      sum = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, sum))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == j) t = sum;
+    todo &= todo - 1;
+  }
   return t;
 }
-__device__ __forceinline__ bool sp_finite(float t) { return fabsf(t) <= 3.402823466e38f; }
+// The same of what this warp has stored as row m of C, columns n0 to n0 + 31 (and on, in steps of 32, up to `columns`).
+__device__ __forceinline__ void sp_stored_again(const Product& p, int m, int n0, int columns) {
+  for (int n = n0 + (threadIdx.x & 31); n < n0 + columns; n += 32) {
+    float* at = p.c + static_cast<size_t>(m) * p.ldc + n;
+    const float v = n < p.n ? *at : 0.0f;
+    const bool again = !sp_settled(v);
+    const float t = sp_again(p.a, p.lda, p.w, p.ldw, p.k, m, n, v, again);
+    if (again) *at = t;
+  }
+}
 
 template <int NT> struct SplitShape {
   static constexpr int WARPS = 16;                                  // that take terms apart and add sums up
@@ -458,6 +502,7 @@ split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   const int first_tile = blockIdx.x / job.ksplit, tile_step = gridDim.x / job.ksplit;
   const int k_lo = rank * job.spans_a_rank * job.span_stages;
   const int k_hi = min(job.stages, k_lo + job.spans_a_rank * job.span_stages);
+  bool again = false;                                               // this thread has stored a sum that is no number
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::RING; ++s) { sp_init(raw_full + s, 1); sp_init(raw_free + s, S::WARPS); }
@@ -652,7 +697,7 @@ split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
       totals([&](int c, float v) {
         const int t = group * S::COLS + c, m = m0 + t;
         if (t < job.tokens && m < p.m && n < p.n) {
-          if (!sp_finite(v)) v = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
+          again = again || !sp_settled(v);
           p.c[static_cast<size_t>(m) * p.ldc + n] = v;
         }
       });
@@ -691,7 +736,7 @@ split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         if (n + e < p.n) {
-          if (!sp_finite(t[e])) t[e] = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n + e) * p.ldw, p.k);
+          again = again || !sp_settled(t[e]);
           p.c[static_cast<size_t>(m) * p.ldc + n + e] = t[e];
         }
     }
@@ -702,6 +747,20 @@ split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ C
   if (warp == S::WARPS) {
     sp_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::TMEM) : "memory");
+  }
+  // Last of all, where the loops' registers are free and no warp waits for another (a call among the stores: 300 rows of 1,024 x
+  // 2,048 28 -> 46 us), each warp the elements that it has stored itself.
+  if (__any_sync(0xffffffffu, again)) {
+    if (job.ksplit > 1) {                                           // (32 threads have one row of the tile, 128 columns of C)
+      const int n0 = first_tile / job.m_tiles * SP_BN, m0 = first_tile % job.m_tiles * job.tokens;
+      for (int i = rank * S::THREADS + warp * 32; i < job.tokens * SP_BN / 4; i += job.ksplit * S::THREADS)
+        if (m0 + i / (SP_BN / 4) < p.m) sp_stored_again(p, m0 + i / (SP_BN / 4), n0, SP_BN);
+    } else {
+      for (int tile = first_tile; tile < job.tiles; tile += tile_step) {
+        const int n0 = tile / job.m_tiles * SP_BN, m0 = tile % job.m_tiles * job.tokens, first = (warp >> 2) * S::COLS;
+        for (int t = first; t < first + S::COLS && t < job.tokens && m0 + t < p.m; ++t) sp_stored_again(p, m0 + t, n0 + (warp & 3) * 32, 32);
+      }
+    }
   }
 }
 
@@ -811,14 +870,16 @@ few_split_kernel(const Product p, int tiles, int stages, int span_stages) {
 #pragma unroll
         for (int i = 0; i < WN / 4; ++i) to[(x * 8 + 2 * c4 + (i & 1)) * WN + r + (i >> 1) * 8] = sum[x][i];
     __syncthreads();
+    static_assert(WN * MR % 32 == 0, "whole warps");
     for (int i = threadIdx.x; i < WN * MR; i += 256) {           // the element: its spans in order
       const int m = m0 + i / WN, n = tile * WN + i % WN;
-      if (m >= p.m || n >= p.n) continue;
+      const bool mine_here = m < p.m && n < p.n;
       const float* from = red + parity * F::WARPS * WN * MR + i;
       float v = from[0];
       for (int s = 1; s < spans; ++s) v += from[s * WN * MR];
-      if (!sp_finite(v)) v = sp_plain(p.a + static_cast<size_t>(m) * p.lda, p.w + static_cast<size_t>(n) * p.ldw, p.k);
-      p.c[static_cast<size_t>(m) * p.ldc + n] = v;
+      const bool again = mine_here && !sp_settled(v);
+      if (__any_sync(0xffffffffu, again)) v = sp_again(p.a, p.lda, p.w, p.ldw, p.k, m, n, v, again);
+      if (mine_here) p.c[static_cast<size_t>(m) * p.ldc + n] = v;
     }
   }
   cp_async_wait<0>();

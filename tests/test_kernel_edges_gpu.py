@@ -76,6 +76,31 @@ def test_32_bit_products_of_infinities_and_the_largest_numbers():
     assert ((ops.gemm_f32(small, w).double() - want).abs() <= 40 * 2.0 ** -24 * size).all()
 
 
+# one kernel each: few rows, a cluster a tile, blocks that walk over tiles
+@pytest.mark.parametrize("m,n,k", [(7, 1024, 4096), (300, 1024, 4096), (1024, 4096, 2048)])
+def test_32_bit_products_whose_rows_are_all_nan_or_infinite(m, n, k):
+    """Every element of such rows is summed again.  No block waits so long for it that another of its warps gives up, and the
+    other rows keep their bits.  (A thread an element took 60 ms a tile and more.)"""
+    from llm_infer_rust_b200.kernels import ops
+    x, w = _rnd(m, k), _rnd(n, k, seed=1)
+    plain = ops.gemm_f32(x, w)
+    for bad in (float("nan"), float("inf")):
+        a = x.clone()
+        a[m // 3:] = bad
+        got = ops.gemm_f32(a, w)
+        torch.cuda.synchronize()
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        ops.gemm_f32(a, w, out=got)
+        end.record()
+        ops.check_errors(a.device)
+        assert torch.equal(got[:m // 3], plain[:m // 3])
+        assert got[m // 3:].isnan().all()                       # (infinities of both signs meet in every sum)
+        # a NaN costs a pass over its row; an infinity one over its row and W's for every element, 1,000 cycles and 16 warps a block
+        if bad != bad:
+            assert begin.elapsed_time(end) < 20.0
+
+
 def test_32_bit_products_of_a_head_each():
     from llm_infer_rust_b200.kernels import ops
     for rows in (3, 70):
