@@ -321,7 +321,8 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
 // softmax of its own over its keys and the four parts of a vector are added up at the end in order.  Which keys a warp takes
 // depends on their positions alone, so a position's result has the same bits however the prompt was cut.
 // The query's terms stay in registers; keys and values are taken apart as they are read, since a block serves two warps only.
-// A tile whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term).
+// A tile whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term), and so is one with
+// sums of weighted values below 2^-80: values below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.
 // Bound by the instructions that take keys and values apart (two warps a scheduler, 22 for a thread's four numbers, six products).  us,
 // CUDA cores / this: 16 heads of 128, 8 KV heads, 300 tokens 59.3 / 30.7, 17 tokens 13.5 / 10.5, 2,000 tokens 991 / 598, 64 behind 2,000
 // cached 343 / 170, 16 rows of 5 behind 100 21.6 / 13.8; heads of 64, 300 tokens 42.3 / 18.7, of 16 37.6 / 11.5.  Error against 64 bits
@@ -337,8 +338,8 @@ struct SplitPrefill {
   static constexpr size_t SMEM = TILES + sizeof(float) * 4 * 32 * 2;
 };
 
-// Two floats as three bfloat16 terms each, packed (the first float in the low half): x = high + mid + low exactly, each term
-// the rest rounded to eight bits.
+// Two floats as three bfloat16 terms each, packed (the first float in the low half): x = high + mid + low, each term the rest
+// rounded to eight bits; exactly from 2^-110 on.
 __device__ __forceinline__ void terms_of(float x, float y, uint32_t& high, uint32_t& mid, uint32_t& low) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(high) : "f"(y), "f"(x));
   x -= __uint_as_float(high << 16);
@@ -534,7 +535,7 @@ prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
       *reinterpret_cast<float2*>(parts + (quarter * 32 + vec) * (D + 4) + 8 * n + 2 * c4) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
   }
   __syncthreads();
-  bool finite = true;
+  bool settled = true;
   for (int i = threadIdx.x; i < nvec * (D / 4); i += PF_WARPS * 32) {
     const int vec = i / (D / 4), at = i - vec * (D / 4);
     float top = -INFINITY;
@@ -552,10 +553,12 @@ prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
     if (sinks != nullptr && sum > 0.0f) sum += expf(sinks[head] - top);
     const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
     const float4 v = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
-    finite = finite && fabsf(sum) < INFINITY && fabsf(acc[0]) < INFINITY && fabsf(acc[1]) < INFINITY && fabsf(acc[2]) < INFINITY && fabsf(acc[3]) < INFINITY;
+    settled = settled && fabsf(sum) < INFINITY;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) settled = settled && fabsf(acc[e]) < INFINITY && (fabsf(acc[e]) >= 8.2718061e-25f || acc[e] == 0.0f);
     *reinterpret_cast<float4*>(out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D + 4 * at) = v;
   }
-  if (__syncthreads_or(finite ? 0 : 1))
+  if (__syncthreads_or(settled ? 0 : 1))
     prefill_tile_again(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window,
                        scale, tile_tokens, head_chunks, softcap, chunk, sinks);
 }

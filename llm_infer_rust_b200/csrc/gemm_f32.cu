@@ -8,8 +8,9 @@
 // spans in order.  That order depends on k alone and both kernels keep to it, split_kernel (tcgen05: many rows) and few_split_kernel
 // (mma.sync, which gives the same bits: the tests compare them), so a token's result is bit-identical however the batch around it
 // is cut.  Error against 64 bits 0.9e-7 of a product's norm (K = 1,024; FFMA in short sums 2.1e-7, in one chain 2.1e-6 for a model's
-// logits).  An element whose terms give no finite sum (an infinity has no second term) is summed again by FFMA; numbers below 2^-110
-// lose their third term to the smallest bfloat16.
+// logits).  An element whose terms give no finite sum (an infinity has no second term) is summed again by FFMA, and so is one
+// below 2^-80: numbers below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.  (What is left: such numbers
+// times others above 2^30, and products that vanish as a whole, below 2^-133.)
 // Measured, us with FFMA tiles / in terms, layers of Qwen3-0.6B: QKV at 4, 32 and 300 rows 9.9 / 5.5, 41.7 / 11.0, 119 / 39 (65 of an
 // ideal 274 TFLOP/s: the terms are taken apart and the sums added up by CUDA cores), O 6.4 / 5.0, 40.8 / 9.7, 63 / 35, gate and up 11.0 / 7.3,
 // 43.2 / 15.6, 127 / 40, down 7.4 / 6.5, 40.8 / 13.6, 65 / 43; one row of large matrices is slower (151,936 x 1,024: 104 / 118).
@@ -404,12 +405,15 @@ __device__ __forceinline__ void sp_split(float x, float y, uint32_t& high, uint3
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(low) : "f"(y), "f"(x));
 }
 
-// Elements for which the terms give no number (an infinity has no second term) are summed again in FFMA, by whole warps: a lane
+// Elements for which the terms give no number (an infinity has no second term), or a very small one, are summed again in FFMA, by whole warps: a lane
 // takes every 32nd piece of four k, the 32 sums meet by halves.  Lane `l` of the warp that calls this has element (m, n) of C and
 // its sum t; it gets t back, or the new sum where `again`.  A row of x that holds a NaN has NaN everywhere and is found in one pass over it: behind
 // the first NaN of a prompt's rows every element of theirs comes here.  (One thread an element, down its row of W alone, would
 // hold a tile of 128 x 128 up for tens of milliseconds at K = 12,288.)
-__device__ __forceinline__ bool sp_settled(float t) { return fabsf(t) <= 3.402823466e38f; }
+__device__ __forceinline__ bool sp_settled(float t) {
+  const float size = fabsf(t);
+  return size <= 3.402823466e38f && (size >= 8.2718061e-25f || size == 0.0f);      // (2^-80; a NaN compares false)
+}
 __device__ __noinline__ float sp_again(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, int k, int m, int n, float t, bool again) {
   const int lane = threadIdx.x & 31;
   unsigned todo = __ballot_sync(0xffffffffu, again);

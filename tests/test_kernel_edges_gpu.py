@@ -76,6 +76,21 @@ def test_32_bit_products_of_infinities_and_the_largest_numbers():
     assert ((ops.gemm_f32(small, w).double() - want).abs() <= 40 * 2.0 ** -24 * size).all()
 
 
+@pytest.mark.parametrize("exponent", [-105, -118, -126])
+@pytest.mark.parametrize("m,n,k", [(5, 130, 64), (200, 300, 1024), (150, 20000, 64)])
+def test_32_bit_products_of_very_small_numbers(m, n, k, exponent):
+    """Above and below 2^-110, where a third term no longer has all its bits."""
+    from llm_infer_rust_b200.kernels import ops
+    for of_w in (False, True):
+        a, w = _rnd(m, k).abs() + 1.0, _rnd(n, k, seed=1)
+        a, w = (a, w * 2.0 ** exponent) if of_w else (a * 2.0 ** exponent, w)
+        got = ops.gemm_f32(a, w)
+        want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+        # as test_32_bit_products_in_three_terms, or k / 32 + 5 roundings of FFMA, and half of the smallest float32 for each of k + 40 sums
+        assert ((got.double() - want).abs() <= (35 + k / 32) * 2.0 ** -24 * size + (k + 40) * 2.0 ** -150).all()
+        assert torch.equal(ops.gemm_f32(a[2:5].contiguous(), w), got[2:5])
+
+
 # one kernel each: few rows, a cluster a tile, blocks that walk over tiles
 @pytest.mark.parametrize("m,n,k", [(7, 1024, 4096), (300, 1024, 4096), (1024, 4096, 2048)])
 def test_32_bit_products_whose_rows_are_all_nan_or_infinite(m, n, k):
@@ -346,6 +361,20 @@ def test_32_bit_prompt_attention(lens, cached, nh, nkv, d, page, form):
             assert torch.equal(torch.cat(parts), got)
         else:                                                   # (a tile's first block follows its first query's window)
             assert (torch.cat(parts) - got).abs().max() <= 2.0 ** -24 * 400 * v.abs().max()
+
+
+@pytest.mark.parametrize("exponent", [-105, -118])
+def test_32_bit_prompt_attention_of_very_small_values(exponent):
+    """Above and below 2^-110, where a third term no longer has all its bits."""
+    from llm_infer_rust_b200.kernels import ops
+    lens, cached, nh, nkv, d, page = [50], [30], 4, 2, 64, 16
+    k, v, table, cu, total, prefix, rows = _paged(lens, cached, nkv, d, page)
+    q, v = _rnd(50, nh * d, seed=3), (v.abs() + 1.0) * 2.0 ** exponent
+    out = torch.empty_like(q)
+    ops.prefill_attention(q, k, v, out, table, cu, total, prefix, rows, 1, 50, nh, nkv, d, page, None, d ** -0.5)
+    want = _attention_64(q, k, v, table, lens, cached, nh, nkv, d, page, d ** -0.5)
+    # values of one sign: as test_32_bit_prompt_attention relative to the result, and the products' roundings below 2^-126
+    assert ((out.double() - want).abs() <= 2.0 ** -24 * 400 * want + 200 * 2.0 ** -150).all()
 
 
 def test_32_bit_prompt_attention_of_infinities():
