@@ -5,15 +5,15 @@
 // numbers (8 + 8 + 8 bits), the product of two floats the sum of nine products of terms, each exact in float, and the six that
 // reach 2^-24 of it are taken.  32 k are summed by the tensor cores from zero, small products first (what an addition there cuts off
 // below a sum's last place stays that of 32 terms); those sums are added in float, an eighth of K (a span) in order, then the eight
-// spans in order.  That order depends on k alone and both kernels keep to it, split_kernel (tcgen05: many rows) and few_split_kernel
-// (mma.sync, which gives the same bits: the tests compare them), so a token's result is bit-identical however the batch around it
-// is cut.  Error against 64 bits 0.9e-7 of a product's norm (K = 1,024; FFMA in short sums 2.1e-7, in one chain 2.1e-6 for a model's
+// spans in order.  That order depends on k alone and the kernels keep to it, split_kernel (tcgen05: many rows), few_split_kernel and
+// pair_split_kernel (mma.sync, which gives the same bits: the tests compare them), so a token's result is bit-identical however the
+// batch around it is cut.  Error against 64 bits 0.9e-7 of a product's norm (K = 1,024; FFMA in short sums 2.1e-7, in one chain 2.1e-6 for a model's
 // logits).  An element whose terms give no finite sum (an infinity has no second term) is summed again by FFMA, and so is one
 // below 2^-80: numbers below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.  (What is left: such numbers
 // times others above 2^30, and products that vanish as a whole, below 2^-133.)
 // Measured, us with FFMA tiles / in terms, layers of Qwen3-0.6B: QKV at 4, 32 and 300 rows 9.9 / 5.5, 41.7 / 11.0, 119 / 39 (65 of an
 // ideal 274 TFLOP/s: the terms are taken apart and the sums added up by CUDA cores), O 6.4 / 5.0, 40.8 / 9.7, 63 / 35, gate and up 11.0 / 7.3,
-// 43.2 / 15.6, 127 / 40, down 7.4 / 6.5, 40.8 / 13.6, 65 / 43; one row of large matrices is slower (151,936 x 1,024: 104 / 118).
+// 43.2 / 15.6, 127 / 40, down 7.4 / 6.5, 40.8 / 13.6, 65 / 43.
 //
 // Other products (K or a distance between rows no multiple of four, unaligned pointers) and batched ones keep to FFMA on CUDA cores,
 // in an order of their own that depends on k alone as well: K is cut into chunks of 128 and spans of four chunks; a chunk is summed
@@ -37,6 +37,7 @@
 #include <cuda.h>
 
 #include <initializer_list>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -889,6 +890,165 @@ few_split_kernel(const Product p, int tiles, int stages, int span_stages) {
   cp_async_wait<0>();
 }
 
+// ------------------------------------------------------------------ up to four rows, in the same terms
+// The same products in the same order once more.  A block takes x apart once, for all the tiles that it walks over (few_split_kernel
+// with every 16 rows of W again).  The instruction's sixteen rows are eight rows of W at one stage and the same eight at the next, its
+// eight columns four rows of x at the one and at the other: two of its four quarters are the two stages' sums, so that tiles have
+// eight rows of W and chains of products half the length.  A chain of twelve takes 255 cycles for 98 of the tensor cores' time, so
+// a step has U pairs of stages side by side.  Which of a 16's k lie in which place of the instruction is the same for both operands, and
+// of no account for a sum's bits.
+// G groups of eight warps (a warp a span, as in few_split_kernel) share x and take every G-th tile; x is asked for before W, which
+// otherwise holds it up (deeper rings of W were slower for that: 1,024 x 3,072 5.9 us with two steps, 6.4 with four).
+// Shared memory: x as [stage][row][c4][half][term][2] words (48 bytes a lane), [G][2][8 spans][rows][8] sums, the rings.
+// Bound by W's bytes where it is large.  One row, us: FFMA / few_split_kernel / this: 24,576 x 4,096 62 / 77 / 63 (6.4 TB/s), 151,936 x 1,024
+// 105 / 118 / 106, 6,144 x 4,096 20.5 / 23.1 / 20.3, 4,096 x 12,288 48 / 44 / 38, 1,024 x 3,072 5.4 / 7.1 / 5.5, 2,048 x 8,192 17.6 / 28.1 / 14.3
+// (FFMA stays ahead at 1,024 x 4,096, 5.8 / 8.8 / 6.5, and with two rows of 151,936 x 1,024, 98.9 / 118 / 106);
+// four rows: 24,576 x 4,096 (x does not fit) 90 / 77, 151,936 x 1,024 134 / 118 / 106, 1,024 x 3,072 7.8 / 7.1 / 6.0.
+constexpr int PAIR_ROWS = 4, PAIR_WN = 8;
+static size_t pair_split_bytes(int m, int stages, int ring, int pairs, int groups) {
+  return (static_cast<size_t>(stages + 2 * pairs) * m * 48 + groups * (2 * SP_SPANS * m * PAIR_WN + SP_SPANS * ring * pairs * 512)) * sizeof(float);
+}
+
+template <int RING, int U, int G>
+__global__ void __launch_bounds__(256 * G, 1)
+pair_split_kernel(const Product p, int tiles, int stages, int span_stages) {
+  extern __shared__ __align__(128) float few_split_smem[];
+  uint32_t* xt = reinterpret_cast<uint32_t*>(few_split_smem);
+  float* red = few_split_smem + (stages + 2 * U) * p.m * 48;
+  const int group = threadIdx.x >> 8, warp = (threadIdx.x >> 5) & 7, lane = threadIdx.x & 31, r = lane >> 2, c4 = lane & 3;
+  float4* ring = reinterpret_cast<float4*>(red + G * 2 * SP_SPANS * p.m * PAIR_WN) + (group * 8 + warp) * RING * U * 128;
+  red += group * 2 * SP_SPANS * p.m * PAIR_WN;
+  const int first_tile = blockIdx.x + group * gridDim.x, tile_step = G * gridDim.x;
+  const int k_lo = min(stages, warp * span_stages), mine = min(stages, k_lo + span_stages) - k_lo;      // this warp's stages of a tile
+  const int spans = (stages + span_stages - 1) / span_stages, units = (mine + 2 * U - 1) / (2 * U);
+  const int k_end = min(p.k, (k_lo + mine) * SP_KS);
+
+  // 2 U stages of the tile's eight rows, whole lines of 128 bytes; an odd row's pieces are exchanged by four, so that the two rows of
+  // a quarter warp's reads lie in different banks.
+  int f_tile = first_tile, f_unit = 0, f_slot = 0;
+  auto fetch = [&]() {
+    if (f_tile < tiles && units > 0) {
+      const int line = lane >> 3, piece = lane & 7, row = f_tile * PAIR_WN + line, kk = (k_lo + 2 * U * f_unit) * SP_KS + 4 * piece;
+      const float* src = p.w + static_cast<size_t>(row) * p.ldw + kk;
+      float4* to = ring + f_slot * U * 128 + line * 8 + (piece ^ (4 * (line & 1)));
+#pragma unroll
+      for (int e = 0; e < 4 * U; ++e) {                             // [stage][four rows]
+        const bool valid = row + 4 * (e & 1) < p.n && kk + SP_KS * (e >> 1) < k_end;
+        cp_async16(to + (e >> 1) * 64 + (e & 1) * 32, valid ? src + (e & 1) * 4 * static_cast<size_t>(p.ldw) + SP_KS * (e >> 1) : p.w, valid);
+      }
+      if (++f_unit == units) { f_unit = 0; f_tile += tile_step; }
+    }
+    if (++f_slot == RING) f_slot = 0;
+    cp_async_commit();
+  };
+  pdl_wait();
+  // x of this span: its warps (one a group) take every G-th 32 pieces each, four at a time
+  const int pieces = mine * 8;                                      // of a row
+  auto take_apart = [&](int i0, bool begin) {
+    float4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = i0 + 32 * G * j, row = i / max(pieces, 1), kk = k_lo * SP_KS + (i - row * pieces) * 4;
+      v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < p.m * pieces && kk < p.k) v[j] = *reinterpret_cast<const float4*>(p.a + static_cast<size_t>(row) * p.lda + kk);
+    }
+    if (begin) {
+      __syncthreads();                                              // W is asked for behind all of x's first pieces, which everything waits for
+#pragma unroll
+      for (int s = 0; s < RING - 1; ++s) fetch();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = i0 + 32 * G * j, row = i / max(pieces, 1), at = i - row * pieces, stage = k_lo + (at >> 3), piece = at & 7;
+      if (i >= p.m * pieces) break;
+      uint2 high, mid, low;
+      sp_split(v[j].x, v[j].y, high.x, mid.x, low.x);
+      sp_split(v[j].z, v[j].w, high.y, mid.y, low.y);
+      uint2* to = reinterpret_cast<uint2*>(xt + ((stage * p.m + row) * 4 + (piece & 3)) * 12 + (piece >> 2) * 6);
+      to[0] = high; to[1] = mid; to[2] = low;
+    }
+  };
+  take_apart(group * 32 + lane, true);
+  for (int i = group * 32 + lane + 128 * G; i < p.m * pieces; i += 128 * G) take_apart(i, false);
+  if (G > 1) asm volatile("bar.sync %0, %1;\n" ::"r"(G + 1 + warp), "r"(32 * G) : "memory"); else __syncwarp();
+
+  const bool has_x = (r & 3) < p.m;
+  const uint4* my_x = reinterpret_cast<const uint4*>(xt + (((k_lo + (r >> 2)) * p.m + (r & 3)) * 4 + c4) * 12);
+  static_assert(U <= 2, "a step of fewer pairs than U has one");
+  // `pairs` pairs of stages from pair `at` of this warp on: their sums to those of the tile
+  auto multiply = [&](auto pairs, int at, int slot, float (&sum)[2]) {
+    constexpr int N = decltype(pairs)::value;
+    uint32_t a[N][2][3][4], b[N][2][3][2];                          // [pair][half][term]
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+      uint4 terms_of_x[3] = {};
+      if (has_x) {
+        const uint4* from = my_x + (at + x) * 2 * p.m * 12;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) terms_of_x[i] = from[i];
+      }
+      memcpy(b[x], terms_of_x, sizeof(b[x]));
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {                               // (stage s: the instruction's rows 8 s to 8 s + 7)
+          const float4 v = ring[(slot * 2 * U + 2 * x + s) * 64 + r * 8 + ((h * 4 + c4) ^ (4 * (r & 1)))];
+          sp_split(v.x, v.y, a[x][h][0][s], a[x][h][1][s], a[x][h][2][s]);
+          sp_split(v.z, v.w, a[x][h][0][2 + s], a[x][h][1][2 + s], a[x][h][2][2 + s]);
+        }
+    }
+    constexpr int WI[6] = {2, 0, 1, 1, 0, 0}, XI[6] = {0, 2, 1, 0, 1, 0};
+    float t[N][4] = {};
+#pragma unroll
+    for (int q = 0; q < 12; ++q)
+#pragma unroll
+      for (int x = 0; x < N; ++x) sp_mma_sync(t[x], a[x][q & 1][WI[q >> 1]], b[x][q & 1][XI[q >> 1]]);
+    // rows 0 to 7 x columns 0 to 3: the first stage; rows 8 to 15 x columns 4 to 7: the second, in the lane two further on
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float second = __shfl_down_sync(0xffffffffu, t[x][2 + i], 2);
+        sum[i] = at + x == 0 ? t[x][i] : sum[i] + t[x][i];
+        if (2 * (at + x) + 1 < mine) sum[i] += second;
+      }
+  };
+  int parity = 0, slot = 0, turn = 0;
+  for (int tile = first_tile; tile < tiles; tile += tile_step, parity ^= 1) {
+    float sum[2] = {};
+    for (int u = 0; u < units; ++u) {
+      __syncwarp();                                                 // (the slot that is filled has been read)
+      fetch();
+      cp_async_wait<RING - 1>();
+      __syncwarp();
+      if (2 * (U * u + U - 1) < mine) multiply(std::integral_constant<int, U>(), U * u, slot, sum);
+      else multiply(std::integral_constant<int, 1>(), U * u, slot, sum);
+      if (++slot == RING) slot = 0;
+    }
+    float* to = red + (parity * SP_SPANS + warp) * PAIR_WN * p.m;
+    if (mine > 0)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (2 * c4 + i < p.m) to[(2 * c4 + i) * PAIR_WN + r] = sum[i];
+    asm volatile("bar.sync %0, 256;\n" ::"r"(group + 1) : "memory");
+    if (warp == turn) {                                             // the elements: their spans in order (at most 4 x 8 of them)
+      const int m = lane / PAIR_WN, n = tile * PAIR_WN + lane % PAIR_WN;
+      const bool mine_here = m < p.m && n < p.n;
+      float v = 0.0f;
+      if (mine_here) {
+        const float* from = red + parity * SP_SPANS * PAIR_WN * p.m + lane;
+        v = from[0];
+        for (int s = 1; s < spans; ++s) v += from[s * PAIR_WN * p.m];
+      }
+      const bool again = mine_here && !sp_settled(v);
+      if (__any_sync(0xffffffffu, again)) v = sp_again(p.a, p.lda, p.w, p.ldw, p.k, m, n, v, again);
+      if (mine_here) p.c[static_cast<size_t>(m) * p.ldc + n] = v;
+    }
+    turn = (turn + 1) & 7;
+  }
+  cp_async_wait<0>();
+}
+
 // ------------------------------------------------------------------ launchers
 constexpr size_t FEW_SMEM_LIMIT = 225 * 1024;
 constexpr int DEVICES = 16;                     // whose launch limits are remembered
@@ -1025,6 +1185,37 @@ static int launch_few_split(const Product& p, int device, int sms, cudaStream_t 
   return b200_launch(few_split_kernel<MR, WN>, grid, dim3(256), F::BYTES, stream, 0, p, tiles, stages, span_stages);
 }
 
+template <int RING, int U, int G>
+static int launch_pair_split(const Product& p, int device, int sms, cudaStream_t stream) {
+  static bool configured[DEVICES];
+  if (device >= DEVICES || !configured[device]) {
+    cudaError_t e = cudaFuncSetAttribute(pair_split_kernel<RING, U, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(FEW_SMEM_LIMIT));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (device < DEVICES) configured[device] = true;
+  }
+  const int tiles = (p.n + PAIR_WN - 1) / PAIR_WN, stages = (p.k + SP_KS - 1) / SP_KS, span_stages = (stages + SP_SPANS - 1) / SP_SPANS;
+  return b200_launch(pair_split_kernel<RING, U, G>, dim3(tiles < sms ? tiles : sms), dim3(256 * G), pair_split_bytes(p.m, stages, RING, U, G), stream, 0,
+                     p, tiles, stages, span_stages);
+}
+// How many groups pair_split_kernel takes a product with, 0: few_split_kernel takes it.  Measured in hundredths of a microsecond on 148
+// SMs, one to four rows of 128 to 8,192 columns and 256 to 16,384 rows of W; ss: stages a span.  few_split_kernel costs 245 and, a round of
+// tiles over the SMs, 84 ss (40 ss with tiles of eight rows of W); this kernel 290 + 20 ss with one group and one round, 335 and a round of
+// 33 (1 + ss) with two, 300 and 20 + 24 ss with one group where shared memory holds no two (two rounds at most: 2,048 x 8,192, two
+// rows, 28.1 / 18.0, but 6,144 x 4,096, four rows, 23.3 / 26.4).  So short rows stay
+// with few_split_kernel (16,384 x 512 9.9 / 11.0, 4,096 x 1,024 5.9 / 6.5; 16,384 x 1,024 16.5 / 14.6, 2,048 x 1,024 5.9 / 5.0).
+static int pair_groups(int m, int n, int k, int sms) {
+  if (m > PAIR_ROWS) return 0;
+  auto rounds = [](long long tiles, long long places) { return (tiles + places - 1) / places; };
+  const int stages = (k + SP_KS - 1) / SP_KS;
+  const long long ss = (stages + SP_SPANS - 1) / SP_SPANS, tiles = (n + 7) / 8, wide = (n + 15) / 16;
+  const long long few = 245 + ss * (wide < sms ? 40 * rounds(tiles, sms) : 84 * rounds(wide, 2 * sms));
+  const bool one = pair_split_bytes(m, stages, 2, 2, 1) <= FEW_SMEM_LIMIT, two = pair_split_bytes(m, stages, 2, 2, 2) <= FEW_SMEM_LIMIT;
+  if (tiles <= sms) return one && 290 + 20 * ss <= few ? 1 : 0;
+  if (two) return 335 + rounds(tiles, 2 * sms) * 33 * (1 + ss) <= few ? 2 : 0;
+  return one && rounds(tiles, sms) <= 2 && 300 + rounds(tiles, sms) * (20 + 24 * ss) <= few ? 1 : 0;
+}
+B200_EXPORT int b200_gemm_f32_pair_groups(int m, int n, int k, int sms) { return pair_groups(m, n, k, sms); }
+
 // Which kernel takes a product in terms: few_split_kernel up to 16 rows, and up to 128 in groups of 32 where that is the shorter way.
 // Its groups cost a tile of 16 rows of W 0.135 us a stage, a block an SM at a time (and 2.7 us to begin), split_kernel's stage costs 0.88
 // us with up to 64 rows of x and 1.1 with 128.  (us on few_split / split, 32 rows: 4,096 x 1,024 11.0 / 17.3, 4,096 x 12,288 95 / 88; 64
@@ -1043,6 +1234,8 @@ static int launch_terms(const Product& p, int* err, int device, int sms, cudaStr
   const SplitWork job = split_work(p, nt, sms, err, cost);
   if (few_split_takes(p, sms, cost, nt)) {
     const bool narrow = (p.n + 15) / 16 < sms;
+    const int groups = pair_groups(p.m, p.n, p.k, sms);
+    if (groups != 0) return groups == 1 ? launch_pair_split<2, 2, 1>(p, device, sms, stream) : launch_pair_split<2, 2, 2>(p, device, sms, stream);
     if (p.m <= 8) return narrow ? launch_few_split<8, 8>(p, device, sms, stream) : launch_few_split<8, 16>(p, device, sms, stream);
     if (p.m <= 16) return narrow ? launch_few_split<16, 8>(p, device, sms, stream) : launch_few_split<16, 16>(p, device, sms, stream);
     return launch_few_split<32, 16>(p, device, sms, stream);

@@ -91,8 +91,27 @@ def test_32_bit_products_of_very_small_numbers(m, n, k, exponent):
         assert torch.equal(ops.gemm_f32(a[2:5].contiguous(), w), got[2:5])
 
 
-# one kernel each: few rows, a cluster a tile, blocks that walk over tiles
-@pytest.mark.parametrize("m,n,k", [(7, 1024, 4096), (300, 1024, 4096), (1024, 4096, 2048)])
+# up to four rows: one group of warps and two, tiles of eight rows of W with a rest, one tile, several a group, fewer than groups; K of odd
+# counts of stages, of one stage more than eight spans, with a rest of a stage; spans that are empty; x that fits beside one ring only
+@pytest.mark.parametrize("m,n,k,groups", [(1, 256, 1024, 1), (4, 1021, 1028, 1), (2, 9, 4100, 1), (3, 1184, 1060, 1), (1, 1185, 1024, 2), (2, 2371, 4128, 2),
+                                          (4, 20003, 1184, 2), (3, 2050, 3076, 2), (1, 4100, 12288, 2), (4, 2048, 4096, 1), (2, 2051, 8192, 1), (1, 700, 2336, 1)])
+def test_32_bit_products_of_up_to_four_rows(m, n, k, groups):
+    """Whichever kernel: the bits that the same rows have beside others."""
+    from llm_infer_rust_b200.kernels import ops
+    from llm_infer_rust_b200.kernels.build import load_cuda_library
+    assert load_cuda_library("gemm_f32.cu").b200_gemm_f32_pair_groups(m, n, k, 148) == groups
+    for spread in (0.0, 4.0):
+        a, w = _rnd(130, k) * torch.exp(spread * _rnd(130, k, seed=2)), _rnd(n, k, seed=1) * torch.exp(spread * _rnd(n, k, seed=3))
+        got = ops.gemm_f32(a[:m].contiguous(), w)
+        want, size = a[:m].double() @ w.double().t(), a[:m].double().abs() @ w.double().abs().t()
+        assert ((got.double() - want).abs() <= (24 + 1 + k / 256 + 10) * 2.0 ** -24 * size).all()      # (as test_32_bit_products_in_three_terms)
+        for rows in (8, 130):
+            assert torch.equal(ops.gemm_f32(a[:rows].contiguous(), w)[:m], got)
+    ops.check_errors(a.device)
+
+
+# one kernel each: a few rows (three kinds), a cluster a tile, blocks that walk over tiles
+@pytest.mark.parametrize("m,n,k", [(3, 1024, 4096), (3, 4100, 4096), (7, 1024, 4096), (300, 1024, 4096), (1024, 4096, 2048)])
 def test_32_bit_products_whose_rows_are_all_nan_or_infinite(m, n, k):
     """Every element of such rows is summed again.  No block waits so long for it that another of its warps gives up, and the
     other rows keep their bits.  (A thread an element took 60 ms a tile and more.)"""

@@ -87,6 +87,15 @@ def test_many_tokens_walk_between_projection_and_attention():
     assert not any(walks(1, threads(t, h)) for t, h in ((777, 32), (500, 32), (45, 48))) and not walks(0, threads(8192, 32))
 
 
+def test_up_to_four_rows_of_32_bit_products():
+    """Which of the two kernels for few rows, by what each costs over the SMs (measured on both sides, 148 SMs)."""
+    groups = lambda m, n, k: build.load_cuda_library("gemm_f32.cu").b200_gemm_f32_pair_groups(m, n, k, 148)
+    assert all(groups(m, n, k) == 1 for m in (1, 4) for n, k in ((1024, 2048), (1024, 3072), (256, 1024)))
+    assert all(groups(m, n, k) == 2 for m in (1, 2) for n, k in ((151936, 1024), (24576, 4096), (6144, 4096), (16384, 1536)))
+    assert groups(1, 4096, 12288) == 2 and groups(2, 2048, 8192) == groups(4, 2048, 4096) == 1
+    assert not any(groups(m, n, k) for m, n, k in ((1, 4096, 1024), (1, 16384, 512), (4, 4096, 512), (4, 24576, 4096), (2, 16384, 8192), (4, 6144, 4096), (5, 1024, 3072)))
+
+
 def test_which_kernel_takes_a_32_bit_product_in_terms():
     """By rows and by what each costs over the SMs (measured on both sides, 148 SMs)."""
     route = build.load_cuda_library("gemm_f32.cu").b200_gemm_f32_route
