@@ -296,8 +296,9 @@ __device__ __forceinline__ void prefill_tile(const T* __restrict__ q, const T* _
   }
 }
 
-// (Heads of 16 are held to three CTAs an SM: with 88 registers instead of 80 they had two, and 2,000 float32 tokens behind 1,000, 40
-// query heads, took 2,949 us for 2,383.  0 leaves the others to the compiler, which stays at 80 or at what shared memory allows;
+// (Reached by bfloat16, and in float by heads above 128, of no multiple of 16, or of another width than their values; others have
+// prefill_split_kernel below.  Builds for heads of 16 are held to three CTAs an SM: with 88 registers instead of 80 they had two, and 2,000
+// float32 tokens behind 1,000, 40 query heads, took 2,949 us for 2,383.  0 leaves the others to the compiler, which stays at 80 or at what shared memory allows;
 // told that one CTA is enough it took all registers, and heads of 32 6,336 us for 2,546.)
 template <typename T>
 __global__ void __launch_bounds__(PF_WARPS * 32, D <= 16 ? 3 : 0)
@@ -743,6 +744,16 @@ B200_EXPORT int b200_prefill_attention_ctas_per_sm(int dtype) {
   return dtype == B200_F32 ? prefill_ctas_per_sm<float>() : prefill_ctas_per_sm<__nv_bfloat16>();
 }
 
+#if HEAD_DIM <= 128
+// Local memory of prefill_split_kernel, whose terms of the query and accumulators take up to all of a thread's registers (one CTA an SM
+// at every head size): anything above zero are spills.
+B200_EXPORT int b200_prefill_split_local_bytes(void) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, prefill_split_kernel);
+  return e == cudaSuccess ? static_cast<int>(a.localSizeBytes) : -static_cast<int>(e);
+}
+#endif
+
 template <typename T>
 static int launch_prefill(const void* q, const void* kc, const void* vc, void* out, const int* block_table,
                           int table_stride, const int* cu_q, const int* kv_len, const int* prefix_len,
@@ -769,12 +780,15 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (hd == D && hd_v == D && (v_stride <= 0 || v_stride == D) && aligned(q) && aligned(kc) && aligned(vc) && aligned(out)) {
       static_assert(SplitPrefill::SMEM >= PrefillShape<float>::FIXED + PrefillShape<float>::BLOCK, "a tile may be done again");
-      static bool split_configured = false;
-      if (!split_configured) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SplitPrefill::SMEM));
-        if (e != cudaSuccess) return static_cast<int>(e);
-        split_configured = true;
+      constexpr int DEVICES = 16;                              // whose launch limit is remembered
+      static bool split_configured[DEVICES];
+      int device = 0;
+      cudaError_t e = cudaGetDevice(&device);
+      if (e == cudaSuccess && (device >= DEVICES || !split_configured[device])) {
+        e = cudaFuncSetAttribute(prefill_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SplitPrefill::SMEM));
+        if (e == cudaSuccess && device < DEVICES) split_configured[device] = true;
       }
+      if (e != cudaSuccess) return static_cast<int>(e);
       prefill_split_kernel<<<grid, PF_WARPS * 32, SplitPrefill::SMEM, stream>>>(
           static_cast<const float*>(q), static_cast<const float*>(kc), static_cast<const float*>(vc), static_cast<float*>(out), block_table,
           table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window, scale, tile_tokens, head_chunks, softcap, chunk, sinks);

@@ -265,6 +265,13 @@ def test_all_sizes_prompt_attention_keeps_its_blocks_on_an_sm(head_dim, ctas, dt
     assert ops._attention(head_dim).b200_prefill_attention_ctas_per_sm(ops.F32 if dtype == torch.float32 else ops.BF16) >= ctas
 
 
+@pytest.mark.parametrize("head_dim", [16, 32, 48, 64, 96, 128])
+def test_32_bit_prompt_attention_keeps_its_numbers_in_registers(head_dim):
+    """(One CTA an SM at every size; the float32 cases above are heads of 24, 40 and the like, which the all-sizes kernel keeps.)"""
+    from llm_infer_rust_b200.kernels import ops
+    assert ops._attention(head_dim).b200_prefill_split_local_bytes() == 0
+
+
 # more steps than the grid has lane groups, with a rest; an odd count of heads (the last step has one); heads of 64 and 256 (8 and 32
 # lanes); without norms, without tables, without a cache
 @pytest.mark.parametrize("tokens,nh,nkv,d,norm,turn,store", [(1020, 16, 8, 128, True, True, True), (2500, 32, 8, 128, True, True, True),
