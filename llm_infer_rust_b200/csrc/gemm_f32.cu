@@ -27,8 +27,8 @@
 //   loads of shared memory for 64 FFMA (4 x 8 elements a thread as packed f32x2 pairs, with one operand stored twice, took
 //   half again as many loads: 25 against 32 TFLOP/s at 1,000 rows).  The blocks of a cluster take different spans of one tile and add
 //   them up in order through distributed shared memory.
-// Measured in a step at the Qwen3-0.6B sizes, mean of a layer's four products, beside one 64 x 64 kernel that summed k in
-// one chain for both: 4 rows 122 -> 9.1 us (1.7 TB/s; the head alone 5 TB/s), 300 rows 145 -> 93 us (25 TFLOP/s).
+// Measured on what is left to them, sixteen products a launch: 4 rows of 128 x 256 5.8 us, 300 rows 22.1 (14 TFLOP/s), 300 of 512 x 128
+// 33.1 (19); eight of 1,500 rows of 320 x 320 79.1 (31 TFLOP/s).
 //
 // The batched form multiplies `batch` independent pairs whose rows may lie apart (leading dimensions lda, ldw, ldc
 // and a distance between consecutive matrices of each operand): per-head products of a mixer, where head h's rows are
@@ -486,8 +486,8 @@ struct SplitWork {
 };
 
 // grid: tiles x ranks of a cluster, or (one rank) at most a block an SM, which walks over tiles.  Warp 16 issues the products, warp 17
-// the copies, the other sixteen take stages apart and add their sums up: of a stage's 1,800 cycles (112 rows of x) they need 900 and
-// 500, beside 1,600 of products, so neither side hides the other whole.
+// the copies, the other sixteen take stages apart and add their sums up.  Bound by those: of a stage's 2,000 cycles (300 rows of 6,144 x
+// 1,024, three tiles of 112 rows of x) the schedulers issue in 69 % and the tensor cores work in 32 %.
 template <int NT>
 __global__ void __launch_bounds__(SplitShape<NT>::THREADS, 1)
 split_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const SplitWork job) {
@@ -1095,15 +1095,46 @@ static int blocks_a_tile(long long tiles, int spans, int sms) {
 }
 B200_EXPORT int b200_gemm_f32_blocks_a_tile(long long tiles, int spans, int sms) { return blocks_a_tile(tiles, spans, sms); }
 
+// How many clusters of `ranks` of split_kernel's blocks (one an SM) a device holds at once; device < 0: a B200 as measured.
+static int clusters_at_once(int ranks, int sms, int device) {
+  static int known[DEVICES][SP_SPANS + 1];
+  constexpr int MEASURED[SP_SPANS + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  if (device < 0) return MEASURED[ranks];
+  if (device < DEVICES && known[device][ranks] > 0) return known[device][ranks];
+  using S = SplitShape<64>;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(ranks);
+  config.blockDim = dim3(S::THREADS);
+  config.dynamicSmemBytes = S::BYTES;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ranks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  int n = 0;
+  cudaError_t e = cudaFuncSetAttribute(split_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, split_kernel<64>, &config);
+  if (e != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = sms / ranks > 0 ? sms / ranks : 1;
+  }
+  if (device < DEVICES) known[device][ranks] = n;
+  return n;
+}
+
 // What a product costs split_kernel, in stages of one block: rounds of blocks over the SMs, each its stages and what begins and ends a
 // block (a cluster's placement and its exchange of sums take as long as nine to eleven stages).  `ranks`: how many blocks share a
-// tile's k, one or two spans each.  (Measured with one, four and eight, the sums exchanged one float a turn: 4,096 x 1,024 at 64 rows
-// 31 / 21 / 38 us, 6,144 x 1,024 at 64 31 / 41 / 50, 1,024 x 3,072 at 300 99 / 43 / 48.)
-static long long split_cost(int tiles, int spans, int stages, int sms, int& ranks) {
+// tile's k, one or two spans each.  How many clusters the SMs hold at once is less than their blocks: a cluster stays within one of the
+// chip's parts, 15 of eight blocks and not 18 (by blocks, 200 rows of 1,024 x 2,048 took eight, 32.3 us; four: 27.2).  Measured with
+// one, four and eight: 4,096 x 1,024 at 64 rows 31.5 / 16.8 / 32.6 us, 6,144 x 1,024 at 64 31.9 / 31.1 / 43.5, 2,048 x 2,048 at 64 56.9 / 22.5 /
+// 28.4, 1,024 x 3,072 at 300 95 / 34.7 / 40.8, at 600 97 / 68 / 62, 6,144 x 4,096 at 64 111 / 70 / 82.
+static long long split_cost(int tiles, int spans, int stages, int sms, int device, int& ranks) {
   ranks = 1;
   long long least = static_cast<long long>((tiles + sms - 1) / sms) * (stages + 3);
   for (int r : {(spans + 1) / 2, spans}) {
-    const long long cost = (static_cast<long long>(tiles) * r + sms - 1) / sms * ((stages + r - 1) / r + 11);
+    const int at_once = clusters_at_once(r, sms, device);
+    const long long cost = static_cast<long long>((tiles + at_once - 1) / at_once) * ((stages + r - 1) / r + 11);
     if (spans >= 3 && cost < least) { ranks = r; least = cost; }
   }
   return least;
@@ -1134,7 +1165,7 @@ static int encode_rows(CUtensorMap* map, const float* base, int rows, int cols, 
   return r == CUDA_SUCCESS ? 0 : 1000 + static_cast<int>(r);
 }
 
-static SplitWork split_work(const Product& p, int nt, int sms, int* err, long long& cost) {
+static SplitWork split_work(const Product& p, int nt, int sms, int device, int* err, long long& cost) {
   SplitWork job = {};
   job.p = p;
   job.err = err;
@@ -1146,7 +1177,7 @@ static SplitWork split_work(const Product& p, int nt, int sms, int* err, long lo
   job.stages = (p.k + SP_KS - 1) / SP_KS;
   job.span_stages = (job.stages + SP_SPANS - 1) / SP_SPANS;
   const int spans = (job.stages + job.span_stages - 1) / job.span_stages;
-  cost = split_cost(job.tiles, spans, job.stages, sms, job.ksplit);
+  cost = split_cost(job.tiles, spans, job.stages, sms, device, job.ksplit);
   job.spans_a_rank = job.ksplit > 1 ? (spans + job.ksplit - 1) / job.ksplit : spans;
   return job;
 }
@@ -1218,8 +1249,9 @@ B200_EXPORT int b200_gemm_f32_pair_groups(int m, int n, int k, int sms) { return
 
 // Which kernel takes a product in terms: few_split_kernel up to 16 rows, and up to 128 in groups of 32 where that is the shorter way.
 // Its groups cost a tile of 16 rows of W 0.135 us a stage, a block an SM at a time (and 2.7 us to begin), split_kernel's stage costs 0.88
-// us with up to 64 rows of x and 1.1 with 128.  (us on few_split / split, 32 rows: 4,096 x 1,024 11.0 / 17.3, 4,096 x 12,288 95 / 88; 64
-// rows: 1,024 x 2,048 9.9 / 16.3, 4,096 x 4,096 67 / 42, 151,936 x 1,024 593 / 252; 96: 1,024 x 2,048 18.6 / 20.3, 6,144 x 1,024 39.4 / 38.8.)
+// us with up to 64 rows of x and 1.1 with 128.  (us on few_split / split, 32 rows: 4,096 x 1,024 11.3 / 15.9, 16,384 x 1,024 34.5 / 32.2; 64
+// rows: 1,024 x 2,048 10.1 / 14.8, 2,048 x 2,048 19.2 / 22.5, 4,096 x 4,096 67 / 36.5, 151,936 x 1,024 593 / 252; 96: 1,024 x 3,072 26.6 / 20.5, and on
+// the line 1,024 x 2,048 18.9 / 16.8, 6,144 x 1,024 40.1 / 37.7.)
 // Tiles of eight rows of W where those of sixteen leave SMs without a block (1,024 x 2,048, one row: 5.6 -> 4.9 us).
 static bool few_split_takes(const Product& p, int sms, long long split_stages, int nt) {
   if (p.m <= 16) return true;
@@ -1231,7 +1263,7 @@ static bool few_split_takes(const Product& p, int sms, long long split_stages, i
 static int launch_terms(const Product& p, int* err, int device, int sms, cudaStream_t stream) {
   const int nt = p.m <= 64 ? 64 : 128;
   long long cost = 0;
-  const SplitWork job = split_work(p, nt, sms, err, cost);
+  const SplitWork job = split_work(p, nt, sms, device, err, cost);
   if (few_split_takes(p, sms, cost, nt)) {
     const bool narrow = (p.n + 15) / 16 < sms;
     const int groups = pair_groups(p.m, p.n, p.k, sms);
@@ -1247,7 +1279,7 @@ B200_EXPORT int b200_gemm_f32_route(int m, int n, int k, int sms) {
   Product p = {};
   p.m = m; p.n = n; p.k = k;
   long long cost = 0;
-  split_work(p, m <= 64 ? 64 : 128, sms, nullptr, cost);
+  split_work(p, m <= 64 ? 64 : 128, sms, -1, nullptr, cost);
   return few_split_takes(p, sms, cost, m <= 64 ? 64 : 128) ? 0 : 1;
 }
 
@@ -1258,6 +1290,7 @@ static int launch(const Product& p, int batch, bool vec, int* err, cudaStream_t 
   if (e != cudaSuccess) return static_cast<int>(e);
   if (vec && batch == 1) return launch_terms(p, err, device, sms, stream);
   const int spans = (p.k + SPAN - 1) / SPAN;
+  // (What is left here are batched and unaligned products; the figures are of single, aligned ones, which these kernels took as well.)
   // Up to 16 rows the weights are streamed, in passes of `mr` rows: as many as fit shared memory beside the rings, 16 to K = 1,536
   // (2,048 where N leaves a block one tile), 8 to 3,072, 4 beyond.  One pass is 2 to 9 times as fast as a tile of 64 that is
   // mostly padding, and three passes or four still are where a span has a warp (16 rows of N x K = 4,096 x 1,024 / 1,024 x 3,072 /

@@ -101,5 +101,6 @@ def test_which_kernel_takes_a_32_bit_product_in_terms():
     route = build.load_cuda_library("gemm_f32.cu").b200_gemm_f32_route
     few = lambda m, n, k: route(m, n, k, 148) == 0
     assert all(few(m, n, k) for m in (1, 8, 16) for n, k in ((1024, 3072), (151936, 1024), (24576, 4096)))
+    assert few(48, 2048, 2048) and few(64, 2048, 2048)          # (clusters of eight would take two rounds)
     assert few(32, 4096, 1024) and few(32, 6144, 1024) and few(64, 1024, 2048) and few(64, 1024, 3072) and few(96, 1024, 2048) and few(128, 64, 1024)
     assert not any(few(m, n, k) for m, n, k in ((32, 151936, 1024), (64, 4096, 4096), (64, 24576, 4096), (128, 6144, 1024), (129, 64, 64), (300, 1024, 2048)))
