@@ -324,7 +324,8 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
 // The query's terms stay in registers; keys and values are taken apart as they are read, since a block serves two warps only.
 // A tile whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term), and so is one with
 // sums of weighted values below 2^-80: values below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.
-// Bound by the instructions that take keys and values apart (two warps a scheduler, 22 for a thread's four numbers, six products).  us,
+// Bound by the latencies of two warps a scheduler (they issue in 34 % of its cycles), most of them those of taking keys and values apart
+// (22 instructions for a thread's four numbers, six products).  us,
 // CUDA cores / this: 16 heads of 128, 8 KV heads, 300 tokens 59.3 / 30.7, 17 tokens 13.5 / 10.5, 2,000 tokens 991 / 598, 64 behind 2,000
 // cached 343 / 170, 16 rows of 5 behind 100 21.6 / 13.8; heads of 64, 300 tokens 42.3 / 18.7, of 16 37.6 / 11.5.  Error against 64 bits
 // 7.2e-7 -> 2.5e-7 (300 tokens).  Heads beyond 128 or of another width than their values stay with prefill_tile.

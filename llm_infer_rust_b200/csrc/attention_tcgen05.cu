@@ -119,7 +119,8 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 // True in one lane of a whole warp.  The warp that issues products walks along as a whole and only the instruction itself is one
 // lane's: what comes before it is then the same in every lane for all the compiler knows, and descriptors are made in uniform
-// registers, where the instruction takes them.  (From one lane's own registers every product waited for eight moves.)
+// registers, where the instruction takes them.  (From one lane's own registers a product took 100 cycles to issue, so 35: 8,192 tokens x
+// 16 heads 299 -> 275 us.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t is;
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(is));
@@ -444,11 +445,6 @@ __device__ __forceinline__ float capped(const ScoreShape& f, float s, float shif
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(fast_exp2(s * (f.tanh_in * 2.8853900817779268f)) + 1.0f));
   return fmaf(-2.0f * f.cap_log2, r, f.cap_log2 + shift);
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 // The same of two scores; NaN stays NaN, a masked score (-inf) does not stay masked.
 __device__ __forceinline__ f32x2 capped2(const ScoreShape& f, f32x2 s, float shift) {

@@ -410,7 +410,7 @@ __device__ __forceinline__ void sp_split(float x, float y, uint32_t& high, uint3
 // takes every 32nd piece of four k, the 32 sums meet by halves.  Lane `l` of the warp that calls this has element (m, n) of C and
 // its sum t; it gets t back, or the new sum where `again`.  A row of x that holds a NaN has NaN everywhere and is found in one pass over it: behind
 // the first NaN of a prompt's rows every element of theirs comes here.  (One thread an element, down its row of W alone, would
-// hold a tile of 128 x 128 up for tens of milliseconds at K = 12,288.)
+// hold a tile of 128 x 128 up for tens of milliseconds at K = 12,288, by estimate.)
 __device__ __forceinline__ bool sp_settled(float t) {
   const float size = fabsf(t);
   return size <= 3.402823466e38f && (size >= 8.2718061e-25f || size == 0.0f);      // (2^-80; a NaN compares false)

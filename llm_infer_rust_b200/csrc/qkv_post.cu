@@ -226,7 +226,7 @@ qkv_post_vec_kernel(const TA* __restrict__ qkv, TA* __restrict__ q_out, TA* __re
 // Many tokens: the same lane groups (HG heads of one token a step) walk over the step's work, and what the next step reads
 // (its heads, its token's position and slot) is on its way while this one is normed, turned and stored.  A thread that comes
 // and goes with one group of heads has loads in flight for a part of its life only, and its index cost a 64-bit division.
-// Bound by latency still (four blocks an SM by registers).  bfloat16, 16 + 2 x 8 heads of 128, us in a graph before / now: 8,192
+// Eight blocks an SM, four at a time by registers; bound by issue (76 % of cycles) more than by bytes (31 % of DRAM).  bfloat16, 16 + 2 x 8 heads of 128, us in a graph before / now: 8,192
 // tokens 51.8 / 35.0 (134 MB: 3.8 TB/s), 2,919 20.2 / 14.1, 1,020 8.7 / 6.5; 32 + 2 x 8 heads, 2,048 tokens 20.3 / 14.6.  One head a
 // lane group: 44.0, 17.6, 7.2, 17.8.
 template <typename TA, typename TW, int HG>

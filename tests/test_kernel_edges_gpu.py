@@ -114,7 +114,7 @@ def test_32_bit_products_of_up_to_four_rows(m, n, k, groups):
 @pytest.mark.parametrize("m,n,k", [(3, 1024, 4096), (3, 4100, 4096), (7, 1024, 4096), (300, 1024, 4096), (1024, 4096, 2048)])
 def test_32_bit_products_whose_rows_are_all_nan_or_infinite(m, n, k):
     """Every element of such rows is summed again.  No block waits so long for it that another of its warps gives up, and the
-    other rows keep their bits.  (A thread an element took 60 ms a tile and more.)"""
+    other rows keep their bits.  (A thread an element would take, by estimate, tens of milliseconds a tile.)"""
     from llm_infer_rust_b200.kernels import ops
     x, w = _rnd(m, k), _rnd(n, k, seed=1)
     plain = ops.gemm_f32(x, w)
