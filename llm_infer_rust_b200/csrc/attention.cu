@@ -201,14 +201,15 @@ __device__ __forceinline__ void load_key_block(T* dst, const T* __restrict__ cac
 // 32 hc ..): tile_tokens * heads <= 32 vectors.
 constexpr int PF_WARPS = 8;
 
-// One tile of a portion, by CUDA cores (shared memory: PrefillShape<T>::SMEM).
+// One tile of a portion, by CUDA cores (shared memory: PrefillShape<T>::SMEM); of its vectors those in `which` are stored.
 template <typename T>
 __device__ __forceinline__ void prefill_tile(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                          T* __restrict__ out, const int* __restrict__ block_table, int table_stride,
                          const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                          const int* __restrict__ prefix_len, const int* __restrict__ rows, int nh, int nkv,
                          int page_size, int window, float scale, int tile_tokens, int head_chunks, int hd,
-                         int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride, int stages) {
+                         int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride, int stages,
+                         uint32_t which) {
   using G = RowGeom<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* qs = reinterpret_cast<float*>(smem_raw);                        // [32][D]
@@ -279,7 +280,7 @@ __device__ __forceinline__ void prefill_tile(const T* __restrict__ q, const T* _
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     const int vec = warp * NV + v;
-    if (vec >= nvec) continue;
+    if (vec >= nvec || (which >> vec & 1) == 0) continue;
     const int tok = vec / group, head = head_base + vec % group;
     T* dst = out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * hd_v;
     float l = st.l[v];
@@ -309,7 +310,7 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
                          int page_size, int window, float scale, int tile_tokens, int head_chunks, int hd,
                          int hd_v, float softcap, int chunk, const float* __restrict__ sinks, int v_stride, int stages) {
   prefill_tile<T>(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window,
-                  scale, tile_tokens, head_chunks, hd, hd_v, softcap, chunk, sinks, v_stride, stages);
+                  scale, tile_tokens, head_chunks, hd, hd_v, softcap, chunk, sinks, v_stride, stages, 0xffffffffu);
 }
 
 #if HEAD_DIM <= 128
@@ -322,8 +323,9 @@ prefill_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
 // softmax of its own over its keys and the four parts of a vector are added up at the end in order.  Which keys a warp takes
 // depends on their positions alone, so a position's result has the same bits however the prompt was cut.
 // The query's terms stay in registers; keys and values are taken apart as they are read, since a block serves two warps only.
-// A tile whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term), and so is one with
-// sums of weighted values below 2^-80: values below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.
+// A vector whose result holds an infinity or a NaN is done again by prefill_tile (an infinity has no second term), and so is one with
+// sums of weighted values below 2^-80: values below 2^-110 lose bits of their third term, for which bfloat16 ends at 2^-133.  The
+// tile's other vectors keep what they have: which they share a tile with follows from how the prompt was cut.
 // Bound by the latencies of two warps a scheduler (they issue in 34 % of its cycles), most of them those of taking keys and values apart
 // (22 instructions for a thread's four numbers, six products).  us,
 // CUDA cores / this: 16 heads of 128, 8 KV heads, 300 tokens 59.3 / 30.7, 17 tokens 13.5 / 10.5, 2,000 tokens 991 / 598, 64 behind 2,000
@@ -337,8 +339,13 @@ struct SplitPrefill {
   static constexpr int STAGE = SPLIT_KEYS * (K_ROW + V_ROW);   // floats
   static constexpr int MERGE = 4 * 32 * (D + 4);               // floats: the four parts of 32 vectors
   static constexpr size_t TILES = sizeof(float) * (2 * STAGE > MERGE ? 2 * STAGE : MERGE);
-  static constexpr size_t SMEM = TILES + sizeof(float) * 4 * 32 * 2;
+  static constexpr size_t AGAIN = TILES + sizeof(float) * 4 * 32 * 2;      // a word: the vectors that are done again
+  static constexpr size_t SMEM = AGAIN + 16;
 };
+__device__ __forceinline__ uint32_t* split_again() {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  return reinterpret_cast<uint32_t*>(smem_raw + SplitPrefill::AGAIN);
+}
 
 // Two floats as three bfloat16 terms each, packed (the first float in the low half): x = high + mid + low, each term the rest
 // rounded to eight bits; exactly from 2^-110 on.
@@ -376,7 +383,7 @@ __device__ __noinline__ void prefill_tile_again(const float* q, const float* k_c
                                                 float scale, int tile_tokens, int head_chunks, float softcap, int chunk,
                                                 const float* sinks) {
   prefill_tile<float>(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size,
-                      window, scale, tile_tokens, head_chunks, D, D, softcap, chunk, sinks, D, 1);
+                      window, scale, tile_tokens, head_chunks, D, D, softcap, chunk, sinks, D, 1, *split_again());
 }
 
 __global__ void __launch_bounds__(PF_WARPS * 32, 1)
@@ -522,6 +529,7 @@ prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
     __syncthreads();                                                     // this block is read: the next copies may overwrite it
   }
   // The four parts of a vector.
+  if (threadIdx.x == 0) *split_again() = 0;
   float* parts = tiles;                                                  // [4][32][D + 4]
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
@@ -537,7 +545,6 @@ prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
       *reinterpret_cast<float2*>(parts + (quarter * 32 + vec) * (D + 4) + 8 * n + 2 * c4) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
   }
   __syncthreads();
-  bool settled = true;
   for (int i = threadIdx.x; i < nvec * (D / 4); i += PF_WARPS * 32) {
     const int vec = i / (D / 4), at = i - vec * (D / 4);
     float top = -INFINITY;
@@ -555,12 +562,14 @@ prefill_split_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
     if (sinks != nullptr && sum > 0.0f) sum += expf(sinks[head] - top);
     const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
     const float4 v = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
-    settled = settled && fabsf(sum) < INFINITY;
+    bool settled = fabsf(sum) < INFINITY;
 #pragma unroll
     for (int e = 0; e < 4; ++e) settled = settled && fabsf(acc[e]) < INFINITY && (fabsf(acc[e]) >= 8.2718061e-25f || acc[e] == 0.0f);
+    if (!settled) atomicOr(split_again(), 1u << vec);
     *reinterpret_cast<float4*>(out + (static_cast<size_t>(q_begin + tok0 + tok) * nh + head) * D + 4 * at) = v;
   }
-  if (__syncthreads_or(settled ? 0 : 1))
+  __syncthreads();
+  if (*split_again() != 0)
     prefill_tile_again(q, k_cache, v_cache, out, block_table, table_stride, cu_q, kv_len, prefix_len, rows, nh, nkv, page_size, window,
                        scale, tile_tokens, head_chunks, softcap, chunk, sinks);
 }
@@ -780,7 +789,7 @@ static int launch_prefill(const void* q, const void* kc, const void* vc, void* o
   if constexpr (sizeof(T) == 4) {
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (hd == D && hd_v == D && (v_stride <= 0 || v_stride == D) && aligned(q) && aligned(kc) && aligned(vc) && aligned(out)) {
-      static_assert(SplitPrefill::SMEM >= PrefillShape<float>::FIXED + PrefillShape<float>::BLOCK, "a tile may be done again");
+      static_assert(SplitPrefill::AGAIN >= PrefillShape<float>::FIXED + PrefillShape<float>::BLOCK, "a tile may be done again");
       constexpr int DEVICES = 16;                              // whose launch limit is remembered
       static bool split_configured[DEVICES];
       int device = 0;

@@ -425,3 +425,33 @@ def test_32_bit_prompt_attention_of_infinities():
             assert out[:32].isfinite().all()
         else:
             assert torch.equal(out.isnan(), want.isnan()) and out.isnan().any() and not out.isnan().all()
+
+
+@pytest.mark.parametrize("what", ["key", "query", "small"])
+def test_32_bit_prompt_attention_beside_rows_that_are_done_again(what):
+    """Rows without a finite result, or with a very small one, leave the bits of the rows and heads in their tile as they are."""
+    from llm_infer_rust_b200.kernels import ops
+    nh, nkv, d, page = 4, 2, 64, 16
+    k, v, table, _, _, _, rows = _paged([90], [0], nkv, d, page)
+    q = _rnd(90, nh * d, seed=3)
+    ints = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def attend(q, first=0):
+        out = torch.empty_like(q)
+        ops.prefill_attention(q, k, v, out, table, ints(0, len(q)), ints(first + len(q)), ints(first), rows, 1, len(q), nh, nkv, d, page, None, d ** -0.5)
+        return out
+    if what == "small":                                         # the first row sees nothing but the first key
+        v[table[0, 0].item(), :, 0] *= 2.0 ** -118
+        got = attend(q)
+        assert 0.0 < got[0].abs().max() < 2.0 ** -80 and got[1:].abs().amin(1).min() > 2.0 ** -80
+        assert torch.equal(got[1:], attend(q[1:].contiguous(), 1))
+        return
+    plain = attend(q)
+    if what == "key":
+        k[table[0, 50 // page].item(), 0, 50 % page, 3] = float("nan")
+    else:
+        q[66, 5] = float("-inf")
+    got = attend(q).view(90, nh, d)
+    other = ~got.isnan()
+    assert other.view(90, -1).sum().item() == ((50 * nh + 40 * 2) if what == "key" else (90 * nh - 1)) * d
+    assert torch.equal(got[other], plain.view(90, nh, d)[other])
